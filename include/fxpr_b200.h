@@ -313,6 +313,17 @@ int fxpr_silu_mul(const void* gate_up, int dtype, void* out, int64_t rows, int64
 int fxpr_silu_mul_pairs(const void* gate_up, int dtype, void* out, int64_t rows, int64_t f,
                         void* stream);
 
+/*
+ * Automatic split counts, from host shapes only (the torch operators ask the same functions; no
+ * choice changes a result).  GEMM K-splits; KV splits of the CUDA-core attention route
+ * (fxpr_vllm/_triton/attention.py:664-689); cluster ranks of the tensor-core attention route.
+ */
+int fxpr_pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int k_tile, int int_bits, int num_sms);
+int fxpr_pick_attention_splits(int requested, int64_t num_requests, int64_t num_q_blocks, int num_heads,
+                               int64_t num_kv_tiles, int num_sms);
+int fxpr_pick_attention_ranks(int requested, int64_t num_requests, int64_t max_query_len, int num_heads,
+                              int num_kv_heads, int64_t max_keys, int num_sms);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,8 +1,9 @@
-"""Build libfxpr_b200.so (sm_100a only) from csrc/*.cu with nvcc, in-tree.
+"""Build, in-tree, libfxpr_b200.so (csrc/*.cu with nvcc, sm_100a only: the C ABI) and
+libfxpr_torch.so (csrc/torch_ops.cpp with g++: the torch operators over it).
 
 Usage: ``python build.py [--force] [--verbose]``.  Objects go to ``build/``, the
-shared library to ``lib/libfxpr_b200.so`` next to this file.  A source is
-recompiled when it or any header is newer than its object.
+shared libraries to ``lib/`` next to this file.  A source is recompiled when it or
+any header is newer than its object.
 """
 from __future__ import annotations
 
@@ -18,6 +19,7 @@ ROOT = Path(__file__).resolve().parent
 CSRC = ROOT / "csrc"
 OBJ = ROOT / "build"
 LIB = ROOT / "lib" / "libfxpr_b200.so"
+TORCH_LIB = ROOT / "lib" / "libfxpr_torch.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -44,11 +46,35 @@ def _stale(src: Path, obj: Path, headers: list[Path]) -> bool:
     return any(p.stat().st_mtime > t for p in [src, *headers])
 
 
+def _torch_cmd(src: Path) -> list[str]:
+    """g++ line of the operator library, against the torch that is installed."""
+    import torch
+    from torch.utils import cpp_extension as ce
+
+    cuda = Path(_nvcc()).resolve().parent.parent
+    inc = [f"-I{p}" for p in [*ce.include_paths(), cuda / "include"]]
+    lib = Path(torch.__file__).resolve().parent / "lib"
+    return [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc, str(src), "-o", str(TORCH_LIB),
+            f"-L{LIB.parent}", f"-L{lib}", f"-L{cuda / 'lib64'}", "-lfxpr_b200", "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_cuda", "-lcudart", "-Wl,-rpath,$ORIGIN"]
+
+
+def _link(nvcc: str, sources: list[Path]) -> None:
+    objs = [str(OBJ / (s.stem + ".o")) for s in sources]
+    cmd = [nvcc, "-shared", "-o", str(LIB), *objs, "-lcudart_static", "-lpthread", "-ldl", "-lrt",
+           "-Xlinker", "-soname=libfxpr_b200.so", "-gencode", "arch=compute_100a,code=sm_100a"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("link failed")
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     nvcc = _nvcc()
     OBJ.mkdir(exist_ok=True)
     LIB.parent.mkdir(exist_ok=True)
-    headers = (sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.inl"))
+    headers = (sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.inl")) + sorted(CSRC.glob("*.h"))
                + sorted((ROOT.parent / "include").glob("*.h")))
     sources = sorted(CSRC.glob("*.cu"))
     jobs = []
@@ -72,14 +98,15 @@ def build(force: bool = False, verbose: bool = False) -> Path:
                 sys.stderr.write(f"--- {src.name}\n{r.stdout}{r.stderr}\n")
             if r.returncode != 0:
                 raise RuntimeError(f"nvcc failed on {src.name}")
-    objs = [str(OBJ / (s.stem + ".o")) for s in sources]
     if jobs or not LIB.exists():
-        cmd = [nvcc, "-shared", "-o", str(LIB), *objs, "-lcudart_static", "-lpthread", "-ldl", "-lrt",
-               "-gencode", "arch=compute_100a,code=sm_100a"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
+        _link(nvcc, sources)
+    src = CSRC / "torch_ops.cpp"
+    deps = [src, CSRC / "host_policy.h", *(ROOT.parent / "include").glob("*.h")]
+    if force or not TORCH_LIB.exists() or any(p.stat().st_mtime > TORCH_LIB.stat().st_mtime for p in deps):
+        r = subprocess.run(_torch_cmd(src), capture_output=True, text=True)
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
-            raise RuntimeError("link failed")
+            raise RuntimeError("g++ failed on torch_ops.cpp")
     return LIB
 
 

@@ -6,6 +6,7 @@
 #include "attention_common.cuh"
 #include "fxp_common.cuh"
 #include "gemm_common.cuh"
+#include "host_policy.h"
 
 using namespace fxpr;
 
@@ -17,6 +18,20 @@ static int default_k_tile(int dtype) {
 extern "C" int64_t fxpr_gemm_scratch_bytes(int64_t M, int64_t N, int int_bits, int split_k) {
   if (split_k <= 1 || M <= 0 || N <= 0) return 0;
   return gemm_tc_scratch_bytes(M, N, int_bits, split_k);
+}
+
+extern "C" int fxpr_pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int k_tile, int int_bits, int num_sms) {
+  return pick_gemm_split_k(M, N, K, k_tile, int_bits, num_sms);
+}
+
+extern "C" int fxpr_pick_attention_splits(int requested, int64_t num_requests, int64_t num_q_blocks, int num_heads,
+                                          int64_t num_kv_tiles, int num_sms) {
+  return (int)pick_attention_splits(requested, num_requests, num_q_blocks, num_heads, num_kv_tiles, num_sms);
+}
+
+extern "C" int fxpr_pick_attention_ranks(int requested, int64_t num_requests, int64_t max_query_len, int num_heads,
+                                         int num_kv_heads, int64_t max_keys, int num_sms) {
+  return (int)pick_attention_ranks(requested, num_requests, max_query_len, num_heads, num_kv_heads, max_keys, num_sms);
 }
 
 static int gemm_entry(const void* a, const void* b, const void* bias, void* c, void* c_int,

@@ -1,0 +1,75 @@
+// Host-shape-only launch policies, shared by the C ABI and the torch operator library.  None of
+// them can change a result: splits of a GEMM or of an attention call are integer partial sums.
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+
+namespace fxpr {
+
+inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// K-split of a GEMM: split when the output tiles alone cannot fill the GPU.
+inline int pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int64_t k_tile, int int_bits, int num_sms) {
+  if (int_bits == 16) return 1;
+  const int64_t tiles = ceil_div(M, 128) * ceil_div(N, 128);
+  const int64_t k_tiles = ceil_div(K, k_tile);
+  if (tiles >= num_sms || k_tiles < 8) return 1;
+  int split = 1;
+  if (M <= 64) {
+    // decode shapes (cluster merge): the largest power of two that fills the SMs once -- clusters
+    // of CTAs that each take a whole SM do not pack the last tenth of the SMs -- and leaves every
+    // rank at least 384 of K (below that the fixed cost of a rank wins)
+    while (split < 8 && tiles * split * 2 <= num_sms * 9 / 10 && K / (split * 2) >= 384) split *= 2;
+    return split;
+  }
+  // one wave of CTAs at most: a second, partly filled wave costs more than it hides
+  while (split < 16 && tiles * split * 2 <= num_sms && k_tiles / (split * 2) >= 4) split *= 2;
+  return split;
+}
+
+// KV splits of the CUDA-core attention route: an explicit request wins; otherwise split only long
+// contexts on an under-filled GPU, power of two, at most 8.
+inline int64_t pick_attention_splits(int64_t requested, int64_t num_requests, int64_t num_q_blocks, int64_t num_heads,
+                                     int64_t num_kv_tiles, int64_t num_sms) {
+  constexpr int64_t kMinTiles = 32, kMaxSplits = 8, kOversub = 2;
+  if (requested >= 1) return requested;
+  if (num_kv_tiles <= kMinTiles) return 1;
+  if (std::max<int64_t>(1, num_requests * num_q_blocks * num_heads) > kOversub * num_sms) return 1;
+  const int64_t split = std::min(num_kv_tiles / kMinTiles, kMaxSplits);
+  if (split < 2) return 1;
+  int64_t p = 1;
+  while (p < split) p *= 2;
+  return p;
+}
+
+// KV splits of the tensor-core attention route, where splits are cluster ranks.  Decode keeps each
+// CTA's key slice near 1024 keys (small score stash -> more resident CTAs) unless fewer clusters
+// than CTA slots call for more ranks; prefill splits only when the row blocks alone cannot fill
+// the SMs.
+inline int64_t pick_attention_ranks(int64_t requested, int64_t num_requests, int64_t max_query_len, int64_t num_heads,
+                                    int64_t num_kv_heads, int64_t max_keys, int64_t num_sms) {
+  if (requested >= 1) return std::min<int64_t>(requested, 16);
+  const int64_t g = num_heads / num_kv_heads;
+  if (max_query_len * g <= 16) {
+    // A rank's score stash must leave room for four CTAs per SM (about 19.5 KB: 19 key tiles at
+    // 16 bytes per key), which sets the least rank count for long contexts.  Few clusters: enough
+    // ranks to fill one wave of 4 CTAs per SM, at least two key tiles each.  Measured on 64
+    // requests x 1152 keys: 8 KV heads 70 -> 63 us with 1 rank instead of 2 (when the block table
+    // is no wider than that), 2 KV heads 30 -> 20.5 us with 4, 1 KV head 25 -> 16 us with 8.
+    const int64_t tiles = ceil_div(max_keys, 64);
+    const int64_t key_bytes = g <= 8 ? 4 * g : 64;
+    const int64_t budget = 19968 + (g <= 8 ? 2048 : 0);      // eight-row Q tiles leave 2 KB more
+    const int64_t cap_tiles = std::max<int64_t>(1, (budget / key_bytes) / 64);
+    const int64_t need = ceil_div(tiles, cap_tiles);
+    const int64_t by_keys = need > 4 ? 8 : std::max<int64_t>(1, need);
+    const int64_t clusters = std::max<int64_t>(1, num_requests * num_kv_heads);
+    const int64_t by_fill = std::max<int64_t>(1, std::min<int64_t>({8, (4 * num_sms) / clusters, tiles / 2}));
+    return std::max(by_keys, by_fill);
+  }
+  const int64_t blocks = num_requests * num_kv_heads * std::max<int64_t>(1, ceil_div(max_query_len * g, 64));
+  if (blocks >= num_sms || max_keys <= 2048) return 1;
+  return std::max<int64_t>(1, std::min<int64_t>(8, num_sms / blocks));
+}
+
+}  // namespace fxpr

@@ -1,7 +1,8 @@
-"""ctypes binding of ``libfxpr_b200.so`` (the C ABI in ``include/fxpr_b200.h``).
+"""Loading of the native libraries: ``libfxpr_b200.so`` (the C ABI in ``include/fxpr_b200.h``, bound
+with ctypes) and ``libfxpr_torch.so`` (the torch operators over it, ``csrc/torch_ops.cpp``).
 
 There is no fallback: if the library is missing the first kernel call raises.
-The library is built in-tree by ``build.py`` next to this package.
+Both are built in-tree by ``build.py`` next to this package.
 """
 from __future__ import annotations
 
@@ -25,6 +26,7 @@ def _find_lib() -> Path:
 
 
 LIB_PATH = _find_lib()
+TORCH_LIB_PATH = LIB_PATH.with_name("libfxpr_torch.so")
 
 FXPR_OK = 0
 FXPR_ERR_BAD_ARG = -1
@@ -93,6 +95,9 @@ SIGNATURES = {
                             _i, _i64, _i, _i, _i, _i, _i,
                             _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64,
                             _i, _i, _d, _d, _i, _i, _i, _i, _vp, _i64, _vp, _vp]),
+    "fxpr_pick_gemm_split_k": (_i, [_i64, _i64, _i64, _i, _i, _i]),
+    "fxpr_pick_attention_splits": (_i, [_i, _i64, _i64, _i, _i64, _i]),
+    "fxpr_pick_attention_ranks": (_i, [_i, _i64, _i64, _i, _i, _i64, _i]),
     "fxpr_attention_static_scratch_capacity": (_i64, []),
     "fxpr_attention_static_scratch": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                                            _i, _i64, _i, _i, _i, _i, _i,
@@ -101,6 +106,41 @@ SIGNATURES = {
 }
 
 _lib = None
+_torch_lib = None
+
+
+@_c.CFUNCTYPE(None)
+def _config_loader():
+    """The native operators ask for the runtime configuration before its first use."""
+    from .config import get_runtime_config
+
+    get_runtime_config()
+
+
+def load_ops(required: bool = True):
+    """Load the operator library (``torch.ops.fxpr.*`` on CUDA tensors) once."""
+    global _torch_lib
+    if _torch_lib is None:
+        if not (TORCH_LIB_PATH.exists() and LIB_PATH.exists()):
+            if required:
+                load()
+                raise RuntimeError(f"fxpr_vllm: operator library {TORCH_LIB_PATH} is missing; run "
+                                   f"`python {_PKG_ROOT / 'build.py'}`")
+            return None
+        load()                           # its symbols resolve the operator library's
+        torch.ops.load_library(str(TORCH_LIB_PATH))
+        lib = ctypes.CDLL(str(TORCH_LIB_PATH))
+        lib.fxpr_torch_set_overrides.argtypes = [_i] * 7
+        lib.fxpr_torch_set_overrides.restype = None
+        lib.fxpr_torch_set_config.argtypes = [_i] * 4
+        lib.fxpr_torch_set_config.restype = None
+        lib.fxpr_torch_set_config_loader.restype = None
+        _torch_lib = lib
+        lib.fxpr_torch_set_config_loader(_config_loader)
+        from . import config
+
+        config.push_to_native(lib)
+    return _torch_lib
 
 
 def load() -> ctypes.CDLL:
@@ -112,7 +152,7 @@ def load() -> ctypes.CDLL:
                 f"fxpr_vllm: CUDA library {LIB_PATH} is missing; run "
                 f"`python {_PKG_ROOT / 'build.py'}` (there is no CPU or Triton fallback)"
             )
-        lib = ctypes.CDLL(str(LIB_PATH))
+        lib = ctypes.CDLL(str(LIB_PATH), mode=ctypes.RTLD_GLOBAL)
         for name, (res, args) in SIGNATURES.items():
             fn = getattr(lib, name)
             fn.restype = res
