@@ -60,18 +60,23 @@ struct TcAttnShape {
   uint32_t idesc_s, idesc_pv;
 };
 
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z,
+                                            uint32_t elected) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(elected) : "memory");
 }
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z,
-                                            int w) {
+                                            int w, uint32_t elected) {
   asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5, %6}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %7, 0;\n\t"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w), "r"(elected) : "memory");
 }
 // generic-proxy writes to shared memory become visible to the tensor core (async proxy)
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -205,14 +210,12 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
   if (warp == 0) {
     // ------------------------------ K / V producer (TMA) ------------------------------
-    // One box per 16-token page piece and half head (2 KB).  Measured on a B200: an SM keeps
-    // only ~15 bytes per clock of such pieces in flight, whether they are fetched as TMA
-    // boxes, as 16-byte cp.async copies from two or four warps, or as both at once; that,
-    // not the tensor core or the conversion work, bounds this kernel at 16-token pages
-    // (48 KB per 128 x 64 tile over the two passes).  The boxes of a tile are issued from 16
-    // lanes in one instruction: issued one by one they cost the issuing thread ~80 clocks
-    // each.  Nothing is copied, and the block table is not read, past the end of the
+    // One box per 16-token page piece and half head (2 KB), 48 KB per 128 x 64 tile over the two
+    // passes.  The boxes are predicated instructions of a uniform warp (see tc_common.cuh): issued
+    // from a divergent branch, one lane or sixteen, each box cost the warp 80-140 clocks.
+    // Nothing is copied, and the block table is not read, past the end of the
     // sequence; V rows there are cleared by the MMA warp before P.V.
+    const uint32_t e = elect_one();
     int stage = 0; uint32_t phase = 1;
     uint32_t q_phase = 1;                                    // qfree: the first wait passes
     // Block-table entries are read 32 at a time (lane L: the 16-key group L of an 8-tile
@@ -230,12 +233,9 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     // warp's last score MMA of the previous item has completed.
     if (!__all_sync(0xffffffffu, mbar_wait(qfree, q_phase, abort_flag))) goto producer_done;
     q_phase ^= 1;
-    if (lane == 0) {
-      mbar_expect_tx(qfull, kQBytes);
-      tma_load_3d(q_s, &map_q, qfull, 0, kvh * G, I.q_start + I.tok0);
-      tma_load_3d(q_s + kQBytes / 2, &map_q, qfull, 64, kvh * G, I.q_start + I.tok0);
-    }
-    __syncwarp();
+    mbar_expect_tx(qfull, kQBytes, e);
+    tma_load_3d(q_s, &map_q, qfull, 0, kvh * G, I.q_start + I.tok0, e);
+    tma_load_3d(q_s + kQBytes / 2, &map_q, qfull, 64, kvh * G, I.q_start + I.tok0, e);
     auto load_entries = [&](int tb) -> int {
       const int n = tb * kTcTileN + lane * 16;
       return (tb < t1 && n < seq_len) ? bt[page_shift >= 0 ? (n >> page_shift) : (n / sh.page_size)] : 0;
@@ -255,18 +255,21 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           const int gs = sh.group_shift, gk = 1 << gs;
           int groups = (seq_len - t * kTcTileN + gk - 1) >> gs;
           groups = min(groups, kTcTileN >> gs);
-          if (lane == 0) mbar_expect_tx(fb, (uint32_t)((groups << (gs + 8)) << pass));
-          __syncwarp();
-          // lane = group * 4 + {K low half, K high half, V low half, V high half}
-          const int g = (lane >> 2) & 3, sel = lane & 3;
-          const int blk = __shfl_sync(0xffffffffu, cur, tt * 4 + (gs == 4 ? g : 0));
-          if (lane < 16 && g < groups && (pass || sel < 2)) {
+          mbar_expect_tx(fb, (uint32_t)((groups << (gs + 8)) << pass), e);
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            if (g >= groups) break;
+            const int blk = __shfl_sync(0xffffffffu, cur, tt * 4 + g);
             const int n = t * kTcTileN + (g << gs);
             const int slot = sh.page_mask ? (n & sh.page_mask) : (n % sh.page_size);
-            const uint32_t dst = ks + (uint32_t)((sel >> 1) * kKBytes + (sel & 1) * 8192 + (g << (gs + 7)));
-            tma_load_4d(dst, (sel >> 1) ? &map_v : &map_k, fb, (sel & 1) * 64, kvh, slot, blk);
+            const uint32_t dst = ks + (uint32_t)(g << (gs + 7));
+            tma_load_4d(dst, &map_k, fb, 0, kvh, slot, blk, e);
+            tma_load_4d(dst + 8192, &map_k, fb, 64, kvh, slot, blk, e);
+            if (pass) {
+              tma_load_4d(dst + kKBytes, &map_v, fb, 0, kvh, slot, blk, e);
+              tma_load_4d(dst + kKBytes + 8192, &map_v, fb, 64, kvh, slot, blk, e);
+            }
           }
-          __syncwarp();
           if (++stage == kTcStages) { stage = 0; phase ^= 1; }
         }
         cur = nxt;
@@ -277,20 +280,18 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------------------
     // S_t = Q . K_t^T: both operands K-major (head dim contiguous), two 64-dim slabs
+    const uint32_t e = elect_one();
     auto issue_s = [&](int stage, int sbuf) {
       const uint32_t d = tmem_base + kColS + (uint32_t)(sbuf * 64);
       const uint64_t qd = make_smem_desc(q_s, 16, 1024);
       const uint64_t kd = make_smem_desc(stage0 + stage * kStageBytes, 16, 1024);
-      if (lane == 0) {
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint64_t ao = (uint64_t)((kk >> 2) * (kQBytes / 2) + (kk & 3) * 32) >> 4;
-          const uint64_t bo = (uint64_t)((kk >> 2) * (kKBytes / 2) + (kk & 3) * 32) >> 4;
-          umma_f16(d, qd + ao, kd + bo, sh.idesc_s, kk ? 1u : 0u);
-        }
-        umma_commit(sfull0 + 8u * sbuf);
+      for (int kk = 0; kk < HD / 16; ++kk) {
+        const uint64_t ao = (uint64_t)((kk >> 2) * (kQBytes / 2) + (kk & 3) * 32) >> 4;
+        const uint64_t bo = (uint64_t)((kk >> 2) * (kKBytes / 2) + (kk & 3) * 32) >> 4;
+        umma_f16(d, qd + ao, kd + bo, sh.idesc_s, kk ? 1u : 0u, e);
       }
-      __syncwarp();
+      umma_commit(sfull0 + 8u * sbuf, e);
     };
     int stage = 0; uint32_t phase = 0;
     int it = 0;                                              // S tiles issued so far (all items, both passes)
@@ -312,8 +313,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (!__all_sync(0xffffffffu, a && b)) goto issuer_done;
         tc_fence_after();
         issue_s(stage, sb);
-        if (lane == 0) umma_commit(empty0 + 8u * stage);
-        __syncwarp();
+        umma_commit(empty0 + 8u * stage, e);
         if (++stage == kTcStages) { stage = 0; phase ^= 1; }
       }
       // pass B: S runs one tile ahead of P.V
@@ -330,13 +330,11 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         return true;
       };
       if (n_tiles > 0 && !issue_s_next()) goto issuer_done;
-      if (n_tiles <= 1 && lane == 0) umma_commit(qfree);     // the item's last score MMA is issued
-      __syncwarp();
+      if (n_tiles <= 1) umma_commit(qfree, e);               // the item's last score MMA is issued
       for (int j = 0; j < n_tiles; ++j, ++jg) {
         if (j + 1 < n_tiles) {
           if (!issue_s_next()) goto issuer_done;
-          if (j + 2 == n_tiles && lane == 0) umma_commit(qfree);
-          __syncwarp();
+          if (j + 2 == n_tiles) umma_commit(qfree, e);
         }
         const int b = jg & 1; const uint32_t ph = (jg >> 1) & 1;
         const bool r1 = mbar_wait(pready0 + 8u * b, ph, abort_flag);
@@ -363,14 +361,11 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const uint32_t d = tmem_base + kColPV + (uint32_t)(b * HD);
         const uint64_t pd = make_smem_desc(p_s0 + b * kPBytes, 16, 1024);
         const uint64_t vd = make_smem_desc(stage0 + stage * kStageBytes + kKBytes, 8192, 1024);
-        if (lane == 0) {
 #pragma unroll
-          for (int kk = 0; kk < kTcTileN / 16; ++kk)
-            umma_f16(d, pd + (uint64_t)(kk * 2), vd + (uint64_t)(kk * 128), sh.idesc_pv, kk ? 1u : 0u);
-          umma_commit(pvfull0 + 8u * b);
-          umma_commit(empty0 + 8u * stage);
-        }
-        __syncwarp();
+        for (int kk = 0; kk < kTcTileN / 16; ++kk)
+          umma_f16(d, pd + (uint64_t)(kk * 2), vd + (uint64_t)(kk * 128), sh.idesc_pv, kk ? 1u : 0u, e);
+        umma_commit(pvfull0 + 8u * b, e);
+        umma_commit(empty0 + 8u * stage, e);
         if (++stage == kTcStages) { stage = 0; phase ^= 1; }
       }
     }
@@ -385,6 +380,9 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const float ninf = -__int_as_float(0x7f800000);
     const bool plain_scores = !(p.cap_log2 > 0.0f) && p.alibi == nullptr;
     const float magic = __uint_as_float(kMagicBits);
+    const uint32_t mbits = q_magic_bits(p.inv_scale), one = (uint32_t)zero + 1u;
+    const uint64_t magic2 = pack2(mbits, mbits);
+    const float screen_limit = q_screen_limit(p.inv_scale);
     uint32_t soft_phase = 0;
     bool ok = true;
     auto soft_sync = [&]() -> bool {                         // bounded barrier over these 8 warps
@@ -469,29 +467,22 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (!warp_wait_relaxed(pvfull0 + 8u * b, ph, abort_flag, lane)) return false;
       tc_fence_after();
       const uint32_t taddr = tmem_base + lane_sel + kColPV + (uint32_t)(b * HD + half * kHalfCols);
-      uint32_t screen = 0, screen_b = 0;
-      {
-        uint32_t v[32];
-        tmem_ld32(taddr, v);
-        tmem_wait_ld();
+      float screen = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const uint32_t ra = __float_as_uint(__fmaf_rn(__uint_as_float(v[i]), p.scale, magic));
-          const uint32_t rb = __float_as_uint(__fmaf_rn(__uint_as_float(v[i + 1]), p.scale, magic));
-          acc[i] += ra;
-          acc[i + 1] += rb;
-          screen |= ra ^ kExpBits;
-          screen_b |= rb ^ kExpBits;
-        }
+      for (int c = 0; c < kHalfCols; c += 16) {
+        uint32_t v[16];
+        tmem_ld16(taddr + c, v);
+        tmem_wait_ld_regs(v);
+        convert16(v, &acc[c], magic2, mbits, one, screen);
       }
-      if (__any_sync(0xffffffffu, ((screen | screen_b) >> 23) != 0)) {
+      if (__any_sync(0xffffffffu, !(screen < screen_limit))) {
         // some partial left the fast range: exact conversion of the offending elements
         if (!corr_used) {
 #pragma unroll 1
           for (int z = 0; z < kHalfCols; ++z) { corr_raw[z + zero] = 0; corr_q[z + zero] = 0; }
           corr_used = true;
         }
-        fixup_tile(taddr, kHalfCols, p.scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
+        fixup_tile(taddr, kHalfCols, mbits, p.scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
       }
       tc_fence_before();
       __syncwarp();
@@ -542,14 +533,14 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       for (int c = 1; c < CG; ++c) dsum += den_s[c * kTcRows + row];
       const float dn = fmaxf(fixed_to_float<long long>(wrap_to_bits(dsum, p.int_bits), p.inv_scale), 1.0e-6f);
       T* op = (T*)p.o + (int64_t)(q_start + tok) * p.o_st + (int64_t)head * p.o_sh + half * kHalfCols;
-      const uint32_t bias_bits = (uint32_t)n_tiles * kMagicBits;
+      const uint32_t bias_bits = (uint32_t)n_tiles * mbits;   // what the multiply-adds summed on top
 #pragma unroll
       for (int g8 = 0; g8 < kHalfCols / 8; ++g8) {
         alignas(16) T out[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int c = g8 * 8 + i;
-          uint32_t raw = acc[c] - bias_bits;
+          uint32_t raw = alu_add(c) ? acc[c] : acc[c] - bias_bits;
           float num;
           if (corr_used) {
             raw -= corr_raw[c + zero];

@@ -99,19 +99,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
             const uint32_t sa = smem_base + stage * L::kStageBytes;
             const uint32_t sb = sa + L::kABytes;
             const int k0 = kt * p.k_tile + ch * kBK;
-            mbar_expect_tx(full_bar(stage), L::kStageBytes);
-            tma_load_2d(sa, &tma_a, full_bar(stage), k0, pm * kBM);
+            mbar_expect_tx(full_bar(stage), L::kStageBytes, 1u);
+            tma_load_2d(sa, &tma_a, full_bar(stage), k0, pm * kBM, 1u);
             if (p.b_kmajor) {
               // B stored (N, K): rows = n, 64 k contiguous; boxes of 64 rows keep the
               // tensor-map box <= 256 and the layout identical to A's
 #pragma unroll
               for (int j = 0; j < BN / 64; ++j)
-                tma_load_2d(sb + j * (64 * kBK * 2), &tma_b, full_bar(stage), k0, pn * BN + j * 64);
+                tma_load_2d(sb + j * (64 * kBK * 2), &tma_b, full_bar(stage), k0, pn * BN + j * 64, 1u);
             } else {
               // B stored (K, N): boxes of 64 n (128 B) x 64 k rows
 #pragma unroll
               for (int j = 0; j < BN / 64; ++j)
-                tma_load_2d(sb + j * (64 * kBK * 2), &tma_b, full_bar(stage), pn * BN + j * 64, k0);
+                tma_load_2d(sb + j * (64 * kBK * 2), &tma_b, full_bar(stage), pn * BN + j * 64, k0, 1u);
             }
             if (++stage == STAGES) { stage = 0; phase ^= 1; }
           }
@@ -143,15 +143,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
             // descriptors differ from stage 0 / k 0 only in the 14-bit address field
             const uint64_t ad = adesc0 + (uint64_t)stage * kStageStep;
             const uint64_t bd = bdesc0 + (uint64_t)stage * kStageStep;
-            umma_f16(d_tmem, ad, bd, idesc, ch ? 1u : 0u);
-            umma_f16(d_tmem, ad + 2, bd + b_kstep, idesc, 1u);
-            umma_f16(d_tmem, ad + 4, bd + 2 * b_kstep, idesc, 1u);
-            umma_f16(d_tmem, ad + 6, bd + 3 * b_kstep, idesc, 1u);
-            umma_commit(empty_bar(stage));   // frees the smem stage when these MMAs finish
+            umma_f16(d_tmem, ad, bd, idesc, ch ? 1u : 0u, 1u);
+            umma_f16(d_tmem, ad + 2, bd + b_kstep, idesc, 1u, 1u);
+            umma_f16(d_tmem, ad + 4, bd + 2 * b_kstep, idesc, 1u, 1u);
+            umma_f16(d_tmem, ad + 6, bd + 3 * b_kstep, idesc, 1u, 1u);
+            umma_commit(empty_bar(stage), 1u);   // frees the smem stage when these MMAs finish
             if (++stage == STAGES) { stage = 0; phase ^= 1; }
           }
           if (!ok) break;
-          umma_commit(tfull_bar(buf));       // K-tile accumulator complete
+          umma_commit(tfull_bar(buf), 1u);       // K-tile accumulator complete
           tphase[buf] ^= 1; buf ^= 1;
         }
       }
@@ -417,14 +417,12 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, TcParams& p, 
 
 bool gemm_tc_fast_supported(const GemmArgs& g, int split_k);
 bool gemm_tc_skinny_supported(const GemmArgs& g, int split_k);
-bool gemm_tc_n256_supported(const GemmArgs& g, int split_k);
-int gemm_tc_n256(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb, cudaStream_t s);
 int gemm_tc_skinny(const GemmArgs& g, TcParams& p, const CUtensorMap& mw, cudaStream_t s);
 int gemm_tc_fast(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb,
                  cudaStream_t s);
 bool gemm_tc_pair_supported(const GemmArgs& g, int split_k);
 int gemm_tc_pair(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb,
-                 int bn, cudaStream_t s);
+                 cudaStream_t s);
 
 int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   const int sms = tc_device_sms();
@@ -452,7 +450,7 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   p.scale = (float)(1ull << g.frac_bits); p.inv_scale = 1.0f / p.scale;
   p.b_kmajor = b_kmajor ? 1 : 0;
   p.idesc = make_idesc(g.dtype == FXPR_BF16 ? 1 : 0, b_kmajor ? 0 : 1, BN, kBM);
-  p.c_vec_ok = (g.c && (((uintptr_t)g.c & 15) == 0) && (g.c_sm % 8 == 0)) ? 1 : 0;
+  p.c_vec_ok = !g.c || ((uintptr_t)g.c & 15) || g.c_sm % 8 ? 0 : ((uintptr_t)g.c & 31) || g.c_sm % 16 ? 1 : 2;
   p.status = g.status;
   p.silu_mul = 0;
   p.best = nullptr; p.n_offset = 0;
@@ -480,17 +478,17 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   }
   if (g.best) return FXPR_ERR_UNSUPPORTED;                          // only the decode-shape kernel
   if (g.flags & FXPR_GEMM_SILU_MUL) return FXPR_ERR_UNSUPPORTED;   // only the decode-shape kernel fuses it
-  // 128 x 256 tiles: measured +6 % at k_tile 128 (two 64-deep stages per accumulator) and -12 %
-  // at k_tile 64 (one MMA group per hand-off with only two accumulators in TMEM), same bits;
-  // so they are the default for k_tile 128 only.  The flags force either shape.
-  if ((g.flags & FXPR_GEMM_PAIR) && !(g.flags & FXPR_GEMM_FORCE_EXACT_TC) && gemm_tc_pair_supported(g, p.split_k)) {
-    int bn = (g.N >= 256) ? 256 : 128;
-    if (g.flags & FXPR_GEMM_TILE_N128) bn = 128;
-    return gemm_tc_pair(g, p, ma, mb, bn, s);
+  if (!(g.flags & FXPR_GEMM_FORCE_EXACT_TC) && gemm_tc_pair_supported(g, p.split_k)) {
+    // 256 x 256 tiles on SM pairs or 128 x 128 tiles on single SMs (same bits).  A full wave of pair
+    // tiles has twice the output of a wave of single tiles and takes 1.7 times as long at K-tile 64
+    // (57 against 34 us at K = 4096), 1.55 times at K-tile 128 (40 against 26 us): count the waves.
+    const int64_t pair_tiles = ((g.M + 255) / 256) * ((g.N + 255) / 256);
+    const int64_t single_tiles = ((g.M + 127) / 128) * ((g.N + 127) / 128);
+    const int64_t pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2), single_waves = (single_tiles + sms - 1) / sms;
+    const bool wide = pair_waves * (g.k_tile == 64 ? 170 : 155) <= single_waves * 100;
+    if ((g.flags & (FXPR_GEMM_PAIR | FXPR_GEMM_TILE_N256)) || (wide && !(g.flags & FXPR_GEMM_TILE_N128)))
+      return gemm_tc_pair(g, p, ma, mb, s);
   }
-  const bool want_n256 = (g.flags & FXPR_GEMM_TILE_N256) || (g.k_tile == 128 && !(g.flags & FXPR_GEMM_TILE_N128));
-  if (want_n256 && !(g.flags & FXPR_GEMM_FORCE_EXACT_TC) && gemm_tc_n256_supported(g, p.split_k))
-    return gemm_tc_n256(g, p, ma, mb, s);
   if (!(g.flags & FXPR_GEMM_FORCE_EXACT_TC) && gemm_tc_fast_supported(g, p.split_k)) {
     return gemm_tc_fast(g, p, ma, mb, s);
   }

@@ -106,9 +106,10 @@ gemm_tc_fast_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   if (warp == 0) {
     // ------------------------------ TMA producer --------------------------------
     // All 32 lanes run the loop (uniform control flow lets the compiler keep addresses
-    // and descriptors in uniform registers); lane 0 alone issues the copies.
+    // and descriptors in uniform registers); one elected lane issues the copies.
     {
       const bool bk = p.b_kmajor != 0;
+      const uint32_t e = elect_one();
       int stage = 0; uint32_t phase = 1;               // "empty" waits start one phase ahead
       int gss = 0;
       for (int item = blockIdx.x; item < items; item += gridDim.x) {
@@ -127,20 +128,17 @@ gemm_tc_fast_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
           const uint32_t fb = full0 + 8u * stage;
           const uint32_t sa = smem_base + stage * kSSBytes;
           const uint32_t sb = sa + kSSBytesA;
-          if (lane == 0) {
-            mbar_expect_tx(fb, two ? kSSBytes : kSSBytes / 2);
-            tma_load_2d(sa, &tma_a, fb, ka, m0);
+          mbar_expect_tx(fb, two ? kSSBytes : kSSBytes / 2, e);
+          tma_load_2d(sa, &tma_a, fb, ka, m0, e);
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j)
+            tma_load_2d(sb + j * 8192, &tma_b, fb, bk ? ka : n0 + j * 64, bk ? n0 + j * 64 : ka, e);
+          if (two) {
+            tma_load_2d(sa + kSSBytesA / 2, &tma_a, fb, kb, m0, e);
 #pragma unroll
             for (int j = 0; j < BN / 64; ++j)
-              tma_load_2d(sb + j * 8192, &tma_b, fb, bk ? ka : n0 + j * 64, bk ? n0 + j * 64 : ka);
-            if (two) {
-              tma_load_2d(sa + kSSBytesA / 2, &tma_a, fb, kb, m0);
-#pragma unroll
-              for (int j = 0; j < BN / 64; ++j)
-                tma_load_2d(sb + kSSBytesB / 2 + j * 8192, &tma_b, fb, bk ? kb : n0 + j * 64, bk ? n0 + j * 64 : kb);
-            }
+              tma_load_2d(sb + kSSBytesB / 2 + j * 8192, &tma_b, fb, bk ? kb : n0 + j * 64, bk ? n0 + j * 64 : kb, e);
           }
-          __syncwarp();
           ++gss;
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -149,11 +147,9 @@ gemm_tc_fast_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------------
-    // One lane feeds the tensor core and its loop is latency-bound (each mbarrier probe,
-    // fence, MMA issue and commit costs 50-100 cycles), so it does as little as possible
-    // per 8 MMAs: two waits, one fence, two commits.  Descriptors are built once; only
-    // their 14-bit address field (bytes >> 4) advances.  All lanes run the loop (uniform
-    // control flow, operands in uniform registers); lane 0 issues.
+    // All lanes run the loop (uniform control flow, operands in uniform registers); the elected
+    // lane issues.  Descriptors are built once; only their 14-bit address field (bytes >> 4)
+    // advances.
     {
       const uint64_t adesc0 = make_smem_desc(smem_base, 16, 1024);
       const uint64_t bdesc0 = p.b_kmajor ? make_smem_desc(smem_base + kSSBytesA, 16, 1024)
@@ -161,7 +157,7 @@ gemm_tc_fast_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
       const uint64_t bks = p.b_kmajor ? 2 : 128;        // (32 B | 2048 B) >> 4 per 16-deep k step
       constexpr uint64_t kStep = kSSBytes >> 4;
       constexpr uint64_t kHalfA = (kSSBytesA / 2) >> 4, kHalfB = (kSSBytesB / 2) >> 4;
-      const uint32_t idesc = p.idesc;
+      const uint32_t idesc = p.idesc, e = elect_one();
       int stage = 0; uint32_t phase = 0; int grp = 0; uint32_t gphase = 1;
       int gss = 0;
       for (int item = blockIdx.x; item < items; item += gridDim.x) {
@@ -180,21 +176,18 @@ gemm_tc_fast_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
           const uint32_t d1 = pairs ? d0 + BN : d0;       // second half: other buffer, or accumulate on
           const uint64_t ad = adesc0 + (uint64_t)stage * kStep;
           const uint64_t bd = bdesc0 + (uint64_t)stage * kStep;
-          if (lane == 0) {
-          umma_f16(d0, ad, bd, idesc, 0u);
-          umma_f16(d0, ad + 2, bd + bks, idesc, 1u);
-          umma_f16(d0, ad + 4, bd + 2 * bks, idesc, 1u);
-          umma_f16(d0, ad + 6, bd + 3 * bks, idesc, 1u);
+          umma_f16(d0, ad, bd, idesc, 0u, e);
+          umma_f16(d0, ad + 2, bd + bks, idesc, 1u, e);
+          umma_f16(d0, ad + 4, bd + 2 * bks, idesc, 1u, e);
+          umma_f16(d0, ad + 6, bd + 3 * bks, idesc, 1u, e);
           if (two) {
-            umma_f16(d1, ad + kHalfA, bd + kHalfB, idesc, pairs ? 0u : 1u);
-            umma_f16(d1, ad + kHalfA + 2, bd + kHalfB + bks, idesc, 1u);
-            umma_f16(d1, ad + kHalfA + 4, bd + kHalfB + 2 * bks, idesc, 1u);
-            umma_f16(d1, ad + kHalfA + 6, bd + kHalfB + 3 * bks, idesc, 1u);
+            umma_f16(d1, ad + kHalfA, bd + kHalfB, idesc, pairs ? 0u : 1u, e);
+            umma_f16(d1, ad + kHalfA + 2, bd + kHalfB + bks, idesc, 1u, e);
+            umma_f16(d1, ad + kHalfA + 4, bd + kHalfB + 2 * bks, idesc, 1u, e);
+            umma_f16(d1, ad + kHalfA + 6, bd + kHalfB + 3 * bks, idesc, 1u, e);
           }
-          umma_commit(empty0 + 8u * stage);            // frees the super-stage when these finish
-          umma_commit(tfull0 + 8u * grp);              // accumulator(s) of this super-stage complete
-          }
-          __syncwarp();
+          umma_commit(empty0 + 8u * stage, e);            // frees the super-stage when these finish
+          umma_commit(tfull0 + 8u * grp, e);              // accumulator(s) of this super-stage complete
           ++gss;
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
           grp ^= 1; if (grp == 0) gphase ^= 1;

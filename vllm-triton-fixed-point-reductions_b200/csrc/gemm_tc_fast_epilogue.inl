@@ -7,7 +7,9 @@
   const int row_in_tile = quarter * 32 + lane;
   const int col0 = cgroup * kCols;
   const uint32_t lane_addr = ((uint32_t)(quarter * 32) << 16) + (uint32_t)col0;
-  const float magic = __uint_as_float(kMagicBits);
+  const uint32_t mbits = q_magic_bits(p.inv_scale), one = (uint32_t)zero + 1u;
+  const uint64_t magic2 = pack2(mbits, mbits);
+  const float screen_limit = q_screen_limit(p.inv_scale);
   const float scale = p.scale;
   int grp = 0; uint32_t gphase = 0; uint32_t epi_phase = 0; bool ok = true;
   int gss = 0;
@@ -42,9 +44,6 @@
       if (!warp_wait(tfull0 + 8u * grp, gphase, abort_flag, lane)) { ok = false; break; }
       tc_fence_after();
       const int nbuf = (pairs && 2 * ss + 1 < n_kt) ? 2 : 1;
-      // Hot path: r = fma(p, 2^f, MAGIC) on the FP32 pipe, raw bit patterns added as
-      // integers, and the OR of the raw fp32 bits as a screen: bit 30 stays clear only if
-      // every |p| < 2, which (f <= 21) implies |p * 2^f| < 2^22.
       // Measured on B200: this plain order (load 16 columns, wait, convert) beats both a
       // software-pipelined order (next load in flight during the conversion: -6 %) and a
       // pairwise order (both K-tiles of a pair per step, one three-input add: -11 %).
@@ -52,14 +51,9 @@
       const uint32_t ta0 = tmem_base + lane_addr + (uint32_t)((grp * 2) * BN);
       const uint32_t ta1 = ta0 + BN;
       uint32_t va[16], vb[16];
-      uint32_t screen0 = 0, screen1 = 0;
-      auto convert = [&](const uint32_t (&v)[16], int c, uint32_t& screen, int h) {
-#pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          acc[c * 16 + i] += __float_as_uint(__fmaf_rn(__uint_as_float(v[i]), scale, magic));
-          acc[c * 16 + i + 1] += __float_as_uint(__fmaf_rn(__uint_as_float(v[i + 1]), scale, magic));
-          screen |= v[i] | v[i + 1];
-        }
+      float screen0 = 0.0f, screen1 = 0.0f;
+      auto convert = [&](const uint32_t (&v)[16], int c, float& screen, int h) {
+        convert16(v, &acc[c * 16], magic2, mbits, one, screen);
         if (DUMP) {
           if (row < p.M) {
             const int kt = pairs ? ks + (2 * ss + h) * p.split_k : ks + ss * p.split_k;
@@ -76,17 +70,17 @@
         tmem_ld16(ta1, va); tmem_wait_ld_regs(va); convert(va, 0, screen1, 1);
         tmem_ld16(ta1 + 16, vb); tmem_wait_ld_regs(vb); convert(vb, 1, screen1, 1);
       }
-      if (__any_sync(0xffffffffu, ((screen0 | screen1) & 0x40000000u) != 0)) {
+      if (__any_sync(0xffffffffu, !(screen0 < screen_limit && screen1 < screen_limit))) {
         // exact fix-up for the K-tile(s) that failed the screen (rare): see fixup_tile
         if (!corr_used) {
 #pragma unroll 1
           for (int z = 0; z < kCols; ++z) { corr_raw[z + zero] = 0; corr_q[z + zero] = 0; }
           corr_used = true;
         }
-        if (__any_sync(0xffffffffu, (screen0 & 0x40000000u) != 0))
-          fixup_tile(ta0, kCols, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
-        if (__any_sync(0xffffffffu, (screen1 & 0x40000000u) != 0))
-          fixup_tile(ta1, kCols, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
+        if (__any_sync(0xffffffffu, !(screen0 < screen_limit)))
+          fixup_tile(ta0, kCols, mbits, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
+        if (__any_sync(0xffffffffu, !(screen1 < screen_limit)))
+          fixup_tile(ta1, kCols, mbits, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
       }
       tc_fence_before();
       __syncwarp();
@@ -96,10 +90,10 @@
     }
     if (!ok) break;
 
-    // every K-tile added MAGIC once
-    const uint32_t bias_bits = (uint32_t)n_kt * kMagicBits;
+    // the multiply-adds summed one magic per K-tile
+    const uint32_t bias_bits = (uint32_t)n_kt * mbits;
     auto total = [&](int i) -> long long {
-      uint32_t raw = acc[i] - bias_bits;
+      uint32_t raw = alu_add(i) ? acc[i] : acc[i] - bias_bits;
       long long t;
       if (corr_used) {
         // the in-range part is < 2^31 in magnitude, so it is the sign extension of the

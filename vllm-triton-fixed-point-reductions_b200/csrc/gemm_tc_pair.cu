@@ -1,33 +1,30 @@
-// Two-SM route of the tensor-core fixed-point GEMM (sm_100a): tcgen05.mma with
-// cta_group::2 on clusters of two CTAs.
+// Two-SM route of the tensor-core fixed-point GEMM (sm_100a): tcgen05.mma with cta_group::2 on
+// clusters of two CTAs, one 256 x 256 output tile per pair.  The default for large products.
 //
-// Why: measured with an idle epilogue, the single-CTA kernels are bound by operand traffic
-// from L2 into shared memory, not by the tensor pipe -- a 128 x 128 tile pulls 32 KB per
-// 64-deep stage (2.1 GB for a 4096^3 problem, ~200 us), a 128 x 256 tile 48 KB (1.6 GB,
-// ~140 us), against 82 us of tensor work.  A CTA pair computes a 256 x BN tile with ONE
-// instruction stream: each CTA loads its own 128 rows of A and its own half of the BN columns
-// of B, the tensor cores of both SMs read both halves of B, and each CTA's tensor memory
-// receives its 128 rows x BN columns of the accumulator.  Per CTA that is 32 KB per stage
-// for a 128 x 256 accumulator (1.07 GB in all), and one MMA-issuing thread per two SMs.
+// What bounds it.  The single-CTA kernels pull 48 KB of operands per 64-deep step of a 128 x 256
+// tile out of L2 (~140 us at 4096^3, against 82 us of tensor work).  Here each CTA loads its own 128
+// rows of A and its own 128 columns of B, 32 KB per step for the same accumulator; the tensor cores
+// of both SMs read both halves of B, and each CTA's tensor memory receives its 128 rows x 256
+// columns: with the conversion left out the kernel runs at 100 us.  The conversion of a K-tile costs
+// each SM about 760 clocks (32768 partials: packed add, integer add, range screen = 2.4 issue slots
+// per partial), the tensor work 512 clocks at K-tile 64 and 1024 at K-tile 128.
 //
-// Roles per CTA (18 warps): warp 0 = TMA producer (both CTAs, each for its own shared
-// memory; the copies of both complete on the leader's "full" barrier), warp 1 = MMA issuer
-// (leader CTA only; its commits arrive on the barriers of both CTAs), warps 2-17 = epilogue
-// (each CTA drains its own tensor memory; the follower's warps arrive on the leader's
-// "accumulator free" barrier through the cluster address space).  Every copy names one
-// destination and one barrier; only tcgen05.commit signals both CTAs at once.
+// What it depends on, measured at 4096^3 with the conversion left out:
+//   - MMAs, commits and copies are predicated instructions of a uniform warp (tc_common.cuh);
+//   - the "accumulator drained" arrival crosses to the leader CTA as a plain mbarrier.arrive: with
+//     .release.cluster on it (a cluster-wide fence behind the TMA traffic) K-tile 64 took 242 us
+//     instead of 126, K-tile 128 156 instead of 109;
+//   - one 256-column accumulator per K-tile and two of them in tensor memory: four of 128 columns
+//     double the hand-offs and measured 175 us instead of 126 at K-tile 64.
 //
-// Barriers: full[stage] (leader), done[stage] (both CTAs: "the MMAs that read this stage
-// have finished" -- the producer refills the stage on it and, for the last stage of a
-// K-tile, the epilogue reads the accumulator on it: one commit per stage serves both),
-// tempty[buffer] (the CTA's 16 epilogue warps have drained the buffer; the follower's idle
-// warp 1 forwards its completion to the leader's as ONE remote arrival.  Measured at 4096^3,
-// K-tile 128: sixteen remote arrivals per K-tile 259 us, the forwarding warp 212 us, a
-// shared-memory counter whose last arriver signals 236 us).
+// Roles per CTA (18 warps): warp 0 = TMA producer (both CTAs, each for its own shared memory; the
+// copies of both complete on the leader's "full" barrier), warp 1 = MMA issuer (leader only; its
+// commits arrive on the barriers of both CTAs), warps 2-17 = epilogue: thread = one row and 64
+// columns, so the running sums fit the 96 registers an 18-warp CTA has.
 //
-// Numerics, the magic-number conversion with its exact fix-up, split-K planes, bounded
-// waits and the persistent grouped tile order are those of gemm_tc_fast.cu; results are
-// bit-identical to it (the fixed-point contract: fxpr_vllm/_triton/gemm.py:183-204).
+// Numerics, the conversion with its range screen and exact fix-up are those of gemm_tc_fast.cu
+// (gemm_tc_fast_common.cuh); results are bit-identical to it (the fixed-point contract:
+// fxpr_vllm/_triton/gemm.py:183-204).  Every wait is bounded.
 #include <cuda.h>
 
 #include "fxp_common.cuh"
@@ -58,15 +55,17 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // TMA tile load whose completion bytes are counted on a barrier that may live in the peer CTA
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster,
-                                                 int x, int y) {
+                                                 int x, int y, uint32_t elected) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(x), "r"(y) : "memory");
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4}], [%2];\n\t}"
+      ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(x), "r"(y), "r"(elected) : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
@@ -78,37 +77,24 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
+                                              uint32_t accumulate, uint32_t elected) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
 }
 // Arrives on the barrier at this shared-memory offset in BOTH CTAs of the pair once every MMA
-// this thread issued so far is done.  One instruction for both: a tcgen05.commit costs the
-// issuing thread ~260 clocks here (measured with no MMA in flight), so commits are rationed.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+// this thread issued so far is done.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t elected) {
   const uint16_t both = 3;
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"(both) : "memory");
-}
-__device__ __forceinline__ void tmem_ld8p(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-      : "r"(taddr) : "memory");
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(bar), "h"(both), "r"(elected) : "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld8p(uint32_t (&r)[8]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
-               :: "memory");
-}
-__device__ __forceinline__ void tmem_ldp(uint32_t taddr, uint32_t (&r)[8]) { tmem_ld8p(taddr, r); }
-__device__ __forceinline__ void tmem_ldp(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
-__device__ __forceinline__ void tmem_wait_ldp(uint32_t (&r)[8]) { tmem_wait_ld8p(r); }
-__device__ __forceinline__ void tmem_wait_ldp(uint32_t (&r)[16]) { tmem_wait_ld_regs(r); }
-
 // Non-blocking probe.  mbarrier.try_wait may park the thread for a hardware time limit, and a
 // parked thread is woken promptly only by arrivals from its own CTA; most barriers here are
 // completed from the peer CTA, so the waits of this kernel poll with test_wait instead.
@@ -139,50 +125,43 @@ __device__ __forceinline__ bool warp_wait_poll(uint32_t bar, uint32_t parity, vo
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
-template <int BN> struct PairCfg {
-  static constexpr int kStages = BN == 256 ? 6 : 8;
-  static constexpr int kABytes = kBM * kBK * 2;             // this CTA's 128 rows of A
-  static constexpr int kBBytes = (BN / 2) * kBK * 2;        // this CTA's half of the B columns
-  static constexpr int kStageBytes = kABytes + kBBytes;     // 32 KB / 24 KB
-  static constexpr int kNBuf = 512 / BN;
-  static constexpr int kSmem = kStages * kStageBytes + 256 + 1024;
-  static constexpr int kChunk = BN == 256 ? 8 : 16;         // columns per tcgen05.ld
-};
+static constexpr int kPrStages = 6;
+static constexpr int kPrABytes = kBM * kBK * 2;            // this CTA's 128 rows of A
+static constexpr int kPrBBytes = 128 * kBK * 2;            // this CTA's 128 columns of B
+static constexpr int kPrStageBytes = kPrABytes + kPrBBytes;
+static constexpr int kPrSmem = kPrStages * kPrStageBytes + 256 + 1024;
+static constexpr int kPrCols = 64;                         // accumulator columns per epilogue thread
 
-template <typename T, int BN, bool DUMP>
+// 32-byte store: every lane of a warp writes another output row, so one full sector per lane
+__device__ __forceinline__ void st_global_32(void* dst, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+}
+
+template <typename T>
 __global__ void __launch_bounds__(kPrThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                     const TcParams p, const int zero /* always 0: keeps the side arrays in local memory */) {
-  using Cfg = PairCfg<BN>;
-  constexpr int STAGES = Cfg::kStages;
-  constexpr int NBUF = Cfg::kNBuf;
-  constexpr int CH = Cfg::kChunk;
-  constexpr int kCols = BN / (kPrEpiW / 4);               // columns per epilogue thread
-  constexpr int NCH = kCols / CH;
-  constexpr int kBarOffset = STAGES * Cfg::kStageBytes;
-
+  constexpr int kBarOffset = kPrStages * kPrStageBytes;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bar_base = smem_base + kBarOffset;
-  const uint32_t full0 = bar_base, done0 = bar_base + 8u * STAGES;
-  const uint32_t tempty0 = bar_base + 8u * (2 * STAGES);
-  constexpr int kMisc = 8 * (2 * STAGES + NBUF);
+  // full[stage]: the leader's arrive plus the bytes of both CTAs; empty[stage], tfull[buffer]: one
+  // commit, in both CTAs; tempty[buffer] (leader): the epilogue warps of both CTAs
+  const uint32_t full0 = bar_base, empty0 = full0 + 8u * kPrStages;
+  const uint32_t tfull0 = empty0 + 8u * kPrStages, tempty0 = tfull0 + 16u;
+  constexpr int kMisc = 16 * kPrStages + 32;
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem_gen + kBarOffset + kMisc);
   volatile int* abort_flag = (volatile int*)(smem_gen + kBarOffset + kMisc + 8);
-  const uint32_t epi_bar = bar_base + kMisc + 16u;
-  volatile int* s_last = (volatile int*)(smem_gen + kBarOffset + kMisc + 24);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();                 // 0 = leader
   const int pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    // full: one arrive (the leader's producer) plus the bytes of both CTAs; done: one commit;
-    // tempty: this CTA's epilogue warps, plus in the leader one arrival forwarded from the follower
-    for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8u * s, 1); mbar_init(done0 + 8u * s, 1); }
-    for (int b = 0; b < NBUF; ++b) mbar_init(tempty0 + 8u * b, rank == 0 ? kPrEpiW + 1 : kPrEpiW);
-    mbar_init(epi_bar, kPrEpiW);
+    for (int s = 0; s < kPrStages; ++s) { mbar_init(full0 + 8u * s, 1); mbar_init(empty0 + 8u * s, 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(tfull0 + 8u * b, 1); mbar_init(tempty0 + 8u * b, 2 * kPrEpiW); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -196,9 +175,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int tiles_mn = p.tiles_m * p.tiles_n;              // pair tiles: 256 rows x BN columns
-  const int items = tiles_mn * p.split_k;
-  const int k_tiles_total = (p.K + p.k_tile - 1) / p.k_tile;
+  const int items = p.tiles_m * p.tiles_n;                 // pair tiles of 256 x 256
+  const int n_kt = (p.K + p.k_tile - 1) / p.k_tile;
   const int halves = p.k_tile / 64;                        // stages per K-tile: 1 or 2
 
   auto tile_coords = [&](int tile, int& pm, int& pn) {
@@ -212,258 +190,174 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ----------------------
+    const uint32_t e = elect_one();
     const bool bk = p.b_kmajor != 0;
+    const uint32_t full_leader = mapa_u32(full0, 0);       // the leader's barriers count both CTAs' bytes
     int stage = 0; uint32_t phase = 1;
     for (int item = pair_id; item < items; item += num_pairs) {
-      int pm, pn; tile_coords(item / p.split_k, pm, pn);
+      int pm, pn; tile_coords(item, pm, pn);
       const int m0 = pm * 256 + (int)rank * kBM;
-      const int n0 = pn * BN + (int)rank * (BN / 2);
-      const int ks = item % p.split_k;
-      const int n_kt = (k_tiles_total - ks + p.split_k - 1) / p.split_k;
-      for (int i = 0; i < n_kt; ++i) {
-        const int kt = ks + i * p.split_k;
-        for (int h = 0; h < halves; ++h) {
-          const int k0 = kt * p.k_tile + h * 64;
-          if (!__all_sync(0xffffffffu, mbar_wait_poll(done0 + 8u * stage, phase, abort_flag))) goto producer_done;
-          const uint32_t fb_local = full0 + 8u * stage;
-          const uint32_t fb = mapa_u32(fb_local, 0);       // the leader's barrier counts both CTAs' bytes
-          const uint32_t sa = smem_base + stage * Cfg::kStageBytes;
-          const uint32_t sb = sa + Cfg::kABytes;
-          if (lane == 0) {
-            if (rank == 0) mbar_expect_tx(fb_local, 2 * Cfg::kStageBytes);
-            tma_load_2d_pair(sa, &tma_a, fb, k0, m0);
-#pragma unroll
-            for (int j = 0; j < BN / 128; ++j)
-              tma_load_2d_pair(sb + j * 8192, &tma_b, fb, bk ? k0 : n0 + j * 64, bk ? n0 + j * 64 : k0);
-          }
-          __syncwarp();
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        }
+      const int n0 = pn * 256 + (int)rank * 128;
+      for (int i = 0; i < n_kt * halves; ++i) {
+        const int k0 = i * 64;
+        if (!__all_sync(0xffffffffu, mbar_wait_poll(empty0 + 8u * stage, phase, abort_flag))) goto producer_done;
+        const uint32_t fb = full_leader + 8u * stage;
+        const uint32_t sa = smem_base + stage * kPrStageBytes;
+        const uint32_t sb = sa + kPrABytes;
+        if (rank == 0) mbar_expect_tx(full0 + 8u * stage, 2 * kPrStageBytes, e);
+        tma_load_2d_pair(sa, &tma_a, fb, k0, m0, e);
+        tma_load_2d_pair(sb, &tma_b, fb, bk ? k0 : n0, bk ? n0 : k0, e);
+        tma_load_2d_pair(sb + 8192, &tma_b, fb, bk ? k0 : n0 + 64, bk ? n0 + 64 : k0, e);
+        if (++stage == kPrStages) { stage = 0; phase ^= 1; }
       }
     }
   producer_done:;
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader only) ----------------------
     if (rank == 0) {
+      const uint32_t e = elect_one();
       const uint64_t adesc0 = make_smem_desc(smem_base, 16, 1024);
-      const uint64_t bdesc0 = p.b_kmajor ? make_smem_desc(smem_base + Cfg::kABytes, 16, 1024)
-                                         : make_smem_desc(smem_base + Cfg::kABytes, 8192, 1024);
+      const uint64_t bdesc0 = p.b_kmajor ? make_smem_desc(smem_base + kPrABytes, 16, 1024)
+                                         : make_smem_desc(smem_base + kPrABytes, 8192, 1024);
       const uint64_t bks = p.b_kmajor ? 2 : 128;          // (32 B | 2048 B) >> 4 per 16-deep k step
-      constexpr uint64_t kStep = Cfg::kStageBytes >> 4;
+      constexpr uint64_t kStep = kPrStageBytes >> 4;
       const uint32_t idesc = p.idesc;
       int stage = 0; uint32_t phase = 0; int buf = 0; uint32_t bphase = 1;
       for (int item = pair_id; item < items; item += num_pairs) {
-        const int ks = item % p.split_k;
-        const int n_kt = (k_tiles_total - ks + p.split_k - 1) / p.split_k;
         for (int i = 0; i < n_kt; ++i) {
-          const uint32_t d = tmem_base + (uint32_t)(buf * BN);
+          const uint32_t d = tmem_base + (uint32_t)(buf * 256);
           for (int h = 0; h < halves; ++h) {
-            bool ok1 = true;
-            if (h == 0) ok1 = mbar_wait_poll(tempty0 + 8u * buf, bphase, abort_flag);
-            const bool ok2 = mbar_wait_poll(full0 + 8u * stage, phase, abort_flag);
-            if (!__all_sync(0xffffffffu, ok1 && ok2)) goto issuer_done;
+            // the operands usually wait for the accumulator, so that is asked last
+            if (!__all_sync(0xffffffffu, mbar_wait_poll(full0 + 8u * stage, phase, abort_flag))) goto issuer_done;
+            if (h == 0 && !__all_sync(0xffffffffu, mbar_wait_poll(tempty0 + 8u * buf, bphase, abort_flag))) goto issuer_done;
             tc_fence_after();
             const uint64_t ad = adesc0 + (uint64_t)stage * kStep;
             const uint64_t bd = bdesc0 + (uint64_t)stage * kStep;
-            if (lane == 0) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) umma_f16_pair(d, ad + 2 * q, bd + q * bks, idesc, (h || q) ? 1u : 0u);
-              // in both CTAs: the stage may be refilled and, after the last stage of a K-tile,
-              // the accumulator may be read, once these MMAs are done
-              umma_commit_pair(done0 + 8u * stage);
-            }
-            __syncwarp();
-            if (++stage == STAGES) { stage = 0; phase ^= 1; }
+            for (int q = 0; q < 4; ++q) umma_f16_pair(d, ad + 2 * q, bd + q * bks, idesc, (h || q) ? 1u : 0u, e);
+            umma_commit_pair(empty0 + 8u * stage, e);
+            if (h == halves - 1) umma_commit_pair(tfull0 + 8u * buf, e);
+            if (++stage == kPrStages) { stage = 0; phase ^= 1; }
           }
-          if (++buf == NBUF) { buf = 0; bphase ^= 1; }
+          buf ^= 1; if (buf == 0) bphase ^= 1;
         }
       }
-    } else {
-      // follower: forward "my epilogue has drained the buffer" to the leader
-      const uint32_t tempty_leader0 = mapa_u32(tempty0, 0);
-      int buf = 0; uint32_t fphase = 0;
-      for (int item = pair_id; item < items; item += num_pairs) {
-        const int ks = item % p.split_k;
-        const int n_kt = (k_tiles_total - ks + p.split_k - 1) / p.split_k;
-        for (int i = 0; i < n_kt; ++i) {
-          if (!__all_sync(0xffffffffu, mbar_wait_poll(tempty0 + 8u * buf, fphase, abort_flag))) goto issuer_done;
-          if (lane == 0) mbar_arrive_cluster(tempty_leader0 + 8u * buf);
-          __syncwarp();
-          if (++buf == NBUF) { buf = 0; fphase ^= 1; }
-        }
-      }
+    issuer_done:;
     }
-  issuer_done:;
   } else {
     // ------------------------------ epilogue warps (both CTAs) --------------------
-    // Warp w owns tensor-memory lanes 32 * (w % 4) .. (one output row per thread) and kCols
-    // consecutive columns of this CTA's 128 x BN accumulator.
     const int quarter = warp & 3;
     const int cgroup = (warp - kPrFirstEpi) >> 2;
-    const int row_in_tile = quarter * 32 + lane;
-    const int col0 = cgroup * kCols;
-    const uint32_t lane_addr = ((uint32_t)(quarter * 32) << 16) + (uint32_t)col0;
+    const uint32_t lane_addr = ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cgroup * kPrCols);
     const float scale = p.scale;
-    uint64_t scale2, magic2;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(scale2) : "r"(__float_as_uint(scale)));
-    asm("mov.b64 %0, {%1, %1};" : "=l"(magic2) : "r"(kMagicBits));
-    auto release_buffer = [&](int b) {     // this warp has drained accumulator buffer b
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(tempty0 + 8u * b);
-    };
-    int buf = 0; uint32_t epi_phase = 0; bool ok = true;
-    int dstage = halves - 1; uint32_t dphase = 0;          // done-barrier of the K-tile's last stage
-    auto epi_sync = [&]() -> bool {   // bounded barrier over this CTA's epilogue warps
-      __syncwarp();
-      if (lane == 0) mbar_arrive(epi_bar);
-      const bool done = warp_wait(epi_bar, epi_phase, abort_flag, lane);
-      epi_phase ^= 1;
-      return done;
-    };
-
-    // Rare-path corrections (local memory, zeroed on first use): wrap-sum of the raw values
-    // the fast add contributed for out-of-range partials, and the exact int64 sum of what
-    // the reference conversion gives for them.
-    uint32_t corr_raw[kCols];
-    long long corr_q[kCols];
+    const uint32_t mbits = q_magic_bits(p.inv_scale);
+    const uint64_t magic2 = pack2(mbits, mbits);
+    const float screen_limit = q_screen_limit(p.inv_scale);
+    const uint32_t one = (uint32_t)zero + 1u;
+    const uint32_t tempty_leader = mapa_u32(tempty0, 0);
+    int buf = 0; uint32_t bphase = 0; bool ok = true;
+    // Rare-path corrections (local memory, zeroed on first use): wrap-sum of the raw values the fast
+    // add contributed for out-of-range partials, and the exact int64 sum of what the reference
+    // conversion gives for them.
+    uint32_t corr_raw[kPrCols];
+    long long corr_q[kPrCols];
     bool corr_used = false;
 
     for (int item = pair_id; item < items && ok; item += num_pairs) {
-      const int tile = item / p.split_k, ks = item % p.split_k;
-      int pm, pn; tile_coords(tile, pm, pn);
-      const int row = pm * 256 + (int)rank * kBM + row_in_tile;
-      const int ncol0 = pn * BN + col0;
-      const int n_kt = (k_tiles_total - ks + p.split_k - 1) / p.split_k;
-      uint32_t acc[kCols];
+      uint32_t acc[kPrCols];
 #pragma unroll
-      for (int i = 0; i < kCols; ++i) acc[i] = 0;
+      for (int i = 0; i < kPrCols; ++i) acc[i] = 0;
       corr_used = false;
-
       for (int kt = 0; kt < n_kt; ++kt) {
-        if (!warp_wait_poll(done0 + 8u * dstage, dphase, abort_flag, lane)) { ok = false; break; }
-        dstage += halves; if (dstage >= STAGES) { dstage -= STAGES; dphase ^= 1; }
+        if (!warp_wait_poll(tfull0 + 8u * buf, bphase, abort_flag, lane)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t taddr = tmem_base + lane_addr + (uint32_t)(buf * BN);
-        // r = fma(p, 2^f, MAGIC) two partials per instruction, raw bit patterns added as
-        // integers; the OR of the raw fp32 bits is the range screen (bit 30 clear: every
-        // |p| < 2, hence |p * 2^f| < 2^22 for f <= 21).  The next chunk's tcgen05.ld is in
-        // flight while the current one is converted.
-        uint32_t v[2][CH];
-        uint32_t screen = 0;
-        tmem_ldp(taddr, v[0]);
+        const uint32_t taddr = tmem_base + lane_addr + (uint32_t)(buf * 256);
+        float screen = 0.0f;
 #pragma unroll
-        for (int c = 0; c < NCH; ++c) {
-          uint32_t (&cur)[CH] = v[c & 1];
-          tmem_wait_ldp(cur);
-          if (c + 1 < NCH) tmem_ldp(taddr + (c + 1) * CH, v[(c + 1) & 1]);
+        for (int c = 0; c < kPrCols / 16; ++c) {
+          uint32_t v[16];
+          tmem_ld16(taddr + c * 16, v);
+          tmem_wait_ld_regs(v);
+          float tail = 0.0f;
+          if (c + 1 == kPrCols / 16) {
+            // the last chunk is in registers: screen it and hand the buffer back before converting it
 #pragma unroll
-          for (int i = 0; i < CH; i += 2) {
-            uint64_t a, r;
-            uint32_t r0, r1;
-            asm("mov.b64 %0, {%1, %2};" : "=l"(a) : "r"(cur[i]), "r"(cur[i + 1]));
-            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(scale2), "l"(magic2));
-            asm("mov.b64 {%0, %1}, %2;" : "=r"(r0), "=r"(r1) : "l"(r));
-            acc[c * CH + i] += r0;
-            acc[c * CH + i + 1] += r1;
-            screen |= cur[i] | cur[i + 1];
-          }
-          if (DUMP) {
-            if (row < p.M) {
-              const int ktg = ks + kt * p.split_k;
-              float* dst = p.partials + ((int64_t)ktg * p.M + row) * p.N + ncol0 + c * CH;
-#pragma unroll
-              for (int i = 0; i < CH; ++i)
-                if (ncol0 + c * CH + i < p.N) dst[i] = __uint_as_float(cur[i]);
-            }
-          }
-        }
-        if (__any_sync(0xffffffffu, (screen & 0x40000000u) != 0)) {
-          // exact fix-up of this K-tile (rare): see fixup_tile
-          if (!corr_used) {
+            for (int i = 0; i < 16; i += 2) screen = max3_abs(screen, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+            if (__any_sync(0xffffffffu, !(screen < screen_limit))) {
+              if (!corr_used) {
 #pragma unroll 1
-            for (int z = 0; z < kCols; ++z) { corr_raw[z + zero] = 0; corr_q[z + zero] = 0; }
-            corr_used = true;
+                for (int z = 0; z < kPrCols; ++z) { corr_raw[z + zero] = 0; corr_q[z + zero] = 0; }
+                corr_used = true;
+              }
+              fixup_tile(taddr, kPrCols, mbits, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(tempty_leader + 8u * buf);
           }
-          fixup_tile(taddr, kCols, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
+          convert16(v, &acc[c * 16], magic2, mbits, one, c + 1 == kPrCols / 16 ? tail : screen);
         }
-        release_buffer(buf);
-        if (++buf == NBUF) buf = 0;
+        buf ^= 1; if (buf == 0) bphase ^= 1;
       }
       if (!ok) break;
 
-      // every K-tile added MAGIC once
-      const uint32_t bias_bits = (uint32_t)n_kt * kMagicBits;
-      auto total = [&](int i) -> long long {
-        uint32_t raw = acc[i] - bias_bits;
-        long long t;
-        if (corr_used) {
-          // the in-range part is < 2^31 in magnitude, so it is the sign extension of the
-          // wrapped sum once the out-of-range raw values are taken out again
-          raw -= corr_raw[i + zero];
-          t = (long long)(int32_t)raw + corr_q[i + zero];
-        } else {
-          t = (long long)(int32_t)raw;
-        }
-        return p.int_bits == 64 ? t : (long long)(int32_t)t;
-      };
-
-      // Split-K: every split leaves its integer partial tile in its own plane of the scratch
-      // (column-major inside this CTA's 128 x BN tile, so every store and load is a full
-      // line); the split that arrives last adds the planes of the others to its registers.
-      // Integer addition is commutative and associative: which split comes last cannot
-      // change the sum.
-      const bool row_ok = row < p.M;
-      bool do_store = true;
-      const int cta_tile = tile * 2 + (int)rank;
-      const int64_t plane_elems = (int64_t)kBM * BN;
-      const int64_t plane_stride = (int64_t)tiles_mn * 2 * plane_elems;
-      const int64_t plane_off = (int64_t)cta_tile * plane_elems + (int64_t)col0 * kBM + row_in_tile;
-      if (p.split_k > 1) {
-        if (p.int_bits == 64) {
-          long long* dst = (long long*)p.acc_scratch + ks * plane_stride + plane_off;
+      int pm, pn; tile_coords(item, pm, pn);
+      const int row = pm * 256 + (int)rank * kBM + quarter * 32 + lane;
+      const int col0 = pn * 256 + cgroup * kPrCols;
+      const uint32_t bias_bits = (uint32_t)n_kt * mbits;   // what the multiply-adds summed on top
+      const T* bias = (const T*)p.bias;
+      // Fast output: with every sum below 2^22 in magnitude, MAGIC + sum is a float whose value minus
+      // MAGIC is the sum, so one fma gives sum * 2^-f exactly (what int -> float -> scale gives).
+      bool fast = !corr_used && !p.c_int && p.c_vec_ok == 2 && col0 + kPrCols <= p.N;
+      if (fast) {
+        uint32_t off = 0;
 #pragma unroll
-          for (int i = 0; i < kCols; ++i) __stcg(dst + i * kBM, total(i));
-        } else {
-          int* dst = (int*)p.acc_scratch + ks * plane_stride + plane_off;
-#pragma unroll
-          for (int i = 0; i < kCols; ++i) __stcg(dst + i * kBM, (int)total(i));
+        for (int i = 0; i < kPrCols; ++i) {
+          acc[i] += alu_add(i) ? kMagicBits : kMagicBits - bias_bits;
+          off |= acc[i] ^ kExpBits;
         }
-        __threadfence();
-        if (!epi_sync()) { ok = false; break; }
-        if (threadIdx.x == kPrFirstEpi * 32) *s_last = (atomicAdd(p.locks + cta_tile, 1) == p.split_k - 1) ? 1 : 0;
-        if (!epi_sync()) { ok = false; break; }
-        do_store = *s_last != 0;
-        if (do_store) __threadfence();
+        fast = !__any_sync(0xffffffffu, (off >> 23) != 0);
+        if (!fast) {
+#pragma unroll
+          for (int i = 0; i < kPrCols; ++i) acc[i] -= alu_add(i) ? kMagicBits : kMagicBits - bias_bits;
+        }
       }
-
-      if (do_store && row_ok) {
-        T* cdst = p.c ? (T*)p.c + (int64_t)row * p.c_sm + ncol0 : nullptr;
-        const T* bias = (const T*)p.bias;
+      if (fast) {
+        if (row < p.M) {
+          const float inv = p.inv_scale, minus = -__fmul_rn(__uint_as_float(kMagicBits), inv);
+          T* cdst = (T*)p.c + (int64_t)row * p.c_sm + col0;
 #pragma unroll
-        for (int g = 0; g < kCols / 8; ++g) {
+          for (int g = 0; g < kPrCols / 16; ++g) {
+            alignas(16) T out[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              float v = __fmaf_rn(__uint_as_float(acc[g * 16 + i]), inv, minus);
+              if (bias) v = __fadd_rn(v, to_f32<T>(bias[col0 + g * 16 + i]));
+              out[i] = from_f32<T>(v);
+            }
+            st_global_32(cdst + g * 16, *reinterpret_cast<const uint32_t(*)[8]>(out));
+          }
+        }
+      } else if (row < p.M) {
+        auto total = [&](int i) -> long long {
+          uint32_t raw = alu_add(i) ? acc[i] : acc[i] - bias_bits;
+          long long t;
+          if (corr_used) {
+            // the in-range part is < 2^31 in magnitude, so it is the sign extension of the wrapped
+            // sum once the out-of-range raw values are taken out again
+            raw -= corr_raw[i + zero];
+            t = (long long)(int32_t)raw + corr_q[i + zero];
+          } else {
+            t = (long long)(int32_t)raw;
+          }
+          return p.int_bits == 64 ? t : (long long)(int32_t)t;
+        };
+#pragma unroll
+        for (int g = 0; g < kPrCols / 8; ++g) {
+          const int colg = col0 + g * 8;
           long long q8[8];
-          const int colg = ncol0 + g * 8;
 #pragma unroll
           for (int i = 0; i < 8; ++i) q8[i] = total(g * 8 + i);
-          if (p.split_k > 1) {
-            for (int s2 = 0; s2 < p.split_k; ++s2) {
-              if (s2 == ks) continue;
-              if (p.int_bits == 64) {
-                const long long* src = (const long long*)p.acc_scratch + s2 * plane_stride + plane_off + (int64_t)g * 8 * kBM;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) q8[i] += __ldcg(src + i * kBM);
-              } else {
-                const int* src = (const int*)p.acc_scratch + s2 * plane_stride + plane_off + (int64_t)g * 8 * kBM;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) q8[i] += (long long)__ldcg(src + i * kBM);
-              }
-            }
-            if (p.int_bits != 64) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) q8[i] = (long long)(int32_t)q8[i];
-            }
-          }
           if (p.c_int) {
             if (p.int_bits == 64) {
               long long* dst = (long long*)p.c_int + (int64_t)row * p.N + colg;
@@ -475,26 +369,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
               for (int i = 0; i < 8; ++i) if (colg + i < p.N) dst[i] = (int32_t)q8[i];
             }
           }
-          if (cdst) {
+          if (p.c) {
+            T* cdst = (T*)p.c + (int64_t)row * p.c_sm + colg;
             alignas(16) T out[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              float v8 = fixed_to_float<long long>(q8[i], p.inv_scale);
-              if (bias && colg + i < p.N) v8 = __fadd_rn(v8, to_f32<T>(bias[colg + i]));
-              out[i] = from_f32<T>(v8);
+              float v = fixed_to_float<long long>(q8[i], p.inv_scale);
+              if (bias && colg + i < p.N) v = __fadd_rn(v, to_f32<T>(bias[colg + i]));
+              out[i] = from_f32<T>(v);
             }
             if (p.c_vec_ok && colg + 8 <= p.N) {
-              *reinterpret_cast<uint4*>(cdst + g * 8) = *reinterpret_cast<const uint4*>(out);
+              *reinterpret_cast<uint4*>(cdst) = *reinterpret_cast<const uint4*>(out);
             } else {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) if (colg + i < p.N) cdst[g * 8 + i] = out[i];
+              for (int i = 0; i < 8; ++i) if (colg + i < p.N) cdst[i] = out[i];
             }
           }
         }
-      }
-      if (p.split_k > 1) {
-        if (do_store && threadIdx.x == kPrFirstEpi * 32) p.locks[cta_tile] = 0;
-        if (!epi_sync()) { ok = false; break; }    // s_last is rewritten only after all have read it
       }
     }
   }
@@ -509,8 +400,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
     if (threadIdx.x == 0 && p.status) atomicExch(p.status, FXPR_ERR_TIMEOUT);
     __syncthreads();
   }
-  // Neither CTA may leave while the other can still signal its barriers or while MMAs that
-  // read its shared memory are in flight (the last tfull commit covers those).
+  // Neither CTA may leave while the other can still signal its barriers or while MMAs that read its
+  // shared memory are in flight (the last tfull commit, which the epilogues wait for, covers those).
   cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
@@ -520,32 +411,32 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
 
 bool gemm_tc_fast_supported(const GemmArgs& g, int split_k);
 
-// Same numeric conditions as gemm_tc_fast.cu; worth it once a pair tile has two real row blocks.
+// Numeric conditions of gemm_tc_fast.cu (int32 / int64 sums, frac_bits <= 21, at most 510 K-tiles);
+// no K-split and no dump of the partials.
 bool gemm_tc_pair_supported(const GemmArgs& g, int split_k) {
-  return g.M > 128 && g.N >= 128 && gemm_tc_fast_supported(g, split_k);
+  return split_k == 1 && g.partials == nullptr && g.M > 128 && g.N >= 128 && gemm_tc_fast_supported(g, split_k);
 }
 
-template <typename T, int BN, bool DUMP>
+template <typename T>
 static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, TcParams& p, int sms, cudaStream_t s) {
-  using Cfg = PairCfg<BN>;
-  auto k = gemm_tc_pair_kernel<T, BN, DUMP>;
+  auto k = gemm_tc_pair_kernel<T>;
   static bool attr_done_dev[64] = {};            // function attributes are per device
   int dev_id = 0;
   cudaGetDevice(&dev_id);
   bool& attr_done = attr_done_dev[dev_id & 63];
   if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
     if (e != cudaSuccess) { set_last_error("gemm_tc_pair smem attribute", e); return FXPR_ERR_CUDA; }
     attr_done = true;
   }
   p.tiles_m = (p.M + 255) / 256;
-  p.tiles_n = (p.N + BN - 1) / BN;
-  const int64_t items = (int64_t)p.tiles_m * p.tiles_n * p.split_k;
+  p.tiles_n = (p.N + 255) / 256;
+  const int64_t items = (int64_t)p.tiles_m * p.tiles_n;
   const int pairs = (int)(items < sms / 2 ? items : sms / 2);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
   cfg.blockDim = dim3(kPrThreads, 1, 1);
-  cfg.dynamicSmemBytes = Cfg::kSmem;
+  cfg.dynamicSmemBytes = kPrSmem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -557,24 +448,12 @@ static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, TcParams& p
 }
 
 // ma, mb: the tensor maps of gemm_tc() (A: 128-row boxes, B: 64-row boxes in either layout).
-int gemm_tc_pair(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb,
-                 int bn, cudaStream_t s) {
+int gemm_tc_pair(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb, cudaStream_t s) {
   const int sms = tc_device_sms();
   if (sms < 0) return FXPR_ERR_ARCH;
-  p.idesc = make_idesc(g.dtype == FXPR_BF16 ? 1 : 0, p.b_kmajor ? 0 : 1, bn, 256);
-  const bool dump = p.partials != nullptr;
-#define FXPR_PAIR(TT)                                                              \
-  do {                                                                             \
-    if (bn == 256) {                                                               \
-      if (dump) return launch_pair<TT, 256, true>(ma, mb, p, sms, s);              \
-      return launch_pair<TT, 256, false>(ma, mb, p, sms, s);                       \
-    }                                                                              \
-    if (dump) return launch_pair<TT, 128, true>(ma, mb, p, sms, s);                \
-    return launch_pair<TT, 128, false>(ma, mb, p, sms, s);                         \
-  } while (0)
-  if (g.dtype == FXPR_BF16) FXPR_PAIR(__nv_bfloat16);
-  FXPR_PAIR(__half);
-#undef FXPR_PAIR
+  p.idesc = make_idesc(g.dtype == FXPR_BF16 ? 1 : 0, p.b_kmajor ? 0 : 1, 256, 256);
+  if (g.dtype == FXPR_BF16) return launch_pair<__nv_bfloat16>(ma, mb, p, sms, s);
+  return launch_pair<__half>(ma, mb, p, sms, s);
 }
 
 }  // namespace fxpr

@@ -98,10 +98,10 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
 
   if (warp == 0) {
     // ------------------------------ TMA producer --------------------------------
+    const uint32_t e = elect_one();
     const bool wk = p.b_kmajor != 0;                     // weights given as an (N, K) row-major view
     // A stage is free again when the MMAs that read it are done, which is also when their
-    // accumulator group is full: the issuer signals both with ONE commit (a tcgen05.commit costs
-    // ~260 clocks of the issuing thread), so super-stage j waits for the group barrier of
+    // accumulator group is full: the issuer signals both with ONE commit, so super-stage j waits for the group barrier of
     // super-stage j - STAGES.
     int stage = 0; int wgrp = 0; uint32_t wphase = 0; int issued = 0;
     // boxes of super-stage ss of an item into shared-memory stage st: weights and/or activations
@@ -115,21 +115,18 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
       const uint32_t fb = full0 + 8u * st;
       const uint32_t sw = smem_base + st * kSkSSBytes;
       const uint32_t sx = sw + kSkWBytes;
-      if (lane == 0) {
-        if (arm) mbar_expect_tx(fb, two ? kSkSSBytes : kSkSSBytes / 2);
+      if (arm) mbar_expect_tx(fb, two ? kSkSSBytes : kSkSSBytes / 2, e);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if (h == 1 && !two) break;
-          const int kk = h ? kb : ka;
-          if (weights) {
+      for (int h = 0; h < 2; ++h) {
+        if (h == 1 && !two) break;
+        const int kk = h ? kb : ka;
+        if (weights) {
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-              tma_load_2d(sw + h * (kSkWBytes / 2) + j * 8192, &tma_w, fb, wk ? kk : n0 + j * 64, wk ? n0 + j * 64 : kk);
-          }
-          if (acts) tma_load_2d(sx + h * (kSkXBytes / 2), &tma_x, fb, kk, 0);
+          for (int j = 0; j < 2; ++j)
+            tma_load_2d(sw + h * (kSkWBytes / 2) + j * 8192, &tma_w, fb, wk ? kk : n0 + j * 64, wk ? n0 + j * 64 : kk, e);
         }
+        if (acts) tma_load_2d(sx + h * (kSkXBytes / 2), &tma_x, fb, kk, 0, e);
       }
-      __syncwarp();
     };
     auto n_ss_of = [&](int item) {
       const int ks = item % p.split_k;
@@ -171,7 +168,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
     const uint64_t wks = p.b_kmajor ? 2 : 128;           // (32 B | 2048 B) >> 4 per 16-deep k step
     constexpr uint64_t kStep = kSkSSBytes >> 4;
     constexpr uint64_t kHalfW = (kSkWBytes / 2) >> 4, kHalfX = (kSkXBytes / 2) >> 4;
-    const uint32_t idesc = p.idesc;
+    const uint32_t idesc = p.idesc, e = elect_one();
     int stage = 0; uint32_t phase = 0; int grp = 0; uint32_t gphase = 1;
     for (int item = first_item; item < items; item += item_step) {
       const int ks = item % p.split_k;
@@ -189,17 +186,14 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
         const uint32_t d1 = pairs ? d0 + MP : d0;
         const uint64_t wd = wdesc0 + (uint64_t)stage * kStep;
         const uint64_t xd = xdesc0 + (uint64_t)stage * kStep;
-        if (lane == 0) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) umma_f16(d0, wd + i * wks, xd + i * 2, idesc, i ? 1u : 0u);
-          if (two) {
+        for (int i = 0; i < 4; ++i) umma_f16(d0, wd + i * wks, xd + i * 2, idesc, i ? 1u : 0u, e);
+        if (two) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-              umma_f16(d1, wd + kHalfW + i * wks, xd + kHalfX + i * 2, idesc, (i || !pairs) ? 1u : 0u);
-          }
-          umma_commit(tfull0 + 8u * grp);              // stage consumed AND accumulator group full
+          for (int i = 0; i < 4; ++i)
+            umma_f16(d1, wd + kHalfW + i * wks, xd + kHalfX + i * 2, idesc, (i || !pairs) ? 1u : 0u, e);
         }
-        __syncwarp();
+        umma_commit(tfull0 + 8u * grp, e);             // stage consumed AND accumulator group full
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
         if (++grp == ngroup) { grp = 0; gphase ^= 1; }
       }

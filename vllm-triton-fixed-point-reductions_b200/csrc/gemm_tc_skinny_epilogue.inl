@@ -7,7 +7,9 @@
   const int n_in_tile = quarter * 32 + lane;
   const int m0 = cgroup * kCols;
   const uint32_t lane_addr = ((uint32_t)(quarter * 32) << 16) + (uint32_t)m0;
-  const float magic = __uint_as_float(kMagicBits);
+  const uint32_t mbits = q_magic_bits(p.inv_scale), one = (uint32_t)zero + 1u;
+  const uint64_t magic2 = pack2(mbits, mbits);
+  const float screen_limit = q_screen_limit(p.inv_scale);
   const float scale = p.scale;
   int grp = 0; uint32_t gphase = 0; uint32_t epi_phase = 0; bool ok = true;
   auto epi_sync = [&]() -> bool {   // bounded barrier over the epilogue warps only
@@ -41,14 +43,9 @@
       const uint32_t ta0 = tmem_base + lane_addr + (uint32_t)grp * group_cols;
       const uint32_t ta1 = ta0 + MP;
       uint32_t va[16], vb[16];
-      uint32_t screen0 = 0, screen1 = 0;
-      auto convert = [&](const uint32_t (&v)[16], int c, uint32_t& screen) {
-#pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          acc[c * 16 + i] += __float_as_uint(__fmaf_rn(__uint_as_float(v[i]), scale, magic));
-          acc[c * 16 + i + 1] += __float_as_uint(__fmaf_rn(__uint_as_float(v[i + 1]), scale, magic));
-          screen |= v[i] | v[i + 1];
-        }
+      float screen0 = 0.0f, screen1 = 0.0f;
+      auto convert = [&](const uint32_t (&v)[16], int c, float& screen) {
+        convert16(v, &acc[c * 16], magic2, mbits, one, screen);
       };
       // both halves of a buffer are requested before the one wait
       tmem_ld16(ta0, va); tmem_ld16(ta0 + 16, vb); tmem_wait_ld_regs2(va, vb);
@@ -57,16 +54,16 @@
         tmem_ld16(ta1, va); tmem_ld16(ta1 + 16, vb); tmem_wait_ld_regs2(va, vb);
         convert(va, 0, screen1); convert(vb, 1, screen1);
       }
-      if (__any_sync(0xffffffffu, ((screen0 | screen1) & 0x40000000u) != 0)) {
+      if (__any_sync(0xffffffffu, !(screen0 < screen_limit && screen1 < screen_limit))) {
         if (!corr_used) {
 #pragma unroll 1
           for (int z = 0; z < kCols; ++z) { corr_raw[z + zero] = 0; corr_q[z + zero] = 0; }
           corr_used = true;
         }
-        if (__any_sync(0xffffffffu, (screen0 & 0x40000000u) != 0))
-          fixup_tile(ta0, kCols, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
-        if (__any_sync(0xffffffffu, (screen1 & 0x40000000u) != 0))
-          fixup_tile(ta1, kCols, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
+        if (__any_sync(0xffffffffu, !(screen0 < screen_limit)))
+          fixup_tile(ta0, kCols, mbits, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
+        if (__any_sync(0xffffffffu, !(screen1 < screen_limit)))
+          fixup_tile(ta1, kCols, mbits, scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
       }
       tc_fence_before();
       __syncwarp();
@@ -75,9 +72,9 @@
     }
     if (!ok) break;
 
-    const uint32_t bias_bits = (uint32_t)n_kt * kMagicBits;   // every K-tile added MAGIC once
+    const uint32_t bias_bits = (uint32_t)n_kt * mbits;   // the multiply-adds summed one magic per K-tile
     auto total = [&](int i) -> long long {
-      uint32_t raw = acc[i] - bias_bits;
+      uint32_t raw = alu_add(i) ? acc[i] : acc[i] - bias_bits;
       long long t;
       if (corr_used) {
         raw -= corr_raw[i + zero];
