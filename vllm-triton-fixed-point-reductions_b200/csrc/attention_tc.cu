@@ -47,7 +47,8 @@ static constexpr int kTcRows = 128;            // query rows per CTA = tensor-me
 static constexpr int kTcColGroups = 4;         // softmax threads per row: each owns 64/4 keys and HD/4 output columns
 static constexpr int kTcSoftWarps = 4 * kTcColGroups;
 static constexpr int kTcFirstSoft = 2;         // warp 0: TMA producer, warp 1: MMA issuer
-static constexpr int kTcThreads = (kTcFirstSoft + kTcSoftWarps) * 32;
+static constexpr int kTcProducer2 = kTcFirstSoft + kTcSoftWarps;   // the second producer warp
+static constexpr int kTcThreads = (kTcProducer2 + 1) * 32;
 static constexpr int kTcStages = 4;
 
 struct TcAttnShape {
@@ -57,7 +58,7 @@ struct TcAttnShape {
   int page_size;
   int group_shift;         // log2 of the keys per TMA box: 6 when pages are multiples of 64 tokens, else 4
   int page_mask;           // page_size - 1 when the page size is a power of two, else 0
-  uint32_t idesc_s, idesc_pv;
+  uint32_t idesc_s, idesc_s2, idesc_pv;    // S of 64 keys, S of 128 keys, P.V
 };
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z,
@@ -86,6 +87,11 @@ __device__ __forceinline__ float ex2_approx_tc(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 template <typename T> __device__ __forceinline__ uint32_t pack2_tc(float lo, float hi);
 template <> __device__ __forceinline__ uint32_t pack2_tc<__nv_bfloat16>(float lo, float hi) {
@@ -129,8 +135,8 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   constexpr int CG = kTcColGroups;
   constexpr int KT = kTcTileN / CG;                        // keys per softmax thread and tile
   constexpr int kHalfCols = HD / CG;                       // P.V columns per thread
-  static_assert(KT == 16 && kHalfCols == 32, "one 16-column and one 32-column tensor-memory load per tile");
-  constexpr uint32_t kColS = 0, kColPV = 128;              // tensor-memory columns: S[2] x 64, PV[2] x 128
+  static_assert(KT == 16 && kHalfCols == 32, "columns per thread");
+  constexpr uint32_t kColS = 0, kColPV = 256;              // tensor-memory columns: S[2] x 128, PV[2] x 128
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -189,7 +195,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   if (threadIdx.x == 0) {
     mbar_init(qfull, 1);
     mbar_init(qfree, 1);
-    for (int s = 0; s < kTcStages; ++s) { mbar_init(full0 + 8u * s, 1); mbar_init(empty0 + 8u * s, 1); }
+    for (int s = 0; s < kTcStages; ++s) { mbar_init(full0 + 8u * s, 2); mbar_init(empty0 + 8u * s, 1); }
     for (int b = 0; b < 2; ++b) {
       mbar_init(sfull0 + 8u * b, 1); mbar_init(sfree0 + 8u * b, kTcSoftWarps);
       mbar_init(pready0 + 8u * b, kTcSoftWarps);
@@ -208,93 +214,103 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    // ------------------------------ K / V producer (TMA) ------------------------------
+  if (warp == 0 || warp == kTcProducer2) {
+    // ------------------------------ K / V producers (TMA) -----------------------------
     // One box per 16-token page piece and half head (2 KB), 48 KB per 128 x 64 tile over the two
-    // passes.  The boxes are predicated instructions of a uniform warp (see tc_common.cuh): issued
-    // from a divergent branch, one lane or sixteen, each box cost the warp 80-140 clocks.
-    // Nothing is copied, and the block table is not read, past the end of the
-    // sequence; V rows there are cleared by the MMA warp before P.V.
+    // passes, issued as predicated instructions of a uniform warp (tc_common.cuh); a box still takes
+    // its warp ~80 clocks, so two warps share them: by page piece, or by half head when a box holds a
+    // whole 64-key tile.  A stage is 32 KB: 128 keys of K in pass A (two 64-dim slabs of 128 rows), 64
+    // keys of K and V in pass B.  Nothing is copied, and the block table is not read, past the end of
+    // the sequence; V rows there are cleared by the MMA warp before P.V.
     const uint32_t e = elect_one();
+    const int me = warp == 0 ? 0 : 1;
     int stage = 0; uint32_t phase = 1;
     uint32_t q_phase = 1;                                    // qfree: the first wait passes
-    // Block-table entries are read 32 at a time (lane L: the 16-key group L of an 8-tile
-    // block), one block ahead of their use, and handed round by shuffle.
+    // Block-table entries are read 32 at a time (lane L: the 16-key group L of an 8-tile block), one
+    // block ahead of their use, and handed round by shuffle.
     int page_shift = -1;
     for (int b = 4; b < 31; ++b) if ((1 << b) == sh.page_size) page_shift = b;
+    const int gs = sh.group_shift;                           // log2 of the keys per box: 4 or 6
     for (int w = blockIdx.x; w < total_items; w += gridDim.x) {
-    const Item I = decode_item(w);
-    if (!I.live) continue;
-    const int kvh = I.kvh, seq_len = I.seq_len, t0 = I.t0, t1 = I.t1;
-    const int32_t* bt = p.block_table + (int64_t)I.req * p.bt_stride;
-    // Q rows: box {64 dims, G heads, 128 / G tokens} -> row = token * G + head.  Tokens past
-    // this request's (they belong to the next one, or lie beyond the tensor: zeros) are rows
-    // whose every key is masked and that are never stored.  The buffer is free once the MMA
-    // warp's last score MMA of the previous item has completed.
-    if (!__all_sync(0xffffffffu, mbar_wait(qfree, q_phase, abort_flag))) goto producer_done;
-    q_phase ^= 1;
-    mbar_expect_tx(qfull, kQBytes, e);
-    tma_load_3d(q_s, &map_q, qfull, 0, kvh * G, I.q_start + I.tok0, e);
-    tma_load_3d(q_s + kQBytes / 2, &map_q, qfull, 64, kvh * G, I.q_start + I.tok0, e);
-    auto load_entries = [&](int tb) -> int {
-      const int n = tb * kTcTileN + lane * 16;
-      return (tb < t1 && n < seq_len) ? bt[page_shift >= 0 ? (n >> page_shift) : (n / sh.page_size)] : 0;
-    };
-    for (int pass = 0; pass < 2; ++pass) {
-      int cur = load_entries(t0);
-      for (int tb = t0; tb < t1; tb += 8) {
-        const int nxt = load_entries(tb + 8);
-        for (int tt = 0; tt < 8 && tb + tt < t1; ++tt) {
-          const int t = tb + tt;
-          if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8u * stage, phase, abort_flag))) goto producer_done;
-          const uint32_t fb = full0 + 8u * stage;
-          const uint32_t ks = stage0 + stage * kStageBytes;
-          // boxes hold group_keys keys (16, or the whole tile when pages are multiples of 64
-          // tokens); only groups that start inside the sequence are copied
-          // (shifts and masks only: this single warp's loop latency is on the critical path)
-          const int gs = sh.group_shift, gk = 1 << gs;
-          int groups = (seq_len - t * kTcTileN + gk - 1) >> gs;
-          groups = min(groups, kTcTileN >> gs);
-          mbar_expect_tx(fb, (uint32_t)((groups << (gs + 8)) << pass), e);
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            if (g >= groups) break;
-            const int blk = __shfl_sync(0xffffffffu, cur, tt * 4 + g);
-            const int n = t * kTcTileN + (g << gs);
-            const int slot = sh.page_mask ? (n & sh.page_mask) : (n % sh.page_size);
-            const uint32_t dst = ks + (uint32_t)(g << (gs + 7));
-            tma_load_4d(dst, &map_k, fb, 0, kvh, slot, blk, e);
-            tma_load_4d(dst + 8192, &map_k, fb, 64, kvh, slot, blk, e);
-            if (pass) {
-              tma_load_4d(dst + kKBytes, &map_v, fb, 0, kvh, slot, blk, e);
-              tma_load_4d(dst + kKBytes + 8192, &map_v, fb, 64, kvh, slot, blk, e);
-            }
-          }
-          if (++stage == kTcStages) { stage = 0; phase ^= 1; }
-        }
-        cur = nxt;
+      const Item I = decode_item(w);
+      if (!I.live) continue;
+      const int kvh = I.kvh, seq_len = I.seq_len, t0 = I.t0, t1 = I.t1;
+      const int32_t* bt = p.block_table + (int64_t)I.req * p.bt_stride;
+      // Q rows: box {64 dims, G heads, 128 / G tokens} -> row = token * G + head.  Tokens past this
+      // request's (they belong to the next one, or lie beyond the tensor: zeros) are rows whose every
+      // key is masked and that are never stored.  The buffer is free once the MMA warp's last score
+      // MMA of the previous item has completed.
+      if (me == 0) {
+        if (!__all_sync(0xffffffffu, mbar_wait(qfree, q_phase, abort_flag))) goto producer_done;
+        q_phase ^= 1;
+        mbar_expect_tx(qfull, kQBytes, e);
+        tma_load_3d(q_s, &map_q, qfull, 0, kvh * G, I.q_start + I.tok0, e);
+        tma_load_3d(q_s + kQBytes / 2, &map_q, qfull, 64, kvh * G, I.q_start + I.tok0, e);
       }
-    }
+      auto load_entries = [&](int tb) -> int {
+        const int n = tb * kTcTileN + lane * 16;
+        return (tb < t1 && n < seq_len) ? bt[page_shift >= 0 ? (n >> page_shift) : (n / sh.page_size)] : 0;
+      };
+      for (int pass = 0; pass < 2; ++pass) {
+        const int step = pass ? 1 : 2;                       // tiles per stage
+        const uint32_t half_bytes = pass ? 8192u : 16384u;   // between the two 64-dim slabs
+        int cur = load_entries(t0);
+        for (int tb = t0; tb < t1; tb += 8) {
+          const int nxt = load_entries(tb + 8);
+          for (int tt = 0; tt < 8 && tb + tt < t1; tt += step) {
+            const int t = tb + tt;
+            if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8u * stage, phase, abort_flag))) goto producer_done;
+            const uint32_t fb = full0 + 8u * stage;
+            const uint32_t ks = stage0 + stage * kStageBytes;
+            // only groups that start inside the sequence are copied
+            const int left = (min(seq_len, t1 * kTcTileN) - t * kTcTileN + (1 << gs) - 1) >> gs;
+            const int groups = min(left, (step * kTcTileN) >> gs);
+            const int first = gs == 4 ? me : 0, stride = gs == 4 ? 2 : 1;
+            const int mine = gs == 4 ? (groups - me + 1) >> 1 : groups;      // my page pieces
+            const int boxes = (gs == 4 ? 2 * mine : mine) << pass;           // of 2^(gs + 7) bytes each
+            mbar_expect_tx(fb, (uint32_t)boxes << (gs + 7), e);
+            for (int g = first; g < groups; g += stride) {
+              const int n = t * kTcTileN + (g << gs);
+              const int blk = __shfl_sync(0xffffffffu, cur, tt * 4 + (g << (gs - 4)));
+              const int slot = sh.page_mask ? (n & sh.page_mask) : (n % sh.page_size);
+              const uint32_t dst = ks + (uint32_t)(g << (gs + 7));
+              if (gs == 4) {
+                tma_load_4d(dst, &map_k, fb, 0, kvh, slot, blk, e);
+                tma_load_4d(dst + half_bytes, &map_k, fb, 64, kvh, slot, blk, e);
+                if (pass) {
+                  tma_load_4d(dst + kKBytes, &map_v, fb, 0, kvh, slot, blk, e);
+                  tma_load_4d(dst + kKBytes + 8192, &map_v, fb, 64, kvh, slot, blk, e);
+                }
+              } else {
+                tma_load_4d(dst + me * half_bytes, &map_k, fb, me * 64, kvh, slot, blk, e);
+                if (pass) tma_load_4d(dst + kKBytes + me * 8192, &map_v, fb, me * 64, kvh, slot, blk, e);
+              }
+            }
+            if (++stage == kTcStages) { stage = 0; phase ^= 1; }
+          }
+          cur = nxt;
+        }
+      }
     }
   producer_done:;
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------------------
-    // S_t = Q . K_t^T: both operands K-major (head dim contiguous), two 64-dim slabs
+    // S = Q . K^T: both operands K-major (head dim contiguous), two 64-dim slabs
     const uint32_t e = elect_one();
-    auto issue_s = [&](int stage, int sbuf) {
-      const uint32_t d = tmem_base + kColS + (uint32_t)(sbuf * 64);
+    auto issue_s = [&](int stage, int sbuf, uint32_t idesc, uint32_t slab_bytes) {
+      const uint32_t d = tmem_base + kColS + (uint32_t)(sbuf * 128);
       const uint64_t qd = make_smem_desc(q_s, 16, 1024);
       const uint64_t kd = make_smem_desc(stage0 + stage * kStageBytes, 16, 1024);
 #pragma unroll
       for (int kk = 0; kk < HD / 16; ++kk) {
         const uint64_t ao = (uint64_t)((kk >> 2) * (kQBytes / 2) + (kk & 3) * 32) >> 4;
-        const uint64_t bo = (uint64_t)((kk >> 2) * (kKBytes / 2) + (kk & 3) * 32) >> 4;
-        umma_f16(d, qd + ao, kd + bo, sh.idesc_s, kk ? 1u : 0u, e);
+        const uint64_t bo = (uint64_t)((kk >> 2) * slab_bytes + (kk & 3) * 32) >> 4;
+        umma_f16(d, qd + ao, kd + bo, idesc, kk ? 1u : 0u, e);
       }
       umma_commit(sfull0 + 8u * sbuf, e);
     };
     int stage = 0; uint32_t phase = 0;
-    int it = 0;                                              // S tiles issued so far (all items, both passes)
+    int it = 0;                                              // S products issued so far (all items, both passes)
     int jg = 0;                                              // P.V tiles issued so far (all items)
     uint32_t q_phase = 0;
     for (int w = blockIdx.x; w < total_items; w += gridDim.x) {
@@ -305,14 +321,14 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (!__all_sync(0xffffffffu, okq)) goto issuer_done;
     q_phase ^= 1;
     {
-      // pass A: scores only
-      for (int t = t0; t < t1; ++t, ++it) {
+      // pass A: scores only, 128 keys at a time
+      for (int t = t0; t < t1; t += 2, ++it) {
         const int sb = it & 1; const uint32_t sph = ((it >> 1) & 1) ^ 1;
         const bool a = mbar_wait(full0 + 8u * stage, phase, abort_flag);
         const bool b = mbar_wait(sfree0 + 8u * sb, sph, abort_flag);
         if (!__all_sync(0xffffffffu, a && b)) goto issuer_done;
         tc_fence_after();
-        issue_s(stage, sb);
+        issue_s(stage, sb, sh.idesc_s2, 16384u);
         umma_commit(empty0 + 8u * stage, e);
         if (++stage == kTcStages) { stage = 0; phase ^= 1; }
       }
@@ -324,7 +340,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const bool b = mbar_wait(sfree0 + 8u * sb, sph, abort_flag);
         if (!__all_sync(0xffffffffu, a && b)) return false;
         tc_fence_after();
-        issue_s(s_stage, sb);
+        issue_s(s_stage, sb, sh.idesc_s, 8192u);
         ++it;
         if (++s_stage == kTcStages) { s_stage = 0; s_phase ^= 1; }
         return true;
@@ -371,7 +387,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     }
   issuer_done:;
-  } else if (warp >= kTcFirstSoft) {
+  } else if (warp < kTcProducer2) {
     // ------------------------------ softmax / conversion warps ------------------------
     const int quarter = warp & 3;
     const int half = (warp - kTcFirstSoft) >> 2;                        // which quarter of the columns
@@ -379,7 +395,9 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
     const float ninf = -__int_as_float(0x7f800000);
     const bool plain_scores = !(p.cap_log2 > 0.0f) && p.alibi == nullptr;
-    const float magic = __uint_as_float(kMagicBits);
+    const bool raw_max = plain_scores && p.ss_log2 > 0.0f;
+    const uint64_t zero2 = pack2((uint32_t)zero, (uint32_t)zero);
+    const uint64_t ss2 = pack2(__float_as_uint(p.ss_log2), __float_as_uint(p.ss_log2));
     const uint32_t mbits = q_magic_bits(p.inv_scale), one = (uint32_t)zero + 1u;
     const uint64_t magic2 = pack2(mbits, mbits);
     const float screen_limit = q_screen_limit(p.inv_scale);
@@ -405,45 +423,56 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const int kend = valid ? (p.causal ? min(seq_len, pos + 1) : seq_len) : 0;
     const int kbeg = valid ? (p.window > 0 ? max(0, pos - p.window + 1) : 0) : 0;
     const float slope = (p.alibi && valid) ? p.alibi[head] : 0.0f;
-    // scores of this thread's 32 keys of tile t, in log2 space, masked (attention.py:103-121, 249-254)
-    auto load_scores = [&](int it, int t, float (&s)[KT]) -> bool {
-      const int sb = it & 1; const uint32_t sph = (it >> 1) & 1;
-      if (!warp_wait_relaxed(sfull0 + 8u * sb, sph, abort_flag, lane)) return false;
-      tc_fence_after();
-      uint32_t v[KT];
-      tmem_ld16(tmem_base + lane_sel + kColS + (uint32_t)(sb * 64 + half * KT), v);
-      tmem_wait_ld();
+    // one score in log2 space with soft-cap and ALiBi (attention.py:103-121, 249-254)
+    auto score = [&](uint32_t v, int n) -> float {
+      float x = __fmul_rn(__uint_as_float(v), p.ss_log2);
+      if (p.cap_log2 > 0.0f) x = __fmul_rn(p.cap_log2, tanhf(__fdiv_rn(x, p.cap_log2)));
+      if (p.alibi) x = __fadd_rn(x, __fmul_rn(slope, __fsub_rn((float)n, (float)pos)));
+      return x;
+    };
+    // hand S buffer sb back to the MMA warp (this warp's share is in registers)
+    auto release_s = [&](int sb) {
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(sfree0 + 8u * sb);          // the buffer may take the tile after next
-      const int n0 = t * kTcTileN + half * KT;
-      if (plain_scores && n0 >= kbeg && n0 + KT <= kend) {
-#pragma unroll
-        for (int i = 0; i < KT; ++i) s[i] = __fmul_rn(__uint_as_float(v[i]), p.ss_log2);
-      } else {
-#pragma unroll
-        for (int i = 0; i < KT; ++i) {
-          const int n = n0 + i;
-          float x = __fmul_rn(__uint_as_float(v[i]), p.ss_log2);
-          if (p.cap_log2 > 0.0f) x = __fmul_rn(p.cap_log2, tanhf(__fdiv_rn(x, p.cap_log2)));
-          if (p.alibi) x = __fadd_rn(x, __fmul_rn(slope, __fsub_rn((float)n, (float)pos)));
-          s[i] = (n >= kbeg && n < kend) ? x : ninf;
-        }
-      }
-      return true;
+      if (lane == 0) mbar_arrive(sfree0 + 8u * sb);
     };
 
     // =============================== pass A: row maxima ===============================
+    // 128 keys per step, 32 per thread.  Scaling by a positive constant is monotonic after rounding
+    // too, so the maximum is taken over the raw products and scaled once.
     float rmax = ninf;
-    for (int t = t0; t < t1 && ok; ++t, ++it) {
-      float s[KT];
-      if (!load_scores(it, t, s)) { ok = false; break; }
-      // max is exact and order-free: a tree keeps the dependency chain short
+    for (int t = t0; t < t1 && ok; t += 2, ++it) {
+      const int sb = it & 1;
+      if (!warp_wait_relaxed(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag, lane)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t v[2 * KT];
+      tmem_ld32(tmem_base + lane_sel + kColS + (uint32_t)(sb * 128 + half * 2 * KT), v);
+      tmem_wait_ld_regs(v);
+      release_s(sb);
+      const int n0 = t * kTcTileN + half * 2 * KT;
+      const bool inside = n0 >= kbeg && n0 + 2 * KT <= kend;
+      float m = ninf;
+      if (raw_max) {
+        if (inside) {
+          float m1 = ninf;                                   // two chains
 #pragma unroll
-      for (int w = KT / 2; w > 0; w >>= 1)
+          for (int i = 0; i < 2 * KT; i += 4) {
+            m = max3(m, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+            m1 = max3(m1, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
+          }
+          m = fmaxf(m, m1);
+        } else {
 #pragma unroll
-        for (int i = 0; i < w; ++i) s[i] = fmaxf(s[i], s[i + w]);
-      rmax = fmaxf(rmax, s[0]);
+          for (int i = 0; i < 2 * KT; ++i)
+            if (n0 + i >= kbeg && n0 + i < kend) m = fmaxf(m, __uint_as_float(v[i]));
+        }
+        m = __fmul_rn(m, p.ss_log2);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 2 * KT; ++i)
+          if (n0 + i >= kbeg && n0 + i < kend) m = fmaxf(m, score(v[i], n0 + i));
+      }
+      rmax = fmaxf(rmax, m);
     }
     rmax_s[half * kTcRows + row] = rmax;
     if (ok && !soft_sync()) ok = false;
@@ -453,7 +482,8 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (gmax == ninf) gmax = 0.0f;                           // rows without keys: exp2 gives 0, not NaN
 
     // =============================== pass B ===========================================
-    uint32_t den32 = 0, den32b = 0;                         // two chains: integer adds commute
+    uint32_t den32 = 0;
+    const uint64_t neg_max2 = pack2(__float_as_uint(-gmax), __float_as_uint(-gmax));
     uint32_t acc[kHalfCols];
 #pragma unroll
     for (int i = 0; i < kHalfCols; ++i) acc[i] = 0;
@@ -492,8 +522,35 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
     for (int j = 0; j < n_tiles && ok; ++j, ++it) {
       const int t = t0 + j;
-      float s[KT];
-      if (!load_scores(it, t, s)) { ok = false; break; }
+      const int sb = it & 1;
+      if (!warp_wait_relaxed(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag, lane)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t v[KT];
+      tmem_ld16(tmem_base + lane_sel + kColS + (uint32_t)(sb * 128 + half * KT), v);
+      tmem_wait_ld_regs(v);
+      release_s(sb);
+      // d = score - max, rounded twice; the product is an fma with a run-time zero because the
+      // assembler contracts a packed multiply and the packed add behind it into one rounding.
+      // The weight of a masked key is exp2(-inf) = 0.
+      const int n0 = t * kTcTileN + half * KT;
+      const bool inside = n0 >= kbeg && n0 + KT <= kend;
+      if (plain_scores) {
+#pragma unroll
+        for (int i = 0; i < KT; i += 2) {
+          uint64_t x;
+          asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x) : "l"(pack2(v[i], v[i + 1])), "l"(ss2), "l"(zero2));
+          asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(neg_max2));
+          asm("mov.b64 {%0, %1}, %2;" : "=r"(v[i]), "=r"(v[i + 1]) : "l"(x));
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < KT; ++i) v[i] = __float_as_uint(__fsub_rn(score(v[i], n0 + i), gmax));
+      }
+      if (!inside) {
+#pragma unroll
+        for (int i = 0; i < KT; ++i)
+          if (n0 + i < kbeg || n0 + i >= kend) v[i] = __float_as_uint(ninf);
+      }
       // weights, integer denominator, P in the io dtype -> shared memory (A operand of P.V):
       // row = 128 bytes of 64 keys, 16-byte chunks XOR-swizzled with the row number
       const int b = (jg + j) & 1;
@@ -503,11 +560,11 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         uint32_t pk[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float s0 = s[c * 8 + e * 2], s1 = s[c * 8 + e * 2 + 1];
-          const float w0 = (s0 == ninf) ? 0.0f : ex2_approx_tc(__fsub_rn(s0, gmax));
-          const float w1 = (s1 == ninf) ? 0.0f : ex2_approx_tc(__fsub_rn(s1, gmax));
-          den32 += __float_as_uint(__fmaf_rn(w0, p.scale, magic));
-          den32b += __float_as_uint(__fmaf_rn(w1, p.scale, magic));
+          const float w0 = ex2_approx_tc(__uint_as_float(v[c * 8 + e * 2]));
+          const float w1 = ex2_approx_tc(__uint_as_float(v[c * 8 + e * 2 + 1]));
+          uint64_t q;
+          asm("add.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(pack2(__float_as_uint(w0), __float_as_uint(w1))), "l"(magic2));
+          den32 = den32 + (uint32_t)q + (uint32_t)(q >> 32);
           pk[e] = pack2_tc<T>(w0, w1);
         }
         const uint32_t chunk = (uint32_t)(half * (KT / 8) + c);
@@ -524,7 +581,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
     // =============================== output ===========================================
     // KT weights per tile went through the fast add in this thread
-    const long long den_half = (long long)(int32_t)(den32 + den32b - (uint32_t)KT * (uint32_t)n_tiles * kMagicBits);
+    const long long den_half = (long long)(int32_t)(den32 - (uint32_t)KT * (uint32_t)n_tiles * mbits);
     den_s[half * kTcRows + row] = den_half;
     if (ok && !soft_sync()) ok = false;
     if (ok && valid) {
@@ -629,6 +686,7 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
   sh.page_mask = (p.page_size & (p.page_size - 1)) == 0 ? p.page_size - 1 : 0;
   const int fmt = dtype == FXPR_BF16 ? 1 : 0;
   sh.idesc_s = make_idesc(fmt, 0, kTcTileN, kTcRows);
+  sh.idesc_s2 = make_idesc(fmt, 0, 2 * kTcTileN, kTcRows);
   sh.idesc_pv = make_idesc(fmt, 1, p.head_dim, kTcRows);
   if ((int64_t)sh.num_q_blocks * p.num_kv_heads > 0x7fffffffLL) return FXPR_ERR_UNSUPPORTED;
 
