@@ -44,10 +44,12 @@ namespace fxpr {
 
 static constexpr int kTcTileN = 64;            // keys per tile (attention.py:32-36)
 static constexpr int kTcRows = 128;            // query rows per CTA = tensor-memory lanes
-static constexpr int kTcColGroups = 4;         // softmax threads per row: each owns 64/4 keys and HD/4 output columns
-static constexpr int kTcSoftWarps = 4 * kTcColGroups;
+static constexpr int kTcGroupWarps = 4;        // softmax group: thread = one row, all keys of every other tile
+static constexpr int kTcSoftWarps = 2 * kTcGroupWarps;
+static constexpr int kTcConvWarps = 8;         // conversion: thread = one row and half of the output columns
 static constexpr int kTcFirstSoft = 2;         // warp 0: TMA producer, warp 1: MMA issuer
-static constexpr int kTcProducer2 = kTcFirstSoft + kTcSoftWarps;   // the second producer warp
+static constexpr int kTcFirstConv = kTcFirstSoft + kTcSoftWarps;
+static constexpr int kTcProducer2 = kTcFirstConv + kTcConvWarps;   // the second producer warp
 static constexpr int kTcThreads = (kTcProducer2 + 1) * 32;
 static constexpr int kTcStages = 4;
 
@@ -58,6 +60,7 @@ struct TcAttnShape {
   int page_size;
   int group_shift;         // log2 of the keys per TMA box: 6 when pages are multiples of 64 tokens, else 4
   int page_mask;           // page_size - 1 when the page size is a power of two, else 0
+  int head_chunks;         // 64-element chunks from one KV head to the next
   uint32_t idesc_s, idesc_s2, idesc_pv;    // S of 64 keys, S of 128 keys, P.V
 };
 
@@ -70,14 +73,14 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       "[%0], [%1, {%3, %4, %5}], [%2];\n\t}"
       ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(elected) : "memory");
 }
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z,
-                                            int w, uint32_t elected) {
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z,
+                                            int w, int v, uint32_t elected) {
   asm volatile(
       "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %7, 0;\n\t"
-      "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w), "r"(elected) : "memory");
+      "setp.ne.b32 q, %8, 0;\n\t"
+      "@q cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n\t}"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w), "r"(v), "r"(elected) : "memory");
 }
 // generic-proxy writes to shared memory become visible to the tensor core (async proxy)
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -103,22 +106,8 @@ template <> __device__ __forceinline__ uint32_t pack2_tc<__half>(float lo, float
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// Wait used by the 16 softmax warps: one lane polls and sleeps between probes, so that the
-// waiting warps leave the issue slots to the two single-lane role warps that they wait for.
-__device__ __forceinline__ bool warp_wait_relaxed(uint32_t bar, uint32_t parity, volatile int* abort_flag, int lane) {
-  int ok = 1;
-  if (lane == 0 && !mbar_try_wait(bar, parity)) {
-    const long long t0 = clock64();
-    int spins = 0;
-    while (!mbar_try_wait(bar, parity)) {
-      __nanosleep(40);
-      if ((++spins & 63) == 0) {
-        if (*abort_flag) { ok = 0; break; }
-        if (clock64() - t0 > kWaitCycles) { *abort_flag = 1; ok = 0; break; }
-      }
-    }
-  }
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+__device__ __forceinline__ bool warp_wait_all(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
 template <typename T, int HD>
@@ -132,10 +121,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   constexpr int kStageBytes = 2 * kKBytes;                 // K then V
   constexpr int kPBytes = kTcRows * kTcTileN * 2;          // 16 KB: 128 rows x 128 B
   constexpr int kBarOffset = kQBytes + kTcStages * kStageBytes + 2 * kPBytes;
-  constexpr int CG = kTcColGroups;
-  constexpr int KT = kTcTileN / CG;                        // keys per softmax thread and tile
-  constexpr int kHalfCols = HD / CG;                       // P.V columns per thread
-  static_assert(KT == 16 && kHalfCols == 32, "columns per thread");
+  constexpr int kHalfCols = HD / 2;                        // P.V columns per conversion thread
   constexpr uint32_t kColS = 0, kColPV = 256;              // tensor-memory columns: S[2] x 128, PV[2] x 128
 
   extern __shared__ uint8_t smem_raw[];
@@ -143,16 +129,17 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t q_s = smem_base, stage0 = smem_base + kQBytes, p_s0 = stage0 + kTcStages * kStageBytes;
   const uint32_t bar_base = smem_base + kBarOffset;
-  // barriers: qfull | full[4] empty[4] | sfull[2] sfree[2] | pready[2] | pvfull[2] pvfree[2] | sync | qfree
+  // barriers: qfull | full[4] empty[4] | sfull[2] sfree[2] | pready[2] | pvfull[2] pvfree[2] | sync | qfree |
+  // denfull[2] denfree[2]
   const uint32_t qfull = bar_base, full0 = bar_base + 8, empty0 = full0 + 8 * kTcStages;
   const uint32_t sfull0 = empty0 + 8 * kTcStages, sfree0 = sfull0 + 16, pready0 = sfree0 + 16;
   const uint32_t pvfull0 = pready0 + 16, pvfree0 = pvfull0 + 16, soft_bar = pvfree0 + 16;
-  const uint32_t qfree = soft_bar + 8;
-  constexpr int kMisc = 8 * (1 + 2 * kTcStages + 10 + 2);
+  const uint32_t qfree = soft_bar + 8, denfull0 = qfree + 8, denfree0 = denfull0 + 16;
+  constexpr int kMisc = 8 * (1 + 2 * kTcStages + 10 + 2 + 4);
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem_gen + kBarOffset + kMisc);
   volatile int* abort_flag = (volatile int*)(smem_gen + kBarOffset + kMisc + 8);
-  float* rmax_s = (float*)(smem_gen + kBarOffset + kMisc + 16);                 // [CG][128]
-  long long* den_s = (long long*)(smem_gen + kBarOffset + kMisc + 16 + 2048);   // [CG][128]
+  float* rmax_s = (float*)(smem_gen + kBarOffset + kMisc + 16);                 // [item parity][group][128]
+  long long* den_s = (long long*)(smem_gen + kBarOffset + kMisc + 16 + 2048);   // [item parity][group][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -197,9 +184,10 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     mbar_init(qfree, 1);
     for (int s = 0; s < kTcStages; ++s) { mbar_init(full0 + 8u * s, 2); mbar_init(empty0 + 8u * s, 1); }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(sfull0 + 8u * b, 1); mbar_init(sfree0 + 8u * b, kTcSoftWarps);
-      mbar_init(pready0 + 8u * b, kTcSoftWarps);
-      mbar_init(pvfull0 + 8u * b, 1); mbar_init(pvfree0 + 8u * b, kTcSoftWarps);
+      mbar_init(sfull0 + 8u * b, 1); mbar_init(sfree0 + 8u * b, kTcGroupWarps);
+      mbar_init(pready0 + 8u * b, kTcGroupWarps);
+      mbar_init(pvfull0 + 8u * b, 1); mbar_init(pvfree0 + 8u * b, kTcConvWarps);
+      mbar_init(denfull0 + 8u * b, kTcSoftWarps); mbar_init(denfree0 + 8u * b, kTcConvWarps);
     }
     mbar_init(soft_bar, kTcSoftWarps);
     *abort_flag = 0;
@@ -216,12 +204,16 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
   if (warp == 0 || warp == kTcProducer2) {
     // ------------------------------ K / V producers (TMA) -----------------------------
-    // One box per 16-token page piece and half head (2 KB), 48 KB per 128 x 64 tile over the two
-    // passes, issued as predicated instructions of a uniform warp (tc_common.cuh); a box still takes
-    // its warp ~80 clocks, so two warps share them: by page piece, or by half head when a box holds a
-    // whole 64-key tile.  A stage is 32 KB: 128 keys of K in pass A (two 64-dim slabs of 128 rows), 64
-    // keys of K and V in pass B.  Nothing is copied, and the block table is not read, past the end of
-    // the sequence; V rows there are cleared by the MMA warp before P.V.
+    // A box is a 16-token page piece, or a whole 64-key tile when pages are multiples of 64 tokens, with
+    // all 128 head dims: [8-row group][64-dim half][8 rows][128 B], 4 or 16 KB.  The 8-row swizzle atoms
+    // of one half then lie 2 KB apart whatever the page size, which is all the MMA descriptors need.
+    // What a box costs is the issuing warp's latency among busy neighbours (~100 clocks, and as much
+    // again for coordinates computed in between), not the copy unit: boxes of one half head (twice as
+    // many) with their coordinates computed one by one took 1760 clocks per stage and bounded the
+    // kernel.  So two warps share the boxes and compute their coordinates before they wait for the
+    // stage.  A stage is 32 KB: 128 keys of K in pass A, 64 keys of K and V in pass B.  Nothing is copied,
+    // and the block table is not read, past the end of the sequence; V rows there are cleared by the
+    // MMA warp before P.V.
     const uint32_t e = elect_one();
     const int me = warp == 0 ? 0 : 1;
     int stage = 0; uint32_t phase = 1;
@@ -253,38 +245,38 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       };
       for (int pass = 0; pass < 2; ++pass) {
         const int step = pass ? 1 : 2;                       // tiles per stage
-        const uint32_t half_bytes = pass ? 8192u : 16384u;   // between the two 64-dim slabs
         int cur = load_entries(t0);
         for (int tb = t0; tb < t1; tb += 8) {
           const int nxt = load_entries(tb + 8);
           for (int tt = 0; tt < 8 && tb + tt < t1; tt += step) {
             const int t = tb + tt;
+            // only pieces that start inside the sequence are copied
+            const int left = (min(seq_len, t1 * kTcTileN) - t * kTcTileN + (1 << gs) - 1) >> gs;
+            const int groups = min(left, (step * kTcTileN) >> gs);
+            // my boxes i < 4: pieces me, me + 2, ... of K (pass A), or of K and V in turn (pass B); with
+            // 64-key boxes the one of my tile (pass A), or of K / V (pass B)
+            int blk[4], piece[4];
+            uint32_t dst[4], mine = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              piece[i] = gs == 4 ? me + 2 * (pass ? i >> 1 : i) : (pass ? 0 : me);
+              const int which = pass ? (gs == 4 ? i & 1 : me) : 0;
+              dst[i] = (uint32_t)(which * kKBytes + (piece[i] << (gs + 8)));
+              mine += (i == 0 || gs == 4) && piece[i] < groups ? 1u : 0u;
+              blk[i] = __shfl_sync(0xffffffffu, cur, (tt * 4 + (piece[i] << (gs - 4))) & 31);
+            }
             if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8u * stage, phase, abort_flag))) goto producer_done;
             const uint32_t fb = full0 + 8u * stage;
             const uint32_t ks = stage0 + stage * kStageBytes;
-            // only groups that start inside the sequence are copied
-            const int left = (min(seq_len, t1 * kTcTileN) - t * kTcTileN + (1 << gs) - 1) >> gs;
-            const int groups = min(left, (step * kTcTileN) >> gs);
-            const int first = gs == 4 ? me : 0, stride = gs == 4 ? 2 : 1;
-            const int mine = gs == 4 ? (groups - me + 1) >> 1 : groups;      // my page pieces
-            const int boxes = (gs == 4 ? 2 * mine : mine) << pass;           // of 2^(gs + 7) bytes each
-            mbar_expect_tx(fb, (uint32_t)boxes << (gs + 7), e);
-            for (int g = first; g < groups; g += stride) {
-              const int n = t * kTcTileN + (g << gs);
-              const int blk = __shfl_sync(0xffffffffu, cur, tt * 4 + (g << (gs - 4)));
+            mbar_expect_tx(fb, mine << (gs + 8), e);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              if (i > 0 && gs != 4) break;
+              const int n = t * kTcTileN + (piece[i] << gs);
               const int slot = sh.page_mask ? (n & sh.page_mask) : (n % sh.page_size);
-              const uint32_t dst = ks + (uint32_t)(g << (gs + 7));
-              if (gs == 4) {
-                tma_load_4d(dst, &map_k, fb, 0, kvh, slot, blk, e);
-                tma_load_4d(dst + half_bytes, &map_k, fb, 64, kvh, slot, blk, e);
-                if (pass) {
-                  tma_load_4d(dst + kKBytes, &map_v, fb, 0, kvh, slot, blk, e);
-                  tma_load_4d(dst + kKBytes + 8192, &map_v, fb, 64, kvh, slot, blk, e);
-                }
-              } else {
-                tma_load_4d(dst + me * half_bytes, &map_k, fb, me * 64, kvh, slot, blk, e);
-                if (pass) tma_load_4d(dst + kKBytes + me * 8192, &map_v, fb, me * 64, kvh, slot, blk, e);
-              }
+              const bool is_v = pass && (gs == 4 ? i & 1 : me);
+              tma_load_5d(ks + dst[i], is_v ? &map_v : &map_k, fb, 0, 0, kvh * sh.head_chunks, slot >> 3, blk[i],
+                          piece[i] < groups ? e : 0u);
             }
             if (++stage == kTcStages) { stage = 0; phase ^= 1; }
           }
@@ -295,16 +287,17 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   producer_done:;
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------------------
-    // S = Q . K^T: both operands K-major (head dim contiguous), two 64-dim slabs
+    // S = Q . K^T: both operands K-major (head dim contiguous); Q in two slabs of 64 dims, K with the two
+    // halves of every 8-row group side by side
     const uint32_t e = elect_one();
-    auto issue_s = [&](int stage, int sbuf, uint32_t idesc, uint32_t slab_bytes) {
+    auto issue_s = [&](int stage, int sbuf, uint32_t idesc) {
       const uint32_t d = tmem_base + kColS + (uint32_t)(sbuf * 128);
       const uint64_t qd = make_smem_desc(q_s, 16, 1024);
-      const uint64_t kd = make_smem_desc(stage0 + stage * kStageBytes, 16, 1024);
+      const uint64_t kd = make_smem_desc(stage0 + stage * kStageBytes, 16, 2048);
 #pragma unroll
       for (int kk = 0; kk < HD / 16; ++kk) {
         const uint64_t ao = (uint64_t)((kk >> 2) * (kQBytes / 2) + (kk & 3) * 32) >> 4;
-        const uint64_t bo = (uint64_t)((kk >> 2) * slab_bytes + (kk & 3) * 32) >> 4;
+        const uint64_t bo = (uint64_t)((kk >> 2) * 1024 + (kk & 3) * 32) >> 4;
         umma_f16(d, qd + ao, kd + bo, idesc, kk ? 1u : 0u, e);
       }
       umma_commit(sfull0 + 8u * sbuf, e);
@@ -328,11 +321,11 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const bool b = mbar_wait(sfree0 + 8u * sb, sph, abort_flag);
         if (!__all_sync(0xffffffffu, a && b)) goto issuer_done;
         tc_fence_after();
-        issue_s(stage, sb, sh.idesc_s2, 16384u);
+        issue_s(stage, sb, sh.idesc_s2);
         umma_commit(empty0 + 8u * stage, e);
         if (++stage == kTcStages) { stage = 0; phase ^= 1; }
       }
-      // pass B: S runs one tile ahead of P.V
+      // pass B: S runs two tiles ahead of P.V, one for each softmax group
       int s_stage = stage; uint32_t s_phase = phase;         // ring position of the next S tile
       auto issue_s_next = [&]() -> bool {
         const int sb = it & 1; const uint32_t sph = ((it >> 1) & 1) ^ 1;
@@ -340,17 +333,18 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const bool b = mbar_wait(sfree0 + 8u * sb, sph, abort_flag);
         if (!__all_sync(0xffffffffu, a && b)) return false;
         tc_fence_after();
-        issue_s(s_stage, sb, sh.idesc_s, 8192u);
+        issue_s(s_stage, sb, sh.idesc_s);
         ++it;
         if (++s_stage == kTcStages) { s_stage = 0; s_phase ^= 1; }
         return true;
       };
-      if (n_tiles > 0 && !issue_s_next()) goto issuer_done;
-      if (n_tiles <= 1) umma_commit(qfree, e);               // the item's last score MMA is issued
+      for (int j = 0; j < 2 && j < n_tiles; ++j)
+        if (!issue_s_next()) goto issuer_done;
+      if (n_tiles <= 2) umma_commit(qfree, e);               // the item's last score MMA is issued
       for (int j = 0; j < n_tiles; ++j, ++jg) {
-        if (j + 1 < n_tiles) {
+        if (j + 2 < n_tiles) {
           if (!issue_s_next()) goto issuer_done;
-          if (j + 2 == n_tiles) umma_commit(qfree, e);
+          if (j + 3 == n_tiles) umma_commit(qfree, e);
         }
         const int b = jg & 1; const uint32_t ph = (jg >> 1) & 1;
         const bool r1 = mbar_wait(pready0 + 8u * b, ph, abort_flag);
@@ -366,7 +360,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             const uint32_t vs = stage0 + stage * kStageBytes + kKBytes;
             for (int idx = lane; idx < (kTcTileN - r0) * 16; idx += 32) {
               const int rr = r0 + (idx >> 4), cc = idx & 15;
-              const uint32_t addr = vs + (uint32_t)((cc >> 3) * 8192 + rr * 128 + (cc & 7) * 16);
+              const uint32_t addr = vs + (uint32_t)((rr >> 3) * 2048 + (cc >> 3) * 1024 + (rr & 7) * 128 + (cc & 7) * 16);
               asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0) : "memory");
             }
             fence_proxy_async_smem();
@@ -376,10 +370,10 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // PV_j = P_j . V_j: P K-major (keys contiguous), V MN-major (head dim contiguous)
         const uint32_t d = tmem_base + kColPV + (uint32_t)(b * HD);
         const uint64_t pd = make_smem_desc(p_s0 + b * kPBytes, 16, 1024);
-        const uint64_t vd = make_smem_desc(stage0 + stage * kStageBytes + kKBytes, 8192, 1024);
+        const uint64_t vd = make_smem_desc(stage0 + stage * kStageBytes + kKBytes, 1024, 2048);
 #pragma unroll
         for (int kk = 0; kk < kTcTileN / 16; ++kk)
-          umma_f16(d, pd + (uint64_t)(kk * 2), vd + (uint64_t)(kk * 128), sh.idesc_pv, kk ? 1u : 0u, e);
+          umma_f16(d, pd + (uint64_t)(kk * 2), vd + (uint64_t)(kk * 256), sh.idesc_pv, kk ? 1u : 0u, e);
         umma_commit(pvfull0 + 8u * b, e);
         umma_commit(empty0 + 8u * stage, e);
         if (++stage == kTcStages) { stage = 0; phase ^= 1; }
@@ -387,10 +381,12 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     }
   issuer_done:;
-  } else if (warp < kTcProducer2) {
-    // ------------------------------ softmax / conversion warps ------------------------
+  } else if (warp < kTcFirstConv) {
+    // ------------------------------ softmax warps -------------------------------------
     const int quarter = warp & 3;
-    const int half = (warp - kTcFirstSoft) >> 2;                        // which quarter of the columns
+    // Two groups take the score products in turn (group = product number & 1 = S buffer): while one
+    // loads or waits, the other keeps the exponential unit busy.
+    const int group = (warp - kTcFirstSoft) >> 2;
     const int row = quarter * 32 + lane;                     // tensor-memory lane = query row
     const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
     const float ninf = -__int_as_float(0x7f800000);
@@ -398,24 +394,25 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const bool raw_max = plain_scores && p.ss_log2 > 0.0f;
     const uint64_t zero2 = pack2((uint32_t)zero, (uint32_t)zero);
     const uint64_t ss2 = pack2(__float_as_uint(p.ss_log2), __float_as_uint(p.ss_log2));
-    const uint32_t mbits = q_magic_bits(p.inv_scale), one = (uint32_t)zero + 1u;
+    const uint32_t mbits = q_magic_bits(p.inv_scale);
     const uint64_t magic2 = pack2(mbits, mbits);
-    const float screen_limit = q_screen_limit(p.inv_scale);
     uint32_t soft_phase = 0;
     bool ok = true;
     auto soft_sync = [&]() -> bool {                         // bounded barrier over these 8 warps
       __syncwarp();
       if (lane == 0) mbar_arrive(soft_bar);
-      const bool done = warp_wait_relaxed(soft_bar, soft_phase, abort_flag, lane);
+      const bool done = warp_wait_all(soft_bar, soft_phase, abort_flag);
       soft_phase ^= 1;
       return done;
     };
-    int it = 0;                                              // S tiles consumed so far (all items, both passes)
-    int jg = 0;                                              // P.V tiles of the items before this one
+    int it = 0;                                              // S products consumed so far (all items, both passes)
+    int jg = 0;                                              // P tiles of the items before this one
+    int k = -1;                                              // live items so far
     for (int w = blockIdx.x; w < total_items && ok; w += gridDim.x) {
     const Item I = decode_item(w);
     if (!I.live) continue;
-    const int kvh = I.kvh, q_start = I.q_start, q_len = I.q_len, tok0 = I.tok0, seq_len = I.seq_len, ctx = I.ctx;
+    ++k;
+    const int kvh = I.kvh, q_len = I.q_len, tok0 = I.tok0, seq_len = I.seq_len, ctx = I.ctx;
     const int t0 = I.t0, t1 = I.t1, n_tiles = I.t1 - I.t0;
     const int tok = tok0 + row / G, head = kvh * G + row % G;
     const bool valid = tok < q_len;
@@ -438,180 +435,213 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     };
 
     // =============================== pass A: row maxima ===============================
-    // 128 keys per step, 32 per thread.  Scaling by a positive constant is monotonic after rounding
+    // 128 keys per step, all of them in one thread.  Scaling by a positive constant is monotonic after rounding
     // too, so the maximum is taken over the raw products and scaled once.
     float rmax = ninf;
     for (int t = t0; t < t1 && ok; t += 2, ++it) {
       const int sb = it & 1;
-      if (!warp_wait_relaxed(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag, lane)) { ok = false; break; }
+      if (sb != group) continue;
+      if (!warp_wait_all(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      uint32_t v[2 * KT];
-      tmem_ld32(tmem_base + lane_sel + kColS + (uint32_t)(sb * 128 + half * 2 * KT), v);
-      tmem_wait_ld_regs(v);
-      release_s(sb);
-      const int n0 = t * kTcTileN + half * 2 * KT;
-      const bool inside = n0 >= kbeg && n0 + 2 * KT <= kend;
       float m = ninf;
-      if (raw_max) {
-        if (inside) {
-          float m1 = ninf;                                   // two chains
 #pragma unroll
-          for (int i = 0; i < 2 * KT; i += 4) {
-            m = max3(m, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
-            m1 = max3(m1, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
+      for (int c = 0; c < 4; ++c) {
+        uint32_t v[32];
+        tmem_ld32(tmem_base + lane_sel + kColS + (uint32_t)(sb * 128 + c * 32), v);
+        tmem_wait_ld_regs(v);
+        if (c == 3) release_s(sb);
+        const int n0 = t * kTcTileN + c * 32;
+        const bool inside = n0 >= kbeg && n0 + 32 <= kend;
+        if (raw_max) {
+          if (inside) {
+            float m1 = ninf;                                 // two chains
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              m = max3(m, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+              m1 = max3(m1, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
+            }
+            m = fmaxf(m, m1);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (n0 + i >= kbeg && n0 + i < kend) m = fmaxf(m, __uint_as_float(v[i]));
           }
-          m = fmaxf(m, m1);
         } else {
 #pragma unroll
-          for (int i = 0; i < 2 * KT; ++i)
-            if (n0 + i >= kbeg && n0 + i < kend) m = fmaxf(m, __uint_as_float(v[i]));
+          for (int i = 0; i < 32; ++i)
+            if (n0 + i >= kbeg && n0 + i < kend) m = fmaxf(m, score(v[i], n0 + i));
         }
-        m = __fmul_rn(m, p.ss_log2);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 2 * KT; ++i)
-          if (n0 + i >= kbeg && n0 + i < kend) m = fmaxf(m, score(v[i], n0 + i));
       }
-      rmax = fmaxf(rmax, m);
+      rmax = fmaxf(rmax, raw_max ? __fmul_rn(m, p.ss_log2) : m);
     }
-    rmax_s[half * kTcRows + row] = rmax;
+    float* rmax_k = rmax_s + (k & 1) * (2 * kTcRows);
+    rmax_k[group * kTcRows + row] = rmax;
     if (ok && !soft_sync()) ok = false;
-    float gmax = rmax_s[row];
-#pragma unroll
-    for (int c = 1; c < CG; ++c) gmax = fmaxf(gmax, rmax_s[c * kTcRows + row]);
+    float gmax = fmaxf(rmax_k[row], rmax_k[kTcRows + row]);
     if (gmax == ninf) gmax = 0.0f;                           // rows without keys: exp2 gives 0, not NaN
 
     // =============================== pass B ===========================================
     uint32_t den32 = 0;
     const uint64_t neg_max2 = pack2(__float_as_uint(-gmax), __float_as_uint(-gmax));
-    uint32_t acc[kHalfCols];
-#pragma unroll
-    for (int i = 0; i < kHalfCols; ++i) acc[i] = 0;
-    uint32_t corr_raw[kHalfCols];                            // rare path, local memory
-    long long corr_q[kHalfCols];
-    bool corr_used = false;
-
-    // round the P.V partial of tile j (this thread's 64 columns) to Q-format and add it
-    auto convert_pv = [&](int j) -> bool {                  // j counts over all items
-      const int b = j & 1; const uint32_t ph = (j >> 1) & 1;
-      if (!warp_wait_relaxed(pvfull0 + 8u * b, ph, abort_flag, lane)) return false;
-      tc_fence_after();
-      const uint32_t taddr = tmem_base + lane_sel + kColPV + (uint32_t)(b * HD + half * kHalfCols);
-      float screen = 0.0f;
-#pragma unroll
-      for (int c = 0; c < kHalfCols; c += 16) {
-        uint32_t v[16];
-        tmem_ld16(taddr + c, v);
-        tmem_wait_ld_regs(v);
-        convert16(v, &acc[c], magic2, mbits, one, screen);
-      }
-      if (__any_sync(0xffffffffu, !(screen < screen_limit))) {
-        // some partial left the fast range: exact conversion of the offending elements
-        if (!corr_used) {
-#pragma unroll 1
-          for (int z = 0; z < kHalfCols; ++z) { corr_raw[z + zero] = 0; corr_q[z + zero] = 0; }
-          corr_used = true;
-        }
-        fixup_tile(taddr, kHalfCols, mbits, p.scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(pvfree0 + 8u * b);
-      return true;
-    };
-
+    int mine = 0;                                            // tiles of this group
     for (int j = 0; j < n_tiles && ok; ++j, ++it) {
       const int t = t0 + j;
       const int sb = it & 1;
-      if (!warp_wait_relaxed(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag, lane)) { ok = false; break; }
+      if (sb != group) continue;
+      ++mine;
+      if (!warp_wait_all(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      uint32_t v[KT];
-      tmem_ld16(tmem_base + lane_sel + kColS + (uint32_t)(sb * 128 + half * KT), v);
-      tmem_wait_ld_regs(v);
-      release_s(sb);
-      // d = score - max, rounded twice; the product is an fma with a run-time zero because the
-      // assembler contracts a packed multiply and the packed add behind it into one rounding.
-      // The weight of a masked key is exp2(-inf) = 0.
-      const int n0 = t * kTcTileN + half * KT;
-      const bool inside = n0 >= kbeg && n0 + KT <= kend;
-      if (plain_scores) {
-#pragma unroll
-        for (int i = 0; i < KT; i += 2) {
-          uint64_t x;
-          asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x) : "l"(pack2(v[i], v[i + 1])), "l"(ss2), "l"(zero2));
-          asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(neg_max2));
-          asm("mov.b64 {%0, %1}, %2;" : "=r"(v[i]), "=r"(v[i + 1]) : "l"(x));
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < KT; ++i) v[i] = __float_as_uint(__fsub_rn(score(v[i], n0 + i), gmax));
-      }
-      if (!inside) {
-#pragma unroll
-        for (int i = 0; i < KT; ++i)
-          if (n0 + i < kbeg || n0 + i >= kend) v[i] = __float_as_uint(ninf);
-      }
-      // weights, integer denominator, P in the io dtype -> shared memory (A operand of P.V):
-      // row = 128 bytes of 64 keys, 16-byte chunks XOR-swizzled with the row number
-      const int b = (jg + j) & 1;
+      const int g = jg + j, b = g & 1;
       const uint32_t prow = p_s0 + b * kPBytes + (uint32_t)row * 128u;
 #pragma unroll
-      for (int c = 0; c < KT / 8; ++c) {
-        uint32_t pk[4];
+      for (int h = 0; h < 2; ++h) {
+        uint32_t v[32];
+        tmem_ld32(tmem_base + lane_sel + kColS + (uint32_t)(sb * 128 + h * 32), v);
+        tmem_wait_ld_regs(v);
+        if (h == 1) release_s(sb);
+        // d = score - max, rounded twice; the product is an fma with a run-time zero because the
+        // assembler contracts a packed multiply and the packed add behind it into one rounding.
+        // The weight of a masked key is exp2(-inf) = 0.
+        const int n0 = t * kTcTileN + h * 32;
+        const bool inside = n0 >= kbeg && n0 + 32 <= kend;
+        if (plain_scores) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float w0 = ex2_approx_tc(__uint_as_float(v[c * 8 + e * 2]));
-          const float w1 = ex2_approx_tc(__uint_as_float(v[c * 8 + e * 2 + 1]));
-          uint64_t q;
-          asm("add.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(pack2(__float_as_uint(w0), __float_as_uint(w1))), "l"(magic2));
-          den32 = den32 + (uint32_t)q + (uint32_t)(q >> 32);
-          pk[e] = pack2_tc<T>(w0, w1);
+          for (int i = 0; i < 32; i += 2) {
+            uint64_t x;
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x) : "l"(pack2(v[i], v[i + 1])), "l"(ss2), "l"(zero2));
+            asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(neg_max2));
+            asm("mov.b64 {%0, %1}, %2;" : "=r"(v[i]), "=r"(v[i + 1]) : "l"(x));
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__fsub_rn(score(v[i], n0 + i), gmax));
         }
-        const uint32_t chunk = (uint32_t)(half * (KT / 8) + c);
-        const uint32_t addr = prow + ((chunk ^ (uint32_t)(row & 7)) << 4);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+        if (!inside) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (n0 + i < kbeg || n0 + i >= kend) v[i] = __float_as_uint(ninf);
+        }
+        // weights, integer denominator, P in the io dtype -> shared memory (A operand of P.V):
+        // row = 128 bytes of 64 keys, 16-byte chunks XOR-swizzled with the row number
+        // (its buffer is free once the P.V product two tiles back has completed)
+        if (h == 0 && g >= 2 && !warp_wait_all(pvfull0 + 8u * b, ((g - 2) >> 1) & 1, abort_flag)) { ok = false; break; }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float w0 = ex2_approx_tc(__uint_as_float(v[c * 8 + e * 2]));
+            const float w1 = ex2_approx_tc(__uint_as_float(v[c * 8 + e * 2 + 1]));
+            uint64_t q;
+            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(pack2(__float_as_uint(w0), __float_as_uint(w1))), "l"(magic2));
+            den32 = den32 + (uint32_t)q + (uint32_t)(q >> 32);
+            pk[e] = pack2_tc<T>(w0, w1);
+          }
+          const uint32_t addr = prow + (((uint32_t)(h * 4 + c) ^ (uint32_t)(row & 7)) << 4);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+        }
       }
+      if (!ok) break;
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(pready0 + 8u * b);
-      if (j > 0 && !convert_pv(jg + j - 1)) { ok = false; break; }
     }
-    if (ok && n_tiles > 0 && !convert_pv(jg + n_tiles - 1)) ok = false;
+    if (!ok) break;
     jg += n_tiles;
-
-    // =============================== output ===========================================
-    // KT weights per tile went through the fast add in this thread
-    const long long den_half = (long long)(int32_t)(den32 - (uint32_t)KT * (uint32_t)n_tiles * mbits);
-    den_s[half * kTcRows + row] = den_half;
-    if (ok && !soft_sync()) ok = false;
-    if (ok && valid) {
-      long long dsum = den_s[row];
-#pragma unroll
-      for (int c = 1; c < CG; ++c) dsum += den_s[c * kTcRows + row];
-      const float dn = fmaxf(fixed_to_float<long long>(wrap_to_bits(dsum, p.int_bits), p.inv_scale), 1.0e-6f);
-      T* op = (T*)p.o + (int64_t)(q_start + tok) * p.o_st + (int64_t)head * p.o_sh + half * kHalfCols;
-      const uint32_t bias_bits = (uint32_t)n_tiles * mbits;   // what the multiply-adds summed on top
-#pragma unroll
-      for (int g8 = 0; g8 < kHalfCols / 8; ++g8) {
-        alignas(16) T out[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int c = g8 * 8 + i;
-          uint32_t raw = alu_add(c) ? acc[c] : acc[c] - bias_bits;
-          float num;
-          if (corr_used) {
-            raw -= corr_raw[c + zero];
-            const long long tot = (long long)(int32_t)raw + corr_q[c + zero];
-            num = fixed_to_float<long long>(wrap_to_bits(tot, p.int_bits), p.inv_scale);
-          } else {
-            // the sum fits 32 bits: the same value through the cheaper 32-bit conversion
-            num = fixed_to_float<int>((int)raw, p.inv_scale);
-          }
-          out[i] = from_f32<T>(__fdiv_rn(num, dn));
-        }
-        *reinterpret_cast<uint4*>(op + g8 * 8) = *reinterpret_cast<const uint4*>(out);
-      }
+    // 64 weights per tile went through the packed add in this thread
+    if (!warp_wait_all(denfree0 + 8u * (k & 1), ((k >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
+    den_s[(k & 1) * (2 * kTcRows) + group * kTcRows + row] =
+        (long long)(int32_t)(den32 - (uint32_t)kTcTileN * (uint32_t)mine * mbits);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(denfull0 + 8u * (k & 1));
     }
+  } else if (warp < kTcProducer2) {
+    // ------------------------------ conversion warps ----------------------------------
+    // Round every P.V partial to Q-format, add, and store the finished rows; the softmax warps are by
+    // then in the next item's maximum pass.
+    const int quarter = warp & 3;
+    const int half = (warp - kTcFirstConv) >> 2;             // which half of the output columns
+    const int row = quarter * 32 + lane;
+    const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
+    const uint32_t mbits = q_magic_bits(p.inv_scale), one = (uint32_t)zero + 1u;
+    const uint64_t magic2 = pack2(mbits, mbits);
+    const float screen_limit = q_screen_limit(p.inv_scale);
+    int jg = 0;                                              // P.V tiles converted so far (all items)
+    int k = -1;                                              // live items so far
+    bool ok = true;
+    for (int w = blockIdx.x; w < total_items && ok; w += gridDim.x) {
+      const Item I = decode_item(w);
+      if (!I.live) continue;
+      ++k;
+      const int n_tiles = I.t1 - I.t0;
+      uint32_t acc[kHalfCols];
+#pragma unroll
+      for (int i = 0; i < kHalfCols; ++i) acc[i] = 0;
+      uint32_t corr_raw[kHalfCols];                          // rare path, local memory
+      long long corr_q[kHalfCols];
+      bool corr_used = false;
+      for (int j = 0; j < n_tiles; ++j, ++jg) {
+        const int b = jg & 1;
+        if (!warp_wait_all(pvfull0 + 8u * b, (jg >> 1) & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + lane_sel + kColPV + (uint32_t)(b * HD + half * kHalfCols);
+        float screen = 0.0f, tail = 0.0f;
+#pragma unroll
+        for (int c = 0; c < kHalfCols; c += 16) {
+          uint32_t v[16];
+          tmem_ld16(taddr + c, v);
+          tmem_wait_ld_regs(v);
+          if (c + 16 == kHalfCols) {
+            // the last chunk is in registers: screen it and hand the buffer back before converting it
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) screen = max3_abs(screen, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+            if (__any_sync(0xffffffffu, !(screen < screen_limit))) {
+              // some partial left the fast range: exact conversion of the offending elements
+              if (!corr_used) {
+#pragma unroll 1
+                for (int z = 0; z < kHalfCols; ++z) { corr_raw[z + zero] = 0; corr_q[z + zero] = 0; }
+                corr_used = true;
+              }
+              fixup_tile(taddr, kHalfCols, mbits, p.scale, p.int_bits, &corr_raw[zero], &corr_q[zero]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(pvfree0 + 8u * b);
+          }
+          convert16(v, &acc[c], magic2, mbits, one, c + 16 == kHalfCols ? tail : screen);
+        }
+      }
+      if (!ok) break;
+      if (!warp_wait_all(denfull0 + 8u * (k & 1), (k >> 1) & 1, abort_flag)) { ok = false; break; }
+      const long long dsum = den_s[(k & 1) * (2 * kTcRows) + row] + den_s[(k & 1) * (2 * kTcRows) + kTcRows + row];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(denfree0 + 8u * (k & 1));
+      const int tok = I.tok0 + row / G, head = I.kvh * G + row % G;
+      if (tok < I.q_len) {
+        const float dn = fmaxf(fixed_to_float<long long>(wrap_to_bits(dsum, p.int_bits), p.inv_scale), 1.0e-6f);
+        T* op = (T*)p.o + (int64_t)(I.q_start + tok) * p.o_st + (int64_t)head * p.o_sh + half * kHalfCols;
+        const uint32_t bias_bits = (uint32_t)n_tiles * mbits;   // what the multiply-adds summed on top
+#pragma unroll
+        for (int g8 = 0; g8 < kHalfCols / 8; ++g8) {
+          alignas(16) T out[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int c = g8 * 8 + i;
+            uint32_t raw = alu_add(c) ? acc[c] : acc[c] - bias_bits;
+            float num;
+            if (corr_used) {
+              raw -= corr_raw[c + zero];
+              const long long tot = (long long)(int32_t)raw + corr_q[c + zero];
+              num = fixed_to_float<long long>(wrap_to_bits(tot, p.int_bits), p.inv_scale);
+            } else {
+              // the sum fits 32 bits: the same value through the cheaper 32-bit conversion
+              num = fixed_to_float<int>((int)raw, p.inv_scale);
+            }
+            out[i] = from_f32<T>(__fdiv_rn(num, dn));
+          }
+          *reinterpret_cast<uint4*>(op + g8 * 8) = *reinterpret_cast<const uint4*>(out);
+        }
+      }
     }
   }
 
@@ -667,7 +697,8 @@ bool attention_tc_supported(const AttnParams& p, int dtype, int max_query_len, b
   const int64_t max_keys = p.bt_stride * (int64_t)p.page_size;
   if ((max_keys + kTcTileN - 1) / kTcTileN > 500) return false;
   const int64_t strides[] = {p.q_st, p.q_sh, p.o_st, p.o_sh, p.kv_sblock, p.kv_sslot, p.kv_shead};
-  for (int64_t st : strides) if (st % 8 != 0 || st <= 0 || st >= (1ll << 38)) return false;
+  for (int64_t st : strides) if (st % 8 != 0 || st <= 0 || st >= (1ll << 35)) return false;
+  if (p.kv_shead % 64 != 0) return false;
   if (((uintptr_t)p.q | (uintptr_t)p.k | (uintptr_t)p.v | (uintptr_t)p.o) & 15) return false;
   if (p.num_reqs > 65535) return false;
   return encode_fn() != nullptr;
@@ -704,15 +735,16 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
       return FXPR_ERR_CUDA;
     }
   }
+  // Cache planes [blocks, 8-slot groups, 64-dim chunks (heads and halves), slots, dims]: see the
+  // producers.  The number of blocks is not known here and only bounds the coordinates, which come from
+  // the block table.
+  sh.head_chunks = (int)(p.kv_shead / 64);
   for (int which = 0; which < 2; ++which) {
-    // cache plane [blocks, slots, kv heads, dims]; the number of blocks is not known here and
-    // only bounds the coordinates, which come from the block table
-    cuuint64_t dims[4] = {(cuuint64_t)p.head_dim, (cuuint64_t)p.num_kv_heads, (cuuint64_t)p.page_size,
+    cuuint64_t dims[5] = {64, 8, (cuuint64_t)((p.num_kv_heads - 1) * (p.kv_shead / 64) + 2), (cuuint64_t)(p.page_size / 8),
                           (cuuint64_t)1 << 31};
-    cuuint64_t strides[3] = {(cuuint64_t)p.kv_shead * 2, (cuuint64_t)p.kv_sslot * 2, (cuuint64_t)p.kv_sblock * 2};
-    cuuint32_t box[4] = {64, 1, (cuuint32_t)(1 << sh.group_shift), 1};
-    cuuint32_t es[4] = {1, 1, 1, 1};
-    if (fn(which ? &mv : &mk, dt, 4, const_cast<void*>(which ? p.v : p.k), dims, strides, box, es,
+    cuuint64_t strides[4] = {(cuuint64_t)p.kv_sslot * 2, 128, (cuuint64_t)p.kv_sslot * 16, (cuuint64_t)p.kv_sblock * 2};
+    cuuint32_t box[5] = {64, 8, 2, 1u << (sh.group_shift - 3), 1}, es[5] = {1, 1, 1, 1, 1};
+    if (fn(which ? &mv : &mk, dt, 5, const_cast<void*>(which ? p.v : p.k), dims, strides, box, es,
            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
       set_last_error("cuTensorMapEncodeTiled(KV)", cudaErrorInvalidValue);
@@ -721,7 +753,7 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
   }
 
   constexpr int kSmem = kTcRows * 128 * 2 + kTcStages * 2 * kTcTileN * 128 * 2 + 2 * kTcRows * kTcTileN * 2 +
-                        8 * (1 + 2 * kTcStages + 10 + 2) + 16 + 2048 + 4096 + 1024;
+                        8 * (1 + 2 * kTcStages + 10 + 2 + 4) + 16 + 2048 + 4096 + 1024;
   // persistent CTAs, one per SM (204 KB of shared memory each), walking the padded item list
   int dev_now = 0, sms = 0;
   cudaGetDevice(&dev_now);
