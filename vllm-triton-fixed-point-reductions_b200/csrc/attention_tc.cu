@@ -33,6 +33,8 @@
 // KV splits are not handled here (the dispatcher sends them to attention_mma.cu: same bits).
 // Every wait is bounded; on a time-out the CTA sets the status word and leaves.
 #include <algorithm>
+#include <type_traits>
+
 #include <cuda.h>
 
 #include "attention_common.cuh"
@@ -49,8 +51,9 @@ static constexpr int kTcSoftWarps = 2 * kTcGroupWarps;
 static constexpr int kTcConvWarps = 8;         // conversion: thread = one row and half of the output columns
 static constexpr int kTcFirstSoft = 2;         // warp 0: TMA producer, warp 1: MMA issuer
 static constexpr int kTcFirstConv = kTcFirstSoft + kTcSoftWarps;
-static constexpr int kTcProducer2 = kTcFirstConv + kTcConvWarps;   // the second producer warp
-static constexpr int kTcThreads = (kTcProducer2 + 1) * 32;
+static constexpr int kTcFirstMore = kTcFirstConv + kTcConvWarps;   // further producer warps
+static constexpr int kTcProducers = 2;
+static constexpr int kTcThreads = (kTcFirstMore + kTcProducers - 1) * 32;
 static constexpr int kTcStages = 4;
 
 struct TcAttnShape {
@@ -144,11 +147,17 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   // ---- work items ---------------------------------------------------------------------
-  // Persistent CTAs: CTA b takes the work items b, b + gridDim.x, ... of the padded space
-  // (request, row block, KV head), later row blocks (more keys) first.  Every role walks the
-  // same list and keeps its ring positions and barrier phases running from one item to the
-  // next, so the producer fetches the next item's Q and first keys and the MMA warp starts its
-  // scores while the softmax warps still convert and store the current item's output.
+  // Persistent CTAs over the padded list (request, row block, KV head), later row blocks (more keys)
+  // first, dealt out there and back again: straight round robin gives the first CTAs the longer item of
+  // every round (16 prompts of 128 to 4096 tokens: the busiest SM 15 % over the mean, 4 % this way).
+  // Drawing items from a counter in global memory balances better still but was slower (16 x 2048 tokens
+  // 1354 against 1223 us): the CTAs then stay in step and read the same cache lines at the same time.
+  // Every role walks the same list and keeps its ring positions and barrier phases running from one item
+  // to the next, so the producers fetch the next item's Q and first keys and the MMA warp starts its
+  // scores while the conversion warps still finish the current item.
+  auto item_of = [&](int r) -> int {
+    return r * (int)gridDim.x + (r & 1 ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+  };
   const int hkv = p.num_kv_heads;
   const int G = sh.rows_per_token;
   const int items_per_req = sh.num_q_blocks * hkv;
@@ -182,7 +191,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   if (threadIdx.x == 0) {
     mbar_init(qfull, 1);
     mbar_init(qfree, 1);
-    for (int s = 0; s < kTcStages; ++s) { mbar_init(full0 + 8u * s, 2); mbar_init(empty0 + 8u * s, 1); }
+    for (int s = 0; s < kTcStages; ++s) { mbar_init(full0 + 8u * s, kTcProducers); mbar_init(empty0 + 8u * s, 1); }
     for (int b = 0; b < 2; ++b) {
       mbar_init(sfull0 + 8u * b, 1); mbar_init(sfree0 + 8u * b, kTcGroupWarps);
       mbar_init(pready0 + 8u * b, kTcGroupWarps);
@@ -202,28 +211,27 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0 || warp == kTcProducer2) {
+  if (warp == 0 || warp >= kTcFirstMore) {
     // ------------------------------ K / V producers (TMA) -----------------------------
     // A box is a 16-token page piece, or a whole 64-key tile when pages are multiples of 64 tokens, with
     // all 128 head dims: [8-row group][64-dim half][8 rows][128 B], 4 or 16 KB.  The 8-row swizzle atoms
     // of one half then lie 2 KB apart whatever the page size, which is all the MMA descriptors need.
-    // What a box costs is the issuing warp's latency among busy neighbours (~100 clocks, and as much
-    // again for coordinates computed in between), not the copy unit: boxes of one half head (twice as
-    // many) with their coordinates computed one by one took 1760 clocks per stage and bounded the
-    // kernel.  So two warps share the boxes and compute their coordinates before they wait for the
-    // stage.  A stage is 32 KB: 128 keys of K in pass A, 64 keys of K and V in pass B.  Nothing is copied,
+    // A 4 KB box takes the copy unit ~100 clocks and its warp about as long again for coordinates and
+    // barriers, with 20 warps on the SM: two warps share the eight boxes of a stage, compute their
+    // coordinates before they wait for it, and run loops without run-time choices.  (One warp with boxes
+    // of one half head, twice as many: 1760 clocks per stage, which bounded the kernel.)
+    // A stage is 32 KB: 128 keys of K in pass A, 64 keys of K and V in pass B.  Nothing is copied,
     // and the block table is not read, past the end of the sequence; V rows there are cleared by the
     // MMA warp before P.V.
     const uint32_t e = elect_one();
-    const int me = warp == 0 ? 0 : 1;
+    const int me = warp == 0 ? 0 : warp - kTcFirstMore + 1;
     int stage = 0; uint32_t phase = 1;
     uint32_t q_phase = 1;                                    // qfree: the first wait passes
     // Block-table entries are read 32 at a time (lane L: the 16-key group L of an 8-tile block), one
     // block ahead of their use, and handed round by shuffle.
     int page_shift = -1;
     for (int b = 4; b < 31; ++b) if ((1 << b) == sh.page_size) page_shift = b;
-    const int gs = sh.group_shift;                           // log2 of the keys per box: 4 or 6
-    for (int w = blockIdx.x; w < total_items; w += gridDim.x) {
+    for (int r = 0, w = blockIdx.x; w < total_items; w = item_of(++r)) {
       const Item I = decode_item(w);
       if (!I.live) continue;
       const int kvh = I.kvh, seq_len = I.seq_len, t0 = I.t0, t1 = I.t1;
@@ -243,46 +251,52 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const int n = tb * kTcTileN + lane * 16;
         return (tb < t1 && n < seq_len) ? bt[page_shift >= 0 ? (n >> page_shift) : (n / sh.page_size)] : 0;
       };
-      for (int pass = 0; pass < 2; ++pass) {
-        const int step = pass ? 1 : 2;                       // tiles per stage
+      // one pass over the item's tiles; PASS and GS (log2 of the keys per box) are compile-time
+      auto walk = [&](auto pass_c, auto gs_c) -> bool {
+        constexpr int PASS = decltype(pass_c)::value, GS = decltype(gs_c)::value;
+        constexpr int kStep = PASS ? 1 : 2;                  // tiles per stage
+        constexpr int kPieces = (kStep * kTcTileN) >> GS;    // page pieces of K (and of V) per stage
+        constexpr int kBoxes = kPieces << PASS;              // box q: piece q of K, or piece q / 2 of K (even q) and V
+        constexpr int kMine = (kBoxes + kTcProducers - 1) / kTcProducers;
         int cur = load_entries(t0);
         for (int tb = t0; tb < t1; tb += 8) {
           const int nxt = load_entries(tb + 8);
-          for (int tt = 0; tt < 8 && tb + tt < t1; tt += step) {
-            const int t = tb + tt;
-            // only pieces that start inside the sequence are copied
-            const int left = (min(seq_len, t1 * kTcTileN) - t * kTcTileN + (1 << gs) - 1) >> gs;
-            const int groups = min(left, (step * kTcTileN) >> gs);
-            // my boxes i < 4: pieces me, me + 2, ... of K (pass A), or of K and V in turn (pass B); with
-            // 64-key boxes the one of my tile (pass A), or of K / V (pass B)
-            int blk[4], piece[4];
-            uint32_t dst[4], mine = 0;
+          for (int tt = 0; tt < 8 && tb + tt < t1; tt += kStep) {
+            const int n0 = (tb + tt) * kTcTileN;
+            // only pieces that start inside the sequence (pass A: and before t1) are copied
+            const int pieces = (min(seq_len, t1 * kTcTileN) - n0 + (1 << GS) - 1) >> GS;
+            int blk[kMine], row8[kMine];
+            uint32_t bytes = 0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              piece[i] = gs == 4 ? me + 2 * (pass ? i >> 1 : i) : (pass ? 0 : me);
-              const int which = pass ? (gs == 4 ? i & 1 : me) : 0;
-              dst[i] = (uint32_t)(which * kKBytes + (piece[i] << (gs + 8)));
-              mine += (i == 0 || gs == 4) && piece[i] < groups ? 1u : 0u;
-              blk[i] = __shfl_sync(0xffffffffu, cur, (tt * 4 + (piece[i] << (gs - 4))) & 31);
+            for (int i = 0; i < kMine; ++i) {
+              const int q = me + i * kTcProducers, piece = PASS ? q >> 1 : q;
+              blk[i] = __shfl_sync(0xffffffffu, cur, (tt * 4 + (piece << (GS - 4))) & 31);
+              const int n = n0 + (piece << GS);
+              row8[i] = (sh.page_mask ? (n & sh.page_mask) : (n % sh.page_size)) >> 3;
+              if (q < kBoxes && piece < pieces) bytes += 256u << GS;
             }
-            if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8u * stage, phase, abort_flag))) goto producer_done;
-            const uint32_t fb = full0 + 8u * stage;
-            const uint32_t ks = stage0 + stage * kStageBytes;
-            mbar_expect_tx(fb, mine << (gs + 8), e);
+            if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8u * stage, phase, abort_flag))) return false;
+            const uint32_t fb = full0 + 8u * stage, ks = stage0 + stage * kStageBytes;
+            mbar_expect_tx(fb, bytes, e);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              if (i > 0 && gs != 4) break;
-              const int n = t * kTcTileN + (piece[i] << gs);
-              const int slot = sh.page_mask ? (n & sh.page_mask) : (n % sh.page_size);
-              const bool is_v = pass && (gs == 4 ? i & 1 : me);
-              tma_load_5d(ks + dst[i], is_v ? &map_v : &map_k, fb, 0, 0, kvh * sh.head_chunks, slot >> 3, blk[i],
-                          piece[i] < groups ? e : 0u);
+            for (int i = 0; i < kMine; ++i) {
+              const int q = me + i * kTcProducers, piece = PASS ? q >> 1 : q;
+              const bool v = PASS && (q & 1);
+              if (q < kBoxes && piece < pieces)
+                tma_load_5d(ks + (uint32_t)((v ? kKBytes : 0) + (piece << (GS + 8))), v ? &map_v : &map_k, fb, 0, 0,
+                            kvh * sh.head_chunks, row8[i], blk[i], e);
             }
             if (++stage == kTcStages) { stage = 0; phase ^= 1; }
           }
           cur = nxt;
         }
-      }
+        return true;
+      };
+      using std::integral_constant;
+      const bool fetched = sh.group_shift == 4
+          ? walk(integral_constant<int, 0>{}, integral_constant<int, 4>{}) && walk(integral_constant<int, 1>{}, integral_constant<int, 4>{})
+          : walk(integral_constant<int, 0>{}, integral_constant<int, 6>{}) && walk(integral_constant<int, 1>{}, integral_constant<int, 6>{});
+      if (!fetched) goto producer_done;
     }
   producer_done:;
   } else if (warp == 1) {
@@ -306,7 +320,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     int it = 0;                                              // S products issued so far (all items, both passes)
     int jg = 0;                                              // P.V tiles issued so far (all items)
     uint32_t q_phase = 0;
-    for (int w = blockIdx.x; w < total_items; w += gridDim.x) {
+    for (int r = 0, w = blockIdx.x; w < total_items; w = item_of(++r)) {
     const Item I = decode_item(w);
     if (!I.live) continue;
     const int seq_len = I.seq_len, t0 = I.t0, t1 = I.t1, n_tiles = I.t1 - I.t0;
@@ -408,7 +422,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     int it = 0;                                              // S products consumed so far (all items, both passes)
     int jg = 0;                                              // P tiles of the items before this one
     int k = -1;                                              // live items so far
-    for (int w = blockIdx.x; w < total_items && ok; w += gridDim.x) {
+    for (int r = 0, w = blockIdx.x; w < total_items && ok; w = item_of(++r)) {
     const Item I = decode_item(w);
     if (!I.live) continue;
     ++k;
@@ -555,7 +569,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     __syncwarp();
     if (lane == 0) mbar_arrive(denfull0 + 8u * (k & 1));
     }
-  } else if (warp < kTcProducer2) {
+  } else {
     // ------------------------------ conversion warps ----------------------------------
     // Round every P.V partial to Q-format, add, and store the finished rows; the softmax warps are by
     // then in the next item's maximum pass.
@@ -569,7 +583,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     int jg = 0;                                              // P.V tiles converted so far (all items)
     int k = -1;                                              // live items so far
     bool ok = true;
-    for (int w = blockIdx.x; w < total_items && ok; w += gridDim.x) {
+    for (int r = 0, w = blockIdx.x; w < total_items && ok; w = item_of(++r)) {
       const Item I = decode_item(w);
       if (!I.live) continue;
       ++k;
