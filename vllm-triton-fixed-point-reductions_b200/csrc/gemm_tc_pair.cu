@@ -120,9 +120,7 @@ __device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, vo
   return true;
 }
 __device__ __forceinline__ bool warp_wait_poll(uint32_t bar, uint32_t parity, volatile int* abort_flag, int lane) {
-  int ok = 1;
-  if (lane == 0) ok = mbar_wait_poll(bar, parity, abort_flag) ? 1 : 0;
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
 static constexpr int kPrStages = 6;
