@@ -234,6 +234,32 @@ def test_tensor_core_route_feature_flags_close_to_oracle(dtype, kwargs, splits):
     assert (got.float().cpu() - exp).abs().max().item() <= tol * max(1.0, float(exp.abs().max()))
 
 
+@pytest.mark.parametrize("page", [16, 48, 64])
+@pytest.mark.parametrize("head_dim,hq,dtype", [(128, 32, torch.bfloat16), (64, 16, torch.float16), (128, 128, torch.bfloat16)])
+def test_decode_kernel_at_tile_edges(page, head_dim, hq, dtype):
+    """One token per request: lengths around the 16-key piece, the 64-key tile, the stage ring and 32 tiles,
+    with NaN in every cache slot past the sequence; each rank count against the float reference."""
+    from fxpr_vllm import synthetic as syn
+
+    sls = [1, 15, 16, 17, 63, 64, 65, 128, 193, 257, 2047, 2049, 2113]
+    q, kv, qsl, sl, bt = syn.paged_attention_inputs(sls, [1] * len(sls), q_heads=hq, kv_heads=8, head_dim=head_dim,
+                                                    page=page, dtype=dtype, seed=5)
+    for i, n in enumerate(sls):                       # the tail of a sequence's last page
+        if n % page:
+            kv[bt[i, n // page].item(), :, n % page:] = float("nan")
+    exp = _float_attention(q.cpu(), kv.cpu().nan_to_num(), qsl.cpu(), sl.cpu(), bt.cpu())
+    outs = []
+    for splits in (1, 2, 8, 16):
+        o = torch.full_like(q, float("nan"))
+        torch.ops.fxpr.unified_attention_fxp(q, kv, o, qsl, sl, bt, 1, None, True, None, 64, 16, 0.0, 0, splits)
+        outs.append(o)
+    L.check_device_status()
+    tol = 2.0 ** -6 if dtype == torch.bfloat16 else 2.0 ** -8
+    assert (outs[0].float().cpu() - exp).abs().max().item() <= tol * max(1.0, float(exp.abs().max()))
+    for o in outs[1:]:
+        assert torch.equal(o.view(torch.int16), outs[0].view(torch.int16))
+
+
 @pytest.mark.parametrize("case", [
     # (seq_lens, q_lens, q heads, kv heads, page, dtype, int_bits, extra arguments)
     ([80, 33], [80, 33], 32, 8, 16, torch.bfloat16, 64, {}),
@@ -247,6 +273,10 @@ def test_tensor_core_route_feature_flags_close_to_oracle(dtype, kwargs, splits):
     ([2100], [2100], 32, 8, 16, torch.bfloat16, 64, {}),
     ([700, 90], [700, 90], 32, 8, 64, torch.bfloat16, 64, {}),                # 64-token pages: one box per tile
     ([700, 90], [300, 90], 32, 8, 128, torch.float16, 32, {}),
+    # one key, and lengths one short of, at and one past the 16-slot piece, the key tile and the score step
+    ([1, 15, 16, 17, 63, 64, 65, 127, 128, 129], [1, 15, 16, 17, 63, 64, 65, 127, 128, 129], 32, 8, 16, torch.bfloat16, 64, {}),
+    ([192, 193, 255, 257], [192, 1, 64, 257], 16, 1, 48, torch.float16, 32, {}),
+    ([385] * 24, [385] * 24, 32, 8, 16, torch.bfloat16, 64, {}),              # several items per CTA, odd tile counts
 ])
 def test_tcgen05_prefill_kernel_equals_mma_sync_kernel(case):
     """The tcgen05 / tensor-memory prefill kernel against the mma.sync kernel it replaces: a

@@ -359,6 +359,26 @@ def test_two_sm_kernel_agrees_on_random_shapes():
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (256, 256, 128), (255, 248, 136), (257, 264, 64), (512, 512, 72), (65, 256, 8), (1025, 2056, 200),
+])
+@pytest.mark.parametrize("kt", [64, 128])
+def test_two_sm_kernel_at_tile_edges(M, N, K, kt):
+    """256 x 256 pair tiles one short of, at and one past their edges; K of one, several and ragged tiles."""
+    from fxpr_vllm import _native as nat
+
+    a = _rand((M, K), torch.bfloat16, M).cuda()
+    b = _rand((K, N), torch.bfloat16, N, 0.05).cuda()
+    a[M - 1, -1] = 2.0e4                              # a partial of the last row leaves the fast range
+    out = []
+    for flags in (nat.GEMM_PAIR, nat.GEMM_FORCE_EXACT_TC):
+        with L.overrides(gemm_k_tile=kt, gemm_split_k=1, gemm_flags=flags):
+            out.append((torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16), _gemm(a, b, None, 32, 16)))
+    assert torch.equal(out[0][0], out[1][0])
+    assert torch.equal(out[0][1].view(torch.int16), out[1][1].view(torch.int16))
+    L.check_device_status()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,f,K", [(64, 1792, 1024), (33, 200, 512), (1, 128, 256), (64, 4096, 2048)])
 @pytest.mark.parametrize("split", [0, 1, 2, 3, 4])
