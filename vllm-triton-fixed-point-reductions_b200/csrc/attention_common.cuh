@@ -1,6 +1,7 @@
 // Launch parameters shared by the attention kernels and their dispatcher.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -46,5 +47,6 @@ bool attention_mma_supported(const AttnParams& p, int dtype);
 // tcgen05 / TMEM / TMA prefill kernel (attention_tc.cu)
 bool attention_tc_supported(const AttnParams& p, int dtype, int max_query_len, bool force_exact);
 int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* status, cudaStream_t s);
+bool attn_kv_map(CUtensorMap* m, const AttnParams& p, int dtype, const void* plane, int box_rows);
 
 }  // namespace fxpr

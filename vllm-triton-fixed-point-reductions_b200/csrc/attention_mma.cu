@@ -24,6 +24,7 @@
 
 #include "attention_common.cuh"
 #include "fxp_common.cuh"
+#include "gemm_tc_fast_common.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -127,19 +128,24 @@ static int launch_mma(const AttnParams& p, const MmaAttnShape& sh, cudaStream_t 
 }
 
 template <typename T, int HD, int NW, bool ACC64, bool ROWS8, int NSTAGE = 2, int MINB = 4>
-static int launch_decode(const AttnParams& p, const MmaAttnShape& sh, cudaStream_t s) {
+static int launch_decode(const AttnParams& p, const MmaAttnShape& sh, int dtype, cudaStream_t s) {
   constexpr int kTileBytes = kTileN * HD * 2;
+  CUtensorMap mk, mv;
+  if (!attn_kv_map(&mk, p, dtype, p.k, 16) || !attn_kv_map(&mv, p, dtype, p.v, 16)) {
+    set_last_error("cuTensorMapEncodeTiled(KV)", cudaErrorInvalidValue);
+    return FXPR_ERR_CUDA;
+  }
   const size_t smem = (size_t)(ROWS8 ? 8 : 16) * HD * 2 + NSTAGE * (size_t)kTileBytes + NW * 16 * 4 + NW * 16 * 8 +
-                      (size_t)sh.stash_keys * stash_bytes_per_key(sh.stash_rows);
+                      8 * (NSTAGE * (NW + 2) + 2) + (size_t)sh.stash_keys * stash_bytes_per_key(sh.stash_rows);
   auto k = attn_decode_kernel<T, HD, NW, ACC64, ROWS8, NSTAGE, MINB>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
   if (e != cudaSuccess) { set_last_error("attention_decode smem attribute", e); return FXPR_ERR_CUDA; }
   if (p.num_splits > 8) {
     e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) { set_last_error("attention_decode cluster attribute", e); return FXPR_ERR_CUDA; }
   }
   e = launch_pdl(k, dim3((unsigned)p.num_splits, (unsigned)(sh.num_q_blocks * p.num_kv_heads), (unsigned)p.num_reqs),
-                 dim3(NW * 32), smem, s, (unsigned)p.num_splits, p, sh);
+                 dim3(NW * 32), smem, s, (unsigned)p.num_splits, mk, mv, p, sh);
   if (e != cudaSuccess) { set_last_error("attention_decode launch", e); return FXPR_ERR_CUDA; }
   return check_launch("attention_decode");
 }
@@ -181,7 +187,9 @@ int attention_mma(const AttnParams& p_in, int dtype, int max_query_len, bool for
   const int64_t tiles = (max_keys + kTileN - 1) / kTileN;
   const int64_t per_rank = (tiles + p.num_splits - 1) / p.num_splits;
   sh.stash_keys = (int)(per_rank * kTileN);
-  const bool stash = small && (int64_t)sh.stash_keys * stash_bytes_per_key(sh.stash_rows) <= 150 * 1024;
+  // the decode kernel fetches page pieces through tensor maps over the cache planes
+  const bool mappable = p.kv_shead % 64 == 0 && p.kv_sblock < (1ll << 35) && p.kv_sslot > 0 && p.kv_sblock > 0;
+  const bool stash = small && mappable && (int64_t)sh.stash_keys * stash_bytes_per_key(sh.stash_rows) <= 150 * 1024;
   if (!stash) sh.stash_keys = 0;
   const bool acc64 = p.int_bits == 64;
   // fast second pass (same bits): scale <= 2^16, 32- or 64-bit sums, bounded tiles per CTA
@@ -191,10 +199,10 @@ int attention_mma(const AttnParams& p_in, int dtype, int max_query_len, bool for
 #define FXPR_ATTN(TT, HDV)                                                                      \
   do {                                                                                          \
     if (small && stash && sh.stash_rows <= 8)                                                   \
-      return acc64 ? launch_decode<TT, HDV, 4, true, true>(p, sh, s)                     \
-                   : launch_decode<TT, HDV, 4, false, true>(p, sh, s);                   \
-    if (small && stash) return acc64 ? launch_decode<TT, HDV, 4, true, false>(p, sh, s)  \
-                                     : launch_decode<TT, HDV, 4, false, false>(p, sh, s);\
+      return acc64 ? launch_decode<TT, HDV, 4, true, true>(p, sh, dtype, s)                     \
+                   : launch_decode<TT, HDV, 4, false, true>(p, sh, dtype, s);                   \
+    if (small && stash) return acc64 ? launch_decode<TT, HDV, 4, true, false>(p, sh, dtype, s)  \
+                                     : launch_decode<TT, HDV, 4, false, false>(p, sh, dtype, s);\
     if (small) return acc64 ? launch_mma<TT, HDV, 1, false, true>(p, sh, s)                     \
                             : launch_mma<TT, HDV, 1, false, false>(p, sh, s);                   \
     if (fast) return launch_mma<TT, HDV, 4, false, false, true>(p, sh, s);                      \

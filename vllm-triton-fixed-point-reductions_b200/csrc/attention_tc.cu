@@ -76,15 +76,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       "[%0], [%1, {%3, %4, %5}], [%2];\n\t}"
       ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(elected) : "memory");
 }
-__device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z,
-                                            int w, int v, uint32_t elected) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %8, 0;\n\t"
-      "@q cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];\n\t}"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w), "r"(v), "r"(elected) : "memory");
-}
 // generic-proxy writes to shared memory become visible to the tensor core (async proxy)
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -696,6 +687,22 @@ static EncodeTiledFnA encode_fn() {
   return fn;
 }
 
+// A plane of the paged cache as [blocks, 8-slot groups, 64-dim chunks (of all heads), 8 slots, 64 dims],
+// boxes of box_rows slots x one head: [8-row group][chunk][8 rows][128 B] in shared memory, 128-byte
+// swizzle.  The number of blocks is not known here and only bounds the coordinates, which come from the
+// block table.
+bool attn_kv_map(CUtensorMap* m, const AttnParams& p, int dtype, const void* plane, int box_rows) {
+  EncodeTiledFnA fn = encode_fn();
+  if (!fn || p.kv_shead % 64 != 0 || p.head_dim % 64 != 0) return false;
+  cuuint64_t dims[5] = {64, 8, (cuuint64_t)((p.num_kv_heads - 1) * (p.kv_shead / 64) + p.head_dim / 64),
+                        (cuuint64_t)(p.page_size / 8), (cuuint64_t)1 << 31};
+  cuuint64_t strides[4] = {(cuuint64_t)p.kv_sslot * 2, 128, (cuuint64_t)p.kv_sslot * 16, (cuuint64_t)p.kv_sblock * 2};
+  cuuint32_t box[5] = {64, 8, (cuuint32_t)(p.head_dim / 64), (cuuint32_t)(box_rows / 8), 1}, es[5] = {1, 1, 1, 1, 1};
+  return fn(m, dtype == FXPR_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5,
+            const_cast<void*>(plane), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // The prefill kernel takes head size 128, bf16/fp16, 32- or 64-bit sums with at most 16
 // fraction bits, no KV split, a sequence short enough for the 32-bit fast sums, and strides
 // a tensor map can express (multiples of 16 bytes, below 2^40).
@@ -749,21 +756,10 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
       return FXPR_ERR_CUDA;
     }
   }
-  // Cache planes [blocks, 8-slot groups, 64-dim chunks (heads and halves), slots, dims]: see the
-  // producers.  The number of blocks is not known here and only bounds the coordinates, which come from
-  // the block table.
   sh.head_chunks = (int)(p.kv_shead / 64);
-  for (int which = 0; which < 2; ++which) {
-    cuuint64_t dims[5] = {64, 8, (cuuint64_t)((p.num_kv_heads - 1) * (p.kv_shead / 64) + 2), (cuuint64_t)(p.page_size / 8),
-                          (cuuint64_t)1 << 31};
-    cuuint64_t strides[4] = {(cuuint64_t)p.kv_sslot * 2, 128, (cuuint64_t)p.kv_sslot * 16, (cuuint64_t)p.kv_sblock * 2};
-    cuuint32_t box[5] = {64, 8, 2, 1u << (sh.group_shift - 3), 1}, es[5] = {1, 1, 1, 1, 1};
-    if (fn(which ? &mv : &mk, dt, 5, const_cast<void*>(which ? p.v : p.k), dims, strides, box, es,
-           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
-      set_last_error("cuTensorMapEncodeTiled(KV)", cudaErrorInvalidValue);
-      return FXPR_ERR_CUDA;
-    }
+  if (!attn_kv_map(&mk, p, dtype, p.k, 1 << sh.group_shift) || !attn_kv_map(&mv, p, dtype, p.v, 1 << sh.group_shift)) {
+    set_last_error("cuTensorMapEncodeTiled(KV)", cudaErrorInvalidValue);
+    return FXPR_ERR_CUDA;
   }
 
   constexpr int kSmem = kTcRows * 128 * 2 + kTcStages * 2 * kTcTileN * 128 * 2 + 2 * kTcRows * kTcTileN * 2 +
