@@ -49,6 +49,21 @@ def test_portable_bit_exact(dtype, M, N, K, int_bits):
     assert torch.equal(got.view(torch.uint8), exp.view(torch.uint8))
 
 
+@pytest.mark.parametrize("M,N,K,kt", [
+    (1, 64, 17, 128), (16, 65, 300, 16), (17, 63, 129, 128), (64, 200, 520, 24), (65, 130, 260, 64), (129, 9600, 40, 64),
+])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_portable_kernel_at_tile_edges(M, N, K, kt, transposed):
+    """Row tiles of 16, 64 and 128, K-tiles dealt to 1 to 8 cluster ranks, ragged chunks, both stride orders."""
+    a = _rand((M, K), torch.float32, M, 0.5)
+    b = _rand((K, N), torch.float32, N, 0.5)
+    ga, gb = (a.t().contiguous().cuda().t(), b.t().contiguous().cuda().t()) if transposed else (a.cuda(), b.cuda())
+    with L.overrides(gemm_portable=True, gemm_k_tile=kt):
+        got = torch.ops.fxpr.gemm_fxp_int(ga, gb, 64, 16).cpu()
+    exp = orc.gemm_fxp(a, b, None, 64, 16, sequential=True, return_int=True, k_tile=kt)
+    assert torch.equal(got.to(torch.int64), exp)
+
+
 def test_portable_strided_operands():
     a = _rand((40, 96), torch.float32, 4)
     w = _rand((24, 96), torch.float32, 5)  # (N, K) weight viewed as (K, N)

@@ -11,96 +11,173 @@
 // multiply and add (bit-reproducible on a CPU), quantised with float_to_fixed and
 // added as an integer; the epilogue converts once, adds the bias in fp32 and
 // rounds to the IO dtype.  The K tail is zero padding (adds nothing).
+//
+// Bound: multiplies and adds are separate instructions, so half the FFMA rate, for large M; reading B for
+// small M.  A thread holds RM x 4 outputs (three 16-byte shared-memory reads per 64 instructions at
+// RM = 8), the next chunk of K travels to registers while this one is multiplied, both operands are
+// read along whichever of their strides is one, and K-tiles are dealt to the ranks of a cluster when
+// the tiles of the output leave the GPU idle (integer sums: no bit depends on it).
+#include <algorithm>
+
+#include <cooperative_groups.h>
+
 #include "fxp_common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace fxpr {
 
-static constexpr int kPT = 64;   // output tile edge
+static constexpr int kPN = 64;   // output columns per CTA
 static constexpr int kPK = 16;   // k chunk staged in shared memory
 
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <int RM>
+constexpr int portable_smem() { return 2 * kPK * (16 * RM + 4 + kPN + 4) * 4 + 16 * RM * kPN * 8; }
+constexpr int portable_ctas(int rm) { return rm == 8 ? 2 : rm == 4 ? 3 : 4; }   // resident per SM
+
+template <typename T, int RM>
+__global__ void __launch_bounds__(256, portable_ctas(RM))
 gemm_portable_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ bias,
                      T* __restrict__ c, void* __restrict__ c_int, float* __restrict__ partials,
                      int M, int N, int K, int64_t a_sm, int64_t a_sk, int64_t b_sk, int64_t b_sn,
-                     int64_t c_sm, int int_bits, float scale, float inv_scale, int k_tile) {
-  __shared__ float sa[kPK][kPT + 1];
-  __shared__ float sb[kPK][kPT + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * kPT, n0 = blockIdx.x * kPT;
-  long long acc[4][4];
+                     int64_t c_sm, int int_bits, float scale, float inv_scale, int k_tile, int splits, float zero /* 0 */) {
+  constexpr int TM = 16 * RM, LA = TM + 4, LB = kPN + 4;
+  extern __shared__ __align__(16) uint8_t smem[];
+  float* sa = reinterpret_cast<float*>(smem);        // [2][kPK][LA]
+  float* sb = sa + 2 * kPK * LA;                      // [2][kPK][LB]
+  // Integer sums, touched once per K-tile, each by the thread that owns it: [RM * 4][256].  In registers
+  // they would leave one CTA per SM at RM = 8.
+  long long* acc = reinterpret_cast<long long*>(sb + 2 * kPK * LB);
+  pdl_wait();
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int rank = blockIdx.x % splits;
+  const int m0 = blockIdx.y * TM, n0 = (blockIdx.x / splits) * kPN;
+  const bool a_along_k = a_sk == 1, b_along_n = b_sn == 1;
+  uint64_t p[RM][2];                                 // pairs of neighbouring columns
+  const uint64_t zero2 = f2_pack(zero, zero);
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+    for (int j = 0; j < 4; ++j) { acc[(i * 4 + j) * 256 + tid] = 0; p[i][j >> 1] = 0; }
 
   const int tiles = (K + k_tile - 1) / k_tile;
-  for (int t = 0; t < tiles; ++t) {
-    float p[4][4];
+  // element `it` of this thread's share of a chunk: its place in the A and in the B chunk
+  auto a_place = [&](int it, int& kk, int& mm) {
+    const int idx = tid + it * 256;
+    if (a_along_k) { kk = idx & (kPK - 1); mm = idx / kPK; } else { mm = idx % TM; kk = idx / TM; }
+  };
+  auto b_place = [&](int it, int& kk, int& nn) {
+    const int idx = tid + it * 256;
+    if (b_along_n) { nn = idx & (kPN - 1); kk = idx / kPN; } else { kk = idx & (kPK - 1); nn = idx / kPK; }
+  };
+  float ra[RM], rb[4];
+  auto fetch = [&](int kc, int kn) {                 // what lies outside is zero and adds nothing
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) p[i][j] = 0.0f;
-    const int k_lo = t * k_tile, k_hi = min(K, k_lo + k_tile);
-    for (int kc = k_lo; kc < k_hi; kc += kPK) {
-      const int kn = min(kPK, k_hi - kc);
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < kPK * kPT; idx += 256) {
-        const int kk = idx / kPT, mm = idx % kPT;  // A: consecutive threads walk m
-        float v = 0.0f;
-        if (kk < kn && m0 + mm < M) v = to_f32<T>(a[(int64_t)(m0 + mm) * a_sm + (int64_t)(kc + kk) * a_sk]);
-        sa[kk][mm] = v;
-      }
-      for (int idx = threadIdx.x; idx < kPK * kPT; idx += 256) {
-        const int kk = idx / kPT, nn = idx % kPT;  // B: consecutive threads walk n
-        float v = 0.0f;
-        if (kk < kn && n0 + nn < N) v = to_f32<T>(b[(int64_t)(kc + kk) * b_sk + (int64_t)(n0 + nn) * b_sn]);
-        sb[kk][nn] = v;
-      }
-      __syncthreads();
-      for (int kk = 0; kk < kn; ++kk) {
-        float av[4], bv[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) av[i] = sa[kk][ty + 16 * i];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bv[j] = sb[kk][tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) p[i][j] = __fadd_rn(p[i][j], __fmul_rn(av[i], bv[j]));
-      }
+    for (int it = 0; it < RM; ++it) {
+      int kk, mm;
+      a_place(it, kk, mm);
+      ra[it] = (kk < kn && m0 + mm < M) ? to_f32<T>(a[(int64_t)(m0 + mm) * a_sm + (int64_t)(kc + kk) * a_sk]) : 0.0f;
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int it = 0; it < 4; ++it) {
+      int kk, nn;
+      b_place(it, kk, nn);
+      rb[it] = (kk < kn && n0 + nn < N) ? to_f32<T>(b[(int64_t)(kc + kk) * b_sk + (int64_t)(n0 + nn) * b_sn]) : 0.0f;
+    }
+  };
+  auto k_end = [&](int t) { return (int)min((int64_t)K, (int64_t)(t + 1) * k_tile); };
+
+  int t = rank, kc = rank * k_tile, buf = 0;
+  if (t < tiles) fetch(kc, k_end(t) - kc);
+  while (t < tiles) {
+    float* ca = sa + buf * kPK * LA;
+    float* cb = sb + buf * kPK * LB;
+    buf ^= 1;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        acc[i][j] += float_to_fixed_any(p[i][j], scale, int_bits);
-        if (partials) {
-          const int m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
-          if (m < M && n < N) partials[((int64_t)t * M + m) * N + n] = p[i][j];
+    for (int it = 0; it < RM; ++it) { int kk, mm; a_place(it, kk, mm); ca[kk * LA + mm] = ra[it]; }
+#pragma unroll
+    for (int it = 0; it < 4; ++it) { int kk, nn; b_place(it, kk, nn); cb[kk * LB + nn] = rb[it]; }
+    __syncthreads();                                 // this chunk is in place, the one before last is free
+    const int t_now = t;
+    kc += kPK;
+    const bool tile_done = kc >= k_end(t);
+    if (tile_done) { t += splits; kc = t < tiles ? t * k_tile : 0; }
+    if (t < tiles) fetch(kc, k_end(t) - kc);
+#pragma unroll
+    for (int kk = 0; kk < kPK; ++kk) {
+      float av[RM];
+      if constexpr (RM >= 4) {
+#pragma unroll
+        for (int i = 0; i < RM; i += 4) *reinterpret_cast<float4*>(av + i) = *reinterpret_cast<const float4*>(ca + kk * LA + ty * RM + i);
+      } else {
+#pragma unroll
+        for (int i = 0; i < RM; ++i) av[i] = ca[kk * LA + ty * RM + i];
+      }
+      const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(cb + kk * LB + tx * 4);
+      // Two columns per instruction.  The product is an fma with a run-time zero: ptxas contracts a packed
+      // multiply and the add behind it, which would round once instead of twice.
+#pragma unroll
+      for (int i = 0; i < RM; ++i) {
+        const uint64_t a2 = f2_pack(av[i], av[i]);
+        p[i][0] = f2_add(p[i][0], f2_fma(a2, bv.x, zero2));
+        p[i][1] = f2_add(p[i][1], f2_fma(a2, bv.y, zero2));
+      }
+    }
+    if (tile_done) {
+#pragma unroll
+      for (int i = 0; i < RM; ++i) {
+        float v[4];
+        f2_unpack(p[i][0], v[0], v[1]);
+        f2_unpack(p[i][1], v[2], v[3]);
+        p[i][0] = p[i][1] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          acc[(i * 4 + j) * 256 + tid] += float_to_fixed_any(v[j], scale, int_bits);
+          if (partials) {
+            const int m = m0 + ty * RM + i, n = n0 + tx * 4 + j;
+            if (m < M && n < N) partials[((int64_t)t_now * M + m) * N + n] = v[j];
+          }
         }
       }
+    }
   }
 
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
-      if (m >= M || n >= N) continue;
-      const long long q = wrap_to_bits(acc[i][j], int_bits);
-      if (c_int) {
-        const int64_t o = (int64_t)m * N + n;
-        if (int_bits == 64) ((long long*)c_int)[o] = q;
-        else if (int_bits == 32) ((int32_t*)c_int)[o] = (int32_t)q;
-        else ((int16_t*)c_int)[o] = (int16_t)q;
-      }
-      if (c) {
-        float v = fixed_to_float<long long>(q, inv_scale);
-        if (bias) v = __fadd_rn(v, to_f32<T>(bias[n]));
-        c[(int64_t)m * c_sm + n] = from_f32<T>(v);
-      }
+  auto write = [&](int m, int n, long long sum) {
+    const long long q = wrap_to_bits(sum, int_bits);
+    if (c_int) {
+      const int64_t o = (int64_t)m * N + n;
+      if (int_bits == 64) ((long long*)c_int)[o] = q;
+      else if (int_bits == 32) ((int32_t*)c_int)[o] = (int32_t)q;
+      else ((int16_t*)c_int)[o] = (int16_t)q;
     }
+    if (c) {
+      float v = fixed_to_float<long long>(q, inv_scale);
+      if (bias) v = __fadd_rn(v, to_f32<T>(bias[n]));
+      c[(int64_t)m * c_sm + n] = from_f32<T>(v);
+    }
+  };
+  // where the idx-th sum of a CTA belongs
+  auto place = [&](int idx, int& m, int& n) {
+    m = m0 + ((idx & 255) >> 4) * RM + (idx >> 10);
+    n = n0 + (idx & 15) * 4 + ((idx >> 8) & 3);
+    return m < M && n < N;
+  };
+  if (splits == 1) {
+    for (int idx = tid; idx < TM * kPN; idx += 256) {
+      int m, n;
+      if (place(idx, m, n)) write(m, n, acc[idx]);
+    }
+    return;
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  for (int idx = rank * 256 + tid; idx < TM * kPN; idx += splits * 256) {
+    int m, n;
+    if (!place(idx, m, n)) continue;
+    long long sum = 0;
+    for (int r = 0; r < splits; ++r) sum += cluster.map_shared_rank(acc, r)[idx];
+    write(m, n, sum);
+  }
+  cluster.sync();                                    // peers may still be reading this CTA's sums
 }
 
 // c = T(fp32(c_int) * 2^-frac + bias)
@@ -124,11 +201,41 @@ int gemm_portable_launch(const void* a, const void* b, const void* bias, void* c
                          int64_t a_sk, int64_t b_sk, int64_t b_sn, int64_t c_sm, int int_bits,
                          int frac_bits, int k_tile, cudaStream_t s) {
   const float scale = (float)(1ull << frac_bits);
-  dim3 grid((unsigned)ceil_div_i(N, kPT), (unsigned)ceil_div_i(M, kPT));
-  gemm_portable_kernel<T><<<grid, 256, 0, s>>>((const T*)a, (const T*)b, (const T*)bias, (T*)c, c_int,
-                                             partials, (int)M, (int)N, (int)K, a_sm, a_sk, b_sk,
-                                             b_sn, c_sm, int_bits, scale, 1.0f / scale, k_tile);
-  return check_launch("gemm_portable");
+  // Rows per CTA: 16 when that covers M.  Otherwise 64 or 128 (whose products cost a sixth less), and for
+  // every choice 1 to 8 cluster ranks that share the K-tiles: whichever gives the shortest rounds, counted
+  // in rows of work per SM.  A doubling of the ranks costs about 3 % (the merge).
+  const int64_t tiles_n = ceil_div_i(N, kPN);
+  int rm = 1, splits = 1;
+  double best = 1e300;
+  for (int r : {1, 4, 8}) {
+    if ((r == 1) != (M <= 16)) continue;
+    const int64_t ctas = tiles_n * ceil_div_i(M, 16 * r);
+    double fee = r == 4 ? 1.17 : 1.0;
+    for (int n = 1; n <= 8 && n <= std::max(1, ceil_div_i(K, k_tile)); n *= 2, fee *= 1.03) {
+      const int per_sm = portable_ctas(r);
+      const int64_t whole = ctas * n / (148 * per_sm), rest = ctas * n % (148 * per_sm);
+      // a last round of fewer CTAs per SM is shorter, but never as short as its share
+      const double rounds = (double)whole * per_sm + (rest ? std::max(0.6 * per_sm, (double)((rest + 147) / 148)) : 0.0);
+      const double cost = rounds * r / n * fee;
+      if (cost < best) { best = cost; rm = r; splits = n; }
+    }
+  }
+  const int64_t tiles_m = ceil_div_i(M, 16 * rm);
+  auto launch = [&](auto kernel, int smem) {
+    if (smem > 48 * 1024) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (e != cudaSuccess) { set_last_error("gemm_portable smem attribute", e); return (int)FXPR_ERR_CUDA; }
+    }
+    const cudaError_t e = launch_pdl(kernel, dim3((unsigned)(tiles_n * splits), (unsigned)tiles_m), dim3(256), smem, s,
+                                     (unsigned)splits, (const T*)a, (const T*)b, (const T*)bias, (T*)c, c_int, partials,
+                                     (int)M, (int)N, (int)K, a_sm, a_sk, b_sk, b_sn, c_sm, int_bits, scale, 1.0f / scale,
+                                     k_tile, splits, 0.0f);
+    if (e != cudaSuccess) { set_last_error("gemm_portable launch", e); return (int)FXPR_ERR_CUDA; }
+    return check_launch("gemm_portable");
+  };
+  if (rm == 1) return launch(gemm_portable_kernel<T, 1>, portable_smem<1>());
+  if (rm == 4) return launch(gemm_portable_kernel<T, 4>, portable_smem<4>());
+  return launch(gemm_portable_kernel<T, 8>, portable_smem<8>());
 }
 
 int gemm_portable(const void* a, const void* b, const void* bias, void* c, void* c_int,
