@@ -34,6 +34,23 @@ template <int RM>
 constexpr int portable_smem() { return 2 * kPK * (16 * RM + 4 + kPN + 4) * 4 + 16 * RM * kPN * 8; }
 constexpr int portable_ctas(int rm) { return rm == 8 ? 2 : rm == 4 ? 3 : 4; }   // resident per SM
 
+template <typename T>
+__device__ __forceinline__ void portable_write(int m, int n, long long sum, const T* bias, T* c, void* c_int, int N,
+                                               int64_t c_sm, int int_bits, float inv_scale) {
+  const long long q = wrap_to_bits(sum, int_bits);
+  if (c_int) {
+    const int64_t o = (int64_t)m * N + n;
+    if (int_bits == 64) ((long long*)c_int)[o] = q;
+    else if (int_bits == 32) ((int32_t*)c_int)[o] = (int32_t)q;
+    else ((int16_t*)c_int)[o] = (int16_t)q;
+  }
+  if (c) {
+    float v = fixed_to_float<long long>(q, inv_scale);
+    if (bias) v = __fadd_rn(v, to_f32<T>(bias[n]));
+    c[(int64_t)m * c_sm + n] = from_f32<T>(v);
+  }
+}
+
 template <typename T, int RM>
 __global__ void __launch_bounds__(256, portable_ctas(RM))
 gemm_portable_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ bias,
@@ -141,20 +158,6 @@ gemm_portable_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* 
     }
   }
 
-  auto write = [&](int m, int n, long long sum) {
-    const long long q = wrap_to_bits(sum, int_bits);
-    if (c_int) {
-      const int64_t o = (int64_t)m * N + n;
-      if (int_bits == 64) ((long long*)c_int)[o] = q;
-      else if (int_bits == 32) ((int32_t*)c_int)[o] = (int32_t)q;
-      else ((int16_t*)c_int)[o] = (int16_t)q;
-    }
-    if (c) {
-      float v = fixed_to_float<long long>(q, inv_scale);
-      if (bias) v = __fadd_rn(v, to_f32<T>(bias[n]));
-      c[(int64_t)m * c_sm + n] = from_f32<T>(v);
-    }
-  };
   // where the idx-th sum of a CTA belongs
   auto place = [&](int idx, int& m, int& n) {
     m = m0 + ((idx & 255) >> 4) * RM + (idx >> 10);
@@ -164,7 +167,7 @@ gemm_portable_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* 
   if (splits == 1) {
     for (int idx = tid; idx < TM * kPN; idx += 256) {
       int m, n;
-      if (place(idx, m, n)) write(m, n, acc[idx]);
+      if (place(idx, m, n)) portable_write(m, n, acc[idx], bias, c, c_int, N, c_sm, int_bits, inv_scale);
     }
     return;
   }
@@ -175,9 +178,98 @@ gemm_portable_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* 
     if (!place(idx, m, n)) continue;
     long long sum = 0;
     for (int r = 0; r < splits; ++r) sum += cluster.map_shared_rank(acc, r)[idx];
-    write(m, n, sum);
+    portable_write(m, n, sum, bias, c, c_int, N, c_sm, int_bits, inv_scale);
   }
   cluster.sync();                                    // peers may still be reading this CTA's sums
+}
+
+// At most 16 rows: bound by reading B, which here goes straight to registers, once, 16 bytes per lane and
+// eight rows of K at a time.  K-tiles are independent up to their integer sums, so every warp of a CTA (and
+// of the cluster) takes its own: a warp is 128 columns x R rows of one K-tile.  fp32, K-tile 128:
+// 8x28672x4096 453 -> see the table of gemm_portable_kernel's figures beside the launch rule.
+template <typename T, int R>
+__global__ void __launch_bounds__(256, 2)
+gemm_portable_rows_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ bias,
+                          T* __restrict__ c, void* __restrict__ c_int, float* __restrict__ partials,
+                          int M, int N, int K, int64_t a_sm, int64_t a_sk, int64_t b_sk,
+                          int64_t c_sm, int int_bits, float scale, float inv_scale, int k_tile, int splits,
+                          float zero /* 0 */) {
+  struct alignas(4 * sizeof(T)) Vec { T v[4]; };
+  __shared__ __align__(16) float sa[8][32][R + 4];   // a warp's slice of A, k-major
+  __shared__ unsigned long long acc[R * 128];
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = blockIdx.x % splits, n0 = (blockIdx.x / splits) * 128;
+  const int n = n0 + lane * 4;
+  for (int i = tid; i < R * 128; i += 256) acc[i] = 0;
+  __syncthreads();
+  const uint64_t zero2 = f2_pack(zero, zero);
+  const int tiles = (K + k_tile - 1) / k_tile;
+  for (int t = rank * 8 + warp; t < tiles; t += splits * 8) {
+    uint64_t p[R][2];
+#pragma unroll
+    for (int i = 0; i < R; ++i) p[i][0] = p[i][1] = 0;
+    const int k_hi = (int)min((int64_t)K, (int64_t)(t + 1) * k_tile);
+    for (int kc = t * k_tile; kc < k_hi; kc += 32) {
+      __syncwarp();
+#pragma unroll
+      for (int m = 0; m < R; ++m)
+        sa[warp][lane][m] = (m < M && kc + lane < k_hi) ? to_f32<T>(a[(int64_t)m * a_sm + (int64_t)(kc + lane) * a_sk]) : 0.0f;
+      __syncwarp();
+#pragma unroll 1
+      for (int k8 = 0; k8 < 32 && kc + k8 < k_hi; k8 += 8) {
+        Vec bv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int k = kc + k8 + u;
+          if (k < k_hi && n < N) bv[u] = *reinterpret_cast<const Vec*>(b + (int64_t)k * b_sk + n);
+          else bv[u] = Vec{};
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const uint64_t b01 = f2_pack(to_f32<T>(bv[u].v[0]), to_f32<T>(bv[u].v[1]));
+          const uint64_t b23 = f2_pack(to_f32<T>(bv[u].v[2]), to_f32<T>(bv[u].v[3]));
+#pragma unroll
+          for (int m4 = 0; m4 < R; m4 += 4) {
+            const float4 av = *reinterpret_cast<const float4*>(&sa[warp][k8 + u][m4]);
+            const float am[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint64_t a2 = f2_pack(am[i], am[i]);
+              p[m4 + i][0] = f2_add(p[m4 + i][0], f2_fma(a2, b01, zero2));
+              p[m4 + i][1] = f2_add(p[m4 + i][1], f2_fma(a2, b23, zero2));
+            }
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < R; ++m) {
+      if (m >= M || n >= N) continue;
+      float v[4];
+      f2_unpack(p[m][0], v[0], v[1]);
+      f2_unpack(p[m][1], v[2], v[3]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        atomicAdd(&acc[m * 128 + lane * 4 + j], (unsigned long long)float_to_fixed_any(v[j], scale, int_bits));
+        if (partials) partials[((int64_t)t * M + m) * N + n + j] = v[j];
+      }
+    }
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  if (splits > 1) cluster.sync(); else __syncthreads();
+  for (int idx = rank * 256 + tid; idx < R * 128; idx += splits * 256) {
+    const int m = idx >> 7, col = n0 + (idx & 127);
+    if (m >= M || col >= N) continue;
+    long long sum = 0;
+    if (splits > 1) {
+      for (int r = 0; r < splits; ++r) sum += (long long)cluster.map_shared_rank(acc, r)[idx];
+    } else {
+      sum = (long long)acc[idx];
+    }
+    portable_write(m, col, sum, bias, c, c_int, N, c_sm, int_bits, inv_scale);
+  }
+  if (splits > 1) cluster.sync();                    // peers may still be reading this CTA's sums
 }
 
 // c = T(fp32(c_int) * 2^-frac + bias)
@@ -201,6 +293,21 @@ int gemm_portable_launch(const void* a, const void* b, const void* bias, void* c
                          int64_t a_sk, int64_t b_sk, int64_t b_sn, int64_t c_sm, int int_bits,
                          int frac_bits, int k_tile, cudaStream_t s) {
   const float scale = (float)(1ull << frac_bits);
+  // Few rows, B readable 4 columns at a time and K-tiles for the eight warps of a CTA: one K-tile per warp.
+  const int k_tiles = ceil_div_i(K, k_tile);
+  if (M <= 16 && k_tiles >= 8 && b_sn == 1 && b_sk % 4 == 0 && N % 4 == 0 && ((uintptr_t)b % (4 * sizeof(T))) == 0) {
+    const int64_t cols = ceil_div_i(N, 128);
+    int splits = 1;
+    while (splits < 8 && splits * 8 < k_tiles && cols * splits * 2 <= 4 * 148) splits *= 2;
+    auto rows = [&](auto kernel) {
+      const cudaError_t e = launch_pdl(kernel, dim3((unsigned)(cols * splits)), dim3(256), 0, s, (unsigned)splits,
+                                       (const T*)a, (const T*)b, (const T*)bias, (T*)c, c_int, partials, (int)M, (int)N,
+                                       (int)K, a_sm, a_sk, b_sk, c_sm, int_bits, scale, 1.0f / scale, k_tile, splits, 0.0f);
+      if (e != cudaSuccess) { set_last_error("gemm_portable launch", e); return (int)FXPR_ERR_CUDA; }
+      return check_launch("gemm_portable");
+    };
+    return M <= 8 ? rows(gemm_portable_rows_kernel<T, 8>) : rows(gemm_portable_rows_kernel<T, 16>);
+  }
   // Rows per CTA: 16 when that covers M.  Otherwise 64 or 128 (whose products cost a sixth less), and for
   // every choice 1 to 8 cluster ranks that share the K-tiles: whichever gives the shortest rounds, counted
   // in rows of work per SM.  A doubling of the ranks costs about 3 % (the merge).
