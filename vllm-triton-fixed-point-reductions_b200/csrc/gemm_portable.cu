@@ -14,7 +14,7 @@
 //
 // Bound: multiplies and adds are separate instructions, so half the FFMA rate, for large M; reading B for
 // small M.  A thread holds RM x 4 outputs (three 16-byte shared-memory reads per 64 instructions at
-// RM = 8), the next chunk of K travels to registers while this one is multiplied, both operands are
+// RM = 8; 512x4096x4096 fp32 2147 -> 897 us, floor 477), the next chunk of K travels to registers while this one is multiplied, both operands are
 // read along whichever of their strides is one, and K-tiles are dealt to the ranks of a cluster when
 // the tiles of the output leave the GPU idle (integer sums: no bit depends on it).
 #include <algorithm>
@@ -185,8 +185,8 @@ gemm_portable_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* 
 
 // At most 16 rows: bound by reading B, which here goes straight to registers, once, 16 bytes per lane and
 // eight rows of K at a time.  K-tiles are independent up to their integer sums, so every warp of a CTA (and
-// of the cluster) takes its own: a warp is 128 columns x R rows of one K-tile.  fp32, K-tile 128:
-// 8x28672x4096 453 -> see the table of gemm_portable_kernel's figures beside the launch rule.
+// of the cluster) takes its own: a warp is 128 columns x R rows of one K-tile.  fp32, K-tile 128, against
+// the tiled kernel above: 1x4096x4096 67 -> 18 us, 8x28672x4096 453 -> 161.
 template <typename T, int R>
 __global__ void __launch_bounds__(256, 2)
 gemm_portable_rows_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* __restrict__ bias,
