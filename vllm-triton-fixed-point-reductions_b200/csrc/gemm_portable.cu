@@ -14,7 +14,8 @@
 //
 // Bound: multiplies and adds are separate instructions, so half the FFMA rate, for large M; reading B for
 // small M.  A thread holds RM x 4 outputs (three 16-byte shared-memory reads per 64 instructions at
-// RM = 8; 512x4096x4096 fp32 2147 -> 897 us, floor 477), the next chunk of K travels to registers while this one is multiplied, both operands are
+// RM = 8; 512x4096x4096 fp32 2147 -> 897 us, floor 477), the next chunk of K travels to registers while
+// this one is multiplied, both operands are
 // read along whichever of their strides is one, and K-tiles are dealt to the ranks of a cluster when
 // the tiles of the output leave the GPU idle (integer sums: no bit depends on it).
 #include <algorithm>
