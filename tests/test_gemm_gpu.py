@@ -51,7 +51,7 @@ def test_portable_bit_exact(dtype, M, N, K, int_bits):
 
 @pytest.mark.parametrize("M,N,K,kt", [
     (1, 64, 17, 128), (16, 65, 300, 16), (17, 63, 129, 128), (64, 200, 520, 24), (65, 130, 260, 64), (129, 9600, 40, 64),
-    (1, 132, 1025, 128), (8, 128, 600, 48), (9, 260, 2100, 64), (16, 4, 300, 16),
+    (1, 132, 1025, 128), (8, 128, 600, 48), (9, 260, 2100, 64), (16, 4, 300, 16), (33, 200, 530, 64),
 ])
 @pytest.mark.parametrize("transposed", [False, True])
 def test_portable_kernel_at_tile_edges(M, N, K, kt, transposed):

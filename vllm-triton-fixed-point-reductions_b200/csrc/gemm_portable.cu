@@ -184,7 +184,7 @@ gemm_portable_kernel(const T* __restrict__ a, const T* __restrict__ b, const T* 
   cluster.sync();                                    // peers may still be reading this CTA's sums
 }
 
-// At most 16 rows: bound by reading B, which here goes straight to registers, once, 16 bytes per lane and
+// Few rows: bound by reading B, which here goes straight to registers, 16 bytes per lane and
 // eight rows of K at a time.  K-tiles are independent up to their integer sums, so every warp of a CTA (and
 // of the cluster) takes its own: a warp is 128 columns x R rows of one K-tile.  fp32, K-tile 128, against
 // the tiled kernel above: 1x4096x4096 67 -> 18 us, 8x28672x4096 453 -> 161.
@@ -201,7 +201,7 @@ gemm_portable_rows_kernel(const T* __restrict__ a, const T* __restrict__ b, cons
   pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = blockIdx.x % splits, n0 = (blockIdx.x / splits) * 128;
-  const int n = n0 + lane * 4;
+  const int n = n0 + lane * 4, m0 = blockIdx.y * R;
   for (int i = tid; i < R * 128; i += 256) acc[i] = 0;
   __syncthreads();
   const uint64_t zero2 = f2_pack(zero, zero);
@@ -215,7 +215,7 @@ gemm_portable_rows_kernel(const T* __restrict__ a, const T* __restrict__ b, cons
       __syncwarp();
 #pragma unroll
       for (int m = 0; m < R; ++m)
-        sa[warp][lane][m] = (m < M && kc + lane < k_hi) ? to_f32<T>(a[(int64_t)m * a_sm + (int64_t)(kc + lane) * a_sk]) : 0.0f;
+        sa[warp][lane][m] = (m0 + m < M && kc + lane < k_hi) ? to_f32<T>(a[(int64_t)(m0 + m) * a_sm + (int64_t)(kc + lane) * a_sk]) : 0.0f;
       __syncwarp();
 #pragma unroll 1
       for (int k8 = 0; k8 < 32 && kc + k8 < k_hi; k8 += 8) {
@@ -246,21 +246,21 @@ gemm_portable_rows_kernel(const T* __restrict__ a, const T* __restrict__ b, cons
     }
 #pragma unroll
     for (int m = 0; m < R; ++m) {
-      if (m >= M || n >= N) continue;
+      if (m0 + m >= M || n >= N) continue;
       float v[4];
       f2_unpack(p[m][0], v[0], v[1]);
       f2_unpack(p[m][1], v[2], v[3]);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         atomicAdd(&acc[m * 128 + lane * 4 + j], (unsigned long long)float_to_fixed_any(v[j], scale, int_bits));
-        if (partials) partials[((int64_t)t * M + m) * N + n + j] = v[j];
+        if (partials) partials[((int64_t)t * M + m0 + m) * N + n + j] = v[j];
       }
     }
   }
   cg::cluster_group cluster = cg::this_cluster();
   if (splits > 1) cluster.sync(); else __syncthreads();
   for (int idx = rank * 256 + tid; idx < R * 128; idx += splits * 256) {
-    const int m = idx >> 7, col = n0 + (idx & 127);
+    const int m = m0 + (idx >> 7), col = n0 + (idx & 127);
     if (m >= M || col >= N) continue;
     long long sum = 0;
     if (splits > 1) {
@@ -294,14 +294,15 @@ int gemm_portable_launch(const void* a, const void* b, const void* bias, void* c
                          int64_t a_sk, int64_t b_sk, int64_t b_sn, int64_t c_sm, int int_bits,
                          int frac_bits, int k_tile, cudaStream_t s) {
   const float scale = (float)(1ull << frac_bits);
-  // Few rows, B readable 4 columns at a time and K-tiles for the eight warps of a CTA: one K-tile per warp.
+  // Few rows, B readable 4 columns at a time and K-tiles for the eight warps of a CTA: one K-tile per warp,
+  // 8 or 16 rows.  Three such row blocks cost less than one 64-row tile (27x28672x4096 fp32 836 -> 499 us).
   const int k_tiles = ceil_div_i(K, k_tile);
-  if (M <= 16 && k_tiles >= 8 && b_sn == 1 && b_sk % 4 == 0 && N % 4 == 0 && ((uintptr_t)b % (4 * sizeof(T))) == 0) {
-    const int64_t cols = ceil_div_i(N, 128);
+  if (M <= 48 && k_tiles >= 8 && b_sn == 1 && b_sk % 4 == 0 && N % 4 == 0 && ((uintptr_t)b % (4 * sizeof(T))) == 0) {
+    const int64_t cols = ceil_div_i(N, 128), blocks = ceil_div_i(M, M <= 8 ? 8 : 16);
     int splits = 1;
-    while (splits < 8 && splits * 8 < k_tiles && cols * splits * 2 <= 4 * 148) splits *= 2;
+    while (splits < 8 && splits * 8 < k_tiles && cols * blocks * splits * 2 <= 4 * 148) splits *= 2;
     auto rows = [&](auto kernel) {
-      const cudaError_t e = launch_pdl(kernel, dim3((unsigned)(cols * splits)), dim3(256), 0, s, (unsigned)splits,
+      const cudaError_t e = launch_pdl(kernel, dim3((unsigned)(cols * splits), (unsigned)blocks), dim3(256), 0, s, (unsigned)splits,
                                        (const T*)a, (const T*)b, (const T*)bias, (T*)c, c_int, partials, (int)M, (int)N,
                                        (int)K, a_sm, a_sk, b_sk, c_sm, int_bits, scale, 1.0f / scale, k_tile, splits, 0.0f);
       if (e != cudaSuccess) { set_last_error("gemm_portable launch", e); return (int)FXPR_ERR_CUDA; }
