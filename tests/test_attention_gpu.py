@@ -303,3 +303,33 @@ def test_tcgen05_prefill_kernel_equals_mma_sync_kernel(case):
     L.check_device_status()
     assert not outs[0].isnan().any()
     assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
+
+
+@pytest.mark.parametrize("hq,head_dim", [(32, 128), (128, 128), (32, 64)])     # 8- and 16-row tiles, both head sizes
+@pytest.mark.parametrize("splits", [1, 4])
+def test_decode_waits_that_give_up_are_reported_and_spoil_no_other_call(hq, head_dim, splits):
+    """With FXPR_ATTN_ABORT_EARLY every block starts as after a time-out in one of its warps: the others give up
+    waiting for what is not there yet.  The call must report it and let what it has requested land in its own
+    shared memory: the call right behind it, whose blocks take over the SMs, is unharmed."""
+    from fxpr_vllm import _native as nat
+    from fxpr_vllm import synthetic as syn
+
+    sls = [2048 - 7 * i for i in range(24)]
+    q, kv, qsl, sl, bt = syn.paged_attention_inputs(sls, [1] * len(sls), q_heads=hq, kv_heads=8, head_dim=head_dim,
+                                                    page=16, dtype=torch.bfloat16, seed=71)
+
+    def call(flags):
+        o = torch.full_like(q, float("nan"))
+        with L.overrides(attn_flags=flags):
+            torch.ops.fxpr.unified_attention_fxp(q, kv, o, qsl, sl, bt, 1, None, True, None, 64, 16, 0.0, 0, splits)
+        return o
+
+    want = call(0)
+    L.check_device_status()
+    for _ in range(3):
+        call(nat.ATTN_ABORT_EARLY)
+        got = call(0)
+        with pytest.raises(RuntimeError, match="(?i)timed out"):
+            L.check_device_status()
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    L.check_device_status()                                        # the word was cleared

@@ -19,6 +19,7 @@ struct AttnParams {
   long long* total_wv;         // [T, H, D]
   int32_t* locks;              // [T, H]
   int32_t* status;             // optional device status word (bounded waits, capacity refusals)
+  int abort_early;             // decode kernel: start as if a wait had given up already (FXPR_ATTN_ABORT_EARLY)
 };
 
 // Scratch carve-up for the split path: [partial_max | total_denom | total_wv | locks],

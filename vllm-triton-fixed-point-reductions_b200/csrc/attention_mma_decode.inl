@@ -58,7 +58,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   if (threadIdx.x == 0) {
     for (int i = 0; i < NSTAGE * NW; ++i) mbar_init(kfull0 + 8u * i, 1);
     for (int i = 0; i < NSTAGE; ++i) { mbar_init(vfull0 + 8u * i, NW); mbar_init(vfree0 + 8u * i, NW); }
-    *abort_s = 0;
+    *abort_s = p.abort_early;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   pdl_launch_dependents();
@@ -136,7 +136,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   int ent = load_entries();
   const uint32_t stage0 = smem_addr(stage_s);
   const int n_tiles = t1 - t0;
-  int req_i = 0, req_st = 0;                         // next tile to request: K tiles, then V tiles, round the stages
+  int req_i = 0, req_st = 0, req_end = 2 * n_tiles;  // next tile to request: K tiles, then V tiles, round the stages
   auto request = [&]() {
     const bool is_v = req_i >= n_tiles;
     const int t = t0 + (is_v ? req_i - n_tiles : req_i);
@@ -154,6 +154,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   };
 
   const uint32_t qs_addr = smem_addr(q_s);
+  // A bounded wait of the whole warp.  A warp that gave up requests no box any more: the stage may still be
+  // waiting for one, and its barrier takes one arrival of this warp a phase.
+  auto wait = [&](uint32_t bar, uint32_t parity) -> bool {
+    const bool done = __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_s));
+    if (!done) req_end = 0;
+    return done;
+  };
   const float ninf = -__int_as_float(0x7f800000);
   const int srows = sh.stash_rows;
   const int slanes = srows <= 8 ? 4 * srows : 32;
@@ -164,7 +171,6 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
 
   // =============================== pass A =============================================
   float rmax[2] = {ninf, ninf};
-  bool ok = true;
   // Scores, later weights: a lane's values of one warp's 16 keys lie together.
   auto stash_at = [&](int t, int w) -> float* {
     return stash_s + ((size_t)((t - t0) * NW + w) * slanes + lane) * (JW * NE);
@@ -172,7 +178,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   {
     __syncthreads();                                 // the barriers exist
 #pragma unroll 1
-    while (req_i < min(NSTAGE, 2 * n_tiles)) request();
+    while (req_i < min(NSTAGE, req_end)) request();
     cp_async_wait<0>();
     __syncthreads();                                 // Q is in shared memory for every warp
     uint32_t qa[HD / 16][ROWS8 ? 2 : 4];
@@ -193,7 +199,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     int st = 0; uint32_t ph = 0;
 #pragma unroll 1
     for (int t = t0; t < t1; ++t) {
-      ok = __all_sync(0xffffffffu, mbar_wait(kfull0 + 8u * (st * NW + warp), ph, abort_s)) && ok;
+      wait(kfull0 + 8u * (st * NW + warp), ph);
       const uint32_t k_addr = stage0 + st * kTileBytes + k_off;
       if (++st == NSTAGE) { st = 0; ph ^= 1; }
       float s[JW][4];
@@ -218,7 +224,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         }
       }
       __syncwarp();
-      if (req_i < 2 * n_tiles) request();            // into the rows of this tile, which only this warp reads
+      if (req_i < req_end) request();            // into the rows of this tile, which only this warp reads
 #pragma unroll
       for (int jj = 0; jj < JW; ++jj) {
         const int j = warp * JW + jj;
@@ -319,9 +325,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     int st = n_tiles % NSTAGE, use = 0, prev = 0; uint32_t ph = 0, ph_prev = 0;
 #pragma unroll 1
     for (int t = t0; t < t1; ++t) {
-      if (t > t0 && req_i < 2 * n_tiles) {             // into the stage of tile t - 1: before the wait for tile t, 6 % faster
-        ok = __all_sync(0xffffffffu, mbar_wait(vfree0 + 8u * prev, ph_prev, abort_s)) && ok;
-        request();
+      if (t > t0 && req_i < req_end) {             // into the stage of tile t - 1: before the wait for tile t, 6 % faster
+        if (wait(vfree0 + 8u * prev, ph_prev)) request();
       }
       uint32_t pa[4][4];
 #pragma unroll
@@ -336,7 +341,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
           pa[w][0] = v.x; pa[w][1] = v.y; pa[w][2] = v.z; pa[w][3] = v.w;
         }
       }
-      ok = __all_sync(0xffffffffu, mbar_wait(vfull0 + 8u * st, ph, abort_s)) && ok;
+      wait(vfull0 + 8u * st, ph);
       const uint32_t v_addr = stage0 + st * kTileBytes;
       if (seq_len - t * kTileN < kTileN) {
         // rows past the sequence hold whatever the page holds, or were not requested: 0 * NaN would
@@ -401,7 +406,6 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       }
     }
   }
-  if (!ok && threadIdx.x == 0 && p.status) atomicExch(p.status, FXPR_ERR_TIMEOUT);
 
   // =============================== merge ==============================================
 #pragma unroll
@@ -410,6 +414,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     den[h] += __shfl_xor_sync(0xffffffffu, den[h], 2);
   }
   __syncthreads();                                   // stages are free: reuse them for wv_s
+  const int gave_up = *abort_s;                      // one for all threads; looked at last, behind the load's latency
 #pragma unroll
   for (int h = 0; h < NH; ++h) {
     const int r = g + 8 * h;
@@ -462,6 +467,12 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
       if (pairs)
         op[d + 1] = from_f32<T>(__fdiv_rn(fixed_to_float<long long>(wrap_to_bits(w1, p.int_bits), p.inv_scale), dn));
     }
+  }
+  if (gave_up) {
+    // boxes still in flight must land in this CTA's shared memory, not in its successor's
+    const long long since = clock64();
+    while (clock64() - since < 200000) { __nanosleep(1000); }
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, FXPR_ERR_TIMEOUT);
   }
   cluster.sync();
 }

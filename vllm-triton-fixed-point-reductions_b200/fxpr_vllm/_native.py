@@ -58,6 +58,7 @@ ATTN_CAUSAL = 1
 ATTN_FORCE_PORTABLE = 2
 ATTN_EXACT_CONVERT = 4
 ATTN_NO_TCGEN05 = 8
+ATTN_ABORT_EARLY = 16
 
 _c = ctypes
 _vp, _i, _i64, _f, _d = _c.c_void_p, _c.c_int, _c.c_int64, _c.c_float, _c.c_double
