@@ -172,7 +172,9 @@ __device__ __forceinline__ uint32_t peer_shared(const void* local, uint32_t rank
   return r;
 }
 // Bounded: a bulk copy of mapped memory always completes; the limit only keeps a fault elsewhere
-// from turning into a hang.
+// from turning into a hang.  A CTA whose wait gave up copies nothing more (its slice may still receive
+// the late piece, and a barrier takes one arrival a phase) but goes on meeting its cluster's barriers;
+// then it lets the late piece land and writes NaN over its slices.
 __device__ __forceinline__ bool lsm_wait(uint32_t bar, uint32_t parity) {
   for (int i = 0; i < (1 << 20); ++i) {
     uint32_t ok;
@@ -206,7 +208,7 @@ log_softmax_bulk_kernel(const T* __restrict__ x, float* __restrict__ y, int64_t 
   const int begin = (int)crank * slice_len;
   const int len = max(0, min(cols, begin + slice_len) - begin);   // multiple of VEC
   const int nvec = len / VEC;
-  const int npieces = (nvec + kLsmThreads - 1) / kLsmThreads;
+  int npieces = (nvec + kLsmThreads - 1) / kLsmThreads;           // 0 once a wait gave up
   const int total_bytes = len * (int)sizeof(T);
   const float ninf = -__int_as_float(0x7f800000);
   const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(bars);
@@ -268,7 +270,7 @@ log_softmax_bulk_kernel(const T* __restrict__ x, float* __restrict__ y, int64_t 
     }
     lmax = warp_max_f32(lmax);
     if (lane == 0) red_f[warp] = lmax;
-    const int failed = __syncthreads_or(!ok);
+    if (__syncthreads_or(!ok)) npieces = 0;
     if (warp == 0) {
       float v = lane < kLsmThreads / 32 ? red_f[lane] : ninf;
       v = warp_max_f32(v);
@@ -322,8 +324,7 @@ log_softmax_bulk_kernel(const T* __restrict__ x, float* __restrict__ y, int64_t 
     cluster_arrive_release();
     cluster_wait_acquire();
     const long long total = warp_sum_i64(lane < (int)csize ? xchg_sum[lane] : 0);
-    float lg = log_det(fixed_to_float<long long>(total, inv_scale));   // once per warp, no block barrier
-    if (failed) lg = __int_as_float(0x7fc00000);
+    const float lg = log_det(fixed_to_float<long long>(total, inv_scale));   // once per warp, no block barrier
     const uint64_t lg2 = f2_pack(lg, lg);
 
     // ---- phase 3: write the slice --------------------------------------------------------------
@@ -345,6 +346,12 @@ log_softmax_bulk_kernel(const T* __restrict__ x, float* __restrict__ y, int64_t 
       __syncthreads();                      // every thread is done reading the slice
       issue_load(row + nclusters);
     }
+  }
+  if (npieces == 0 && nvec > 0) {
+    const long long since = clock64();
+    while (clock64() - since < 200000) { __nanosleep(1000); }
+    for (row = blockIdx.x / csize; row < rows; row += nclusters)
+      for (int i = (int)threadIdx.x; i < len; i += kLsmThreads) y[row * (int64_t)cols + begin + i] = __int_as_float(0x7fc00000);
   }
 }
 
