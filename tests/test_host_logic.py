@@ -148,3 +148,58 @@ def test_overrides_context_restores_state():
     with L.overrides(gemm_k_tile=64, gemm_split_k=4, gemm_portable=True):
         assert (L._ovr.gemm_k_tile, L._ovr.gemm_split_k, L._ovr.gemm_portable) == (64, 4, True)
     assert (L._ovr.gemm_k_tile, L._ovr.gemm_split_k, L._ovr.gemm_portable) == (None, None, False)
+
+
+_MISSING_LIBRARY_PROBE = """
+import shutil, sys
+sys.path.insert(0, %(pkg)r)
+import torch
+import fxpr_vllm
+from fxpr_vllm import _lib as L, _native as nat
+
+def call(op, *args):        # a CPU tensor sent to the CUDA implementation: no device needed to reach it
+    return op.default.redispatch(torch._C.DispatchKeySet(torch._C.DispatchKey.CUDA), *args)
+
+x = torch.ones(4, 8)
+cases = [("float_to_fixed", (x, 32, 16)), ("fixed_to_float", (x.int(), 32, 16)), ("rms_norm_fxp", (x, x[0], 1e-6)),
+         ("rms_norm_fxp_residual", (x, x, x[0], 1e-6)), ("rms_norm_fxp_from_int", (x.int(), x, x[0], None, 1e-6, 16)),
+         ("log_softmax_fxp", (x, 16)), ("gemm_fxp", (x, x.t(), None, 32, 16)), ("gemm_fxp_int", (x, x.t(), 32, 16)),
+         ("gemm_fxp_epilogue", (x.int(), None, torch.float32, 16)),
+         ("unified_attention_fxp", (x, x, x, x, x, x, 1, None, True, None, 32, 16, 0.0, 0, 1))]
+calls = [lambda n=n, a=a: call(getattr(torch.ops.fxpr, n), *a) for n, a in cases]
+calls += [lambda: L.silu_mul(x), lambda: L.gemm_silu_mul(x, x.t(), 32, 16), lambda: L.gemm_fxp_argmax(x, x.t(), None, 32, 16),
+          lambda: L.overrides(gemm_k_tile=64).__enter__()]
+for c in calls:
+    try:
+        c()
+    except RuntimeError as e:
+        assert "missing" in str(e) and "build.py" in str(e), e
+    else:
+        raise AssertionError("no error")
+L._ovr.__dict__.clear()
+for name in %(present)r:                     # built after the import
+    shutil.copy(%(lib)r + "/" + name, nat.LIB_PATH.parent)
+try:
+    call(torch.ops.fxpr.float_to_fixed, x, 32, 16)
+except RuntimeError as e:
+    assert "missing" not in str(e), e        # the library's own: it refuses a CPU device
+assert nat._torch_lib is not None
+print("PROBE ok")
+"""
+
+
+@pytest.mark.parametrize("have", [[], ["libfxpr_b200.so"]])
+def test_every_operator_names_the_build_command_while_a_library_is_missing(tmp_path, have):
+    import os
+    import shutil
+    import subprocess
+    import sys
+
+    lib = nat.LIB_PATH.parent
+    for name in have:
+        shutil.copy(lib / name, tmp_path)
+    left = [n for n in ("libfxpr_b200.so", "libfxpr_torch.so") if n not in have]
+    code = _MISSING_LIBRARY_PROBE % {"pkg": str(CSRC.parent), "lib": str(lib), "present": left}
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600,
+                       env=dict(os.environ, FXPR_B200_LIB=str(tmp_path / "libfxpr_b200.so")))
+    assert r.returncode == 0 and "PROBE ok" in r.stdout, r.stdout + r.stderr[-3000:]

@@ -62,8 +62,35 @@ BLOCK_K_BY_DTYPE = {torch.float16: 128, torch.bfloat16: 128, torch.float32: 64}
 BLOCK_N_BY_DTYPE = {torch.float16: 64, torch.bfloat16: 64, torch.float32: 32}
 
 
-_native_ops = torch.ops.fxpr_b200
-nat.load_ops(required=False)     # absent only before the first build; nat.load_ops() then reports it
+class _NativeOps:
+    """``torch.ops.fxpr_b200``, loaded at the first use (which raises if the library is not built)."""
+
+    def __getattr__(self, name):
+        nat.load_ops()
+        op = getattr(torch.ops.fxpr_b200, name)
+        setattr(self, name, op)
+        return op
+
+
+_native_ops = _NativeOps()
+
+
+def _report_missing_library() -> None:
+    """CUDA implementations that raise nat.load_ops()'s error, which names the build command, instead of
+    the dispatcher's "no kernel for CUDA".  Built after the import, the library's own take their place."""
+    def stand_in(name):
+        def op(*args):
+            nat.load_ops()
+            return getattr(torch.ops.fxpr, name)(*args)
+        return op
+
+    for name in ("float_to_fixed", "fixed_to_float", "rms_norm_fxp", "rms_norm_fxp_residual", "rms_norm_fxp_from_int",
+                 "log_softmax_fxp", "gemm_fxp", "gemm_fxp_int", "gemm_fxp_epilogue", "unified_attention_fxp"):
+        _lib.impl(name, stand_in(name), "CUDA")
+
+
+if nat.load_ops(required=False) is None:
+    _report_missing_library()
 
 
 @contextlib.contextmanager
