@@ -203,3 +203,43 @@ def test_every_operator_names_the_build_command_while_a_library_is_missing(tmp_p
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600,
                        env=dict(os.environ, FXPR_B200_LIB=str(tmp_path / "libfxpr_b200.so")))
     assert r.returncode == 0 and "PROBE ok" in r.stdout, r.stdout + r.stderr[-3000:]
+
+
+def _build_module():
+    import importlib.util
+
+    spec = importlib.util.spec_from_file_location("fxpr_build", CSRC.parent / "build.py")
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
+def test_operator_library_is_rebuilt_for_another_torch(tmp_path, monkeypatch):
+    """The C++ interface of torch changes between versions, so a library that is newer than its sources is
+    still stale when another torch, or another command line, built it."""
+    mod = _build_module()
+    monkeypatch.setattr(mod, "OBJ", tmp_path / "build")
+    monkeypatch.setattr(mod, "LIB", tmp_path / "lib" / "libfxpr_b200.so")
+    monkeypatch.setattr(mod, "TORCH_LIB", tmp_path / "lib" / "libfxpr_torch.so")
+    ran = []
+
+    def fake_run(cmd, **_):
+        out = next((cmd[i + 1] for i, a in enumerate(cmd) if a == "-o"))
+        ran.append(out.rsplit("/", 1)[1])
+        open(out, "w").close()
+        return type("R", (), dict(returncode=0, stdout="", stderr=""))()
+
+    monkeypatch.setattr(mod.subprocess, "run", fake_run)
+    mod.build()
+    assert "libfxpr_torch.so" in ran and "libfxpr_b200.so" in ran
+    ran.clear()
+    mod.build()
+    assert ran == []                                          # nothing changed
+    monkeypatch.setattr(torch, "__version__", "0.0.0+other")
+    mod.build()
+    assert ran == ["libfxpr_torch.so"]
+    ran.clear()
+    real = mod._torch_cmd
+    monkeypatch.setattr(mod, "_torch_cmd", lambda src: [*real(src), "-DOTHER"])
+    mod.build()
+    assert ran == ["libfxpr_torch.so"]

@@ -3,7 +3,8 @@ libfxpr_torch.so (csrc/torch_ops.cpp with g++: the torch operators over it).
 
 Usage: ``python build.py [--force] [--verbose]``.  Objects go to ``build/``, the
 shared libraries to ``lib/`` next to this file.  A source is recompiled when it or
-any header is newer than its object.
+any header is newer than its object, the operator library also when its command line
+or the installed torch is another one than it was built with (``build/torch_ops.stamp``).
 """
 from __future__ import annotations
 
@@ -60,6 +61,13 @@ def _torch_cmd(src: Path) -> list[str]:
             "-ltorch_cuda", "-lcudart", "-Wl,-rpath,$ORIGIN"]
 
 
+def _torch_stamp(cmd: list[str]) -> str:
+    """What the operator library's binary interface depends on besides its sources."""
+    import torch
+
+    return "\n".join([torch.__version__, str(torch.version.git_version), *cmd]) + "\n"
+
+
 def _link(nvcc: str, sources: list[Path]) -> None:
     objs = [str(OBJ / (s.stem + ".o")) for s in sources]
     cmd = [nvcc, "-shared", "-o", str(LIB), *objs, "-lcudart_static", "-lpthread", "-ldl", "-lrt",
@@ -102,11 +110,16 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         _link(nvcc, sources)
     src = CSRC / "torch_ops.cpp"
     deps = [src, CSRC / "host_policy.h", *(ROOT.parent / "include").glob("*.h")]
-    if force or not TORCH_LIB.exists() or any(p.stat().st_mtime > TORCH_LIB.stat().st_mtime for p in deps):
-        r = subprocess.run(_torch_cmd(src), capture_output=True, text=True)
+    cmd, stamp_file = _torch_cmd(src), OBJ / "torch_ops.stamp"
+    stamp = _torch_stamp(cmd)
+    same = stamp_file.exists() and stamp_file.read_text() == stamp
+    if force or not same or not TORCH_LIB.exists() or any(p.stat().st_mtime > TORCH_LIB.stat().st_mtime for p in deps):
+        stamp_file.unlink(missing_ok=True)
+        r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("g++ failed on torch_ops.cpp")
+        stamp_file.write_text(stamp)
     return LIB
 
 
