@@ -29,11 +29,11 @@ def pytest_collection_modifyitems(config, items):
 
 @pytest.fixture(scope="session", autouse=True)
 def _built_library():
-    """Every test may assume the C-ABI library exists (it is built in-tree)."""
+    """Every test may assume that the C-ABI and the operator library exist (they are built in-tree)."""
     import importlib.util
 
     lib = PKG / "lib" / "libfxpr_b200.so"
-    if not lib.exists():
+    if not (lib.exists() and lib.with_name("libfxpr_torch.so").exists()):
         spec = importlib.util.spec_from_file_location("fxpr_build", PKG / "build.py")
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
