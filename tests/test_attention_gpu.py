@@ -333,3 +333,22 @@ def test_decode_waits_that_give_up_are_reported_and_spoil_no_other_call(hq, head
             L.check_device_status()
         assert torch.equal(got.view(torch.int16), want.view(torch.int16))
     L.check_device_status()                                        # the word was cleared
+
+
+def test_more_requests_than_a_grid_dimension_holds():
+    """Above 65535 requests the tensor-core kernels' grids end and the CUDA-core route takes the call; the
+    operator has to plan splits and scratch for that route (a wide block table asks the other one for ranks)."""
+    n = 65600
+    g = torch.Generator(device="cuda").manual_seed(5)
+    kv = torch.randn((9, 2, 16, 1, 64), generator=g, device="cuda", dtype=torch.float16)
+    q = torch.randn((n, 2, 64), generator=g, device="cuda", dtype=torch.float16)
+    sl = torch.randint(1, 17, (n,), generator=g, device="cuda", dtype=torch.int32)
+    bt = torch.zeros((n, 512), device="cuda", dtype=torch.int32)
+    bt[:, 0] = torch.randint(1, 9, (n,), generator=g, device="cuda", dtype=torch.int32)
+    qsl = torch.arange(n + 1, device="cuda", dtype=torch.int32)
+    got = _h().run_attention(q, kv, qsl, sl, bt, 1, int_bits=64, splits=0)
+    half = n // 2
+    with L.overrides(attn_portable=True):
+        for a in (0, half):
+            exp = _h().run_attention(q[a:a + half], kv, qsl[:half + 1], sl[a:a + half], bt[a:a + half], 1, int_bits=64)
+            assert torch.equal(got[a:a + half].view(torch.int16), exp.view(torch.int16))

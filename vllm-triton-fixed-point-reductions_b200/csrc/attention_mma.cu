@@ -25,6 +25,7 @@
 #include "attention_common.cuh"
 #include "fxp_common.cuh"
 #include "gemm_tc_fast_common.cuh"
+#include "host_policy.h"
 
 namespace cg = cooperative_groups;
 
@@ -150,19 +151,10 @@ static int launch_decode(const AttnParams& p, const MmaAttnShape& sh, int dtype,
   return check_launch("attention_decode");
 }
 
-static bool pow2_le16(int v) { return v == 1 || v == 2 || v == 4 || v == 8 || v == 16; }
-
 bool attention_mma_supported(const AttnParams& p, int dtype) {
-  if (dtype != FXPR_F16 && dtype != FXPR_BF16) return false;
-  if (p.head_dim != 64 && p.head_dim != 128) return false;
-  if (p.page_size % 16 != 0) return false;
-  if (!pow2_le16(p.num_heads / p.num_kv_heads)) return false;
-  // 16-byte cp.async: every row start must be 16-byte aligned
-  const int64_t strides[] = {p.q_st, p.q_sh, p.kv_sblock, p.kv_sslot, p.kv_shead};
-  for (int64_t st : strides) if (st % 8 != 0) return false;
-  if (((uintptr_t)p.q | (uintptr_t)p.k | (uintptr_t)p.v) & 15) return false;
-  if (p.num_kv_heads > 4096 || p.num_reqs > 65535) return false;
-  return true;
+  return attention_tensor_core_route({dtype == FXPR_F16 || dtype == FXPR_BF16, p.head_dim, p.page_size, p.num_heads,
+                                      p.num_kv_heads, p.num_reqs, p.q_st, p.q_sh, p.kv_sblock, p.kv_sslot, p.kv_shead,
+                                      p.q, p.k, p.v});
 }
 
 int attention_mma(const AttnParams& p_in, int dtype, int max_query_len, bool force_exact, cudaStream_t s) {

@@ -9,6 +9,24 @@ namespace fxpr {
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// What the tensor-core attention route takes.  Types, geometry and alignment only, nothing of the batch but
+// the grid's limits, so that a token's bits do not depend on the other requests.
+struct AttnRoute {
+  bool half;                                             // fp16 or bf16
+  int64_t head_dim, page_size, num_heads, num_kv_heads, num_reqs;
+  int64_t q_st, q_sh, kv_sblock, kv_sslot, kv_shead;     // strides in elements
+  const void *q, *k, *v;
+};
+inline bool attention_tensor_core_route(const AttnRoute& r) {
+  const int64_t g = r.num_heads / r.num_kv_heads;
+  if (!r.half || (r.head_dim != 64 && r.head_dim != 128) || r.page_size % 16 != 0) return false;
+  if (g != 1 && g != 2 && g != 4 && g != 8 && g != 16) return false;
+  // 16-byte copies: every row must start on 16 bytes
+  if ((r.q_st | r.q_sh | r.kv_sblock | r.kv_sslot | r.kv_shead) % 8 != 0) return false;
+  if (((uintptr_t)r.q | (uintptr_t)r.k | (uintptr_t)r.v) & 15) return false;
+  return r.num_kv_heads <= 4096 && r.num_reqs <= 65535;  // grid dimensions
+}
+
 // K-split of a GEMM: split when the output tiles alone cannot fill the GPU.
 inline int pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int64_t k_tile, int int_bits, int num_sms) {
   if (int_bits == 16) return 1;

@@ -444,21 +444,6 @@ Tensor rope_kv_write(const Tensor& qkv, const Tensor& cos, const Tensor& sin, co
 }
 
 // ------------------------------------------------------------------ attention
-bool pow2_up_to_16(int64_t g) { return g == 1 || g == 2 || g == 4 || g == 8 || g == 16; }
-
-// Mirror of the C side's routing rule (dtype and geometry only, never the batch).
-bool tensor_core_route(const Tensor& q, const Tensor& kv, int64_t g) {
-  const auto t = q.scalar_type();
-  const int64_t d = q.size(2);
-  if (!((t == at::kHalf || t == at::kBFloat16) && (d == 64 || d == 128) && kv.size(2) % 16 == 0 && pow2_up_to_16(g)) ||
-      t_ovr.attn_portable)
-    return false;
-  // 16-byte copies: row starts must be 16-byte aligned
-  if ((q.stride(0) | q.stride(1) | kv.stride(0) | kv.stride(2) | kv.stride(3)) % 8) return false;
-  const auto base = (uintptr_t)kv.data_ptr();
-  return (((uintptr_t)q.data_ptr() | base | (base + kv.stride(1) * kv.element_size())) & 15) == 0;
-}
-
 void unified_attention_fxp(const Tensor& q, const Tensor& kv, const Tensor& o, const Tensor& query_start_loc,
                            const Tensor& seq_lens, const Tensor& block_table_in, int64_t max_query_len,
                            const optional<Tensor>& alibi_slopes, bool is_causal, optional<double> softmax_scale,
@@ -489,7 +474,12 @@ void unified_attention_fxp(const Tensor& q, const Tensor& kv, const Tensor& o, c
   const double ss = softmax_scale.has_value() ? *softmax_scale : 1.0 / std::sqrt((double)head_dim);
   const bool table2d = block_table_in.dim() == 2;
   const int64_t max_keys = std::max<int64_t>(1, (table2d ? block_table_in.size(1) : 0) * page);
-  const bool tc = tensor_core_route(q, kv, num_heads / num_kv_heads);
+  const char* k_base = (const char*)kv.data_ptr();
+  const char* v_base = k_base + kv.stride(1) * kv.element_size();
+  const bool tc = !t_ovr.attn_portable && !(t_ovr.attn_flags & FXPR_ATTN_FORCE_PORTABLE) &&
+                  fxpr::attention_tensor_core_route({t == at::kHalf || t == at::kBFloat16, head_dim, page, num_heads, num_kv_heads,
+                                                     num_requests, q.stride(0), q.stride(1), kv.stride(0), kv.stride(2),
+                                                     kv.stride(3), q.data_ptr(), k_base, v_base});
   int64_t splits;
   if (tc) {
     splits = fxpr::pick_attention_ranks(num_kv_splits, num_requests, max_query_len, num_heads, num_kv_heads, max_keys,
@@ -513,9 +503,8 @@ void unified_attention_fxp(const Tensor& q, const Tensor& kv, const Tensor& o, c
   const int flags = (is_causal ? FXPR_ATTN_CAUSAL : 0) | (t_ovr.attn_portable ? FXPR_ATTN_FORCE_PORTABLE : 0) | t_ovr.attn_flags;
   const Tensor qsl = query_start_loc.contiguous(), sl = seq_lens.contiguous();
   const Tensor bt = table2d && block_table_in.stride(1) != 1 ? block_table_in.contiguous() : block_table_in;
-  const char* k_base = (const char*)kv.data_ptr();
   check_status(
-      fxpr_attention(q.data_ptr(), k_base, k_base + kv.stride(1) * kv.element_size(), o.data_ptr(), qsl.data_ptr<int32_t>(),
+      fxpr_attention(q.data_ptr(), k_base, v_base, o.data_ptr(), qsl.data_ptr<int32_t>(),
                      sl.data_ptr<int32_t>(), bt.data_ptr<int32_t>(), has_alibi ? alibi.data_ptr<float>() : nullptr, dtype_code(t),
                      tokens, (int)num_requests, (int)num_heads, (int)num_kv_heads, (int)head_dim, (int)page, q.stride(0),
                      q.stride(1), o.stride(0), o.stride(1), kv.stride(0), kv.stride(2), kv.stride(3), table2d ? bt.stride(0) : 0,
