@@ -314,6 +314,9 @@ int fxpr_silu_mul(const void* gate_up, int dtype, void* out, int64_t rows, int64
 int fxpr_silu_mul_pairs(const void* gate_up, int dtype, void* out, int64_t rows, int64_t f,
                         void* stream);
 
+/* The K-tile of a GEMM that names none: 128 for f16/bf16, 64 for f32. */
+int fxpr_gemm_default_k_tile(int dtype);
+
 /*
  * Automatic split counts, from host shapes only (the torch operators ask the same functions; no
  * choice changes a result).  GEMM K-splits; KV splits of the CUDA-core attention route

@@ -2,6 +2,7 @@
 the same bits) and the arg-max key arithmetic of the fused lm_head GEMM."""
 from __future__ import annotations
 
+import pytest
 import torch
 
 import fxpr_vllm  # noqa: F401
@@ -57,3 +58,10 @@ def test_interleave_gate_up_layout():
     p = L.interleave_gate_up(wg, wu)
     assert p.shape == (3, 8)
     assert torch.equal(p[:, 0::2], wg) and torch.equal(p[:, 1::2], wu)
+
+
+def test_default_k_tiles_are_the_reference_ones():
+    # fxpr_vllm/_triton/gemm.py:26-30; one table for the operators, the C ABI and Python callers
+    assert dict(L.BLOCK_K_BY_DTYPE) == {torch.float16: 128, torch.bfloat16: 128, torch.float32: 64}
+    with pytest.raises(KeyError):
+        L.BLOCK_K_BY_DTYPE[torch.float64]

@@ -10,10 +10,7 @@
 
 using namespace fxpr;
 
-static int default_k_tile(int dtype) {
-  // fxpr_vllm/_triton/gemm.py:26-30: 128 for 16-bit inputs, 64 for fp32
-  return dtype == FXPR_F32 ? 64 : 128;
-}
+extern "C" int fxpr_gemm_default_k_tile(int dtype) { return default_k_tile(dtype == FXPR_F32); }
 
 extern "C" int64_t fxpr_gemm_scratch_bytes(int64_t M, int64_t N, int int_bits, int split_k) {
   if (split_k <= 1 || M <= 0 || N <= 0) return 0;
@@ -47,7 +44,7 @@ static int gemm_entry(const void* a, const void* b, const void* bias, void* c, v
   if ((K > 0 && (!a || !b)) || (!c && !c_int)) return FXPR_ERR_BAD_ARG;
   if (M > 0x7fffffffLL || N > 0x7fffffffLL || K > 0x7fffffffLL) return FXPR_ERR_BAD_ARG;
   if (dtype != FXPR_F16 && dtype != FXPR_BF16 && dtype != FXPR_F32) return FXPR_ERR_UNSUPPORTED;
-  if (k_tile <= 0) k_tile = default_k_tile(dtype);
+  if (k_tile <= 0) k_tile = default_k_tile(dtype == FXPR_F32);
   if (split_k < 1) split_k = 1;
   if (split_k > 1 && partials_out) return FXPR_ERR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;

@@ -9,6 +9,9 @@ namespace fxpr {
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// K-tile of a GEMM that names none (fxpr_vllm/_triton/gemm.py:26-30).
+inline int default_k_tile(bool fp32) { return fp32 ? 64 : 128; }
+
 // What the tensor-core attention route takes.  Types, geometry and alignment only, nothing of the batch but
 // the grid's limits, so that a token's bits do not depend on the other requests.
 struct AttnRoute {

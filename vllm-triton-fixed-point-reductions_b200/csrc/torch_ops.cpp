@@ -315,7 +315,7 @@ GemmOut gemm_common(const Tensor& a, const Tensor& b, const optional<Tensor>& bi
   const Overrides& o = t_ovr;
   const Config& cfg = config();
   int k_tile = o.gemm_k_tile >= 0 ? o.gemm_k_tile : cfg.gemm_k_tile.load();
-  if (k_tile <= 0) k_tile = t == at::kFloat ? 64 : 128;
+  if (k_tile <= 0) k_tile = fxpr::default_k_tile(t == at::kFloat);
   const int64_t k_tiles = fxpr::ceil_div(K, k_tile);
   int flags = (o.gemm_portable ? FXPR_GEMM_FORCE_PORTABLE : 0) | o.gemm_flags | (want.silu_pairs ? FXPR_GEMM_SILU_MUL : 0);
   optional<Tensor> bias = bias_in;

@@ -53,13 +53,6 @@ _lib.define(
 )
 
 _INT_DTYPE = {16: torch.int16, 32: torch.int32, 64: torch.int64}
-_IO_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
-
-# K-tile = determinism granularity per dtype (gemm.py:26-30 of the reference);
-# tests read this the way the reference's test reads _BLOCK_K_BY_DTYPE.
-BLOCK_K_BY_DTYPE = {torch.float16: 128, torch.bfloat16: 128, torch.float32: 64}
-# key-tile width of the attention kernels (attention.py:32-36)
-BLOCK_N_BY_DTYPE = {torch.float16: 64, torch.bfloat16: 64, torch.float32: 32}
 
 
 class _NativeOps:
@@ -89,8 +82,24 @@ def _report_missing_library() -> None:
         _lib.impl(name, stand_in(name), "CUDA")
 
 
+class _KTileTable(dict):
+    """The library's default K-tile (determinism granularity, gemm.py:26-30 of the reference) of each io
+    dtype; tests read it the way the reference's test reads ``_BLOCK_K_BY_DTYPE``."""
+
+    def __missing__(self, dtype):
+        if dtype not in (torch.float16, torch.bfloat16, torch.float32):
+            raise KeyError(dtype)
+        self[dtype] = nat.load().fxpr_gemm_default_k_tile(nat.DTYPE_CODE[dtype])
+        return self[dtype]
+
+
+BLOCK_K_BY_DTYPE = _KTileTable()
+
 if nat.load_ops(required=False) is None:
     _report_missing_library()
+else:
+    for _dt in (torch.float16, torch.bfloat16, torch.float32):
+        BLOCK_K_BY_DTYPE[_dt]
 
 
 @contextlib.contextmanager

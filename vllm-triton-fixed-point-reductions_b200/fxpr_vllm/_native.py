@@ -96,6 +96,7 @@ SIGNATURES = {
                             _i, _i64, _i, _i, _i, _i, _i,
                             _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64,
                             _i, _i, _d, _d, _i, _i, _i, _i, _vp, _i64, _vp, _vp]),
+    "fxpr_gemm_default_k_tile": (_i, [_i]),
     "fxpr_pick_gemm_split_k": (_i, [_i64, _i64, _i64, _i, _i, _i]),
     "fxpr_pick_attention_splits": (_i, [_i, _i64, _i64, _i, _i64, _i]),
     "fxpr_pick_attention_ranks": (_i, [_i, _i64, _i64, _i, _i, _i64, _i]),
