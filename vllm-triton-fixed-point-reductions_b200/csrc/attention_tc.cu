@@ -98,10 +98,6 @@ template <> __device__ __forceinline__ uint32_t pack2_tc<__half>(float lo, float
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-__device__ __forceinline__ bool warp_wait_all(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
-}
-
 template <typename T, int HD>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -404,7 +400,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     auto soft_sync = [&]() -> bool {                         // bounded barrier over these 8 warps
       __syncwarp();
       if (lane == 0) mbar_arrive(soft_bar);
-      const bool done = warp_wait_all(soft_bar, soft_phase, abort_flag);
+      const bool done = warp_wait(soft_bar, soft_phase, abort_flag);
       soft_phase ^= 1;
       return done;
     };
@@ -444,7 +440,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     for (int t = t0; t < t1 && ok; t += 2, ++it) {
       const int sb = it & 1;
       if (sb != group) continue;
-      if (!warp_wait_all(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!warp_wait(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       float m = ninf;
 #pragma unroll
@@ -492,7 +488,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int sb = it & 1;
       if (sb != group) continue;
       ++mine;
-      if (!warp_wait_all(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!warp_wait(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int g = jg + j, b = g & 1;
       const uint32_t prow = p_s0 + b * kPBytes + (uint32_t)row * 128u;
@@ -527,7 +523,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // weights, integer denominator, P in the io dtype -> shared memory (A operand of P.V):
         // row = 128 bytes of 64 keys, 16-byte chunks XOR-swizzled with the row number
         // (its buffer is free once the P.V product two tiles back has completed)
-        if (h == 0 && g >= 2 && !warp_wait_all(pvfull0 + 8u * b, ((g - 2) >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (h == 0 && g >= 2 && !warp_wait(pvfull0 + 8u * b, ((g - 2) >> 1) & 1, abort_flag)) { ok = false; break; }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           uint32_t pk[4];
@@ -552,7 +548,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (!ok) break;
     jg += n_tiles;
     // 64 weights per tile went through the packed add in this thread
-    if (!warp_wait_all(denfree0 + 8u * (k & 1), ((k >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
+    if (!warp_wait(denfree0 + 8u * (k & 1), ((k >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
     den_s[(k & 1) * (2 * kTcRows) + group * kTcRows + row] =
         (long long)(int32_t)(den32 - (uint32_t)kTcTileN * (uint32_t)mine * mbits);
     __syncwarp();
@@ -585,7 +581,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       bool corr_used = false;
       for (int j = 0; j < n_tiles; ++j, ++jg) {
         const int b = jg & 1;
-        if (!warp_wait_all(pvfull0 + 8u * b, (jg >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (!warp_wait(pvfull0 + 8u * b, (jg >> 1) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t taddr = tmem_base + lane_sel + kColPV + (uint32_t)(b * HD + half * kHalfCols);
         float screen = 0.0f, tail = 0.0f;
@@ -615,7 +611,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
       }
       if (!ok) break;
-      if (!warp_wait_all(denfull0 + 8u * (k & 1), (k >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!warp_wait(denfull0 + 8u * (k & 1), (k >> 1) & 1, abort_flag)) { ok = false; break; }
       const long long dsum = den_s[(k & 1) * (2 * kTcRows) + row] + den_s[(k & 1) * (2 * kTcRows) + kTcRows + row];
       __syncwarp();
       if (lane == 0) mbar_arrive(denfree0 + 8u * (k & 1));

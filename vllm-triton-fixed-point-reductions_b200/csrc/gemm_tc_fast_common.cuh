@@ -8,8 +8,6 @@
 
 namespace fxpr {
 
-static __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
-
 static constexpr uint32_t kMagicBits = 0x4B400000u;      // 1.5 * 2^23
 static constexpr uint32_t kExpBits = 0x4B000000u;        // exponent pattern of [2^23, 2^24)
 
@@ -85,7 +83,7 @@ static __device__ __noinline__ void fixup_tile(uint32_t taddr, int ncols, uint32
 }
 
 // The whole warp probes: 1-7 % faster than one lane probing and a shuffle behind it.
-static __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int lane) {
+static __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 

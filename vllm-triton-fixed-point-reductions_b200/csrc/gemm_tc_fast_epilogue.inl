@@ -16,7 +16,7 @@
   auto epi_sync = [&]() -> bool {   // bounded barrier over the epilogue warps only
     __syncwarp();
     if (lane == 0) mbar_arrive(epi_bar);
-    const bool done = warp_wait(epi_bar, epi_phase, abort_flag, lane);
+    const bool done = warp_wait(epi_bar, epi_phase, abort_flag);
     epi_phase ^= 1;
     return done;
   };
@@ -41,7 +41,7 @@
 
     const int n_ss = pairs ? (n_kt + 1) >> 1 : n_kt;
     for (int ss = 0; ss < n_ss; ++ss) {
-      if (!warp_wait(tfull0 + 8u * grp, gphase, abort_flag, lane)) { ok = false; break; }
+      if (!warp_wait(tfull0 + 8u * grp, gphase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int nbuf = (pairs && 2 * ss + 1 < n_kt) ? 2 : 1;
       // Measured on B200: this plain order (load 16 columns, wait, convert) beats both a

@@ -95,9 +95,12 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t elected)
       "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
       ::"r"(bar), "h"(both), "r"(elected) : "memory");
 }
-// Non-blocking probe.  mbarrier.try_wait may park the thread for a hardware time limit, and a
-// parked thread is woken promptly only by arrivals from its own CTA; most barriers here are
-// completed from the peer CTA, so the waits of this kernel poll with test_wait instead.
+// Non-blocking probe, for the waits of the producers and the issuer.  mbarrier.try_wait may park the
+// thread for a hardware time limit, and a parked thread is woken promptly only by arrivals from its own
+// CTA; most of these barriers are completed from the peer CTA.  The sixteen epilogue warps wait with
+// try_wait all the same: they share the issue slots with the conversion, and polling takes more of them
+// than a late wake-up costs (polling everywhere: 4096^3 at K-tile 64 200.4 -> 201.4 us, at K-tile 128
+// 140.7 -> 143.0, 8192 x 14336 x 4096 945 -> 962).
 __device__ __forceinline__ uint32_t mbar_test_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -118,9 +121,6 @@ __device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, vo
     }
   }
   return true;
-}
-__device__ __forceinline__ bool warp_wait_poll(uint32_t bar, uint32_t parity, volatile int* abort_flag, int lane) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
 static constexpr int kPrStages = 6;
@@ -267,7 +267,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
       for (int i = 0; i < kPrCols; ++i) acc[i] = 0;
       corr_used = false;
       for (int kt = 0; kt < n_kt; ++kt) {
-        if (!warp_wait_poll(tfull0 + 8u * buf, bphase, abort_flag, lane)) { ok = false; break; }
+        if (!warp_wait(tfull0 + 8u * buf, bphase, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t taddr = tmem_base + lane_addr + (uint32_t)(buf * 256);
         float screen = 0.0f;
