@@ -221,9 +221,9 @@ def test_tp_sharding_single_gpu_equals_unsharded():
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("int_bits", [32, 64])
-@pytest.mark.parametrize("kt,split", [(64, 1), (128, 1), (64, 3), (128, 2)])
-@pytest.mark.parametrize("tile", ["n128", "n256", "pair128", "pair256"])
-def test_fast_epilogue_equals_plain_conversion_with_outliers(dtype, int_bits, kt, split, tile):
+@pytest.mark.parametrize("tile,kt,split", [("n128", 64, 1), ("n128", 128, 1), ("n128", 64, 3), ("n128", 128, 2),
+                                           ("pair", 64, 1), ("pair", 128, 1)])
+def test_fast_epilogue_equals_plain_conversion_with_outliers(dtype, int_bits, tile, kt, split):
     """The magic-number epilogue with its exact fix-up gives the same integers as the
     tensor-core kernel that converts every partial with cvt.rni (saturating), including
     rows whose partials leave the fast range, saturate int32 or overflow the 32-bit sum."""
@@ -236,10 +236,8 @@ def test_fast_epilogue_equals_plain_conversion_with_outliers(dtype, int_bits, kt
     a[M - 1, 5::7] = -3000.0
     a[M // 2, :64] = 6.0e4
     a[7, 100] = float("inf") if int_bits == 32 else 5.0e4
-    # every tile shape, whatever the default: 128 x 128, 128 x 256, and the two-SM kernel's
-    # 256 x 128 / 256 x 256 pair tiles
-    shape_flag = {"n128": nat.GEMM_TILE_N128, "n256": nat.GEMM_TILE_N256,
-                  "pair128": nat.GEMM_PAIR | nat.GEMM_TILE_N128, "pair256": nat.GEMM_PAIR}[tile]
+    # both tile shapes, whatever the default: 128 x 128, and 256 x 256 on SM pairs (unsplit K only)
+    shape_flag = {"n128": nat.GEMM_TILE_N128, "pair": nat.GEMM_PAIR}[tile]
     with L.overrides(gemm_k_tile=kt, gemm_split_k=split, gemm_flags=shape_flag):
         fast_i = torch.ops.fxpr.gemm_fxp_int(a, b, int_bits, 16)
         fast_c = _gemm(a, b, None, int_bits, 16)
@@ -315,7 +313,7 @@ def test_decode_row_bits_do_not_depend_on_the_batch():
 
 def test_routes_agree_on_random_shapes():
     """Seeded sweep over ragged shapes: whichever kernel the dispatcher picks (decode-shape,
-    128x128 or 128x256 tiles, cluster or plane split-K) must give the integers of the
+    128x128 tiles or 256x256 on SM pairs, cluster or plane split-K) must give the integers of the
     tensor-core kernel with plain cvt.rni conversion, for both weight layouts."""
     from fxpr_vllm import _native as nat
 
@@ -343,55 +341,97 @@ def test_routes_agree_on_random_shapes():
     L.check_device_status()
 
 
+def _kernels_launched(fn):
+    """Names of the CUDA kernels ``fn`` launches; empty where the profiler cannot see them."""
+    from torch.profiler import ProfilerActivity, profile
+
+    fn()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    return [e.key for e in prof.key_averages()]
+
+
+@pytest.mark.parametrize("M,N,K,split,flag,want", [
+    (129, 128, 64, 1, "pair", "gemm_tc_pair_kernel"),           # the smallest call the two-SM kernel takes
+    (128, 512, 256, 1, "pair", "gemm_tc_fast_kernel"),          # one row, column or K-tile split short of it
+    (300, 120, 256, 1, "pair", "gemm_tc_fast_kernel"),
+    (300, 512, 512, 2, "pair", "gemm_tc_fast_kernel"),
+    (4096, 4096, 256, 0, "", "gemm_tc_pair_kernel"),            # by size
+    (4096, 4096, 256, 0, "n128", "gemm_tc_fast_kernel"),
+])
+def test_which_kernel_takes_a_call(M, N, K, split, flag, want):
+    """What the flags and the dispatch rule say about the wide kernels, seen in the launches: the comparisons
+    below prove nothing if both of their sides run the same kernel."""
+    from fxpr_vllm import _native as nat
+
+    a, b = _rand((M, K), torch.bfloat16, 1).cuda(), _rand((K, N), torch.bfloat16, 2, 0.05).cuda()
+    flags = {"pair": nat.GEMM_PAIR, "n128": nat.GEMM_TILE_N128, "": 0}[flag]
+    kw = {"gemm_split_k": split} if split else {}
+    with L.overrides(gemm_flags=flags, **kw):
+        names = [n for n in _kernels_launched(lambda: _gemm(a, b, None, 64, 16)) if "gemm" in n]
+    if not names:
+        pytest.skip("no kernel activity from the profiler")
+    assert any(want in n for n in names), names
+
+
 def test_two_sm_kernel_agrees_on_random_shapes():
-    """The cta_group::2 kernel (CTA pairs, 256-row tiles) gives the integers of the plain-conversion
-    tensor-core kernel on ragged shapes, with and without split-K, for both weight layouts."""
+    """The cta_group::2 kernel (CTA pairs, 256-row tiles, unsplit K) gives the integers and outputs of the
+    plain-conversion tensor-core kernel on ragged shapes: every mix of K-tile, accumulator width, io dtype,
+    layout of B and bias, each with N a multiple of 16 (wide stores) and not."""
     from fxpr_vllm import _native as nat
 
     g = torch.Generator().manual_seed(77)
-    for case in range(24):
+    for case in range(64):
         M = int(torch.randint(129, 900, (1,), generator=g))
-        N = 8 * int(torch.randint(16, 130, (1,), generator=g))
+        N = 16 * int(torch.randint(8, 65, (1,), generator=g)) + 8 * ((case // 32) % 2)
         K = 8 * int(torch.randint(8, 300, (1,), generator=g))
         kt = (64, 128)[case % 2]
-        split = (1, 2, 3, 5)[case % 4]
         int_bits = (64, 32)[(case // 2) % 2]
         dtype = (torch.bfloat16, torch.float16)[(case // 4) % 2]
-        flag = nat.GEMM_PAIR | (nat.GEMM_TILE_N128 if case % 3 == 0 else 0)
         a = _rand((M, K), dtype, 3000 + case).cuda()
         b = _rand((K, N), dtype, 4000 + case, 0.05).cuda()
         if case % 5 == 0:
             a[M // 2, : min(64, K)] = 3.0e4
-        bb = b if case % 2 else b.t().contiguous().t()
-        bias = _rand((N,), dtype, 5000 + case).cuda() if case % 2 else None
-        with L.overrides(gemm_k_tile=kt, gemm_split_k=split, gemm_flags=flag):
+        bb = b if (case // 8) % 2 else b.t().contiguous().t()
+        bias = _rand((N,), dtype, 5000 + case).cuda() if (case // 16) % 2 else None
+        with L.overrides(gemm_k_tile=kt, gemm_split_k=1, gemm_flags=nat.GEMM_PAIR):
             got = torch.ops.fxpr.gemm_fxp_int(a, bb, int_bits, 16)
             got_c = _gemm(a, bb, bias, int_bits, 16)
         with L.overrides(gemm_k_tile=kt, gemm_split_k=1, gemm_flags=nat.GEMM_FORCE_EXACT_TC):
             exp = torch.ops.fxpr.gemm_fxp_int(a, bb, int_bits, 16)
             exp_c = _gemm(a, bb, bias, int_bits, 16)
-        assert torch.equal(got, exp), (case, M, N, K, kt, split, int_bits, dtype)
+        assert torch.equal(got, exp), (case, M, N, K, kt, int_bits, dtype)
         assert torch.equal(got_c.view(torch.int16), exp_c.view(torch.int16)), case
     L.check_device_status()
 
 
 @pytest.mark.parametrize("M,N,K", [
-    (256, 256, 128), (255, 248, 136), (257, 264, 64), (512, 512, 72), (65, 256, 8), (1025, 2056, 200),
+    (256, 256, 128), (255, 248, 136), (257, 264, 64), (512, 512, 72), (129, 128, 64), (1025, 2056, 200),
 ])
 @pytest.mark.parametrize("kt", [64, 128])
-def test_two_sm_kernel_at_tile_edges(M, N, K, kt):
-    """256 x 256 pair tiles one short of, at and one past their edges; K of one, several and ragged tiles."""
+@pytest.mark.parametrize("kmajor", [False, True])
+def test_two_sm_kernel_at_tile_edges(M, N, K, kt, kmajor):
+    """256 x 256 pair tiles one short of, at and one past their edges, and the smallest the kernel takes; K of
+    one, several and ragged tiles; both layouts of B; with and without bias (whose sums need not fit the
+    shortcut of the wide stores)."""
     from fxpr_vllm import _native as nat
 
     a = _rand((M, K), torch.bfloat16, M).cuda()
     b = _rand((K, N), torch.bfloat16, N, 0.05).cuda()
+    if kmajor:
+        b = b.t().contiguous().t()
+    bias = _rand((N,), torch.bfloat16, 7, 30.0).cuda()
+    clean = a.clone()
     a[M - 1, -1] = 2.0e4                              # a partial of the last row leaves the fast range
     out = []
     for flags in (nat.GEMM_PAIR, nat.GEMM_FORCE_EXACT_TC):
         with L.overrides(gemm_k_tile=kt, gemm_split_k=1, gemm_flags=flags):
-            out.append((torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16), _gemm(a, b, None, 32, 16)))
+            out.append((torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16), _gemm(a, b, None, 32, 16), _gemm(a, b, bias, 64, 16),
+                        _gemm(clean, b, None, 64, 16), _gemm(clean, b, bias, 32, 16)))
     assert torch.equal(out[0][0], out[1][0])
-    assert torch.equal(out[0][1].view(torch.int16), out[1][1].view(torch.int16))
+    for got, exp in zip(out[0][1:], out[1][1:]):
+        assert torch.equal(got.view(torch.int16), exp.view(torch.int16))
     L.check_device_status()
 
 

@@ -486,7 +486,7 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
     const int64_t single_tiles = ((g.M + 127) / 128) * ((g.N + 127) / 128);
     const int64_t pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2), single_waves = (single_tiles + sms - 1) / sms;
     const bool wide = pair_waves * (g.k_tile == 64 ? 170 : 155) <= single_waves * 100;
-    if ((g.flags & (FXPR_GEMM_PAIR | FXPR_GEMM_TILE_N256)) || (wide && !(g.flags & FXPR_GEMM_TILE_N128)))
+    if ((g.flags & FXPR_GEMM_PAIR) || (wide && !(g.flags & FXPR_GEMM_TILE_N128)))
       return gemm_tc_pair(g, p, ma, mb, s);
   }
   if (!(g.flags & FXPR_GEMM_FORCE_EXACT_TC) && gemm_tc_fast_supported(g, p.split_k)) {

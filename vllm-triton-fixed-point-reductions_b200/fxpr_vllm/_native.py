@@ -52,7 +52,6 @@ GEMM_PAIR = 512
 GEMM_SILU_MUL = 1024
 GEMM_WEIGHTS_STATIC = 2048
 TP_LOCAL_RESIDUAL = 1
-GEMM_TILE_N256 = 64
 GEMM_TILE_N128 = 128
 ATTN_CAUSAL = 1
 ATTN_FORCE_PORTABLE = 2
