@@ -759,12 +759,9 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
   constexpr int kSmem = kTcRows * 128 * 2 + kTcStages * 2 * kTcTileN * 128 * 2 + 2 * kTcRows * kTcTileN * 2 +
                         8 * (1 + 2 * kTcStages + 10 + 2 + 4) + 16 + 2048 + 4096 + 1024;
   // persistent CTAs, one per SM (204 KB of shared memory each), walking the padded item list
-  int dev_now = 0, sms = 0;
-  cudaGetDevice(&dev_now);
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_now) != cudaSuccess || sms < 1) sms = 148;
   const int64_t total_items = (int64_t)sh.num_q_blocks * p.num_kv_heads * p.num_reqs;
   if (total_items > 0x7fffffffLL) return FXPR_ERR_UNSUPPORTED;
-  dim3 grid((unsigned)std::min<int64_t>(total_items, sms), 1, 1);
+  dim3 grid((unsigned)std::min<int64_t>(total_items, device_sms()), 1, 1);
 #define FXPR_TC_ATTN(TT)                                                                              \
   do {                                                                                                \
     auto k = attn_tc_prefill_kernel<TT, 128>;                                                         \

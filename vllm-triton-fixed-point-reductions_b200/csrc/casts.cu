@@ -80,23 +80,10 @@ fixed_to_float_kernel(const TIn* __restrict__ x, TOut* __restrict__ y, int64_t n
   }
 }
 
-static int num_sms() {
-  static int cached[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (cached[dev] == 0) {
-    int n = 0;
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    cached[dev] = n > 0 ? n : 148;
-  }
-  return cached[dev];
-}
-
 static int cast_grid(int64_t n, int vec) {
   vec *= kCastU;
   int64_t want = (n + (int64_t)kCastThreads * vec - 1) / ((int64_t)kCastThreads * vec);
-  int64_t cap = (int64_t)num_sms() * kCastCtasPerSm;
+  int64_t cap = (int64_t)device_sms() * kCastCtasPerSm;
   return (int)(want < cap ? (want < 1 ? 1 : want) : cap);
 }
 

@@ -31,6 +31,19 @@ int check_launch(const char* what) {
   return FXPR_OK;
 }
 
+int device_sms() {
+  static int cached[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  if (cached[dev] == 0) {
+    int n = 0;
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    cached[dev] = n > 0 ? n : 148;
+  }
+  return cached[dev];
+}
+
 bool pdl_enabled() {
   static const bool on = [] {
     const char* v = getenv("FXPR_NO_PDL");

@@ -10,6 +10,8 @@
 //
 // No reductions here: every output element depends on one or two input elements, so these
 // kernels cannot affect batch / split / tensor-parallel invariance.
+#include <algorithm>
+
 #include "fxp_common.cuh"
 
 namespace fxpr {
@@ -105,7 +107,7 @@ static void launch_silu(const void* gu, void* out, int64_t rows, int64_t f, cuda
   constexpr int V = 16 / (int)sizeof(T);
   const bool vec = (f % V == 0) && ((((uintptr_t)gu | (uintptr_t)out) & 15) == 0);
   const int64_t n = rows * (vec ? f / V : f);
-  const unsigned grid = (unsigned)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
+  const unsigned grid = (unsigned)(std::min<int64_t>((n + 255) / 256, device_sms() * 16));
   if (vec) (void)launch_pdl(silu_mul_kernel<T, V>, dim3(grid), dim3(256), 0, s, 1u, (const T*)gu, (T*)out, rows, f);
   else (void)launch_pdl(silu_mul_kernel<T, 1>, dim3(grid), dim3(256), 0, s, 1u, (const T*)gu, (T*)out, rows, f);
 }
@@ -130,7 +132,7 @@ extern "C" int fxpr_rope_kv_write(const void* qkv, int dtype, const float* cos_t
   // enough CTAs for ~4 per SM at decode sizes, one per token for long prefills
   const int work = (q_heads + kv_heads) * (head_dim / 2);
   int parts = (work + 255) / 256;
-  while (parts > 1 && tokens * parts > 148 * 8) parts = (parts + 1) / 2;
+  while (parts > 1 && tokens * parts > device_sms() * 8) parts = (parts + 1) / 2;
   const dim3 grid((unsigned)tokens, (unsigned)parts);
 #define FXPR_ROPE(TT)                                                                                  \
   (void)launch_pdl(rope_kv_write_kernel<TT>, grid, dim3(256), 0, s, 1u,                                \
@@ -167,7 +169,7 @@ extern "C" int fxpr_silu_mul_pairs(const void* gate_up, int dtype, void* out, in
   if (!gate_up || !out) return FXPR_ERR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t n = rows * f;
-  const unsigned grid = (unsigned)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
+  const unsigned grid = (unsigned)(std::min<int64_t>((n + 255) / 256, device_sms() * 16));
 #define FXPR_SILU_PAIRS(TT)                                                                         \
   (void)launch_pdl(silu_mul_pairs_kernel<TT>, dim3(grid), dim3(256), 0, s, 1u, (const TT*)gate_up,  \
                    (TT*)out, rows, f)

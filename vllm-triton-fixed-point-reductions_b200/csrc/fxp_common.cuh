@@ -20,6 +20,7 @@ namespace fxpr {
 // ---- host-side error plumbing ------------------------------------------------
 void set_last_error(const char* what, cudaError_t err);
 int check_launch(const char* what);
+int device_sms();                        // of the current device
 
 inline int ceil_div_i(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 

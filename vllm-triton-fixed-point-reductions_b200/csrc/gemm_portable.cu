@@ -296,11 +296,11 @@ int gemm_portable_launch(const void* a, const void* b, const void* bias, void* c
   const float scale = (float)(1ull << frac_bits);
   // Few rows, B readable 4 columns at a time and K-tiles for the eight warps of a CTA: one K-tile per warp,
   // 8 or 16 rows.  Three such row blocks cost less than one 64-row tile (27x28672x4096 fp32 836 -> 499 us).
-  const int k_tiles = ceil_div_i(K, k_tile);
+  const int k_tiles = ceil_div_i(K, k_tile), sms = device_sms();
   if (M <= 48 && k_tiles >= 8 && b_sn == 1 && b_sk % 4 == 0 && N % 4 == 0 && ((uintptr_t)b % (4 * sizeof(T))) == 0) {
     const int64_t cols = ceil_div_i(N, 128), blocks = ceil_div_i(M, M <= 8 ? 8 : 16);
     int splits = 1;
-    while (splits < 8 && splits * 8 < k_tiles && cols * blocks * splits * 2 <= 4 * 148) splits *= 2;
+    while (splits < 8 && splits * 8 < k_tiles && cols * blocks * splits * 2 <= 4 * sms) splits *= 2;
     auto rows = [&](auto kernel) {
       const cudaError_t e = launch_pdl(kernel, dim3((unsigned)(cols * splits), (unsigned)blocks), dim3(256), 0, s, (unsigned)splits,
                                        (const T*)a, (const T*)b, (const T*)bias, (T*)c, c_int, partials, (int)M, (int)N,
@@ -322,9 +322,9 @@ int gemm_portable_launch(const void* a, const void* b, const void* bias, void* c
     double fee = r == 4 ? 1.17 : 1.0;
     for (int n = 1; n <= 8 && n <= std::max(1, ceil_div_i(K, k_tile)); n *= 2, fee *= 1.03) {
       const int per_sm = portable_ctas(r);
-      const int64_t whole = ctas * n / (148 * per_sm), rest = ctas * n % (148 * per_sm);
+      const int64_t whole = ctas * n / (sms * per_sm), rest = ctas * n % (sms * per_sm);
       // a last round of fewer CTAs per SM is shorter, but never as short as its share
-      const double rounds = (double)whole * per_sm + (rest ? std::max(0.6 * per_sm, (double)((rest + 147) / 148)) : 0.0);
+      const double rounds = (double)whole * per_sm + (rest ? std::max(0.6 * per_sm, (double)ceil_div_i(rest, sms)) : 0.0);
       const double cost = rounds * r / n * fee;
       if (cost < best) { best = cost; rm = r; splits = n; }
     }
@@ -367,7 +367,7 @@ static int epilogue_dispatch(const void* c_int, int int_bits, const void* bias, 
                              int64_t N, int64_t c_sm, float inv, cudaStream_t s) {
   const int64_t total = M * N;
   int grid = (int)((total + 255) / 256);
-  if (grid > 148 * 16) grid = 148 * 16;
+  grid = std::min(grid, device_sms() * 16);
   if (int_bits == 64)
     epilogue_from_int_kernel<T, long long><<<grid, 256, 0, s>>>((const long long*)c_int, (const T*)bias, (T*)c, M, N, c_sm, inv);
   else if (int_bits == 32)

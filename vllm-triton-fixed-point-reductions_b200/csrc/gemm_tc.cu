@@ -353,17 +353,16 @@ bool tc_make_map(CUtensorMap* m, int dtype, const void* base, int64_t rows, int6
 }
 
 int tc_device_sms() {
-  static int cached[64] = {0};
+  static int cached[64] = {0};             // 1: compute capability 10.x, -1: another
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
   if (!cached[dev]) {
-    int n = 0, major = 0;
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    int major = 0;
     cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
-    cached[dev] = (major == 10 && n > 0) ? n : -1;
+    cached[dev] = major == 10 ? 1 : -1;
   }
-  return cached[dev];
+  return cached[dev] > 0 ? device_sms() : -1;
 }
 
 bool gemm_tc_supported(const GemmArgs& g) {
