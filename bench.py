@@ -39,9 +39,10 @@ METRIC = "fxp GEMM TFLOP/s + split-K decode attn GB/s (% roofline); bitwise-inva
 GEMM = dict(M=4096, N=4096, K=4096, k_tile=64, int_bits=64, frac_bits=16)
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
 NOMINAL = {"hbm_gbs": 8000.0, "bf16_tflops": 2250.0}
-# DRAM bytes of one launch of the headline kernel, from its ncu capture (71.4 MB read + 16.2 MB
-# written); a profiler cannot run inside the timed bench, so the captured figure is quoted
-GEMM_DRAM_TRAFFIC_BYTES = 87.6e6
+# DRAM bytes of one launch of the headline kernel (gemm_tc_pair_kernel) on this workload, from an ncu
+# capture of this program (107.8 MB read + 33.9 MB written); a profiler cannot run inside the timed
+# bench, so the captured figure is quoted
+GEMM_DRAM_TRAFFIC_BYTES = 141.7e6
 
 
 def load_peaks():
@@ -366,8 +367,8 @@ def run_gpu_arm(args):
         "roofline": {"bound": "tensor", "achieved": per_gpu, "peak": peak, "unit": "TFLOP/s",
                      "frac": per_gpu / peak, "traffic": GEMM_DRAM_TRAFFIC_BYTES,
                      "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of "
-                                       "this kernel on this workload: A and B once (67.1 MB) plus the part "
-                                       "of C that left L2 during the launch",
+                                       "this kernel on this workload: A and B (67.1 MB, read 1.6 times) "
+                                       "and C (33.5 MB)",
                      "peak_source": f"{peaks['source']} cuBLAS bf16 burst",
                      "frac_of_nominal_2250": per_gpu / NOMINAL["bf16_tflops"],
                      "algorithmic": "2*M*N*K = 137.44 GFLOP per launch"},

@@ -26,8 +26,11 @@
 //   conversion  eight warps: P.V partials to Q-format on the FP32 and integer pipes (packed add of
 //               1.5 * 2^(23-f), raw bits summed in 32-bit registers, magnitude screen, exact fix-up
 //               from tensor memory) while the other roles work on the next tiles.
-// Bound: the conversion and softmax arithmetic of a tile on the ALU, FMA and MUFU pipes,
-// not its tensor work (768 clocks in two passes).  16 prompts of 128 to 4096 tokens, 32/8 heads: 2570 -> 1340 us.
+// Bound: the softmax groups, as chains of dependent steps and not by any unit's rate.  A tile takes an SM about
+// 2430 clocks (its tensor work is 768); a group spends 4860 clocks on a tile of its own and the other group's, of
+// which 2050 make weights and P, 565 maxima, 1420 are waits for scores and buffers, and the MMA warp waits for
+// copies a tenth of the time.  Issue slots are half busy, ALU 40 %, MUFU 28 %, tensor pipe 27 %.
+// 16 prompts of 128 to 4096 tokens, 32/8 heads: 2570 -> 1410 us.
 // KV splits are not handled here (the dispatcher sends them to attention_mma.cu: same bits).
 // Every wait is bounded; on a time-out the CTA sets the status word and leaves.
 #include <algorithm>

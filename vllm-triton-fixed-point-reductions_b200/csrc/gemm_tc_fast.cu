@@ -3,34 +3,31 @@
 // fp32 partial has to be rounded to Q-format and integer-added for every 2*k_tile
 // flops, i.e. ~64 elements per clock per SM at k_tile = 64.
 //
-//   * rounding runs on the FP32 pipe: r = fma(p, 2^f, 1.5*2^23) has rint-half-even of
-//     p*2^f in its mantissa whenever |p*2^f| < 2^22, so float_as_int(r) = MAGIC + q.
-//     The raw bit patterns are summed in int32 and MAGIC * (#tiles) is subtracted once.
-//   * a one-instruction-per-two-partials screen (OR of the raw fp32 bits, test bit 30,
-//     i.e. "some |p| >= 2") sends a K-tile to an exact fix-up that uses the reference's
-//     cvt.rni conversion (fxpr_vllm/_triton/fxp.py:92-108) for every out-of-range
-//     partial, so results equal the plain conversion for every input.
+//   * rounding runs on the FP32 pipe: p + 1.5*2^(23-f) has rint-half-even of p*2^f in its
+//     mantissa whenever |p*2^f| < 2^22.  The raw bit patterns are summed in int32 and the
+//     constant * (#tiles) is taken out (gemm_tc_fast_common.cuh).
+//   * a three-input maximum per two partials screens a K-tile's magnitudes; one beyond the
+//     range sends it to an exact fix-up that uses the reference's cvt.rni conversion
+//     (fxpr_vllm/_triton/fxp.py:92-108) for every out-of-range partial, so results equal
+//     the plain conversion for every input.
 //   * int64 semantics with 32-bit registers: in-range addends are < 2^22, so up to 510
 //     K-tiles cannot overflow int32; out-of-range addends go to per-thread side arrays
 //     in local memory that are touched only on that rare path.
 //
 // Tile 128 x 128, one persistent CTA per SM.  Warp 0 = TMA producer, warp 1 = MMA issuer,
-// then 16 epilogue warps (TMEM lane quarter x 32-column group).  The single-lane roles are
-// latency-bound: an mbarrier probe, a tcgen05 fence, an MMA issue and a commit each take
-// 50-100 cycles of the issuing thread, so the pipeline hands over 128 of K at a time
-// ("super-stage": for k_tile 64 a pair of K-tiles into two TMEM buffers, each with a fresh
-// accumulator; for k_tile 128 one K-tile): one full/empty and one tensor-full/empty
-// hand-off per 8 MMAs.  Every index (stage, TMEM group, barrier phase) is a function of the
-// running super-stage number, so the roles need no communication beyond the barriers.
+// then 16 epilogue warps (TMEM lane quarter x 32-column group).  The pipeline hands over
+// 128 of K at a time ("super-stage": for k_tile 64 a pair of K-tiles into two TMEM buffers,
+// each with a fresh accumulator; for k_tile 128 one K-tile): one full/empty and one
+// tensor-full/empty hand-off per 8 MMAs.  Every index (stage, TMEM group, barrier phase) is
+// a function of the running super-stage number, so the roles need no communication beyond
+// the barriers.
 //
-// Measured with clock64 stamps of CTA 0 at 4096^3, k_tile 64:
-// a super-stage takes ~1700 cycles against 512 cycles of tensor work; the issuer spends
-// ~1250 of them between "operands landed" and "committed" (MMA issue is paced at 65-80
-// cycles per MMA when nothing else runs and ~125 when the 16 epilogue warps convert), the
-// rest waiting for the epilogue to hand the TMEM group back.  Tried and measured slower or
-// equal: two issuer warps (one per TMEM group; correct, -10 %), four single-buffer groups
-// for k_tile 128 (equal), software-pipelined or pairwise TMEM loads in the epilogue
-// (-6 % / -11 %), no TMA copies at all (equal: shared-memory bandwidth is not the limit).
+// It serves 65 to some 700 rows, split K and the dumps; large products take the two-SM kernel
+// (gemm_tc_pair.cu).  Bound: operands out of L2, since each tile fetches its own 128 rows and 128
+// columns.  333 x 6144 x 4096: 302 MB in 29 us = 10.4 TB/s; issue slots 52 % busy, tensor pipe 38 %.
+// Tried and measured slower or equal: two issuer warps (one per TMEM group, -10 %), four
+// single-buffer groups for k_tile 128 (equal), software-pipelined or pairwise TMEM loads in
+// the epilogue (-6 % / -11 %).
 // Split-K: per-split integer partial planes, summed by the last arriver.  All waits bounded.
 #include <cuda.h>
 
@@ -237,8 +234,9 @@ static int launch_fast(const CUtensorMap& ma, const CUtensorMap& mb, TcParams& p
 }
 
 // The fast route covers int32 / int64 accumulation while no item has more than 510
-// K-tiles (in-range addends are < 2^22, so their int32 sum cannot overflow) and the
-// "|p| < 2" screen implies "|p * 2^f| < 2^22" (f <= 21).
+// K-tiles (in-range addends are < 2^22, so their int32 sum cannot overflow).  Above 21 fraction
+// bits the range ends below |p| = 2 and ordinary partials would take the fix-up: the plain
+// conversion (gemm_tc.cu) serves those.
 bool gemm_tc_fast_supported(const GemmArgs& g, int split_k) {
   if (g.int_bits == 16) return false;
   if (g.frac_bits > 21) return false;

@@ -1,6 +1,6 @@
-// Pieces shared by the fast tensor-core GEMM kernels (gemm_tc_fast.cu, gemm_tc_skinny.cu):
-// the magic-number conversion constants, the exact fix-up of a K-tile accumulator and the
-// one-lane barrier wait.
+// Pieces shared by the fast tensor-core kernels (gemm_tc_fast.cu, gemm_tc_pair.cu, gemm_tc_skinny.cu,
+// attention_tc.cu, the decode attention): the magic-number conversion, the exact fix-up of a K-tile
+// accumulator and the barrier wait of a whole warp.
 #pragma once
 
 #include "fxp_common.cuh"
@@ -46,7 +46,7 @@ static __device__ __forceinline__ float q_screen_limit(float inv_scale) { return
 // 16 fp32 partials -> Q-format, added to acc; screen keeps the largest magnitude (valid while below
 // q_screen_limit).  Per partial half a packed add, one integer add and half a three-input maximum.
 // Integer adds run at half rate on the ALU pipe and multiply-adds at half rate on the FMA pipe, so
-// they are dealt out evenly: on 128 x 256 partials per SM 760-830 clocks, against 960 with scalar fma
+// they are dealt out evenly: on 128 x 256 partials per SM 760-830 clocks by itself, against 960 with scalar fma
 // and the adds left to the compiler (which puts them all on the FMA pipe).
 static __device__ __forceinline__ void convert16(const uint32_t (&v)[16], uint32_t* acc, uint64_t magic2,
                                                  uint32_t magic_bits, uint32_t one, float& screen) {

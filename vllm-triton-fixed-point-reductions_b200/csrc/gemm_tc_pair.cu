@@ -5,9 +5,13 @@
 // tile out of L2 (~140 us at 4096^3, against 82 us of tensor work).  Here each CTA loads its own 128
 // rows of A and its own 128 columns of B, 32 KB per step for the same accumulator; the tensor cores
 // of both SMs read both halves of B, and each CTA's tensor memory receives its 128 rows x 256
-// columns: with the conversion left out the kernel runs at 100 us.  The conversion of a K-tile costs
-// each SM about 760 clocks (32768 partials: packed add, integer add, range screen = 2.4 issue slots
-// per partial), the tensor work 512 clocks at K-tile 64 and 1024 at K-tile 128.
+// columns: with the conversion left out the kernel runs at 100 us.  What is left is the conversion.  By
+// itself a K-tile's 32768 partials take an SM about 760 clocks (packed add, integer add, range screen =
+// 2.4 issue slots per partial); in the kernel its warps need about 1150, as the four tcgen05.ld of a warp
+// are waited for one after the other (103 clocks each) and the other warps take issue slots.  At K-tile 64
+// (512 clocks of tensor work, 1350 a K-tile all in) they are at work 84 % of the time, ALU pipe 64 %, and
+// the tensor core waits for accumulators; at K-tile 128 (1024 clocks of tensor work) they wait a quarter
+// of the time and the tensor pipe is busy 63 %: the hand-over.  Times: 200 us and 141 us at 4096^3.
 //
 // What it depends on, measured at 4096^3 with the conversion left out:
 //   - MMAs, commits and copies are predicated instructions of a uniform warp (tc_common.cuh);
