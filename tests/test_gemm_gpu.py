@@ -520,3 +520,49 @@ def test_static_weights_promise_changes_no_bit(split):
                 x = (x0 * sc).to(torch.bfloat16)            # written by the kernel right before the GEMM
                 assert torch.equal(torch.ops.fxpr.gemm_fxp(x, w, None, 64, 16), wants[sc])
         assert torch.equal(torch.ops.fxpr.gemm_fxp(x0.to(torch.bfloat16), w, None, 64, 16), wants[1.0])
+
+
+def _split_calls(n):
+    """Operands of `n` products of more than 64 rows that split K through the scratch, and their results."""
+    out = []
+    for i in range(n):
+        M, N, K = (200, 300, 65, 128)[i % 4], (512, 384, 640)[i % 3], (4096, 2048)[i % 2]
+        a, b = _rand((M, K), torch.bfloat16, 300 + i).cuda(), _rand((K, N), torch.bfloat16, 400 + i, 0.05).cuda()
+        with L.overrides(gemm_split_k=1):
+            out.append((a, b, torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16)))
+    torch.cuda.synchronize()
+    return out
+
+
+def test_streams_that_split_k_at_the_same_time_do_not_share_scratch():
+    """Split products on more streams than scratch is kept for, all in flight together, round after round."""
+    streams = [torch.cuda.Stream() for _ in range(20)]
+    calls = _split_calls(len(streams))
+    with L.overrides(gemm_split_k=8):
+        for _ in range(5):
+            got = []
+            for s, (a, b, _) in zip(streams, calls):
+                with torch.cuda.stream(s):
+                    got += [torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16) for _ in range(3)]
+            torch.cuda.synchronize()
+            for i, g in enumerate(got):
+                assert torch.equal(g, calls[i // 3][2]), i
+
+
+def test_a_graph_that_splits_k_does_not_share_scratch_with_eager_calls():
+    (a, b, want), (a2, b2, want2) = _split_calls(2)
+    with L.overrides(gemm_split_k=8):
+        torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16)                  # sizes the scratch, as a warm-up does
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = [torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16) for _ in range(8)]
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        for _ in range(5):
+            with torch.cuda.stream(side):
+                graph.replay()
+            eager = [torch.ops.fxpr.gemm_fxp_int(a2, b2, 64, 16) for _ in range(8)]
+            torch.cuda.synchronize()
+            assert all(torch.equal(o, want) for o in outs)
+            assert all(torch.equal(o, want2) for o in eager)

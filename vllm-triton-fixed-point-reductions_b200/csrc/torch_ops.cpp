@@ -12,6 +12,7 @@
 #include <c10/util/Exception.h>
 #include <torch/library.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <mutex>
@@ -58,9 +59,14 @@ struct DeviceState {
   std::atomic<int32_t*> status_ptr{nullptr};
   std::atomic<int> sms{0};
   Tensor status;                       // int32 the kernels set when a bounded wait gives up
-  Tensor scratch;                      // zero-initialised split-K scratch, grown on demand
-  std::vector<Tensor> retired;         // replaced scratch: graphs captured with it stay valid
+  // Zero-initialised split-K scratch, grown on demand: one buffer for each of the streams that used one last,
+  // and one for all graphs.
+  struct StreamScratch { cudaStream_t stream; Tensor buffer; };
+  std::vector<StreamScratch> scratch;  // most recent use last, at most kScratchStreams
+  Tensor graph_scratch;
+  std::vector<Tensor> retired;         // replaced graph scratch: graphs captured with it stay valid
 };
+constexpr size_t kScratchStreams = 16;
 // never destroyed: the tensors must not outlive the CUDA context at process exit
 DeviceState* const g_dev = new DeviceState[kMaxDevices];
 
@@ -98,20 +104,40 @@ bool capturing() {
          st != cudaStreamCaptureStatusNone;
 }
 
-// The kernels re-zero the counters they used, so one buffer serves call after call.  A buffer that
-// was replaced stays alive for graphs captured with it; growing during a capture would allocate
-// and zero-fill inside the graph, so that is refused.
+// The kernels re-zero the counters they used, so one buffer serves call after call -- of ONE stream: calls that
+// overlap would take each other's partial sums and arrivals, so every stream has its own.  A stream's buffer is
+// allocated, cleared and used on that stream alone, so the allocator's own ordering makes dropping it safe, and the
+// stream not used for longest gives its buffer back.  Graphs share one further buffer, which outlives them
+// (graphs that run at the same time must not both split); growing it during a capture would allocate and
+// zero-fill inside the graph, so that is refused.
 Tensor gemm_scratch(int dev, int64_t bytes) {
   DeviceState& d = device_state(dev);
+  const auto cleared = [&] {
+    return at::zeros({std::max<int64_t>(bytes, 1 << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
+  };
   std::lock_guard<std::mutex> lock(d.mu);
-  const int64_t have = d.scratch.defined() ? d.scratch.numel() : 0;
-  if (have < bytes || !d.scratch.defined()) {
-    TORCH_CHECK(!capturing(), "gemm_fxp: split-K scratch of ", bytes, " bytes needed during CUDA-graph capture but only ",
-                have, " are allocated; run the shape once (or warmup_gemm) before capturing");
-    if (d.scratch.defined()) d.retired.push_back(d.scratch);
-    d.scratch = at::zeros({std::max<int64_t>(bytes, 1 << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
+  const int64_t for_graphs = d.graph_scratch.defined() ? d.graph_scratch.numel() : 0;
+  if (capturing()) {
+    TORCH_CHECK(for_graphs >= std::max<int64_t>(bytes, 1), "gemm_fxp: split-K scratch of ", bytes,
+                " bytes needed during CUDA-graph capture but only ", for_graphs,
+                " are allocated; run the shape once (or warmup_gemm) before capturing");
+    return d.graph_scratch;
   }
-  return d.scratch;
+  if (for_graphs < std::max<int64_t>(bytes, 1)) {
+    if (d.graph_scratch.defined()) d.retired.push_back(d.graph_scratch);
+    d.graph_scratch = cleared();
+  }
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev).stream();
+  auto& v = d.scratch;
+  auto it = std::find_if(v.begin(), v.end(), [&](const auto& s) { return s.stream == stream; });
+  if (it == v.end()) {
+    if (v.size() == kScratchStreams) v.erase(v.begin());
+    v.push_back({stream, cleared()});
+  } else {
+    if (it->buffer.numel() < bytes) it->buffer = cleared();
+    std::rotate(it, it + 1, v.end());
+  }
+  return v.back().buffer;
 }
 
 // ------------------------------------------------------------------ small helpers

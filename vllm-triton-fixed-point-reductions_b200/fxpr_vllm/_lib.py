@@ -194,9 +194,9 @@ def silu_mul_pairs(gate_up):
 # --------------------------------------------------------------------------
 
 def _get_gemm_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Persistent zero-initialised split-K scratch per device, grown on demand (the kernel
-    re-zeroes what it used; gemm.py:86-107 of the reference keeps one such buffer too).
-    ``warmup_gemm`` sizes it before CUDA-graph capture."""
+    """The current stream's persistent zero-initialised split-K scratch, grown on demand (the
+    kernel re-zeroes what it used; gemm.py:86-107 of the reference keeps one such buffer per device),
+    and with it the one of the device's CUDA graphs: ``warmup_gemm`` sizes both before capture."""
     nat.load_ops()
     return _native_ops.gemm_scratch(_device_index(device), nbytes)
 
