@@ -233,7 +233,7 @@ def run_reference_arm(args):
         "note": "the reference has no CPU path of its own (CUDA-only Triton kernels); unless "
                 "FXPR_REFERENCE_PATH is set this arm is the torch CPU restatement of its algorithm "
                 "from oracle/, so its ratio to the GPU arm compares devices, not kernels "
-                "(the reference's Triton kernel on a B200 of this pool: 264 TFLOP/s at K-tile 64)",
+                "(the reference's Triton kernel on a B200: 264 TFLOP/s at K-tile 64)",
     }
     print(json.dumps(line))
 
