@@ -302,6 +302,30 @@ def test_decode_shape_kernel_equals_wide_tile_kernel(dtype, M, kt, split, int_bi
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M", [3, 16, 17, 32, 63])
+@pytest.mark.parametrize("kt,split", [(64, 1), (128, 1), (64, 4), (128, 8), (64, 3), (128, 5)])
+def test_decode_shape_row_tiles(M, kt, split):
+    """Row tiles of 16, 32 and 64 at their edges, with more stages of K than the ring holds and, in the
+    cluster merge, ranks with fewer rows than the others or none: the integers of the wide kernel."""
+    from fxpr_vllm import _native as nat
+
+    N, K = 392, 4168
+    a = _rand((M, K), torch.bfloat16, 221).cuda()
+    b = _rand((K, N), torch.bfloat16, 222, 0.05).cuda()
+    a[M - 1, 700:764] = 3.0e4                      # one K-tile beyond the fast conversion's range
+    with L.overrides(gemm_k_tile=kt, gemm_split_k=split):
+        got = torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16)
+        best = L.gemm_fxp_argmax(a, b, None, 64, 16) if split == 1 else None
+    with L.overrides(gemm_k_tile=kt, gemm_split_k=1, gemm_flags=nat.GEMM_NO_SKINNY):
+        want = torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16)
+        want_c = torch.ops.fxpr.gemm_fxp(a, b, None, 64, 16)
+    assert torch.equal(got, want)
+    if best is not None:
+        assert torch.equal(best[0].view(torch.int16), want_c.view(torch.int16))
+        assert torch.equal(L.argmax_from_keys(best[1]), want_c.argmax(dim=-1))
+    L.check_device_status()
+
+
 def test_decode_row_bits_do_not_depend_on_the_batch():
     """Row r of a 64-row launch (decode-shape kernel) equals row r of a 300-row launch."""
     a = _rand((300, 1024), torch.bfloat16, 211).cuda()

@@ -43,17 +43,18 @@ static __device__ __forceinline__ float max3_abs(float a, float b, float c) {
 // Partials below this magnitude keep rint(p * 2^f) within +-(2^22 - 1).
 static __device__ __forceinline__ float q_screen_limit(float inv_scale) { return __fmul_rn(4194303.0f, inv_scale); }
 
-// 16 fp32 partials -> Q-format, added to acc; screen keeps the largest magnitude (valid while below
+// N fp32 partials -> Q-format, added to acc; screen keeps the largest magnitude (valid while below
 // q_screen_limit).  Per partial half a packed add, one integer add and half a three-input maximum.
 // Integer adds run at half rate on the ALU pipe and multiply-adds at half rate on the FMA pipe, so
 // they are dealt out evenly: on 128 x 256 partials per SM 760-830 clocks by itself, against 960 with scalar fma
 // and the adds left to the compiler (which puts them all on the FMA pipe).
-static __device__ __forceinline__ void convert16(const uint32_t (&v)[16], uint32_t* acc, uint64_t magic2,
+template <int N>
+static __device__ __forceinline__ void convert_n(const uint32_t (&v)[N], uint32_t* acc, uint64_t magic2,
                                                  uint32_t magic_bits, uint32_t one, float& screen) {
 #pragma unroll
-  for (int i = 0; i < 16; i += 2) screen = max3_abs(screen, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+  for (int i = 0; i < N; i += 2) screen = max3_abs(screen, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
 #pragma unroll
-  for (int i = 0; i < 16; i += 2) {
+  for (int i = 0; i < N; i += 2) {
     uint64_t r;
     uint32_t r0, r1;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(v[i], v[i + 1])), "l"(magic2));
@@ -63,6 +64,10 @@ static __device__ __forceinline__ void convert16(const uint32_t (&v)[16], uint32
     if (alu_add(i + 1)) acc[i + 1] = acc[i + 1] + r1 - magic_bits;
     else asm("mad.lo.u32 %0, %1, %2, %0;" : "+r"(acc[i + 1]) : "r"(r1), "r"(one));
   }
+}
+static __device__ __forceinline__ void convert16(const uint32_t (&v)[16], uint32_t* acc, uint64_t magic2,
+                                                 uint32_t magic_bits, uint32_t one, float& screen) {
+  convert_n<16>(v, acc, magic2, magic_bits, one, screen);
 }
 
 // Rare path, entered by a whole warp (tcgen05.ld is warp-collective): for `ncols` columns of one
