@@ -305,6 +305,51 @@ def test_tcgen05_prefill_kernel_equals_mma_sync_kernel(case):
     assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
 
 
+@pytest.mark.parametrize("head_dim,case", [
+    # (seq_lens, q_lens, q heads, kv heads, page, dtype, int_bits, extra arguments)
+    (64, ([1, 16, 63, 64, 65, 127, 128, 129, 385], [1, 16, 63, 64, 65, 127, 128, 129, 385], 32, 8, 16, torch.bfloat16, 64, {})),
+    (64, ([700, 90, 1000], [300, 90, 1], 32, 8, 16, torch.float16, 32, {})),  # chunked prefill beside a decode row
+    (64, ([500, 129], [100, 129], 8, 8, 32, torch.float16, 64, {})),
+    (64, ([192, 193, 257], [192, 64, 257], 16, 1, 48, torch.bfloat16, 64, {})),
+    (64, ([700, 90], [700, 90], 32, 8, 64, torch.bfloat16, 64, dict(window=100))),
+    (64, ([300, 257], [300, 200], 16, 2, 16, torch.bfloat16, 64, dict(softcap=30.0, alibi=True))),
+    (64, ([300, 257], [300, 200], 32, 8, 16, torch.bfloat16, 64, dict(causal=False))),
+    (64, ([385] * 24, [385] * 24, 32, 8, 16, torch.bfloat16, 64, {})),
+    (128, ([65] * 300, [65] * 300, 4, 1, 16, torch.bfloat16, 64, {})),         # one and two tiles, many items a CTA
+    (128, ([1500, 20, 900], [1500, 20, 900], 32, 8, 16, torch.bfloat16, 64, dict(softcap=50.0, window=128))),
+    (128, ([1200, 700], [1200, 700], 16, 4, 16, torch.bfloat16, 64, dict(outliers=True))),
+    (64, ([1200, 700], [1200, 700], 16, 4, 16, torch.bfloat16, 64, dict(outliers=True))),
+])
+def test_prefill_kernel_forms(head_dim, case):
+    """Both head sizes, score products with one or two tiles, items shorter than the pipeline is deep, strided
+    Q and O, V values whose partials leave the fast conversion's range: the bits of the mma.sync kernel."""
+    from fxpr_vllm import _native as nat
+    from fxpr_vllm import synthetic as syn
+
+    sls, qls, hq, hkv, page, dtype, int_bits, kw = case
+    kw = dict(kw)
+    q, kv, qsl, sl, bt = syn.paged_attention_inputs(sls, qls, q_heads=hq, kv_heads=hkv, head_dim=head_dim, page=page,
+                                                    dtype=dtype, seed=300 + len(sls) + hq)
+    if kw.pop("outliers", False):
+        kv[3::5, 1, 3, :, 5] = 5000.0
+    wide = torch.zeros(q.shape[0], hq, head_dim + 64, dtype=dtype, device="cuda")
+    wide[..., :head_dim] = q
+    q = wide[..., :head_dim]
+    alibi = None
+    if kw.pop("alibi", False):
+        alibi = torch.arange(1, hq + 1, device="cuda", dtype=torch.float32) * 0.01 * orc.RCP_LN2
+    outs = []
+    for flags in (0, nat.ATTN_NO_TCGEN05):
+        o = torch.full_like(wide, float("nan"))[..., :head_dim]
+        with L.overrides(attn_flags=flags):
+            torch.ops.fxpr.unified_attention_fxp(q, kv, o, qsl, sl, bt, max(qls), alibi, kw.get("causal", True), None,
+                                                 int_bits, 16, kw.get("softcap", 0.0), kw.get("window", 0), 1)
+        outs.append(o.contiguous())
+    L.check_device_status()
+    assert not outs[0].isnan().any()
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
+
+
 @pytest.mark.parametrize("hq,head_dim", [(32, 128), (128, 128), (32, 64)])     # 8- and 16-row tiles, both head sizes
 @pytest.mark.parametrize("splits", [1, 4])
 def test_decode_waits_that_give_up_are_reported_and_spoil_no_other_call(hq, head_dim, splits):

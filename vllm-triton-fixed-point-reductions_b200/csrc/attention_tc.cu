@@ -15,22 +15,25 @@
 // a decode step" (the decode kernel stays on mma.sync) and is what the tests assert.
 //
 // One CTA = 128 query rows of one KV head: a row is a (token, query head of the GQA group)
-// pair, so a K/V tile is fetched once for the whole group.  Roles:
-//   producers   two warps: Q by one box per item, K / V pages by one box per page piece (16 or 64
-//               slots) and whole head, 128-byte swizzle (attn_kv_map)
-//   issuer      one warp: S = Q.K^T (128 x 64 per tile, two tiles ahead in pass B) and P.V (128 x 128,
-//               a fresh accumulator per tile), P read from shared memory where the softmax warps put it
-//   softmax     two groups of four warps, a thread is one row, a group takes every other key tile.
-//               Pass A: row maxima straight from tensor memory, 128 keys a step (a row lives in one
-//               lane: no shuffles).  Pass B: weights, integer denominator, P -> shared memory
+// pair, so a K/V tile is fetched once for the whole group.  Roles, 24 warps:
+//   producers   two warps for V, four for K: a box per page piece (16 or 64 slots) and whole head, 128-byte
+//               swizzle (attn_kv_map); Q by one box per 64 dims.  The first V producer also makes the item list
+//   issuers     one warp for S = Q.K^T (128 keys a product in pass A, 64 in pass B), one for P.V (a fresh
+//               accumulator per tile); P is the tensor-memory operand, written over the scores it came from
+//   softmax     two groups of four warps, a thread is one row.  Pass A: row maxima straight from tensor memory
+//               (a row lives in one lane: no shuffles).  Pass B: a group takes every other tile: weights, integer
+//               denominator, P
 //   conversion  eight warps: P.V partials to Q-format on the FP32 and integer pipes (packed add of
 //               1.5 * 2^(23-f), raw bits summed in 32-bit registers, magnitude screen, exact fix-up
 //               from tensor memory) while the other roles work on the next tiles.
-// Bound: the softmax groups, as chains of dependent steps and not by any unit's rate.  A tile takes an SM about
-// 2430 clocks (its tensor work is 768); a group spends 4860 clocks on a tile of its own and the other group's, of
-// which 2050 make weights and P, 565 maxima, 1420 are waits for scores and buffers, and the MMA warp waits for
-// copies a tenth of the time.  Issue slots are half busy, ALU 40 %, MUFU 28 %, tensor pipe 27 %.
-// 16 prompts of 128 to 4096 tokens, 32/8 heads: 2570 -> 1410 us.
+// Bound: no unit's rate but instructions in flight.  A tile takes an SM about 2000 clocks; its tensor work is 900 (a
+// 128 x 64 x 16 product from shared memory takes 48 clocks and not 32: 6 KB of operands at 128 bytes a clock), its
+// exponentials 512 on the special-function unit, its copies about 1200 at the rate L2 gives all SMs at once.  The
+// schedulers issue 53 % of the time with six warps each, an instruction of a warp at work takes 6 clocks, and the
+// softmax warps wait a third of the time for scores, the conversion warps for P.V.
+// 16 prompts of 128 to 4096 tokens, 32/8 heads (one box, both sides): 1333 -> 1034 us against a kernel with P through
+// shared memory, one issuer for both products, every role decoding every item, and exact divisions per output.
+// With head size 64 882 us, where the mma.sync kernel takes 3114.
 // KV splits are not handled here (the dispatcher sends them to attention_mma.cu: same bits).
 // Every wait is bounded; on a time-out the CTA sets the status word and leaves.
 #include <algorithm>
@@ -46,19 +49,32 @@
 namespace fxpr {
 
 static constexpr int kTcTileN = 64;            // keys per tile (attention.py:32-36)
+static constexpr int kTcOpN = 2 * kTcTileN;    // keys per score product, in both passes
 static constexpr int kTcRows = 128;            // query rows per CTA = tensor-memory lanes
-static constexpr int kTcGroupWarps = 4;        // softmax group: thread = one row, all keys of every other tile
-static constexpr int kTcSoftWarps = 2 * kTcGroupWarps;
+static constexpr int kTcSoftWarps = 8;         // two groups of four warps, one per half of the score buffers: thread = one row
 static constexpr int kTcConvWarps = 8;         // conversion: thread = one row and half of the output columns
-static constexpr int kTcFirstSoft = 2;         // warp 0: TMA producer, warp 1: MMA issuer
+// warps 0, 1: score and P.V issuers; 2, 3: V producers (the first also decodes the item list); 4-7: K producers
+static constexpr int kTcVProducers = 2, kTcKProducers = 4;
+static constexpr int kTcFirstV = 2, kTcFirstK = kTcFirstV + kTcVProducers;
+static constexpr int kTcFirstSoft = kTcFirstK + kTcKProducers;
 static constexpr int kTcFirstConv = kTcFirstSoft + kTcSoftWarps;
-static constexpr int kTcFirstMore = kTcFirstConv + kTcConvWarps;   // further producer warps
-static constexpr int kTcProducers = 2;
-static constexpr int kTcThreads = (kTcFirstMore + kTcProducers - 1) * 32;
-static constexpr int kTcStages = 4;
+static constexpr int kTcThreads = (kTcFirstConv + kTcConvWarps) * 32;
+static constexpr int kTcItems = 4;             // ring of work items in shared memory
+static constexpr int kTcListGroup = 8;         // requests whose row blocks are dealt out together
+static constexpr int kTcItemReaders = kTcThreads / 32;
+// Registers: 24 warps, six per scheduler, launch with 80 a thread.  Conversion keeps 64 sums and two loads of
+// 16 in registers; the first eight warps give up what that takes.  Per scheduler: 2 x 48 + 2 x 88 + 2 x 104 = 6 x 80.
+static constexpr int kTcRegsLaunch = 80, kTcRegsFront = 48, kTcRegsSoft = 88, kTcRegsConv = 104;
+static_assert(kTcFirstSoft / 4 * kTcRegsFront + kTcSoftWarps / 4 * kTcRegsSoft + kTcConvWarps / 4 * kTcRegsConv <=
+              kTcThreads / 128 * kTcRegsLaunch, "setmaxnreg draws on the registers of the launch");
+static_assert(kTcFirstSoft % 4 == 0, "register shares go by groups of four warps");
+// (setmaxnreg.dec to more, or .inc to fewer, registers than a warp has is an illegal instruction)
+static_assert(kTcRegsFront <= kTcRegsLaunch && kTcRegsSoft >= kTcRegsLaunch && kTcRegsConv >= kTcRegsLaunch,
+              "the first eight warps give, the others take");
 
 struct TcAttnShape {
   int rows_per_token;      // GQA group size
+  int row_shift;           // log2 of it
   int tokens_per_block;    // 128 / rows_per_token
   int num_q_blocks;
   int page_size;
@@ -97,75 +113,104 @@ template <> __device__ __forceinline__ uint32_t pack2_tc<__half>(float lo, float
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <typename T, int HD>
+// D (tensor memory) = A (tensor memory, packed 16-bit pairs) . B (shared memory)
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate, uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// Bounded wait of a whole warp.  Eight to twelve warps of this kernel wait at any time, so a probe is few
+// instructions and little code: it parks for up to a microsecond (an arrival of its own CTA wakes it), probes are
+// counted instead of clocks, and the abort flag is looked at every 64.
+static constexpr int kParkProbes = 1 << 22;
+__device__ __forceinline__ bool mbar_park(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return __all_sync(0xffffffffu, ok);
+}
+__device__ __forceinline__ bool park_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
+  for (int probes = 0; probes < kParkProbes; ++probes) {
+    if (mbar_park(bar, parity)) return true;
+    if ((probes & 63) == 63 && __any_sync(0xffffffffu, *abort_flag)) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+
+template <int HD> struct TcAttnSmem {
+  static constexpr int kQBytes = kTcRows * HD * 2;             // slabs of 64 dims: 128 rows x 128 B
+  static constexpr int kKBytes = kTcOpN * HD * 2;              // [8-key group][64-dim half][8 keys][128 B]
+  static constexpr int kVBytes = kTcTileN * HD * 2;
+  static constexpr int kKStages = 3, kVStages = 3;
+  static constexpr int kQOff = 0, kKOff = 2 * kQBytes, kVOff = kKOff + kKStages * kKBytes;
+  static constexpr int kItemOff = kVOff + kVStages * kVBytes;                    // [kTcItems][8] ints
+  static constexpr int kMaxOff = kItemOff + kTcItems * 32;                       // [item parity][group][128] floats
+  static constexpr int kDenOff = kMaxOff + 2 * 2 * kTcRows * 4;      // [item parity][group][128] int64
+  static constexpr int kGoOff = kDenOff + 2 * 2 * kTcRows * 8;       // [group][item parity] ints
+  static constexpr int kBarOff = kGoOff + 64;
+  static constexpr int kBars = 4 + 2 * kKStages + 2 * kVStages + 2 * kTcItems + 2 + 4 + 2 + 4 + 4 + 4 + 1 + 4;
+  static constexpr int kTotal = kBarOff + kBars * 8 + 16 + 1024;
+  static_assert(kTotal <= 227 * 1024, "shared memory of an SM");
+};
+
+// PLAIN: scores are the scaled products (no soft-cap, no ALiBi) and the scale is positive, so a row's maximum
+// is the maximum of the raw products, scaled.
+template <typename T, int HD, bool PLAIN>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                        const __grid_constant__ CUtensorMap map_v, const AttnParams p, const TcAttnShape sh,
                        int32_t* status, const int zero /* always 0: keeps the side arrays in local memory */) {
-  static_assert(HD == 128, "head size 128");
-  constexpr int kQBytes = kTcRows * HD * 2;                // 32 KB: two 64-dim slabs of 128 rows x 128 B
-  constexpr int kKBytes = kTcTileN * HD * 2;               // 16 KB: two slabs of 64 keys x 128 B
-  constexpr int kStageBytes = 2 * kKBytes;                 // K then V
-  constexpr int kPBytes = kTcRows * kTcTileN * 2;          // 16 KB: 128 rows x 128 B
-  constexpr int kBarOffset = kQBytes + kTcStages * kStageBytes + 2 * kPBytes;
+  static_assert(HD == 64 || HD == 128, "head size 64 or 128");
+  using Sm = TcAttnSmem<HD>;
+  constexpr int KST = Sm::kKStages, VST = Sm::kVStages;
   constexpr int kHalfCols = HD / 2;                        // P.V columns per conversion thread
-  constexpr uint32_t kColS = 0, kColPV = 256;              // tensor-memory columns: S[2] x 128, PV[2] x 128
+  // Tensor-memory columns: scores in four buffers of 64 keys (the maximum pass fills two neighbours, "half" 0 or
+  // 1; in the weight pass P of a tile replaces the first 32 columns of its scores), then two P.V accumulators
+  constexpr uint32_t kColS = 0, kColPV = 256;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t q_s = smem_base, stage0 = smem_base + kQBytes, p_s0 = stage0 + kTcStages * kStageBytes;
-  const uint32_t bar_base = smem_base + kBarOffset;
-  // barriers: qfull | full[4] empty[4] | sfull[2] sfree[2] | pready[2] | pvfull[2] pvfree[2] | sync | qfree |
-  // denfull[2] denfree[2]
-  const uint32_t qfull = bar_base, full0 = bar_base + 8, empty0 = full0 + 8 * kTcStages;
-  const uint32_t sfull0 = empty0 + 8 * kTcStages, sfree0 = sfull0 + 16, pready0 = sfree0 + 16;
-  const uint32_t pvfull0 = pready0 + 16, pvfree0 = pvfull0 + 16, soft_bar = pvfree0 + 16;
-  const uint32_t qfree = soft_bar + 8, denfull0 = qfree + 8, denfree0 = denfull0 + 16;
-  constexpr int kMisc = 8 * (1 + 2 * kTcStages + 10 + 2 + 4);
-  volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem_gen + kBarOffset + kMisc);
-  volatile int* abort_flag = (volatile int*)(smem_gen + kBarOffset + kMisc + 8);
-  float* rmax_s = (float*)(smem_gen + kBarOffset + kMisc + 16);                 // [item parity][group][128]
-  long long* den_s = (long long*)(smem_gen + kBarOffset + kMisc + 16 + 2048);   // [item parity][group][128]
+  const uint32_t q_s0 = smem_base + Sm::kQOff, k_s0 = smem_base + Sm::kKOff, v_s0 = smem_base + Sm::kVOff;
+  const uint32_t qfull0 = smem_base + Sm::kBarOff, qfree0 = qfull0 + 16;          // [2] each
+  const uint32_t kfull0 = qfree0 + 16, kempty0 = kfull0 + 8 * KST;
+  const uint32_t vfull0 = kempty0 + 8 * KST, vempty0 = vfull0 + 8 * VST;
+  const uint32_t ifull0 = vempty0 + 8 * VST, iempty0 = ifull0 + 8 * kTcItems;
+  const uint32_t sfa0 = iempty0 + 8 * kTcItems;            // [half]: scores of the maximum pass
+  const uint32_t sfb0 = sfa0 + 16;                         // [buffer]: scores of the weight pass
+  const uint32_t afree0 = sfb0 + 32;                       // [half]: maximum pass has read the scores
+  const uint32_t pready0 = afree0 + 16;                    // [buffer]: P is written
+  const uint32_t pdone0 = pready0 + 32;                    // [buffer]: P.V has read it
+  const uint32_t pvfull0 = pdone0 + 32, pvfree0 = pvfull0 + 16;                   // [accumulator]
+  const uint32_t soft_bar = pvfree0 + 16, denfull0 = soft_bar + 8, denfree0 = denfull0 + 16;
+  volatile uint32_t* tmem_slot = (volatile uint32_t*)(smem_gen + Sm::kBarOff + Sm::kBars * 8);
+  volatile int* abort_flag = (volatile int*)(smem_gen + Sm::kBarOff + Sm::kBars * 8 + 8);
+  float* rmax_s = (float*)(smem_gen + Sm::kMaxOff);
+  long long* den_s = (long long*)(smem_gen + Sm::kDenOff);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-  // ---- work items ---------------------------------------------------------------------
-  // Persistent CTAs over the padded list (request, row block, KV head), later row blocks (more keys)
-  // first, dealt out there and back again: straight round robin gives the first CTAs the longer item of
-  // every round (16 prompts of 128 to 4096 tokens: the busiest SM 15 % over the mean, 4 % this way).
-  // Drawing items from a counter in global memory balances better still but was slower (16 x 2048 tokens
-  // 1354 against 1223 us): the CTAs then stay in step and read the same cache lines at the same time.
-  // Every role walks the same list and keeps its ring positions and barrier phases running from one item
-  // to the next, so the producers fetch the next item's Q and first keys and the MMA warp starts its
-  // scores while the conversion warps still finish the current item.
-  auto item_of = [&](int r) -> int {
-    return r * (int)gridDim.x + (r & 1 ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
-  };
   const int hkv = p.num_kv_heads;
   const int G = sh.rows_per_token;
-  const int items_per_req = sh.num_q_blocks * hkv;
-  const int total_items = items_per_req * p.num_reqs;
-  struct Item { int live, req, kvh, q_start, q_len, tok0, seq_len, ctx, t0, t1; };
-  auto decode_item = [&](int w) -> Item {
-    Item I;
-    I.req = w / items_per_req;
-    const int rem = w - I.req * items_per_req;
-    const int qb = sh.num_q_blocks - 1 - rem / hkv;
-    I.kvh = rem % hkv;
-    I.q_start = p.qsl[I.req];
-    I.q_len = p.qsl[I.req + 1] - I.q_start;
-    I.tok0 = qb * sh.tokens_per_block;
-    I.live = I.tok0 < I.q_len;
-    I.seq_len = I.live ? p.seq_lens[I.req] : 0;
-    I.ctx = I.seq_len - I.q_len;
-    const int tok_end = min(I.q_len, I.tok0 + sh.tokens_per_block);
-    const int hi_key = p.causal ? min(I.seq_len, I.ctx + tok_end) : I.seq_len;
-    const int lo_key = p.window > 0 ? max(0, I.ctx + I.tok0 - p.window + 1) : 0;
-    I.t0 = lo_key / kTcTileN;
-    I.t1 = max(I.t0, (hi_key + kTcTileN - 1) / kTcTileN);
-    return I;
-  };
 
   if (threadIdx.x == 32) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
@@ -173,20 +218,19 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
   }
   if (threadIdx.x == 0) {
-    mbar_init(qfull, 1);
-    mbar_init(qfree, 1);
-    for (int s = 0; s < kTcStages; ++s) { mbar_init(full0 + 8u * s, kTcProducers); mbar_init(empty0 + 8u * s, 1); }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(sfull0 + 8u * b, 1); mbar_init(sfree0 + 8u * b, kTcGroupWarps);
-      mbar_init(pready0 + 8u * b, kTcGroupWarps);
-      mbar_init(pvfull0 + 8u * b, 1); mbar_init(pvfree0 + 8u * b, kTcConvWarps);
-      mbar_init(denfull0 + 8u * b, kTcSoftWarps); mbar_init(denfree0 + 8u * b, kTcConvWarps);
-    }
+    for (int i = 0; i < 2; ++i) { mbar_init(qfull0 + 8u * i, 1); mbar_init(qfree0 + 8u * i, 1); }
+    for (int i = 0; i < KST; ++i) { mbar_init(kfull0 + 8u * i, kTcKProducers); mbar_init(kempty0 + 8u * i, 1); }
+    for (int i = 0; i < VST; ++i) { mbar_init(vfull0 + 8u * i, kTcVProducers); mbar_init(vempty0 + 8u * i, 1); }
+    for (int i = 0; i < kTcItems; ++i) { mbar_init(ifull0 + 8u * i, 1); mbar_init(iempty0 + 8u * i, kTcItemReaders); }
+    for (int i = 0; i < 2; ++i) { mbar_init(sfa0 + 8u * i, 1); mbar_init(afree0 + 8u * i, 4); }
+    for (int i = 0; i < 4; ++i) { mbar_init(sfb0 + 8u * i, 1); mbar_init(pready0 + 8u * i, 4); mbar_init(pdone0 + 8u * i, 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(pvfull0 + 8u * i, 1); mbar_init(pvfree0 + 8u * i, kTcConvWarps); }
     mbar_init(soft_bar, kTcSoftWarps);
+    for (int i = 0; i < 2; ++i) { mbar_init(denfull0 + 8u * i, kTcSoftWarps); mbar_init(denfree0 + 8u * i, kTcConvWarps); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
+  if (warp == 0) {
     tmem_alloc(smem_u32((const void*)tmem_slot), 512);
     tmem_relinquish();
   }
@@ -195,368 +239,488 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0 || warp >= kTcFirstMore) {
-    // ------------------------------ K / V producers (TMA) -----------------------------
-    // A box is a 16-token page piece, or a whole 64-key tile when pages are multiples of 64 tokens, with
-    // all 128 head dims: [8-row group][64-dim half][8 rows][128 B], 4 or 16 KB.  The 8-row swizzle atoms
-    // of one half then lie 2 KB apart whatever the page size, which is all the MMA descriptors need.
-    // A 4 KB box takes the copy unit ~100 clocks and its warp about as long again for coordinates and
-    // barriers, with 20 warps on the SM: two warps share the eight boxes of a stage, compute their
-    // coordinates before they wait for it, and run loops without run-time choices.  (One warp with boxes
-    // of one half head, twice as many: 1760 clocks per stage, which bounded the kernel.)
-    // A stage is 32 KB: 128 keys of K in pass A, 64 keys of K and V in pass B.  Nothing is copied,
-    // and the block table is not read, past the end of the sequence; V rows there are cleared by the
-    // MMA warp before P.V.
-    const uint32_t e = elect_one();
-    const int me = warp == 0 ? 0 : warp - kTcFirstMore + 1;
-    int stage = 0; uint32_t phase = 1;
-    uint32_t q_phase = 1;                                    // qfree: the first wait passes
-    // Block-table entries are read 32 at a time (lane L: the 16-key group L of an 8-tile block), one
-    // block ahead of their use, and handed round by shuffle.
-    int page_shift = -1;
-    for (int b = 4; b < 31; ++b) if ((1 << b) == sh.page_size) page_shift = b;
-    for (int r = 0, w = blockIdx.x; w < total_items; w = item_of(++r)) {
-      const Item I = decode_item(w);
-      if (!I.live) continue;
-      const int kvh = I.kvh, seq_len = I.seq_len, t0 = I.t0, t1 = I.t1;
-      const int32_t* bt = p.block_table + (int64_t)I.req * p.bt_stride;
-      // Q rows: box {64 dims, G heads, 128 / G tokens} -> row = token * G + head.  Tokens past this
-      // request's (they belong to the next one, or lie beyond the tensor: zeros) are rows whose every
-      // key is masked and that are never stored.  The buffer is free once the MMA warp's last score
-      // MMA of the previous item has completed.
-      if (me == 0) {
-        if (!__all_sync(0xffffffffu, mbar_wait(qfree, q_phase, abort_flag))) goto producer_done;
-        q_phase ^= 1;
-        mbar_expect_tx(qfull, kQBytes, e);
-        tma_load_3d(q_s, &map_q, qfull, 0, kvh * G, I.q_start + I.tok0, e);
-        tma_load_3d(q_s + kQBytes / 2, &map_q, qfull, 64, kvh * G, I.q_start + I.tok0, e);
-      }
-      auto load_entries = [&](int tb) -> int {
-        const int n = tb * kTcTileN + lane * 16;
-        return (tb < t1 && n < seq_len) ? bt[page_shift >= 0 ? (n >> page_shift) : (n / sh.page_size)] : 0;
-      };
-      // one pass over the item's tiles; PASS and GS (log2 of the keys per box) are compile-time
-      auto walk = [&](auto pass_c, auto gs_c) -> bool {
-        constexpr int PASS = decltype(pass_c)::value, GS = decltype(gs_c)::value;
-        constexpr int kStep = PASS ? 1 : 2;                  // tiles per stage
-        constexpr int kPieces = (kStep * kTcTileN) >> GS;    // page pieces of K (and of V) per stage
-        constexpr int kBoxes = kPieces << PASS;              // box q: piece q of K, or piece q / 2 of K (even q) and V
-        constexpr int kMine = (kBoxes + kTcProducers - 1) / kTcProducers;
-        int cur = load_entries(t0);
-        for (int tb = t0; tb < t1; tb += 8) {
-          const int nxt = load_entries(tb + 8);
-          for (int tt = 0; tt < 8 && tb + tt < t1; tt += kStep) {
-            const int n0 = (tb + tt) * kTcTileN;
-            // only pieces that start inside the sequence (pass A: and before t1) are copied
-            const int pieces = (min(seq_len, t1 * kTcTileN) - n0 + (1 << GS) - 1) >> GS;
-            int blk[kMine], row8[kMine];
-            uint32_t bytes = 0;
-#pragma unroll
-            for (int i = 0; i < kMine; ++i) {
-              const int q = me + i * kTcProducers, piece = PASS ? q >> 1 : q;
-              blk[i] = __shfl_sync(0xffffffffu, cur, (tt * 4 + (piece << (GS - 4))) & 31);
-              const int n = n0 + (piece << GS);
-              row8[i] = (sh.page_mask ? (n & sh.page_mask) : (n % sh.page_size)) >> 3;
-              if (q < kBoxes && piece < pieces) bytes += 256u << GS;
-            }
-            if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8u * stage, phase, abort_flag))) return false;
-            const uint32_t fb = full0 + 8u * stage, ks = stage0 + stage * kStageBytes;
-            mbar_expect_tx(fb, bytes, e);
-#pragma unroll
-            for (int i = 0; i < kMine; ++i) {
-              const int q = me + i * kTcProducers, piece = PASS ? q >> 1 : q;
-              const bool v = PASS && (q & 1);
-              if (q < kBoxes && piece < pieces)
-                tma_load_5d(ks + (uint32_t)((v ? kKBytes : 0) + (piece << (GS + 8))), v ? &map_v : &map_k, fb, 0, 0,
-                            kvh * sh.head_chunks, row8[i], blk[i], e);
-            }
-            if (++stage == kTcStages) { stage = 0; phase ^= 1; }
-          }
-          cur = nxt;
-        }
-        return true;
-      };
-      using std::integral_constant;
-      const bool fetched = sh.group_shift == 4
-          ? walk(integral_constant<int, 0>{}, integral_constant<int, 4>{}) && walk(integral_constant<int, 1>{}, integral_constant<int, 4>{})
-          : walk(integral_constant<int, 0>{}, integral_constant<int, 6>{}) && walk(integral_constant<int, 1>{}, integral_constant<int, 6>{});
-      if (!fetched) goto producer_done;
+  // ---- work items ---------------------------------------------------------------------
+  // Persistent CTAs over the live (row block, request, KV head) of eight requests at a time, the last row blocks
+  // (most keys) of all of them first, dealt out there and back again.  That gives every CTA about the same work:
+  // request by request, a request's last, short items and the next one's long ones fall into one round.  All requests
+  // together balance best but spread the CTAs over more keys than L2 holds (16 prompts of 128 to 4096 tokens:
+  // requests by 32 1071 us, 8 1046, 1 1062; a static list with the dead entries in it left the busiest SM 10 % over the
+  // mean).
+  // The first V producer makes the list and leaves it in a ring in shared memory; every
+  // role reads them there in order.  (Decoded by each role for itself, two dependent global loads and a
+  // division per entry, dead ones included, took the softmax warps some 400 of 4860 clocks per two tiles.)
+  // Ring positions and barrier phases run on from one item to the next, so the producers fetch the next item's
+  // Q and first keys, and its scores are made, while the current one is still finished.
+  struct Item { int req, kvh, q_start, q_len, tok0, seq_len, t0, t1; };
+  int ipos = 0; uint32_t iphase = 0;                       // this role's position in the ring
+  auto read_item = [&](Item& I) -> bool {                  // ifull[ipos] has been waited for; false: no more items
+    const int4* src = reinterpret_cast<const int4*>(smem_gen + Sm::kItemOff + ipos * 32);
+    const int4 a = src[0], b = src[1];
+    I.req = a.x; I.kvh = a.y; I.q_start = a.z; I.q_len = a.w;
+    I.tok0 = b.x; I.seq_len = b.y; I.t0 = b.z; I.t1 = b.w;
+    __syncwarp();
+    mbar_arrive_if(iempty0 + 8u * ipos, lane == 0);
+    if (++ipos == kTcItems) { ipos = 0; iphase ^= 1; }
+    return __all_sync(0xffffffffu, I.req >= 0);
+  };
+  auto next_item = [&](Item& I) -> bool {
+    return park_wait(ifull0 + 8u * ipos, iphase, abort_flag) && read_item(I);
+  };
+  // Softmax and conversion warps work in groups of four, one on each scheduler.  One warp of a group probes the
+  // barrier, the others sleep in a hardware barrier: with all 20 probing, half of the issued instructions were
+  // probes.  After a wait that gave up a group goes on through its item, on whatever it reads (later waits then
+  // fail at once), so that its four warps always meet the same barriers; it leaves, all four, at the next item.
+  const int grp = (warp - kTcFirstSoft) >> 2;              // 0, 1 softmax, 2, 3 conversion
+  const bool prober = (warp & 3) == grp;
+  auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); };
+  auto group_wait = [&](uint32_t bar, uint32_t parity) {
+    if (prober) (void)park_wait(bar, parity, abort_flag);
+    group_sync();
+  };
+  volatile int* go = (volatile int*)(smem_gen + Sm::kGoOff) + 2 * grp;   // [item parity]: is there an item
+  auto group_next = [&](Item& I, int k) -> bool {
+    if (prober) {
+      const bool ok = park_wait(ifull0 + 8u * ipos, iphase, abort_flag);
+      if (lane == 0) go[k & 1] = ok;
     }
-  producer_done:;
-  } else if (warp == 1) {
-    // ------------------------------ MMA issuer ----------------------------------------
-    // S = Q . K^T: both operands K-major (head dim contiguous); Q in two slabs of 64 dims, K with the two
-    // halves of every 8-row group side by side
-    const uint32_t e = elect_one();
-    auto issue_s = [&](int stage, int sbuf, uint32_t idesc) {
-      const uint32_t d = tmem_base + kColS + (uint32_t)(sbuf * 128);
-      const uint64_t qd = make_smem_desc(q_s, 16, 1024);
-      const uint64_t kd = make_smem_desc(stage0 + stage * kStageBytes, 16, 2048);
-#pragma unroll
-      for (int kk = 0; kk < HD / 16; ++kk) {
-        const uint64_t ao = (uint64_t)((kk >> 2) * (kQBytes / 2) + (kk & 3) * 32) >> 4;
-        const uint64_t bo = (uint64_t)((kk >> 2) * 1024 + (kk & 3) * 32) >> 4;
-        umma_f16(d, qd + ao, kd + bo, idesc, kk ? 1u : 0u, e);
-      }
-      umma_commit(sfull0 + 8u * sbuf, e);
-    };
-    int stage = 0; uint32_t phase = 0;
-    int it = 0;                                              // S products issued so far (all items, both passes)
-    int jg = 0;                                              // P.V tiles issued so far (all items)
-    uint32_t q_phase = 0;
-    for (int r = 0, w = blockIdx.x; w < total_items; w = item_of(++r)) {
-    const Item I = decode_item(w);
-    if (!I.live) continue;
-    const int seq_len = I.seq_len, t0 = I.t0, t1 = I.t1, n_tiles = I.t1 - I.t0;
-    bool okq = mbar_wait(qfull, q_phase, abort_flag);
-    if (!__all_sync(0xffffffffu, okq)) goto issuer_done;
-    q_phase ^= 1;
-    {
-      // pass A: scores only, 128 keys at a time
-      for (int t = t0; t < t1; t += 2, ++it) {
-        const int sb = it & 1; const uint32_t sph = ((it >> 1) & 1) ^ 1;
-        const bool a = mbar_wait(full0 + 8u * stage, phase, abort_flag);
-        const bool b = mbar_wait(sfree0 + 8u * sb, sph, abort_flag);
-        if (!__all_sync(0xffffffffu, a && b)) goto issuer_done;
-        tc_fence_after();
-        issue_s(stage, sb, sh.idesc_s2);
-        umma_commit(empty0 + 8u * stage, e);
-        if (++stage == kTcStages) { stage = 0; phase ^= 1; }
-      }
-      // pass B: S runs two tiles ahead of P.V, one for each softmax group
-      int s_stage = stage; uint32_t s_phase = phase;         // ring position of the next S tile
-      auto issue_s_next = [&]() -> bool {
-        const int sb = it & 1; const uint32_t sph = ((it >> 1) & 1) ^ 1;
-        const bool a = mbar_wait(full0 + 8u * s_stage, s_phase, abort_flag);
-        const bool b = mbar_wait(sfree0 + 8u * sb, sph, abort_flag);
-        if (!__all_sync(0xffffffffu, a && b)) return false;
-        tc_fence_after();
-        issue_s(s_stage, sb, sh.idesc_s);
-        ++it;
-        if (++s_stage == kTcStages) { s_stage = 0; s_phase ^= 1; }
-        return true;
+    group_sync();
+    return go[k & 1] != 0 && read_item(I);
+  };
+
+  if (warp < kTcFirstSoft) {
+    regs_dec<kTcRegsFront>();
+    if (warp == 0) {
+      // ------------------------------ score issuer ------------------------------------
+      // Item by item the maximum pass, 128 keys a product into alternating halves of the score buffers, then the
+      // weight pass, 64 keys into the next of the four buffers: a softmax group then finds its next tile's scores
+      // in one buffer while P.V still reads the other (with products of 128 keys here too, a group waited 1250
+      // clocks per product for P.V and the next scores, next to 3700 at work).  Scores and P.V have a warp each:
+      // in one warp, in turn, the 12 MMAs, 5 commits and 5 waits of a tile were a chain of 1700 clocks next to 770
+      // of tensor work.  Everything here is warp-uniform also for the compiler (votes, values read by shuffle).
+      const uint32_t e = elect_one();
+      int half = 0;                                        // of the next maximum-pass product
+      int kst = 0; uint32_t kph = 0;
+      int qb = 0; uint32_t qph = 0;
+      uint32_t a_pend = 0, a_ph = 0, p_pend = 0, p_ph = 0; // what a half, a buffer is still waited for; phases
+      const uint64_t qd0 = make_smem_desc(q_s0, 16, 1024), kd0 = make_smem_desc(k_s0, 16, HD * 16);
+      auto half_free = [&](int h) -> bool {                // the maximum pass has read it
+        if (!(a_pend >> h & 1)) return true;
+        a_pend ^= 1u << h;
+        const uint32_t ph = a_ph >> h & 1;
+        a_ph ^= 1u << h;
+        return park_wait(afree0 + 8u * h, ph, abort_flag);
       };
-      for (int j = 0; j < 2 && j < n_tiles; ++j)
-        if (!issue_s_next()) goto issuer_done;
-      if (n_tiles <= 2) umma_commit(qfree, e);               // the item's last score MMA is issued
-      for (int j = 0; j < n_tiles; ++j, ++jg) {
-        if (j + 2 < n_tiles) {
-          if (!issue_s_next()) goto issuer_done;
-          if (j + 3 == n_tiles) umma_commit(qfree, e);
+      auto buffer_free = [&](int b) -> bool {              // P.V has read it
+        if (!(p_pend >> b & 1)) return true;
+        p_pend ^= 1u << b;
+        const uint32_t ph = p_ph >> b & 1;
+        p_ph ^= 1u << b;
+        return park_wait(pdone0 + 8u * b, ph, abort_flag);
+      };
+      // S = Q . K^T: both operands K-major (head dim contiguous); Q in slabs of 64 dims, K with the 64-dim
+      // halves of every 8-key group side by side
+      auto issue = [&](int column, uint64_t qd, uint64_t kd, uint32_t idesc) {
+        const uint32_t d = tmem_base + kColS + (uint32_t)column;
+#pragma unroll
+        for (int kk = 0; kk < HD / 16; ++kk) {
+          const uint64_t ao = (uint64_t)((kk >> 2) * (kTcRows * 128) + (kk & 3) * 32) >> 4;
+          const uint64_t bo = (uint64_t)((kk >> 2) * 1024 + (kk & 3) * 32) >> 4;
+          umma_f16(d, qd + ao, kd + bo, idesc, kk ? 1u : 0u, e);
         }
-        const int b = jg & 1; const uint32_t ph = (jg >> 1) & 1;
-        const bool r1 = mbar_wait(pready0 + 8u * b, ph, abort_flag);
-        const bool r2 = mbar_wait(pvfree0 + 8u * b, ph ^ 1, abort_flag);
-        if (!__all_sync(0xffffffffu, r1 && r2)) goto issuer_done;
-        tc_fence_after();
-        {
-          // Keys at or past the end of the sequence: their V rows were not copied (or come
-          // from slots nobody wrote) and 0 * NaN would poison the accumulator, so the rows
-          // are cleared.  Only the last tile of a sequence has any.
-          const int r0 = seq_len - (t0 + j) * kTcTileN;
-          if (r0 < kTcTileN) {
-            const uint32_t vs = stage0 + stage * kStageBytes + kKBytes;
-            for (int idx = lane; idx < (kTcTileN - r0) * 16; idx += 32) {
-              const int rr = r0 + (idx >> 4), cc = idx & 15;
-              const uint32_t addr = vs + (uint32_t)((rr >> 3) * 2048 + (cc >> 3) * 1024 + (rr & 7) * 128 + (cc & 7) * 16);
+      };
+      auto next_stage = [&]() {
+        umma_commit(kempty0 + 8u * kst, e);
+        if (++kst == KST) { kst = 0; kph ^= 1; }
+      };
+      Item I;
+      while (next_item(I)) {
+        const int tiles = __shfl_sync(0xffffffffu, I.t1 - I.t0, 0);
+        const uint64_t qd = qd0 + (uint64_t)(qb * (Sm::kQBytes >> 4));
+        if (!park_wait(qfull0 + 8u * qb, qph, abort_flag)) goto scores_done;
+#pragma unroll 1
+        for (int j = 0; j < tiles; j += 2) {
+          if (!half_free(half) || !buffer_free(2 * half) || !buffer_free(2 * half + 1)) goto scores_done;
+          if (!park_wait(kfull0 + 8u * kst, kph, abort_flag)) goto scores_done;
+          tc_fence_after();
+          issue(half * 128, qd, kd0 + (uint64_t)(kst * (Sm::kKBytes >> 4)), sh.idesc_s2);
+          umma_commit(sfa0 + 8u * half, e);
+          a_pend |= 1u << half;
+          next_stage();
+          half ^= 1;
+        }
+        int b = 2 * half;
+#pragma unroll 1
+        for (int j = 0; j < tiles; ++j) {
+          if (!half_free(b >> 1) || !buffer_free(b)) goto scores_done;
+          if (!(j & 1) && !park_wait(kfull0 + 8u * kst, kph, abort_flag)) goto scores_done;
+          tc_fence_after();
+          issue(b * 64, qd, kd0 + (uint64_t)(kst * (Sm::kKBytes >> 4) + (j & 1) * (kTcTileN * HD * 2 >> 4)), sh.idesc_s);
+          umma_commit(sfb0 + 8u * b, e);
+          p_pend |= 1u << b;
+          if ((j & 1) || j + 1 == tiles) next_stage();
+          half = (b >> 1) ^ 1;                             // not the half of the last tile
+          b = (b + 1) & 3;
+        }
+        umma_commit(qfree0 + 8u * qb, e);
+        qb ^= 1; if (qb == 0) qph ^= 1;
+      }
+    scores_done:;
+    } else if (warp == 1) {
+      // ------------------------------ P.V issuer --------------------------------------
+      const uint32_t e = elect_one();
+      int half = 0, acc = 0; uint32_t r_ph = 0, acc_ph = 1;   // half: of the next maximum-pass product
+      int vst = 0; uint32_t vph = 0;
+      const uint64_t vd0 = make_smem_desc(v_s0, 1024, HD * 16);
+      Item I;
+      while (next_item(I)) {
+        const int tiles = __shfl_sync(0xffffffffu, I.t1 - I.t0, 0);
+        const int keys = __shfl_sync(0xffffffffu, I.seq_len - I.t0 * kTcTileN, 0);
+        half ^= ((tiles + 1) >> 1) & 1;                    // the maximum pass's products
+        int b = 2 * half;
+#pragma unroll 1
+        for (int j = 0; j < tiles; ++j) {
+          if (!park_wait(vfull0 + 8u * vst, vph, abort_flag)) goto pv_done;
+          if (!park_wait(pvfree0 + 8u * acc, acc_ph, abort_flag)) goto pv_done;
+          if (!park_wait(pready0 + 8u * b, r_ph >> b & 1, abort_flag)) goto pv_done;
+          tc_fence_after();
+          // Keys at or past the end of the sequence: their V rows were not copied (or come from slots
+          // nobody wrote) and 0 * NaN would poison the accumulator, so the rows are cleared.  Only the
+          // last tile of a sequence has any.
+          const int n0 = keys - j * kTcTileN;
+          if (n0 < kTcTileN) {
+            const uint32_t vs = v_s0 + vst * Sm::kVBytes;
+#pragma unroll 1
+            for (int idx = lane; idx < (kTcTileN - n0) * (HD / 8); idx += 32) {
+              const int rr = n0 + idx / (HD / 8), cc = idx % (HD / 8);
+              const uint32_t addr = vs + (uint32_t)((rr >> 3) * (HD * 16) + (cc >> 3) * 1024 + (rr & 7) * 128 + (cc & 7) * 16);
               asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0) : "memory");
             }
             fence_proxy_async_smem();
             __syncwarp();
           }
-        }
-        // PV_j = P_j . V_j: P K-major (keys contiguous), V MN-major (head dim contiguous)
-        const uint32_t d = tmem_base + kColPV + (uint32_t)(b * HD);
-        const uint64_t pd = make_smem_desc(p_s0 + b * kPBytes, 16, 1024);
-        const uint64_t vd = make_smem_desc(stage0 + stage * kStageBytes + kKBytes, 1024, 2048);
+          // PV_j = P_j . V_j: P from tensor memory, V MN-major (head dim contiguous)
+          const uint32_t d = tmem_base + kColPV + (uint32_t)(acc * HD), pa = tmem_base + kColS + (uint32_t)(b * 64);
+          const uint64_t vd = vd0 + (uint64_t)(vst * (Sm::kVBytes >> 4));
 #pragma unroll
-        for (int kk = 0; kk < kTcTileN / 16; ++kk)
-          umma_f16(d, pd + (uint64_t)(kk * 2), vd + (uint64_t)(kk * 256), sh.idesc_pv, kk ? 1u : 0u, e);
-        umma_commit(pvfull0 + 8u * b, e);
-        umma_commit(empty0 + 8u * stage, e);
-        if (++stage == kTcStages) { stage = 0; phase ^= 1; }
+          for (int kk = 0; kk < kTcTileN / 16; ++kk)
+            umma_f16_ts(d, pa + (uint32_t)(kk * 8), vd + (uint64_t)(kk * (HD * 32 >> 4)), sh.idesc_pv, kk ? 1u : 0u, e);
+          umma_commit(pvfull0 + 8u * acc, e);
+          umma_commit(vempty0 + 8u * vst, e);
+          umma_commit(pdone0 + 8u * b, e);
+          r_ph ^= 1u << b;
+          half = (b >> 1) ^ 1;
+          b = (b + 1) & 3;
+          acc ^= 1; if (acc == 0) acc_ph ^= 1;
+          if (++vst == VST) { vst = 0; vph ^= 1; }
+        }
+      }
+    pv_done:;
+    } else {
+      // ------------------------------ K / V producers (TMA) ---------------------------
+      // A box is a 16-token page piece, or 64 keys when pages are multiples of 64 tokens, with all head
+      // dims.  The 8-row swizzle atoms of one 64-dim half lie HD * 16 bytes apart whatever the page size, which
+      // is all the MMA descriptors need.  Nothing is copied, and the block table is not read, past the end of
+      // the sequence or of the item's tiles; V rows there are cleared by the P.V issuer, scores there belong
+      // to no tile or are masked.
+      const uint32_t e = elect_one();
+      const bool is_v = warp < kTcFirstK, lists = warp == kTcFirstV;
+      const int me = is_v ? warp - kTcFirstV : warp - kTcFirstK;
+      const CUtensorMap* map = is_v ? &map_v : &map_k;
+      const uint32_t ring0 = is_v ? v_s0 : k_s0, full0 = is_v ? vfull0 : kfull0, empty0 = is_v ? vempty0 : kempty0;
+      const int step = is_v ? kTcTileN : kTcOpN, stages = is_v ? VST : KST, passes = is_v ? 1 : 2;
+      const int stage_bytes = is_v ? Sm::kVBytes : Sm::kKBytes;
+      int stage = 0; uint32_t phase = 1;
+      int qb = 0; uint32_t q_phase = 1;                    // qfree: the first waits pass
+      int page_shift = -1;
+#pragma unroll 1
+      for (int b = 4; b < 31; ++b) if ((1 << b) == sh.page_size) page_shift = b;
+      // ---- item list (first V producer): kTcListGroup requests at a time, one a lane
+      int l_start = 0, l_q = 0, l_seq = 0, l_blocks = 0;     // this lane's request
+      int group = -kTcListGroup, level = -1;                 // first of these requests; row block, from the last down
+      uint32_t round = 0, base = 0, target = blockIdx.x;     // live items before this level; this CTA's next one
+      bool ended = false;                                    // the end mark (req -1) is written
+      int wpos = 0, ahead = 0; uint32_t wphase = 1;          // ahead: items written and not yet read by this warp
+      auto fill_list = [&]() -> bool {
+        while (!ended && ahead < kTcItems) {
+          // wait only for a slot that this warp itself has to read next
+          if (ahead == 0) {
+            if (!park_wait(iempty0 + 8u * wpos, wphase, abort_flag)) return false;
+          } else if (!__all_sync(0xffffffffu, mbar_test_wait(iempty0 + 8u * wpos, wphase))) {
+            return true;
+          }
+          uint32_t live = 0;
+          while (!ended) {
+            if (level < 0) {
+              group += kTcListGroup;
+              if (group >= p.num_reqs) { ended = true; break; }
+              const int req = group + lane;
+              l_q = 0;
+              if (lane < kTcListGroup && req < p.num_reqs) { l_start = p.qsl[req]; l_q = p.qsl[req + 1] - l_start; l_seq = p.seq_lens[req]; }
+              l_blocks = min(sh.num_q_blocks, (l_q + sh.tokens_per_block - 1) / sh.tokens_per_block);
+              level = __reduce_max_sync(0xffffffffu, l_blocks) - 1;
+              continue;
+            }
+            live = __ballot_sync(0xffffffffu, l_blocks > level);
+            const uint32_t count = (uint32_t)(__popc(live) * hkv);
+            if (target < base + count) break;
+            base += count;
+            --level;
+          }
+          int who = 0, kvh = 0;
+          if (!ended) {
+            const int off = (int)(target - base), nth = off / hkv;
+            kvh = off - nth * hkv;
+            who = __ffs(__ballot_sync(0xffffffffu, (live >> lane & 1) && __popc(live & ((1u << lane) - 1)) == nth)) - 1;
+            ++round;
+            target = round * gridDim.x + (round & 1 ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+          }
+          if (lane == who) {
+            const int tok0 = level * sh.tokens_per_block;
+            const int ctx = l_seq - l_q, tok_end = min(l_q, tok0 + sh.tokens_per_block);
+            const int hi_key = p.causal ? min(l_seq, ctx + tok_end) : l_seq;
+            const int lo_key = p.window > 0 ? max(0, ctx + tok0 - p.window + 1) : 0;
+            const int t0 = lo_key / kTcTileN, t1 = max(t0, (hi_key + kTcTileN - 1) / kTcTileN);
+            int4* dst = reinterpret_cast<int4*>(smem_gen + Sm::kItemOff + wpos * 32);
+            dst[0] = make_int4(ended ? -1 : group + lane, kvh, l_start, l_q);
+            dst[1] = make_int4(tok0, l_seq, t0, t1);
+            mbar_arrive(ifull0 + 8u * wpos);
+          }
+          __syncwarp();
+          ++ahead;
+          if (++wpos == kTcItems) { wpos = 0; wphase ^= 1; }
+        }
+        return true;
+      };
+      Item I;
+      while ((!lists || fill_list()) && next_item(I)) {
+        --ahead;
+        const int32_t* bt = p.block_table + (int64_t)I.req * p.bt_stride;
+        const int end = min(I.seq_len, I.t1 * kTcTileN);   // keys to copy
+        // Q rows: box {64 dims, G heads, 128 / G tokens} -> row = token * G + head.  Tokens past this
+        // request's (they belong to the next one, or lie beyond the tensor: zeros) are rows whose every
+        // key is masked and that are never stored.
+        if (!is_v && me == 0) {
+          if (!park_wait(qfree0 + 8u * qb, q_phase, abort_flag)) break;
+          const uint32_t fb = qfull0 + 8u * qb;
+          mbar_expect_tx(fb, Sm::kQBytes, e);
+#pragma unroll
+          for (int c = 0; c < HD / 64; ++c)
+            tma_load_3d(q_s0 + qb * Sm::kQBytes + c * (kTcRows * 128), &map_q, fb, c * 64, I.kvh * G, I.q_start + I.tok0, e);
+          qb ^= 1; if (qb == 0) q_phase ^= 1;
+        }
+        // `passes` walks over the item's keys, `step` keys a stage; GS = log2 of the keys per box, `mine` boxes of
+        // a stage from `first` on are this warp's.  Block-table entries are read 32 at a time (lane L: the 16-key
+        // group L of a 512-key block), one block ahead of their use, and handed round by shuffle with the row in
+        // the page.
+        auto walk = [&](auto gs_c) -> bool {
+          constexpr int GS = decltype(gs_c)::value;
+          constexpr int kBoxBytes = (HD * 2) << GS;
+          constexpr int kMine = GS == 4 ? 2 : 1;             // 8 boxes of K over 4 warps, 4 of V over 2; or 2 and 1
+          static_assert((kTcOpN >> 4) / kTcKProducers == 2 && (kTcTileN >> 4) / kTcVProducers == 2, "boxes per warp");
+          const int first = me * kMine, start = I.t0 * kTcTileN, stop = I.t1 * kTcTileN;
+#pragma unroll 1
+          for (int pass = 0; pass < passes; ++pass) {
+            int cur = 0, cur_row = 0, nxt, nxt_row;
+#pragma unroll 1
+            for (int nb = start - 512; nb < stop; nb += 512) {
+              {
+                const int n = nb + 512 + lane * 16, pg = page_shift >= 0 ? n >> page_shift : n / sh.page_size;
+                nxt = n < end ? bt[pg] : 0;
+                nxt_row = (n - pg * sh.page_size) >> 3;
+              }
+              const int top = nb < start ? 0 : min(512, stop - nb);
+#pragma unroll 1
+              for (int off = 0; off < top; off += step) {
+                int blk[kMine], row8[kMine];
+                // of its boxes, those that start before the end
+                const int left = (end - (nb + off) + (1 << GS) - 1) >> GS;
+                const int boxes = max(0, min(kMine, min(step >> GS, left) - first));
+#pragma unroll
+                for (int i = 0; i < kMine; ++i) {
+                  const int from = ((off >> 4) + ((first + i) << (GS - 4))) & 31;
+                  blk[i] = __shfl_sync(0xffffffffu, cur, from);
+                  row8[i] = __shfl_sync(0xffffffffu, cur_row, from);
+                }
+                const uint32_t fb = full0 + 8u * stage;
+                const uint32_t dst = ring0 + (uint32_t)(stage * stage_bytes + first * kBoxBytes);
+                if (!park_wait(empty0 + 8u * stage, phase, abort_flag)) return false;
+                mbar_expect_tx(fb, (uint32_t)(boxes * kBoxBytes), e);
+#pragma unroll
+                for (int i = 0; i < kMine; ++i)
+                  if (i < boxes)
+                    tma_load_5d(dst + (uint32_t)(i * kBoxBytes), map, fb, 0, 0, I.kvh * sh.head_chunks, row8[i], blk[i], e);
+                if (++stage == stages) { stage = 0; phase ^= 1; }
+              }
+              cur = nxt; cur_row = nxt_row;
+            }
+          }
+          return true;
+        };
+        const bool fetched = sh.group_shift == 4 ? walk(std::integral_constant<int, 4>{}) : walk(std::integral_constant<int, 6>{});
+        if (!fetched) break;
       }
     }
-    }
-  issuer_done:;
   } else if (warp < kTcFirstConv) {
     // ------------------------------ softmax warps -------------------------------------
+    regs_inc<kTcRegsSoft>();
     const int quarter = warp & 3;
-    // Two groups take the score products in turn (group = product number & 1 = S buffer): while one
-    // loads or waits, the other keeps the exponential unit busy.
-    const int group = (warp - kTcFirstSoft) >> 2;
     const int row = quarter * 32 + lane;                     // tensor-memory lane = query row
-    const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
+    const uint32_t s_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + kColS;
     const float ninf = -__int_as_float(0x7f800000);
-    const bool plain_scores = !(p.cap_log2 > 0.0f) && p.alibi == nullptr;
-    const bool raw_max = plain_scores && p.ss_log2 > 0.0f;
     const uint64_t zero2 = pack2((uint32_t)zero, (uint32_t)zero);
     const uint64_t ss2 = pack2(__float_as_uint(p.ss_log2), __float_as_uint(p.ss_log2));
     const uint32_t mbits = q_magic_bits(p.inv_scale);
     const uint64_t magic2 = pack2(mbits, mbits);
-    uint32_t soft_phase = 0;
-    bool ok = true;
-    auto soft_sync = [&]() -> bool {                         // bounded barrier over these 8 warps
-      __syncwarp();
-      if (lane == 0) mbar_arrive(soft_bar);
-      const bool done = warp_wait(soft_bar, soft_phase, abort_flag);
-      soft_phase ^= 1;
-      return done;
-    };
-    int it = 0;                                              // S products consumed so far (all items, both passes)
-    int jg = 0;                                              // P tiles of the items before this one
-    int k = -1;                                              // live items so far
-    for (int r = 0, w = blockIdx.x; w < total_items && ok; w = item_of(++r)) {
-    const Item I = decode_item(w);
-    if (!I.live) continue;
-    ++k;
-    const int kvh = I.kvh, q_len = I.q_len, tok0 = I.tok0, seq_len = I.seq_len, ctx = I.ctx;
-    const int t0 = I.t0, t1 = I.t1, n_tiles = I.t1 - I.t0;
-    const int tok = tok0 + row / G, head = kvh * G + row % G;
-    const bool valid = tok < q_len;
-    const int pos = ctx + tok;
-    const int kend = valid ? (p.causal ? min(seq_len, pos + 1) : seq_len) : 0;
-    const int kbeg = valid ? (p.window > 0 ? max(0, pos - p.window + 1) : 0) : 0;
-    const float slope = (p.alibi && valid) ? p.alibi[head] : 0.0f;
-    // one score in log2 space with soft-cap and ALiBi (attention.py:103-121, 249-254)
-    auto score = [&](uint32_t v, int n) -> float {
-      float x = __fmul_rn(__uint_as_float(v), p.ss_log2);
-      if (p.cap_log2 > 0.0f) x = __fmul_rn(p.cap_log2, tanhf(__fdiv_rn(x, p.cap_log2)));
-      if (p.alibi) x = __fadd_rn(x, __fmul_rn(slope, __fsub_rn((float)n, (float)pos)));
-      return x;
-    };
-    // hand S buffer sb back to the MMA warp (this warp's share is in registers)
-    auto release_s = [&](int sb) {
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(sfree0 + 8u * sb);
-    };
+    // Group 0 takes the maximum-pass products in half 0 and, in the weight pass, the buffers 0 and 2, that is every
+    // other tile, group 1 the others.
+    const uint32_t s_half = s_addr + (uint32_t)(grp * 128);
+    uint32_t soft_phase = 0, a_phase = 0, b_phase = 0;       // b_phase: a bit for either buffer
+    int half = 0;                                            // of the next maximum-pass product
+    int k = -1;                                              // items so far
+    Item I;
+    while (group_next(I, ++k)) {
+      const int n_tiles = I.t1 - I.t0, n_ops = (n_tiles + 1) >> 1;
+      const int tok = I.tok0 + (row >> sh.row_shift);
+      const bool valid = tok < I.q_len;
+      const int pos = I.seq_len - I.q_len + tok;
+      const int kend = valid ? (p.causal ? min(I.seq_len, pos + 1) : I.seq_len) : 0;
+      const int kbeg = valid ? (p.window > 0 ? max(0, pos - p.window + 1) : 0) : 0;
+      const float slope = (!PLAIN && p.alibi && valid) ? p.alibi[I.kvh * G + (row & (G - 1))] : 0.0f;
+      // one score in log2 space with soft-cap and ALiBi (attention.py:103-121, 249-254)
+      auto score = [&](uint32_t v, int n) -> float {
+        float x = __fmul_rn(__uint_as_float(v), p.ss_log2);
+        if (p.cap_log2 > 0.0f) x = __fmul_rn(p.cap_log2, tanhf(__fdiv_rn(x, p.cap_log2)));
+        if (p.alibi) x = __fadd_rn(x, __fmul_rn(slope, __fsub_rn((float)n, (float)pos)));
+        return x;
+      };
 
-    // =============================== pass A: row maxima ===============================
-    // 128 keys per step, all of them in one thread.  Scaling by a positive constant is monotonic after rounding
-    // too, so the maximum is taken over the raw products and scaled once.
-    float rmax = ninf;
-    for (int t = t0; t < t1 && ok; t += 2, ++it) {
-      const int sb = it & 1;
-      if (sb != group) continue;
-      if (!warp_wait(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      float m = ninf;
+      // =============================== pass A: row maxima ===============================
+      // 128 keys per step, all of them in one thread.  Scaling by a positive constant is monotonic after
+      // rounding too, so the maximum is taken over the raw products and scaled once.
+      float rmax = ninf;
+#pragma unroll 1
+      for (int i = half ^ grp; i < n_ops; i += 2) {
+        group_wait(sfa0 + 8u * grp, a_phase);
+        a_phase ^= 1;
+        tc_fence_after();
+        float m = ninf;
+        const int first = I.t0 * kTcTileN + i * kTcOpN;
+        if (PLAIN && __all_sync(0xffffffffu, first >= kbeg && first + kTcOpN <= kend)) {
+          // no row of the warp is masked here
+          float m1 = ninf;                                   // two chains
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        tmem_ld32(tmem_base + lane_sel + kColS + (uint32_t)(sb * 128 + c * 32), v);
-        tmem_wait_ld_regs(v);
-        if (c == 3) release_s(sb);
-        const int n0 = t * kTcTileN + c * 32;
-        const bool inside = n0 >= kbeg && n0 + 32 <= kend;
-        if (raw_max) {
-          if (inside) {
-            float m1 = ninf;                                 // two chains
+          for (int c = 0; c < 4; ++c) {
+            uint32_t v[32];
+            tmem_ld32(s_half + (uint32_t)(c * 32), v);
+            tmem_wait_ld_regs(v);
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              m = max3(m, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
-              m1 = max3(m1, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
+            for (int x = 0; x < 32; x += 4) {
+              m = max3(m, __uint_as_float(v[x]), __uint_as_float(v[x + 1]));
+              m1 = max3(m1, __uint_as_float(v[x + 2]), __uint_as_float(v[x + 3]));
             }
-            m = fmaxf(m, m1);
+          }
+          m = fmaxf(m, m1);
+        } else {
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v[32];
+          tmem_ld32(s_half + (uint32_t)(c * 32), v);
+          tmem_wait_ld_regs(v);
+          const int n0 = first + c * 32;
+          if (n0 < kend && n0 + 32 > kbeg) {
+#pragma unroll
+            for (int x = 0; x < 32; ++x)
+              if (n0 + x >= kbeg && n0 + x < kend) m = fmaxf(m, PLAIN ? __uint_as_float(v[x]) : score(v[x], n0 + x));
+          }
+        }
+        }
+        // all of it has been read: hand the half back
+        tc_fence_before();
+        __syncwarp();
+        mbar_arrive_if(afree0 + 8u * grp, lane == 0);
+        rmax = fmaxf(rmax, PLAIN ? __fmul_rn(m, p.ss_log2) : m);
+      }
+      half ^= n_ops & 1;
+      float* rmax_k = rmax_s + (k & 1) * (2 * kTcRows);
+      rmax_k[grp * kTcRows + row] = rmax;
+      __syncwarp();
+      mbar_arrive_if(soft_bar, lane == 0);
+      group_wait(soft_bar, soft_phase);
+      soft_phase ^= 1;
+      float gmax = fmaxf(rmax_k[row], rmax_k[kTcRows + row]);
+      if (gmax == ninf) gmax = 0.0f;                         // rows without keys: exp2 gives 0, not NaN
+
+      // =============================== pass B ===========================================
+      uint32_t den32 = 0;
+      const uint64_t neg_max2 = pack2(__float_as_uint(-gmax), __float_as_uint(-gmax));
+      int done = 0;                                          // tiles of this group
+#pragma unroll 1
+      for (int j = grp; j < n_tiles; j += 2) {
+        const int b = (2 * half + j) & 3;
+        group_wait(sfb0 + 8u * b, b_phase >> (b >> 1) & 1);
+        b_phase ^= 1u << (b >> 1);
+        tc_fence_after();
+        const uint32_t sb = s_addr + (uint32_t)(b * 64);
+        const int first = (I.t0 + j) * kTcTileN;
+        const bool masks = __any_sync(0xffffffffu, first < kbeg || first + kTcTileN > kend);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t v[32];
+          tmem_ld32(sb + (uint32_t)(c * 32), v);
+          tmem_wait_ld_regs(v);
+          // d = score - max, rounded twice; the product is an fma with a run-time zero because the
+          // assembler contracts a packed multiply and the packed add behind it into one rounding.
+          // The weight of a masked key is exp2(-inf) = 0.
+          const int n0 = first + c * 32;
+          if (PLAIN) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+              uint64_t x;
+              asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x) : "l"(pack2(v[i], v[i + 1])), "l"(ss2), "l"(zero2));
+              asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(neg_max2));
+              asm("mov.b64 {%0, %1}, %2;" : "=r"(v[i]), "=r"(v[i + 1]) : "l"(x));
+            }
           } else {
 #pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__fsub_rn(score(v[i], n0 + i), gmax));
+          }
+          if (masks) {
+#pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (n0 + i >= kbeg && n0 + i < kend) m = fmaxf(m, __uint_as_float(v[i]));
+              if (n0 + i < kbeg || n0 + i >= kend) v[i] = __float_as_uint(ninf);
           }
-        } else {
+          // weights, integer denominator, P in the io dtype over the scores that were read (A operand of
+          // P.V: two keys a column)
+          uint32_t pk[16];
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (n0 + i >= kbeg && n0 + i < kend) m = fmaxf(m, score(v[i], n0 + i));
-        }
-      }
-      rmax = fmaxf(rmax, raw_max ? __fmul_rn(m, p.ss_log2) : m);
-    }
-    float* rmax_k = rmax_s + (k & 1) * (2 * kTcRows);
-    rmax_k[group * kTcRows + row] = rmax;
-    if (ok && !soft_sync()) ok = false;
-    float gmax = fmaxf(rmax_k[row], rmax_k[kTcRows + row]);
-    if (gmax == ninf) gmax = 0.0f;                           // rows without keys: exp2 gives 0, not NaN
-
-    // =============================== pass B ===========================================
-    uint32_t den32 = 0;
-    const uint64_t neg_max2 = pack2(__float_as_uint(-gmax), __float_as_uint(-gmax));
-    int mine = 0;                                            // tiles of this group
-    for (int j = 0; j < n_tiles && ok; ++j, ++it) {
-      const int t = t0 + j;
-      const int sb = it & 1;
-      if (sb != group) continue;
-      ++mine;
-      if (!warp_wait(sfull0 + 8u * sb, (it >> 1) & 1, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      const int g = jg + j, b = g & 1;
-      const uint32_t prow = p_s0 + b * kPBytes + (uint32_t)row * 128u;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t v[32];
-        tmem_ld32(tmem_base + lane_sel + kColS + (uint32_t)(sb * 128 + h * 32), v);
-        tmem_wait_ld_regs(v);
-        if (h == 1) release_s(sb);
-        // d = score - max, rounded twice; the product is an fma with a run-time zero because the
-        // assembler contracts a packed multiply and the packed add behind it into one rounding.
-        // The weight of a masked key is exp2(-inf) = 0.
-        const int n0 = t * kTcTileN + h * 32;
-        const bool inside = n0 >= kbeg && n0 + 32 <= kend;
-        if (plain_scores) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            uint64_t x;
-            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x) : "l"(pack2(v[i], v[i + 1])), "l"(ss2), "l"(zero2));
-            asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(neg_max2));
-            asm("mov.b64 {%0, %1}, %2;" : "=r"(v[i]), "=r"(v[i + 1]) : "l"(x));
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__fsub_rn(score(v[i], n0 + i), gmax));
-        }
-        if (!inside) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (n0 + i < kbeg || n0 + i >= kend) v[i] = __float_as_uint(ninf);
-        }
-        // weights, integer denominator, P in the io dtype -> shared memory (A operand of P.V):
-        // row = 128 bytes of 64 keys, 16-byte chunks XOR-swizzled with the row number
-        // (its buffer is free once the P.V product two tiles back has completed)
-        if (h == 0 && g >= 2 && !warp_wait(pvfull0 + 8u * b, ((g - 2) >> 1) & 1, abort_flag)) { ok = false; break; }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t pk[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float w0 = ex2_approx_tc(__uint_as_float(v[c * 8 + e * 2]));
-            const float w1 = ex2_approx_tc(__uint_as_float(v[c * 8 + e * 2 + 1]));
+          for (int i = 0; i < 16; ++i) {
+            const float w0 = ex2_approx_tc(__uint_as_float(v[2 * i]));
+            const float w1 = ex2_approx_tc(__uint_as_float(v[2 * i + 1]));
             uint64_t q;
             asm("add.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(pack2(__float_as_uint(w0), __float_as_uint(w1))), "l"(magic2));
             den32 = den32 + (uint32_t)q + (uint32_t)(q >> 32);
-            pk[e] = pack2_tc<T>(w0, w1);
+            pk[i] = pack2_tc<T>(w0, w1);
           }
-          const uint32_t addr = prow + (((uint32_t)(h * 4 + c) ^ (uint32_t)(row & 7)) << 4);
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]), "r"(pk[3]) : "memory");
+          tmem_st16(sb + (uint32_t)(c * 16), pk);            // over scores that have been read
         }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        mbar_arrive_if(pready0 + 8u * b, lane == 0);
+        ++done;
       }
-      if (!ok) break;
-      fence_proxy_async_smem();
+      if (n_tiles) half = (((2 * half + n_tiles - 1) & 3) >> 1) ^ 1;   // not the half of the last tile
+      // 64 weights per tile went through the packed add in this thread
+      group_wait(denfree0 + 8u * (k & 1), ((k >> 1) & 1) ^ 1);
+      den_s[((k & 1) * 2 + grp) * kTcRows + row] = (long long)(int32_t)(den32 - (uint32_t)kTcTileN * (uint32_t)done * mbits);
       __syncwarp();
-      if (lane == 0) mbar_arrive(pready0 + 8u * b);
-    }
-    if (!ok) break;
-    jg += n_tiles;
-    // 64 weights per tile went through the packed add in this thread
-    if (!warp_wait(denfree0 + 8u * (k & 1), ((k >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
-    den_s[(k & 1) * (2 * kTcRows) + group * kTcRows + row] =
-        (long long)(int32_t)(den32 - (uint32_t)kTcTileN * (uint32_t)mine * mbits);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(denfull0 + 8u * (k & 1));
+      mbar_arrive_if(denfull0 + 8u * (k & 1), lane == 0);
     }
   } else {
     // ------------------------------ conversion warps ----------------------------------
     // Round every P.V partial to Q-format, add, and store the finished rows; the softmax warps are by
     // then in the next item's maximum pass.
+    regs_inc<kTcRegsConv>();
     const int quarter = warp & 3;
     const int half = (warp - kTcFirstConv) >> 2;             // which half of the output columns
     const int row = quarter * 32 + lane;
@@ -565,12 +729,9 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const uint64_t magic2 = pack2(mbits, mbits);
     const float screen_limit = q_screen_limit(p.inv_scale);
     int jg = 0;                                              // P.V tiles converted so far (all items)
-    int k = -1;                                              // live items so far
-    bool ok = true;
-    for (int r = 0, w = blockIdx.x; w < total_items && ok; w = item_of(++r)) {
-      const Item I = decode_item(w);
-      if (!I.live) continue;
-      ++k;
+    int k = -1;                                              // items so far
+    Item I;
+    while (group_next(I, ++k)) {
       const int n_tiles = I.t1 - I.t0;
       uint32_t acc[kHalfCols];
 #pragma unroll
@@ -578,21 +739,25 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       uint32_t corr_raw[kHalfCols];                          // rare path, local memory
       long long corr_q[kHalfCols];
       bool corr_used = false;
+#pragma unroll 1
       for (int j = 0; j < n_tiles; ++j, ++jg) {
         const int b = jg & 1;
-        if (!warp_wait(pvfull0 + 8u * b, (jg >> 1) & 1, abort_flag)) { ok = false; break; }
+        group_wait(pvfull0 + 8u * b, (jg >> 1) & 1);
         tc_fence_after();
         const uint32_t taddr = tmem_base + lane_sel + kColPV + (uint32_t)(b * HD + half * kHalfCols);
         float screen = 0.0f, tail = 0.0f;
+        uint32_t v[2][16];                                   // the next load is under way while one is converted
+        tmem_ld16(taddr, v[0]);
 #pragma unroll
-        for (int c = 0; c < kHalfCols; c += 16) {
-          uint32_t v[16];
-          tmem_ld16(taddr + c, v);
-          tmem_wait_ld_regs(v);
-          if (c + 16 == kHalfCols) {
+        for (int c = 0; c < kHalfCols / 16; ++c) {
+          uint32_t (&cur)[16] = v[c & 1];
+          tmem_wait_ld_regs(cur);
+          if (c + 1 < kHalfCols / 16) {
+            tmem_ld16(taddr + (c + 1) * 16, v[(c + 1) & 1]);
+          } else {
             // the last chunk is in registers: screen it and hand the buffer back before converting it
 #pragma unroll
-            for (int i = 0; i < 16; i += 2) screen = max3_abs(screen, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+            for (int i = 0; i < 16; i += 2) screen = max3_abs(screen, __uint_as_float(cur[i]), __uint_as_float(cur[i + 1]));
             if (__any_sync(0xffffffffu, !(screen < screen_limit))) {
               // some partial left the fast range: exact conversion of the offending elements
               if (!corr_used) {
@@ -604,46 +769,72 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(pvfree0 + 8u * b);
+            mbar_arrive_if(pvfree0 + 8u * b, lane == 0);
           }
-          convert16(v, &acc[c], magic2, mbits, one, c + 16 == kHalfCols ? tail : screen);
+          convert16(cur, &acc[c * 16], magic2, mbits, one, c + 1 == kHalfCols / 16 ? tail : screen);
         }
       }
-      if (!ok) break;
-      if (!warp_wait(denfull0 + 8u * (k & 1), (k >> 1) & 1, abort_flag)) { ok = false; break; }
-      const long long dsum = den_s[(k & 1) * (2 * kTcRows) + row] + den_s[(k & 1) * (2 * kTcRows) + kTcRows + row];
+      group_wait(denfull0 + 8u * (k & 1), (k >> 1) & 1);
+      const long long dsum = den_s[(k & 1) * 2 * kTcRows + row] + den_s[((k & 1) * 2 + 1) * kTcRows + row];
       __syncwarp();
-      if (lane == 0) mbar_arrive(denfree0 + 8u * (k & 1));
-      const int tok = I.tok0 + row / G, head = I.kvh * G + row % G;
-      if (tok < I.q_len) {
-        const float dn = fmaxf(fixed_to_float<long long>(wrap_to_bits(dsum, p.int_bits), p.inv_scale), 1.0e-6f);
-        T* op = (T*)p.o + (int64_t)(I.q_start + tok) * p.o_st + (int64_t)head * p.o_sh + half * kHalfCols;
-        const uint32_t bias_bits = (uint32_t)n_tiles * mbits;   // what the multiply-adds summed on top
+      mbar_arrive_if(denfree0 + 8u * (k & 1), lane == 0);
+      const int tok = I.tok0 + (row >> sh.row_shift), head = I.kvh * G + (row & (G - 1));
+      const bool store = tok < I.q_len && !*abort_flag;
+      const float dn = fmaxf(fixed_to_float<long long>(wrap_to_bits(dsum, p.int_bits), p.inv_scale), 1.0e-6f);
+      T* op = (T*)p.o + (int64_t)(I.q_start + tok) * p.o_st + (int64_t)head * p.o_sh + half * kHalfCols;
+      const uint32_t bias_bits = (uint32_t)n_tiles * mbits;  // what the multiply-adds summed on top
+      // With every sum below 2^22 in magnitude MAGIC + sum is a float whose value minus MAGIC is the sum.
+      uint32_t off = 0;
+#pragma unroll
+      for (int i = 0; i < kHalfCols; ++i) {
+        acc[i] += alu_add(i) ? kMagicBits : kMagicBits - bias_bits;
+        off |= acc[i] ^ kExpBits;
+      }
+      if (__all_sync(0xffffffffu, !corr_used && (off >> 23) == 0)) {
+        // num / dn correctly rounded from the row's one reciprocal (Markstein, IBM J. Res. Dev. 34, 1990: with y the
+        // correctly rounded 1 / b and q within an ulp of a / b, q + (a - b q) y, the remainder by fma, rounds
+        // correctly; the first step brings q there).  num = sum * 2^-f over dn is sum over dn * 2^f.
+        const float b = __fmul_rn(dn, p.scale), y = __frcp_rn(b);
+        const uint64_t y2 = pack2(__float_as_uint(y), __float_as_uint(y)), nb2 = pack2(__float_as_uint(-b), __float_as_uint(-b));
+        const uint64_t minus2 = pack2(kMagicBits | 0x80000000u, kMagicBits | 0x80000000u);
 #pragma unroll
         for (int g8 = 0; g8 < kHalfCols / 8; ++g8) {
-          alignas(16) T out[8];
+          uint32_t out[4];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int c = g8 * 8 + i;
-            uint32_t raw = alu_add(c) ? acc[c] : acc[c] - bias_bits;
-            float num;
-            if (corr_used) {
-              raw -= corr_raw[c + zero];
-              const long long tot = (long long)(int32_t)raw + corr_q[c + zero];
-              num = fixed_to_float<long long>(wrap_to_bits(tot, p.int_bits), p.inv_scale);
-            } else {
-              // the sum fits 32 bits: the same value through the cheaper 32-bit conversion
-              num = fixed_to_float<int>((int)raw, p.inv_scale);
-            }
-            out[i] = from_f32<T>(__fdiv_rn(num, dn));
+          for (int i = 0; i < 4; ++i) {
+            const int c = g8 * 8 + i * 2;
+            uint64_t a, q, r;
+            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(a) : "l"(pack2(acc[c], acc[c + 1])), "l"(minus2));
+            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(a), "l"(y2));
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(q), "l"(nb2), "l"(a));
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(q) : "l"(r), "l"(y2), "l"(q));
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(q), "l"(nb2), "l"(a));
+            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(q) : "l"(r), "l"(y2), "l"(q));
+            out[i] = pack2_tc<T>(__uint_as_float((uint32_t)q), __uint_as_float((uint32_t)(q >> 32)));
           }
-          *reinterpret_cast<uint4*>(op + g8 * 8) = *reinterpret_cast<const uint4*>(out);
+          if (store) *reinterpret_cast<uint4*>(op + g8 * 8) = make_uint4(out[0], out[1], out[2], out[3]);
+        }
+      } else {
+        // large sums or corrections: element by element out of local memory, in a loop, as unrolled it was most
+        // of the kernel's code
+        uint32_t sums[kHalfCols];
+#pragma unroll
+        for (int i = 0; i < kHalfCols; ++i) sums[i + zero] = acc[i] - kMagicBits;
+        if (store) {
+#pragma unroll 1
+          for (int c = 0; c < kHalfCols; ++c) {
+            long long tot = (long long)(int32_t)sums[c + zero];
+            if (corr_used)
+              tot = wrap_to_bits((long long)(int32_t)(sums[c + zero] - corr_raw[c + zero]) + corr_q[c + zero], p.int_bits);
+            op[c] = from_f32<T>(__fdiv_rn(fixed_to_float<long long>(tot, p.inv_scale), dn));
+          }
         }
       }
     }
   }
 
   // ------------------------------ teardown ----------------------------------------
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (*abort_flag) {
@@ -653,7 +844,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (threadIdx.x == 0 && status) atomicExch(status, FXPR_ERR_TIMEOUT);
     __syncthreads();
   }
-  if (warp == 1) {
+  if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
@@ -696,13 +887,13 @@ bool attn_kv_map(CUtensorMap* m, const AttnParams& p, int dtype, const void* pla
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The prefill kernel takes head size 128, bf16/fp16, 32- or 64-bit sums with at most 16
+// The prefill kernel takes head sizes 64 and 128, bf16/fp16, 32- or 64-bit sums with at most 16
 // fraction bits, no KV split, a sequence short enough for the 32-bit fast sums, and strides
 // a tensor map can express (multiples of 16 bytes, below 2^40).
 bool attention_tc_supported(const AttnParams& p, int dtype, int max_query_len, bool force_exact) {
   if (force_exact || p.num_splits != 1) return false;
   if (dtype != FXPR_F16 && dtype != FXPR_BF16) return false;
-  if (p.head_dim != 128 || p.page_size % 16 != 0) return false;
+  if ((p.head_dim != 64 && p.head_dim != 128) || p.page_size % 16 != 0) return false;
   const int G = p.num_heads / p.num_kv_heads;
   if (G != 1 && G != 2 && G != 4 && G != 8 && G != 16) return false;
   if ((int64_t)max_query_len * G <= 16) return false;      // decode shapes: attention_mma.cu
@@ -724,6 +915,7 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
   const int G = p.num_heads / p.num_kv_heads;
   TcAttnShape sh;
   sh.rows_per_token = G;
+  sh.row_shift = G == 1 ? 0 : G == 2 ? 1 : G == 4 ? 2 : G == 8 ? 3 : 4;
   sh.tokens_per_block = kTcRows / G;
   sh.num_q_blocks = (max_query_len + sh.tokens_per_block - 1) / sh.tokens_per_block;
   sh.page_size = p.page_size;
@@ -731,7 +923,7 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
   sh.page_mask = (p.page_size & (p.page_size - 1)) == 0 ? p.page_size - 1 : 0;
   const int fmt = dtype == FXPR_BF16 ? 1 : 0;
   sh.idesc_s = make_idesc(fmt, 0, kTcTileN, kTcRows);
-  sh.idesc_s2 = make_idesc(fmt, 0, 2 * kTcTileN, kTcRows);
+  sh.idesc_s2 = make_idesc(fmt, 0, kTcOpN, kTcRows);
   sh.idesc_pv = make_idesc(fmt, 1, p.head_dim, kTcRows);
   if ((int64_t)sh.num_q_blocks * p.num_kv_heads > 0x7fffffffLL) return FXPR_ERR_UNSUPPORTED;
 
@@ -755,29 +947,36 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
     return FXPR_ERR_CUDA;
   }
 
-  constexpr int kSmem = kTcRows * 128 * 2 + kTcStages * 2 * kTcTileN * 128 * 2 + 2 * kTcRows * kTcTileN * 2 +
-                        8 * (1 + 2 * kTcStages + 10 + 2 + 4) + 16 + 2048 + 4096 + 1024;
-  // persistent CTAs, one per SM (204 KB of shared memory each), walking the padded item list
+  // persistent CTAs, one per SM, walking the padded item list
   const int64_t total_items = (int64_t)sh.num_q_blocks * p.num_kv_heads * p.num_reqs;
   if (total_items > 0x7fffffffLL) return FXPR_ERR_UNSUPPORTED;
   dim3 grid((unsigned)std::min<int64_t>(total_items, device_sms()), 1, 1);
-#define FXPR_TC_ATTN(TT)                                                                              \
-  do {                                                                                                \
-    auto k = attn_tc_prefill_kernel<TT, 128>;                                                         \
-    static bool attr_done_dev[64] = {};                                                               \
-    int dev_id = 0;                                                                                   \
-    cudaGetDevice(&dev_id);                                                                           \
-    if (!attr_done_dev[dev_id & 63]) {                                                                \
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);    \
-      if (e != cudaSuccess) { set_last_error("attention_tc smem attribute", e); return FXPR_ERR_CUDA; } \
-      attr_done_dev[dev_id & 63] = true;                                                              \
-    }                                                                                                 \
-    k<<<grid, kTcThreads, kSmem, s>>>(mq, mk, mv, p, sh, status, 0);                                  \
+  const bool plain = !(p.cap_log2 > 0.0f) && p.alibi == nullptr && p.ss_log2 > 0.0f;
+  auto launch = [&](auto k, int smem, bool (&attr_done_dev)[64]) -> int {
+    int dev_id = 0;
+    cudaGetDevice(&dev_id);
+    if (!attr_done_dev[dev_id & 63]) {
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (e != cudaSuccess) { set_last_error("attention_tc smem attribute", e); return FXPR_ERR_CUDA; }
+      attr_done_dev[dev_id & 63] = true;
+    }
+    k<<<grid, kTcThreads, smem, s>>>(mq, mk, mv, p, sh, status, 0);
+    return check_launch("attention_tc");
+  };
+#define FXPR_TC_ATTN(TT, HD, PLAIN)                                                              \
+  do {                                                                                           \
+    static bool attr_done_dev[64] = {};      /* function attributes are per device */            \
+    return launch(attn_tc_prefill_kernel<TT, HD, PLAIN>, TcAttnSmem<HD>::kTotal, attr_done_dev); \
   } while (0)
-  if (dtype == FXPR_BF16) FXPR_TC_ATTN(__nv_bfloat16);
-  else FXPR_TC_ATTN(__half);
+#define FXPR_TC_ATTN_T(TT)                                                                       \
+  do {                                                                                           \
+    if (p.head_dim == 128) { if (plain) FXPR_TC_ATTN(TT, 128, true); else FXPR_TC_ATTN(TT, 128, false); } \
+    if (plain) FXPR_TC_ATTN(TT, 64, true); else FXPR_TC_ATTN(TT, 64, false);                     \
+  } while (0)
+  if (dtype == FXPR_BF16) FXPR_TC_ATTN_T(__nv_bfloat16);
+  FXPR_TC_ATTN_T(__half);
+#undef FXPR_TC_ATTN_T
 #undef FXPR_TC_ATTN
-  return check_launch("attention_tc");
 }
 
 }  // namespace fxpr

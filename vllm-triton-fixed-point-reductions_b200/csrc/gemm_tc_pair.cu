@@ -85,21 +85,12 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t elected)
       "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
       ::"r"(bar), "h"(both), "r"(elected) : "memory");
 }
-// Non-blocking probe, for the waits of the producers and the issuer.  mbarrier.try_wait may park the
+// Wait by non-blocking probes, for the producers and the issuer.  mbarrier.try_wait may park the
 // thread for a hardware time limit, and a parked thread is woken promptly only by arrivals from its own
 // CTA; most of these barriers are completed from the peer CTA.  The sixteen epilogue warps wait with
 // try_wait all the same: they share the issue slots with the conversion, and polling takes more of them
 // than a late wake-up costs (polling everywhere: 4096^3 at K-tile 64 200.4 -> 201.4 us, at K-tile 128
 // 140.7 -> 143.0, 8192 x 14336 x 4096 945 -> 962).
-__device__ __forceinline__ uint32_t mbar_test_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  return ok;
-}
 __device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_test_wait(bar, parity)) return true;
   const long long t0 = clock64();
