@@ -459,6 +459,26 @@ def test_two_sm_kernel_at_tile_edges(M, N, K, kt, kmajor):
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M,N", [(129, 130), (300, 136), (256, 161), (290, 552), (417, 288)])
+@pytest.mark.parametrize("big", [False, True])
+def test_two_sm_kernel_output_paths(M, N, big):
+    """Outputs that leave by TMA (rows on 16 bytes: boxes of 32 rows and columns, clipped at every edge), those the
+    threads store (odd N), and sums beyond the shortcut's 2^22, with a bias: the plain-conversion kernel's bits."""
+    from fxpr_vllm import _native as nat
+
+    K = 256
+    a = _rand((M, K), torch.bfloat16, M, 3.0 if big else 1.0).cuda()
+    b = _rand((N, K), torch.bfloat16, N, 1.5 if big else 0.05).cuda().t()
+    bias = _rand((N,), torch.bfloat16, 9).cuda()
+    out = []
+    for flags in (nat.GEMM_PAIR, nat.GEMM_FORCE_EXACT_TC):
+        with L.overrides(gemm_k_tile=64, gemm_split_k=1, gemm_flags=flags):
+            out.append([_gemm(a, b, x, bits, 16) for x in (None, bias) for bits in (32, 64)])
+    for got, exp in zip(*out):
+        assert torch.equal(got.view(torch.int16), exp.view(torch.int16))
+    L.check_device_status()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,f,K", [(64, 1792, 1024), (33, 200, 512), (1, 128, 256), (64, 4096, 2048)])
 @pytest.mark.parametrize("split", [0, 1, 2, 3, 4])

@@ -336,18 +336,19 @@ static EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// 2-D row-major tensor [rows, cols] (cols contiguous), box [box_rows, 64 cols], 128 B swizzle.
+// 2-D row-major tensor [rows, cols] (cols contiguous), box [box_rows, box_cols], swizzled over a box row:
+// 64 columns are 128 bytes, 32 are 64.
 bool tc_make_map(CUtensorMap* m, int dtype, const void* base, int64_t rows, int64_t cols,
-                     int64_t row_stride_elems, int box_rows) {
+                     int64_t row_stride_elems, int box_rows, int box_cols) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)row_stride_elems * 2};
-  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(m, dtype == FXPR_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                   2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
 }
@@ -449,8 +450,9 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   p.scale = (float)(1ull << g.frac_bits); p.inv_scale = 1.0f / p.scale;
   p.b_kmajor = b_kmajor ? 1 : 0;
   p.idesc = make_idesc(g.dtype == FXPR_BF16 ? 1 : 0, b_kmajor ? 0 : 1, BN, kBM);
-  p.c_vec_ok = !g.c || ((uintptr_t)g.c & 15) || g.c_sm % 8 ? 0 : ((uintptr_t)g.c & 31) || g.c_sm % 16 ? 1 : 2;
+  p.c_vec_ok = g.c && !((uintptr_t)g.c & 15) && g.c_sm % 8 == 0;
   p.status = g.status;
+  p.c_tma = 0;
   p.silu_mul = 0;
   p.best = nullptr; p.n_offset = 0;
   p.w_static = (g.flags & FXPR_GEMM_WEIGHTS_STATIC) ? 1 : 0;

@@ -11,7 +11,9 @@
 // are waited for one after the other (103 clocks each) and the other warps take issue slots.  At K-tile 64
 // (512 clocks of tensor work, 1350 a K-tile all in) they are at work 84 % of the time, ALU pipe 64 %, and
 // the tensor core waits for accumulators; at K-tile 128 (1024 clocks of tensor work) they wait a quarter
-// of the time and the tensor pipe is busy 63 %: the hand-over.  Times: 200 us and 141 us at 4096^3.
+// of the time and the tensor pipe is busy 63 %: the hand-over, next to operands at 8.4 TB/s out of L2.  Outputs
+// leave by TMA: stored by the threads they held the epilogue warps for 7700-8400 clocks a tile.  4096^3, outputs
+// by the threads -> by TMA: K-tile 64 196 -> 186 us, K-tile 128 139 -> 134.
 //
 // What it depends on, measured at 4096^3 with the conversion left out:
 //   - MMAs, commits and copies are predicated instructions of a uniform warp (tc_common.cuh);
@@ -108,20 +110,16 @@ static constexpr int kPrStages = 6;
 static constexpr int kPrABytes = kBM * kBK * 2;            // this CTA's 128 rows of A
 static constexpr int kPrBBytes = 128 * kBK * 2;            // this CTA's 128 columns of B
 static constexpr int kPrStageBytes = kPrABytes + kPrBBytes;
-static constexpr int kPrSmem = kPrStages * kPrStageBytes + 256 + 1024;
+static constexpr int kPrOutBytes = 32 * 64;                // half of a warp's output: 32 rows of 32 columns
+static constexpr int kPrSmem = kPrStages * kPrStageBytes + kPrEpiW * kPrOutBytes + 256 + 1024;
+static_assert(kPrSmem <= 227 * 1024, "shared memory of an SM");
 static constexpr int kPrCols = 64;                         // accumulator columns per epilogue thread
-
-// 32-byte store: every lane of a warp writes another output row, so one full sector per lane
-__device__ __forceinline__ void st_global_32(void* dst, const uint32_t (&w)[8]) {
-  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-               ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
-}
 
 template <typename T>
 __global__ void __launch_bounds__(kPrThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                    const TcParams p, const int zero /* always 0: keeps the side arrays in local memory */) {
-  constexpr int kBarOffset = kPrStages * kPrStageBytes;
+                    const __grid_constant__ CUtensorMap tma_c, const TcParams p, const int zero /* always 0: keeps the side arrays in local memory */) {
+  constexpr int kOutOffset = kPrStages * kPrStageBytes, kBarOffset = kOutOffset + kPrEpiW * kPrOutBytes;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -286,8 +284,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
       const uint32_t bias_bits = (uint32_t)n_kt * mbits;   // what the multiply-adds summed on top
       const T* bias = (const T*)p.bias;
       // Fast output: with every sum below 2^22 in magnitude, MAGIC + sum is a float whose value minus
-      // MAGIC is the sum, so one fma gives sum * 2^-f exactly (what int -> float -> scale gives).
-      bool fast = !corr_used && !p.c_int && p.c_vec_ok == 2 && col0 + kPrCols <= p.N;
+      // MAGIC is the sum, so one fma gives sum * 2^-f exactly (what int -> float -> scale gives).  The rows go
+      // through shared memory and leave by TMA, which clips them to the matrix, while the next tile is
+      // converted.  (Stored by the threads, a row each, an output took the epilogue warps 7700-8400 clocks a tile:
+      // all SMs write at the same time, and the stores wait.)
+      bool fast = !corr_used && p.c_tma;
       if (fast) {
         uint32_t off = 0;
 #pragma unroll
@@ -302,71 +303,66 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
         }
       }
       if (fast) {
-        if (row < p.M) {
+        if (col0 < p.N && row - lane < p.M) {
           const float inv = p.inv_scale, minus = -__fmul_rn(__uint_as_float(kMagicBits), inv);
-          T* cdst = (T*)p.c + (int64_t)row * p.c_sm + col0;
+          const uint32_t out_s = smem_base + kOutOffset + (uint32_t)((warp - kPrFirstEpi) * kPrOutBytes);
 #pragma unroll
-          for (int g = 0; g < kPrCols / 16; ++g) {
-            alignas(16) T out[16];
+          for (int h = 0; h < kPrCols; h += 32) {
+            tma_store_wait_read();                         // the last store has read the staging
+            __syncwarp();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              float v = __fmaf_rn(__uint_as_float(acc[g * 16 + i]), inv, minus);
-              if (bias) v = __fadd_rn(v, to_f32<T>(bias[col0 + g * 16 + i]));
-              out[i] = from_f32<T>(v);
+            for (int g = 0; g < 4; ++g) {
+              alignas(16) T out[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int c = h + g * 8 + i;
+                float v = __fmaf_rn(__uint_as_float(acc[c]), inv, minus);
+                if (bias) v = __fadd_rn(v, col0 + c < p.N ? to_f32<T>(bias[col0 + c]) : 0.0f);
+                out[i] = from_f32<T>(v);
+              }
+              const uint32_t* w = reinterpret_cast<const uint32_t*>(out);
+              // 16-byte chunks swizzled with the row, as the tensor map says
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                           ::"r"(out_s + (uint32_t)(lane * 64 + ((g ^ ((lane >> 1) & 3)) << 4))), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
             }
-            st_global_32(cdst + g * 16, *reinterpret_cast<const uint32_t(*)[8]>(out));
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0 && col0 + h < p.N) {
+              tma_store_2d(&tma_c, out_s, col0 + h, row);
+              tma_store_commit();
+            }
           }
         }
-      } else if (row < p.M) {
-        auto total = [&](int i) -> long long {
-          uint32_t raw = alu_add(i) ? acc[i] : acc[i] - bias_bits;
-          long long t;
-          if (corr_used) {
-            // the in-range part is < 2^31 in magnitude, so it is the sign extension of the wrapped
-            // sum once the out-of-range raw values are taken out again
-            raw -= corr_raw[i + zero];
-            t = (long long)(int32_t)raw + corr_q[i + zero];
-          } else {
-            t = (long long)(int32_t)raw;
-          }
-          return p.int_bits == 64 ? t : (long long)(int32_t)t;
-        };
+      } else {
+        // integer output, corrections, large sums or an unaligned matrix: element by element out of local
+        // memory, in a loop (unrolled it was most of the kernel's code)
+        uint32_t sums[kPrCols];
 #pragma unroll
-        for (int g = 0; g < kPrCols / 8; ++g) {
-          const int colg = col0 + g * 8;
-          long long q8[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) q8[i] = total(g * 8 + i);
-          if (p.c_int) {
-            if (p.int_bits == 64) {
-              long long* dst = (long long*)p.c_int + (int64_t)row * p.N + colg;
-#pragma unroll
-              for (int i = 0; i < 8; ++i) if (colg + i < p.N) dst[i] = q8[i];
-            } else {
-              int32_t* dst = (int32_t*)p.c_int + (int64_t)row * p.N + colg;
-#pragma unroll
-              for (int i = 0; i < 8; ++i) if (colg + i < p.N) dst[i] = (int32_t)q8[i];
+        for (int i = 0; i < kPrCols; ++i) sums[i + zero] = alu_add(i) ? acc[i] : acc[i] - bias_bits;
+        if (row < p.M) {
+#pragma unroll 4
+          for (int c = 0; c < kPrCols; ++c) {
+            const int col = col0 + c;
+            if (col >= p.N) break;
+            // with corrections the in-range part is < 2^31 in magnitude, so it is the sign extension of the
+            // wrapped sum once the out-of-range raw values are taken out again
+            long long t = (long long)(int32_t)(corr_used ? sums[c + zero] - corr_raw[c + zero] : sums[c + zero]);
+            if (corr_used) t += corr_q[c + zero];
+            if (p.int_bits != 64) t = (long long)(int32_t)t;
+            if (p.c_int) {
+              if (p.int_bits == 64) ((long long*)p.c_int)[(int64_t)row * p.N + col] = t;
+              else ((int32_t*)p.c_int)[(int64_t)row * p.N + col] = (int32_t)t;
             }
-          }
-          if (p.c) {
-            T* cdst = (T*)p.c + (int64_t)row * p.c_sm + colg;
-            alignas(16) T out[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              float v = fixed_to_float<long long>(q8[i], p.inv_scale);
-              if (bias && colg + i < p.N) v = __fadd_rn(v, to_f32<T>(bias[colg + i]));
-              out[i] = from_f32<T>(v);
-            }
-            if (p.c_vec_ok && colg + 8 <= p.N) {
-              *reinterpret_cast<uint4*>(cdst) = *reinterpret_cast<const uint4*>(out);
-            } else {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) if (colg + i < p.N) cdst[i] = out[i];
+            if (p.c) {
+              float v = fixed_to_float<long long>(t, p.inv_scale);
+              if (bias) v = __fadd_rn(v, to_f32<T>(bias[col]));
+              ((T*)p.c)[(int64_t)row * p.c_sm + col] = from_f32<T>(v);
             }
           }
         }
       }
     }
+    tma_store_wait_read();                                 // the staging is this CTA's until its stores have read it
   }
 
   // ------------------------------ teardown ----------------------------------------
@@ -397,7 +393,8 @@ bool gemm_tc_pair_supported(const GemmArgs& g, int split_k) {
 }
 
 template <typename T>
-static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, TcParams& p, int sms, cudaStream_t s) {
+static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, TcParams& p, int sms,
+                       cudaStream_t s) {
   auto k = gemm_tc_pair_kernel<T>;
   static bool attr_done_dev[64] = {};            // function attributes are per device
   int dev_id = 0;
@@ -421,7 +418,7 @@ static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, TcParams& p
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, k, ma, mb, (const TcParams)p, 0);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, k, ma, mb, mc, (const TcParams)p, 0);
   if (e != cudaSuccess) { set_last_error("gemm_tc_pair launch", e); return FXPR_ERR_CUDA; }
   return check_launch("gemm_tc_pair");
 }
@@ -431,8 +428,11 @@ int gemm_tc_pair(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CU
   const int sms = tc_device_sms();
   if (sms < 0) return FXPR_ERR_ARCH;
   p.idesc = make_idesc(g.dtype == FXPR_BF16 ? 1 : 0, p.b_kmajor ? 0 : 1, 256, 256);
-  if (g.dtype == FXPR_BF16) return launch_pair<__nv_bfloat16>(ma, mb, p, sms, s);
-  return launch_pair<__half>(ma, mb, p, sms, s);
+  // C by TMA where a tensor map can say where it is: rows that start on 16 bytes
+  CUtensorMap mc = ma;
+  p.c_tma = !p.c_int && p.c_vec_ok && tc_make_map(&mc, g.dtype, g.c, g.M, g.N, g.c_sm, 32, 32);
+  if (g.dtype == FXPR_BF16) return launch_pair<__nv_bfloat16>(ma, mb, mc, p, sms, s);
+  return launch_pair<__half>(ma, mb, mc, p, sms, s);
 }
 
 }  // namespace fxpr

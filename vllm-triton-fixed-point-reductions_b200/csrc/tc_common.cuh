@@ -88,6 +88,14 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       "[%0], [%1, {%3, %4}], [%2];\n\t}"
       ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(elected) : "memory");
 }
+// shared memory -> global tile, in the issuing thread's bulk group; the smem may be written again after
+// tma_store_wait_read, and must live until then.  Rows and columns past the tensor are not written.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z,
                                             int w, int v, uint32_t elected) {
   asm volatile(
@@ -280,7 +288,8 @@ struct TcParams {
   void* acc_scratch; int32_t* locks; int32_t* status;
   int M, N, K; int64_t c_sm;
   int k_tile, split_k, int_bits; float scale, inv_scale;
-  int tiles_m, tiles_n; uint32_t idesc; int b_kmajor; int c_vec_ok;   // 1: rows of c start on 16 bytes, 2: on 32
+  int tiles_m, tiles_n; uint32_t idesc; int b_kmajor; int c_vec_ok;   // rows of c start on 16 bytes
+  int c_tma;             // two-SM kernel: c leaves by TMA
   int silu_mul;          // decode-shape kernel only: c[m, n / 2] = silu(out[m, n]) * out[m, n + 1], n even
   // decode-shape kernel only: best[m] = max over columns of argmax_key(out[m, n], n_offset + n)
   unsigned long long* best; unsigned int n_offset;
@@ -311,7 +320,7 @@ struct SmemLayout {
 
 // Host-side helpers implemented in gemm_tc.cu.
 bool tc_make_map(CUtensorMap* m, int dtype, const void* base, int64_t rows, int64_t cols,
-                 int64_t row_stride_elems, int box_rows);
+                 int64_t row_stride_elems, int box_rows, int box_cols = 64);
 int tc_device_sms();
 
 }  // namespace fxpr
