@@ -479,6 +479,50 @@ def test_two_sm_kernel_output_paths(M, N, big):
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M,N,K", [
+    (65, 128, 64), (96, 256, 200), (97, 264, 1096), (128, 392, 640), (129, 520, 1096), (192, 256, 2056), (193, 1000, 328),
+    (257, 384, 712), (333, 776, 456), (700, 520, 136),
+])
+@pytest.mark.parametrize("kt,split", [(64, 1), (128, 1), (64, 2), (128, 3), (64, 4)])
+def test_medium_batch_kernel(M, N, K, kt, split):
+    """Row tiles of 96 to 256 at and past their edges, ragged columns and K, one to four K-splits in a cluster (some
+    with fewer rows to merge than others), both weight layouts, and partials beyond the fast conversion's range in
+    some tiles only: the integers and outputs of the plain-conversion kernel."""
+    from fxpr_vllm import _native as nat
+
+    split = min(split, -(-K // kt))
+    dtype = torch.float16 if N % 16 else torch.bfloat16
+    a = _rand((M, K), dtype, M).cuda()
+    b = _rand((K, N), dtype, N, 0.05).cuda()
+    bias = _rand((N,), dtype, 7).cuda()
+    far = a.clone()
+    far[M - 1, :64] = 3.0e4
+    for bb in (b, b.t().contiguous().t()):
+        out = []
+        for flags, sp in ((nat.GEMM_MID, split), (nat.GEMM_FORCE_EXACT_TC, 1)):
+            with L.overrides(gemm_k_tile=kt, gemm_split_k=sp, gemm_flags=flags):
+                out.append([torch.ops.fxpr.gemm_fxp_int(a, bb, 64, 16), torch.ops.fxpr.gemm_fxp_int(far, bb, 64, 16),
+                            torch.ops.fxpr.gemm_fxp_int(far, bb, 32, 16), _gemm(a, bb, bias, 64, 16).view(torch.int16),
+                            _gemm(far, bb, None, 64, 16).view(torch.int16)])
+        for got, exp in zip(*out):
+            assert torch.equal(got, exp)
+    L.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K,flag,want", [
+    (80, 4096, 4096, 0, "gemm_tc_mid_kernel"), (333, 6144, 4096, 0, "gemm_tc_mid_kernel"),
+    (64, 4096, 4096, 0, "gemm_tc_skinny_kernel"), (4096, 4096, 4096, 0, "gemm_tc_pair_kernel"),
+    (333, 6144, 4096, 128, "gemm_tc_fast_kernel"),                # GEMM_TILE_N128
+])
+def test_which_kernel_a_medium_batch_takes(M, N, K, flag, want):
+    a, b = _rand((M, K), torch.bfloat16, 1).cuda(), _rand((K, N), torch.bfloat16, 2, 0.05).cuda()
+    with L.overrides(gemm_flags=flag):
+        names = [n for n in _kernels_launched(lambda: _gemm(a, b, None, 64, 16)) if "gemm" in n]
+    if not names:
+        pytest.skip("no kernel activity from the profiler")
+    assert any(want in n for n in names), names
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,f,K", [(64, 1792, 1024), (33, 200, 512), (1, 128, 256), (64, 4096, 2048)])
 @pytest.mark.parametrize("split", [0, 1, 2, 3, 4])

@@ -23,6 +23,22 @@ def test_decode_gemm_split_policy_fills_the_sms_once():
     assert L.pick_split_k(4096, 4096, 4096, 64, 64, sms) == 1     # the output tiles fill the GPU
 
 
+def test_medium_batches_split_into_clusters():
+    """65 rows and more: K-splits that a cluster merges (at most four) where those are cheaper than planes in
+    scratch, none where the tiles fill the pairs, powers of two up to 16 for the CUDA-core and int16 callers' old rule."""
+    sms = 148
+    assert L.pick_split_k(80, 4096, 4096, 128, 64, sms) == 3      # 16 column tiles: clusters of six
+    assert L.pick_split_k(80, 6144, 4096, 128, 64, sms) == 2
+    assert L.pick_split_k(333, 6144, 4096, 128, 64, sms) == 1
+    assert L.pick_split_k(700, 6144, 4096, 128, 64, sms) == 1
+    assert L.pick_split_k(80, 4096, 4096, 128, 16, sms) == 1
+    for kt in (64, 128):
+        for m in (65, 100, 200, 400, 700):
+            for n, k in ((768, 4096), (4096, 14336), (28672, 4096), (1064, 2376)):
+                got = L.pick_split_k(m, n, k, kt, 64, sms)
+                assert 1 <= got <= 16 and got <= -(-k // kt)
+
+
 def test_decode_attention_rank_policy():
     f = L.pick_num_splits_b200
     assert f(5, 64, 1, 32, 8, 8192, 148) == 5                     # an explicit request is kept

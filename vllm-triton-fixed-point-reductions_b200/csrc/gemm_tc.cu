@@ -25,6 +25,7 @@
 
 #include "fxp_common.cuh"
 #include "gemm_common.cuh"
+#include "host_policy.h"
 #include "tc_common.cuh"
 
 namespace fxpr {
@@ -353,6 +354,19 @@ bool tc_make_map(CUtensorMap* m, int dtype, const void* base, int64_t rows, int6
   return r == CUDA_SUCCESS;
 }
 
+bool tc_make_map_groups(CUtensorMap* m, int dtype, const void* base, int64_t rows, int64_t cols,
+                        int64_t row_stride_elems, int box_rows) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn || cols % 64 != 0) return false;
+  cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
+  cuuint64_t strides[2] = {(cuuint64_t)row_stride_elems * 2, 128};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 2}, estr[3] = {1, 1, 1};
+  return fn(m, dtype == FXPR_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
+            const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int tc_device_sms() {
   static int cached[64] = {0};             // 1: compute capability 10.x, -1: another
   int dev = 0;
@@ -421,6 +435,8 @@ int gemm_tc_skinny(const GemmArgs& g, TcParams& p, const CUtensorMap& mw, cudaSt
 int gemm_tc_fast(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb,
                  cudaStream_t s);
 bool gemm_tc_pair_supported(const GemmArgs& g, int split_k);
+bool gemm_tc_mid_supported(const GemmArgs& g, int split_k);
+int gemm_tc_mid(const GemmArgs& g, TcParams& p, const CUtensorMap& mw, int row_tiles, cudaStream_t s);
 int gemm_tc_pair(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb,
                  cudaStream_t s);
 
@@ -479,6 +495,12 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   }
   if (g.best) return FXPR_ERR_UNSUPPORTED;                          // only the decode-shape kernel
   if (g.flags & FXPR_GEMM_SILU_MUL) return FXPR_ERR_UNSUPPORTED;   // only the decode-shape kernel fuses it
+  // medium batches: weights on the M side of SM pairs (same bits, see gemm_tc_mid.cu)
+  if (!(g.flags & (FXPR_GEMM_FORCE_EXACT_TC | FXPR_GEMM_TILE_N128 | FXPR_GEMM_PAIR)) && gemm_tc_mid_supported(g, p.split_k)) {
+    const int rows = (g.flags & FXPR_GEMM_MID) ? plan_mid_rows(g.M, g.N, g.K, g.k_tile, p.split_k, sms).row_tiles
+                                               : mid_route(g.M, g.N, g.K, g.k_tile, p.split_k, sms);
+    if (rows) return gemm_tc_mid(g, p, mb, rows, s);
+  }
   if (!(g.flags & FXPR_GEMM_FORCE_EXACT_TC) && gemm_tc_pair_supported(g, p.split_k)) {
     // 256 x 256 tiles on SM pairs or 128 x 128 tiles on single SMs (same bits).  A full wave of pair
     // tiles has twice the output of a wave of single tiles and takes 1.7 times as long at K-tile 64

@@ -22,9 +22,9 @@
 // a function of the running super-stage number, so the roles need no communication beyond
 // the barriers.
 //
-// It serves 65 to some 700 rows, split K and the dumps; large products take the two-SM kernel
-// (gemm_tc_pair.cu).  Bound: operands out of L2, since each tile fetches its own 128 rows and 128
-// columns.  333 x 6144 x 4096: 302 MB in 29 us = 10.4 TB/s; issue slots 52 % busy, tensor pipe 38 %.
+// It serves splits through scratch, the dumps and the calls above 64 rows that neither the medium-batch
+// kernel (gemm_tc_mid.cu) nor the two-SM kernel (gemm_tc_pair.cu) does faster (host_policy.h).  Bound: operands out of
+// L2, since each tile fetches its own 128 rows and 128 columns.
 // Tried and measured slower or equal: two issuer warps (one per TMEM group, -10 %), four
 // single-buffer groups for k_tile 128 (equal), software-pipelined or pairwise TMEM loads in
 // the epilogue (-6 % / -11 %).

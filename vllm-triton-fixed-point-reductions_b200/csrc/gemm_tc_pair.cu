@@ -45,67 +45,6 @@ static constexpr int kPrFirstEpi = 2;
 static constexpr int kPrThreads = (kPrFirstEpi + kPrEpiW) * 32;
 static constexpr int kPrGroupM = 4;        // pair-tile rows (256 each) per L2 group
 
-// ---- cluster / cta_group::2 PTX ---------------------------------------------------------
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// TMA tile load whose completion bytes are counted on a barrier that may live in the peer CTA
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster,
-                                                 int x, int y, uint32_t elected) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4}], [%2];\n\t}"
-      ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(x), "r"(y), "r"(elected) : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate, uint32_t elected) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
-}
-// Arrives on the barrier at this shared-memory offset in BOTH CTAs of the pair once every MMA
-// this thread issued so far is done.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint32_t elected) {
-  const uint16_t both = 3;
-  asm volatile(
-      "{\n\t.reg .pred q;\n\t"
-      "setp.ne.b32 q, %2, 0;\n\t"
-      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
-      ::"r"(bar), "h"(both), "r"(elected) : "memory");
-}
-// Wait by non-blocking probes, for the producers and the issuer.  mbarrier.try_wait may park the
-// thread for a hardware time limit, and a parked thread is woken promptly only by arrivals from its own
-// CTA; most of these barriers are completed from the peer CTA.  The sixteen epilogue warps wait with
-// try_wait all the same: they share the issue slots with the conversion, and polling takes more of them
-// than a late wake-up costs (polling everywhere: 4096^3 at K-tile 64 200.4 -> 201.4 us, at K-tile 128
-// 140.7 -> 143.0, 8192 x 14336 x 4096 945 -> 962).
-__device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_test_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  int spins = 0;
-  while (!mbar_test_wait(bar, parity)) {
-    if ((++spins & 255) == 0) {
-      if (*abort_flag) return false;
-      if (clock64() - t0 > kWaitCycles) { *abort_flag = 1; return false; }
-    }
-  }
-  return true;
-}
-
 static constexpr int kPrStages = 6;
 static constexpr int kPrABytes = kBM * kBK * 2;            // this CTA's 128 rows of A
 static constexpr int kPrBBytes = 128 * kBK * 2;            // this CTA's 128 columns of B
@@ -212,8 +151,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
             const uint64_t bd = bdesc0 + (uint64_t)stage * kStep;
 #pragma unroll
             for (int q = 0; q < 4; ++q) umma_f16_pair(d, ad + 2 * q, bd + q * bks, idesc, (h || q) ? 1u : 0u, e);
-            umma_commit_pair(empty0 + 8u * stage, e);
-            if (h == halves - 1) umma_commit_pair(tfull0 + 8u * buf, e);
+            umma_commit_pair(empty0 + 8u * stage, 3, e);
+            if (h == halves - 1) umma_commit_pair(tfull0 + 8u * buf, 3, e);
             if (++stage == kPrStages) { stage = 0; phase ^= 1; }
           }
           buf ^= 1; if (buf == 0) bphase ^= 1;

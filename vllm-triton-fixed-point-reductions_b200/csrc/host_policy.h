@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <climits>
 
 namespace fxpr {
 
@@ -30,6 +31,52 @@ inline bool attention_tensor_core_route(const AttnRoute& r) {
   return r.num_kv_heads <= 4096 && r.num_reqs <= 65535;  // grid dimensions
 }
 
+// ---- which wide GEMM kernel, by estimated microseconds -----------------------------------------
+// Above 64 rows three kernels give the same bits: 128 x 128 tiles on single SMs (gemm_tc_fast.cu, K-splits through
+// scratch), 256 x 256 on pairs (gemm_tc_pair.cu, unsplit) and 256 weight columns x 96 to 256 rows on pairs
+// (gemm_tc_mid.cu, up to four splits in a cluster).  The estimates are clocks per 128 of K at 1850 MHz, fitted to
+// sweeps of 80 to 700 rows over ten weight shapes (within 15 % of the measured times, most within 8 %):
+//   128 x 128     1300 (K-tile 128) or 1665 (64), 3.5 us a call, 8 + splits for the planes of a split
+//   256 x 256     1936 or 2690
+//   256 x rows    copies: (256 + rows) requests of 128 bytes a CTA at 2.4 clocks, 3.05 when most SMs fetch; or the
+//                 conversion, 7 (14) clocks a row; 3 us a call, 8 a wave when there are several (its waves do not
+//                 overlap), 2 to 4.5 for the merge
+inline double est_single_us(int64_t M, int64_t N, int64_t K, int64_t k_tile, int split, int num_sms) {
+  const double waves = (double)ceil_div(ceil_div(M, 128) * ceil_div(N, 128) * split, num_sms);
+  return waves * ((double)K / 128 / split * (k_tile == 64 ? 1665 : 1300) / 1850) + 3.5 + (split > 1 ? 8.0 + split : 0.0);
+}
+inline double est_pair_us(int64_t M, int64_t N, int64_t K, int64_t k_tile, int num_sms) {
+  const double waves = (double)ceil_div(ceil_div(M, 256) * ceil_div(N, 256), std::max(1, num_sms / 2));
+  return waves * ((double)K / 128 * (k_tile == 64 ? 2690 : 1936) / 1850) + 3.5;
+}
+
+// Row tiles of gemm_tc_mid.cu for a given split (0: it does not take the call) and their estimate.
+struct MidPlan { int row_tiles; double us; };
+inline MidPlan plan_mid_rows(int64_t M, int64_t N, int64_t K, int64_t k_tile, int split, int num_sms) {
+  MidPlan best = {0, 1e30};
+  if (M <= 64 || N < 128 || split < 1 || split > 4 || (k_tile != 64 && k_tile != 128)) return best;
+  const int64_t cols = ceil_div(N, 256), pairs = std::max(1, num_sms / 2), most = split > 1 ? 128 : 256;
+  // clusters of 4, 6 and 8 whole SMs that are resident at once: they do not pack a GPC
+  const int64_t room = split == 1 ? pairs : split == 2 ? num_sms * 34 / 148 : split == 3 ? num_sms * 20 / 148 : num_sms * 14 / 148;
+  for (int64_t t = ceil_div(M, most); t <= ceil_div(M, 64) && t <= 65535; ++t) {
+    const int64_t rows = std::max<int64_t>(96, ceil_div(ceil_div(M, t), 32) * 32);
+    const double waves = (double)ceil_div(cols * t, std::max<int64_t>(1, room));
+    const double copies = (double)(256 + rows) * (cols * t * split * 2 * 3 >= num_sms * 2 ? 3.05 : 2.4);
+    const double convert = (double)rows * (k_tile == 64 ? 14 : 7);
+    const double us = waves * ((double)K / 128 / split * std::max(copies, convert) / 1850 + (waves > 1 ? 8 : 3)) +
+                      (split == 1 ? 0.0 : split == 2 ? 2.0 : split == 3 ? 3.0 : 4.5);
+    if (us < best.us) best = {(int)t, us};
+  }
+  return best;
+}
+// Row tiles of gemm_tc_mid.cu when it is the kernel for the call, else 0.
+inline int mid_route(int64_t M, int64_t N, int64_t K, int64_t k_tile, int split, int num_sms) {
+  const MidPlan mid = plan_mid_rows(M, N, K, k_tile, split, num_sms);
+  double other = est_single_us(M, N, K, k_tile, split, num_sms);
+  if (split == 1) other = std::min(other, est_pair_us(M, N, K, k_tile, num_sms));
+  return mid.row_tiles && mid.us < 0.95 * other ? mid.row_tiles : 0;
+}
+
 // K-split of a GEMM: split when the output tiles alone cannot fill the GPU.
 inline int pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int64_t k_tile, int int_bits, int num_sms) {
   if (int_bits == 16) return 1;
@@ -46,7 +93,14 @@ inline int pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int64_t k_tile, in
   }
   // one wave of CTAs at most: a second, partly filled wave costs more than it hides
   while (split < 16 && tiles * split * 2 <= num_sms && k_tiles / (split * 2) >= 4) split *= 2;
-  return split;
+  // the splits of a cluster are cheaper to merge
+  int best = split;
+  double us = est_single_us(M, N, K, k_tile, split, num_sms);
+  for (int s = 1; s <= 4 && k_tiles / s >= 2; ++s) {
+    const MidPlan mid = plan_mid_rows(M, N, K, k_tile, s, num_sms);
+    if (mid.row_tiles && mid.us < us && mid_route(M, N, K, k_tile, s, num_sms)) { best = s; us = mid.us; }
+  }
+  return best;
 }
 
 // KV splits of the CUDA-core attention route: an explicit request wins; otherwise split only long

@@ -257,6 +257,75 @@ __device__ __forceinline__ void tmem_wait_ld_regs2(uint32_t (&a)[16], uint32_t (
                :: "memory");
 }
 
+// ---- cta_group::2: two CTAs with neighbouring ranks work on one MMA ----
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// TMA tile load whose completion bytes are counted on a barrier that may live in the peer CTA
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster,
+                                                 int x, int y, uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4}], [%2];\n\t}"
+      ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(x), "r"(y), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster,
+                                                 int x, int y, int z, uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+      ::"r"(dst), "l"(map), "r"(bar_cluster), "r"(x), "r"(y), "r"(z), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                              uint32_t accumulate, uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
+}
+// Arrives on the barrier at this shared-memory offset in BOTH CTAs of the pair (`both`: their two bits of the
+// cluster) once every MMA this thread issued so far is done.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t both, uint32_t elected) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(bar), "h"(both), "r"(elected) : "memory");
+}
+// Wait by non-blocking probes, for the producers and the issuer.  mbarrier.try_wait may park the
+// thread for a hardware time limit, and a parked thread is woken promptly only by arrivals from its own
+// CTA; most of these barriers are completed from the peer CTA.  The sixteen epilogue warps wait with
+// try_wait all the same: they share the issue slots with the conversion, and polling takes more of them
+// than a late wake-up costs (polling everywhere: 4096^3 at K-tile 64 200.4 -> 201.4 us, at K-tile 128
+// 140.7 -> 143.0, 8192 x 14336 x 4096 945 -> 962).
+__device__ __forceinline__ bool mbar_wait_poll(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_test_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  int spins = 0;
+  while (!mbar_test_wait(bar, parity)) {
+    if ((++spins & 255) == 0) {
+      if (*abort_flag) return false;
+      if (clock64() - t0 > kWaitCycles) { *abort_flag = 1; return false; }
+    }
+  }
+  return true;
+}
+
 // Shared-memory matrix descriptor (sm_100 format): start address, leading / stride
 // byte offsets (all >> 4), version 1, 128-byte swizzle.
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
@@ -321,6 +390,10 @@ struct SmemLayout {
 // Host-side helpers implemented in gemm_tc.cu.
 bool tc_make_map(CUtensorMap* m, int dtype, const void* base, int64_t rows, int64_t cols,
                  int64_t row_stride_elems, int box_rows, int box_cols = 64);
+// The same tensor as [groups of 64 columns][rows][64], boxes of 2 groups x box_rows: two neighbouring boxes of
+// tc_make_map in one copy.  cols must be a multiple of 64 (a ragged last group would reach past the last row).
+bool tc_make_map_groups(CUtensorMap* m, int dtype, const void* base, int64_t rows, int64_t cols,
+                        int64_t row_stride_elems, int box_rows);
 int tc_device_sms();
 
 }  // namespace fxpr

@@ -49,6 +49,7 @@ GEMM_FORCE_EXACT_TC = 2
 GEMM_NO_SKINNY = 8
 GEMM_NO_CLUSTER = 16
 GEMM_PAIR = 512
+GEMM_MID = 4096
 GEMM_SILU_MUL = 1024
 GEMM_WEIGHTS_STATIC = 2048
 TP_LOCAL_RESIDUAL = 1
