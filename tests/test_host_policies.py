@@ -54,6 +54,20 @@ def test_decode_attention_rank_policy():
     assert f(0, 16, 4096, 32, 8, 4096, 148) == 1                  # prefill with enough row blocks
 
 
+def test_decode_ranks_of_small_batches_and_last_waves():
+    f = L.pick_num_splits_b200
+    assert f(0, 25, 1, 32, 8, 3168, 148) == 2                     # three ranks would be a full wave and eight CTAs
+    assert f(0, 64, 1, 32, 8, 2048, 148) == 2                     # nearly two full waves stay
+    assert f(0, 5, 1, 32, 8, 704, 148) == 5                       # two key tiles a rank
+    assert f(0, 1, 1, 32, 8, 3584, 148) == 16                     # a CTA per SM
+    assert f(0, 2, 1, 32, 8, 3584, 148) == 8
+    assert f(0, 1, 1, 4, 1, 64, 148) == 1                         # one key tile
+    for n in (1, 7, 64, 300):
+        for hq, hkv in ((32, 8), (16, 4), (4, 1), (32, 32), (16, 1)):
+            for keys in (16, 100, 1000, 9600, 40000):
+                assert 1 <= f(0, n, 1, hq, hkv, keys, 148) <= 16
+
+
 def test_argmax_keys_pick_the_first_maximum_and_combine_across_shards():
     g = torch.Generator().manual_seed(0)
     for dtype in (torch.bfloat16, torch.float16):

@@ -140,7 +140,17 @@ inline int64_t pick_attention_ranks(int64_t requested, int64_t num_requests, int
     const int64_t by_keys = need > 4 ? 8 : std::max<int64_t>(1, need);
     const int64_t clusters = std::max<int64_t>(1, num_requests * num_kv_heads);
     const int64_t by_fill = std::max<int64_t>(1, std::min<int64_t>({8, (4 * num_sms) / clusters, tiles / 2}));
-    return std::max(by_keys, by_fill);
+    // A few clusters with long contexts: sixteen, one CTA per SM (1 request x 3588 keys, 8 KV heads: 14.1 us with
+    // eight, 11.3).
+    if (clusters * 16 <= num_sms && tiles >= 48) return 16;
+    int64_t ranks = std::max(by_keys, by_fill);
+    // No last wave of a handful of CTAs: one rank less where that fits one wave at three CTAs per SM (25 requests x
+    // 3160 keys, 8 KV heads: 600 CTAs of three ranks 76.6 us, 400 of two 56.7; 64 x 2048, 1024 CTAs, stays).
+    const int64_t over = clusters * ranks - 4 * num_sms;
+    if (ranks > 1 && over > 0 && over * 8 < 4 * num_sms && clusters * (ranks - 1) <= 3 * num_sms &&
+        ceil_div(tiles, ranks - 1) * 64 * key_bytes <= 32 * 1024)
+      --ranks;
+    return ranks;
   }
   const int64_t blocks = num_requests * num_kv_heads * std::max<int64_t>(1, ceil_div(max_query_len * g, 64));
   if (blocks >= num_sms || max_keys <= 2048) return 1;
