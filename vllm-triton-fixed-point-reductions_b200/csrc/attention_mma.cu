@@ -1,5 +1,6 @@
 // Unified prefill + decode paged attention on tensor cores for fp16/bf16, head size
-// 64/128, page sizes that are multiples of 16 and GQA groups of 1/2/4/8/16.
+// 64/128, page sizes that are multiples of 16 and GQA groups of 1/2/4/8/16.  Prefill without KV splits
+// goes to attention_tc.cu where TMA can take the cache (same bits).
 //
 // Semantics: fxpr_vllm/_triton/attention.py of the reference (scores in log2 space
 // :103-121, masks :199-215, exact row maximum first :233-257, w = exp2(s - max),

@@ -49,11 +49,11 @@
 namespace fxpr {
 
 static constexpr int kTcTileN = 64;            // keys per tile (attention.py:32-36)
-static constexpr int kTcOpN = 2 * kTcTileN;    // keys per score product, in both passes
+static constexpr int kTcOpN = 2 * kTcTileN;    // keys per K stage; pass A scores them in one product, pass B in two
 static constexpr int kTcRows = 128;            // query rows per CTA = tensor-memory lanes
-static constexpr int kTcSoftWarps = 8;         // two groups of four warps, one per half of the score buffers: thread = one row
+static constexpr int kTcSoftWarps = 8;         // two groups of four warps, a group takes every other tile: thread = one row
 static constexpr int kTcConvWarps = 8;         // conversion: thread = one row and half of the output columns
-// warps 0, 1: score and P.V issuers; 2, 3: V producers (the first also decodes the item list); 4-7: K producers
+// warps 0, 1: score and P.V issuers; 2, 3: V producers (the first also makes the item list); 4-7: K producers
 static constexpr int kTcVProducers = 2, kTcKProducers = 4;
 static constexpr int kTcFirstV = 2, kTcFirstK = kTcFirstV + kTcVProducers;
 static constexpr int kTcFirstSoft = kTcFirstK + kTcKProducers;
