@@ -58,6 +58,8 @@ def test_decode_ranks_of_small_batches_and_last_waves():
     f = L.pick_num_splits_b200
     assert f(0, 25, 1, 32, 8, 3168, 148) == 2                     # three ranks would be a full wave and eight CTAs
     assert f(0, 64, 1, 32, 8, 2048, 148) == 2                     # nearly two full waves stay
+    assert f(0, 40, 1, 32, 8, 2000, 148) == 2                     # one rank would leave mixed lengths unbalanced
+    assert f(0, 10, 1, 32, 32, 8192, 148) == 2
     assert f(0, 5, 1, 32, 8, 704, 148) == 5                       # two key tiles a rank
     assert f(0, 1, 1, 32, 8, 3584, 148) == 16                     # a CTA per SM
     assert f(0, 2, 1, 32, 8, 3584, 148) == 8

@@ -144,10 +144,12 @@ inline int64_t pick_attention_ranks(int64_t requested, int64_t num_requests, int
     // eight, 11.3).
     if (clusters * 16 <= num_sms && tiles >= 48) return 16;
     int64_t ranks = std::max(by_keys, by_fill);
-    // No last wave of a handful of CTAs: one rank less where that fits one wave at three CTAs per SM (25 requests x
-    // 3160 keys, 8 KV heads: 600 CTAs of three ranks 76.6 us, 400 of two 56.7; 64 x 2048, 1024 CTAs, stays).
+    // No last wave of a handful of CTAs: two ranks and not three where two fit one wave at three CTAs per SM (600
+    // CTAs of three against 400 of two, 25 requests x 3160 keys, 8 KV heads: 76.6 -> 56.7 us, lengths of 790 to 3160
+    // 50.3 -> 43.1).  One and not two: uniform lengths gain as much, mixed ones lose (40 x 2000 74.0 -> 59.8, 400 to
+    // 2000 46.2 -> 49.5; 10 x 1640 to 8192 with 32 KV heads 115 -> 162), so two stay.
     const int64_t over = clusters * ranks - 4 * num_sms;
-    if (ranks > 1 && over > 0 && over * 8 < 4 * num_sms && clusters * (ranks - 1) <= 3 * num_sms &&
+    if (ranks > 2 && over > 0 && over * 8 < 4 * num_sms && clusters * (ranks - 1) <= 3 * num_sms &&
         ceil_div(tiles, ranks - 1) * 64 * key_bytes <= 32 * 1024)
       --ranks;
     return ranks;
