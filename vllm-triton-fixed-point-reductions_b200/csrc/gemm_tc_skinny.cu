@@ -257,6 +257,7 @@ static int route_skinny(const GemmArgs& g, const CUtensorMap& mw, TcParams& p, i
   // with one CTA and tile after tile per SM, 38.8 with two).  64 x 4096 x 4096 on 128 CTAs: 11.3 us with the
   // whole ring, 12.1 with half of it; 64 x 6144 x 4096 13.7 / 15.9.  With 16 rows half of it holds as many
   // weights as are needed in flight: 16 x 4096 x 4096 10.5 / 9.9, 16 x 4096 x 14336 23.9 / 21.8.
+  // A thousand tiles of 64 rows pay for a CTA's set-up each: 64 x 128256 x 4096 166.6 us with persistent CTAs, 170.5.
   if constexpr (MP > 16) {
     if ((int64_t)p.tiles_n * p.split_k <= sms)
       return cluster ? launch_skinny<T, MP, true, 1>(g, mw, p, s) : launch_skinny<T, MP, false, 1>(g, mw, p, s);
