@@ -479,6 +479,25 @@ def test_two_sm_kernel_output_paths(M, N, big):
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M", [33, 62, 63, 64])
+@pytest.mark.parametrize("split", [2, 5, 6, 7, 8])
+@pytest.mark.parametrize("K", [896, 1064])
+def test_decode_shape_cluster_merge_at_every_rank_count(M, split, K):
+    """What the ranks of a merge send each other has room at every rank count: seven ranks of 64 rows receive the
+    most, also where eight are asked for and there are seven K-tiles.  The unsplit integers and outputs."""
+    a, b = _rand((M, K), torch.bfloat16, M).cuda(), _rand((K, 392), torch.bfloat16, split, 0.05).cuda()
+    far = a.clone()
+    far[M - 1, :64] = 3.0e5                            # sums beyond 32 bits in one of the splits
+    out = []
+    for sp in (split, 1):
+        with L.overrides(gemm_k_tile=128, gemm_split_k=sp):
+            out.append([torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16), torch.ops.fxpr.gemm_fxp_int(a, b, 32, 16),
+                        torch.ops.fxpr.gemm_fxp_int(far, b, 64, 16), _gemm(a, b, None, 64, 16).view(torch.int16)])
+    for got, exp in zip(*out):
+        assert torch.equal(got, exp)
+    L.check_device_status()
+
+
 @pytest.mark.parametrize("M,N,K", [
     (65, 128, 64), (96, 256, 200), (97, 264, 1096), (128, 392, 640), (129, 520, 1096), (192, 256, 2056), (193, 1000, 328),
     (257, 384, 712), (333, 776, 456), (700, 520, 136),

@@ -32,6 +32,17 @@ static constexpr int kSkWarps = 2 + 8;                    // producer, issuer, 8
 static constexpr int kSkWBytes = 128 * kBK * 2;           // weights of a stage: 64 of K, 128 columns
 static constexpr int kSkTmemCols = 256;                   // two CTAs share an SM's 512
 
+// Most rows that one rank of a cluster merge receives, all its peers together, over 2 to 8 ranks: with 64 rows it
+// is seven ranks of ten rows (60), not eight of eight.
+constexpr int sk_most_received(int rows) {
+  int most = 0;
+  for (int ranks = 2; ranks <= 8; ++ranks) {
+    const int got = (ranks - 1) * ((rows + ranks - 1) / ranks);
+    if (got > most) most = got;
+  }
+  return most;
+}
+
 // MP = activation rows of the tile (MMA N).  PER_SM = CTAs that share an SM's memory.
 template <int MP, int PER_SM> struct SkShape {
   static constexpr int kStages = (MP == 16 ? 12 : MP == 32 ? 10 : 8) / PER_SM;
@@ -42,9 +53,10 @@ template <int MP, int PER_SM> struct SkShape {
   static constexpr int kBarBytes = 448;
   static constexpr int kSmem = kBarOffset + kBarBytes + 1024;   // barriers, alignment slack
   // over the stages once they are done: the finished sums, [row][128 columns] of 32 bits; what the
-  // peers send for this rank's rows (7/8 as much at most), their flags, this rank's high words
-  static constexpr int kRecvOffset = 32 * 1024, kFlagOffset = 60 * 1024, kHighOffset = 64 * 1024;
-  static_assert(MP * 512 <= kRecvOffset && kRecvOffset + MP * 448 <= kFlagOffset, "sums and received slices");
+  // peers send for this rank's rows, their flags, this rank's high words
+  static constexpr int kRecvOffset = 32 * 1024, kFlagOffset = 62 * 1024, kHighOffset = 64 * 1024;
+  static_assert(MP * 512 <= kRecvOffset && kRecvOffset + sk_most_received(MP) * 512 <= kFlagOffset, "sums and received slices");
+  static_assert(kFlagOffset + 7 * 16 <= kHighOffset, "a flag of 16 bytes from each peer");
   static_assert(kHighOffset + MP * 512 <= kBarOffset, "the merge fits the stages");
   static_assert(PER_SM * (kSmem + 1024) <= 228 * 1024, "shared memory of an SM");
   static_assert(kGroups * MP <= kSkTmemCols, "tensor memory");
