@@ -498,6 +498,23 @@ def test_decode_shape_cluster_merge_at_every_rank_count(M, split, K):
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M,split", [(5, 8), (16, 3), (33, 2), (64, 7), (64, 8), (80, 2), (100, 3), (128, 4)])
+@pytest.mark.parametrize("wide", ["one", "some", "all"])
+def test_cluster_merges_of_sums_beyond_32_bits(M, split, wide):
+    """High words cross the cluster by plain loads: from one split, from some and from all of them, call after call."""
+    K = 64 * 16
+    a, b = _rand((M, K), torch.bfloat16, M).cuda(), _rand((K, 392), torch.bfloat16, split, 0.05).cuda()
+    for t in {"one": [3], "some": [0, 1, 5], "all": range(16)}[wide]:
+        a[t % M::3, 64 * t:64 * t + 64] = 3.0e5                      # partials of about 1.2e5 * 2^16
+    with L.overrides(gemm_k_tile=64, gemm_split_k=1):
+        exp = torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16)
+    assert exp.abs().max().item() > 1 << 32
+    with L.overrides(gemm_k_tile=64, gemm_split_k=split, gemm_flags=4096):     # GEMM_MID above 64 rows
+        for got in [torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16) for _ in range(20)]:
+            assert torch.equal(got, exp)
+    L.check_device_status()
+
+
 @pytest.mark.parametrize("M,N,K", [
     (65, 128, 64), (96, 256, 200), (97, 264, 1096), (128, 392, 640), (129, 520, 1096), (192, 256, 2056), (193, 1000, 328),
     (257, 384, 712), (333, 776, 456), (700, 520, 136),

@@ -75,7 +75,8 @@ gemm_tc_mid_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   volatile int* abort_flag = (volatile int*)(smem_gen + kBarOffset + kMisc + 8);
   const uint32_t epi_bar = bar_base + kMisc + 16u, recv_bar = bar_base + kMisc + 24u;
   volatile int* s_wide = (volatile int*)(smem_gen + kBarOffset + kMisc + 32);   // 16 bytes, copied to the peers
-  static_assert(kMisc + 48 <= Shape::kBarBytes, "barrier block");
+  const uint32_t high_bar = bar_base + kMisc + 48u;
+  static_assert(kMisc + 56 <= Shape::kBarBytes, "barrier block");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = (int)blockIdx.x, parity = rank & 1, ks = rank >> 1, S = p.split_k;
@@ -96,6 +97,7 @@ gemm_tc_mid_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     for (int b = 0; b < GROUPS; ++b) { mbar_init(tfull0 + 8u * b, 1); mbar_init(tempty0 + 8u * b, 2 * EPIW); }
     mbar_init(epi_bar, EPIW);
     mbar_init(recv_bar, 1);
+    if constexpr (SPLIT) mbar_init(high_bar, (uint32_t)(S - 1));
     *abort_flag = 0;
     for (int i = 0; i < 4; ++i) s_wide[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -353,7 +355,7 @@ gemm_tc_mid_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         if (to < S && to != ks && lane == 0 && rows_of(to) > 0) {
           const int slot = ks < to ? ks : ks - 1;
           const uint32_t peer = (uint32_t)(2 * to + parity), bar = mapa_u32(recv_bar, peer);
-          if (*s_wide) fence_acq_rel_cluster();            // peers read the high words with plain loads
+          if (*s_wide) mbar_arrive_release_cluster(mapa_u32(high_bar, peer));   // peers read the high words with plain loads
           bulk_copy_cluster(mapa_u32(smem_base + Shape::kRecvOffset + (uint32_t)(slot * rows_of(to) * 512), peer),
                             smem_base + (uint32_t)(to * rows_per * 512), (uint32_t)(rows_of(to) * 512), bar);
           bulk_copy_cluster(mapa_u32(smem_base + Shape::kFlagOffset + (uint32_t)(slot * 16), peer),
@@ -368,8 +370,18 @@ gemm_tc_mid_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         wide = (unsigned long long)(uint32_t)*s_wide << (16 * ks);
         for (int rr = 0; rr < S - 1; ++rr) wide |= (unsigned long long)(uint32_t)flags[rr * 4] << (16 * (rr < ks ? rr : rr + 1));
       }
-      if (wide) fence_acq_rel_cluster();
-      else cluster_arrive();                               // this CTA has what was sent to it
+      if (wide) {
+        // the high words of every peer that has some; its own arrivals stand for the other peers
+        if (warp == 2 && lane == 0) {
+          int none = S - 1;
+          for (int s = 0; s < S; ++s) none -= s != ks && ((wide >> (16 * s)) & 0xffff);
+          if (none) mbar_arrive_n(high_bar, (uint32_t)none);
+        }
+        __syncwarp();
+        ok = __all_sync(0xffffffffu, mbar_wait_acquire_cluster(high_bar, 0, abort_flag));
+      } else {
+        cluster_arrive();                                  // this CTA has what was sent to it
+      }
       if (ok) {
         const int* mine = stage32 + ks * rows_per * 128;
         const int* recv = reinterpret_cast<const int*>(smem_gen + Shape::kRecvOffset);

@@ -86,7 +86,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
   volatile int* abort_flag = (volatile int*)(smem_gen + kBarOffset + kMisc + 8);
   const uint32_t epi_bar = bar_base + kMisc + 16u;
   volatile int* s_last = (volatile int*)(smem_gen + kBarOffset + kMisc + 24);
-  const uint32_t recv_bar = bar_base + kMisc + 32u;
+  const uint32_t recv_bar = bar_base + kMisc + 32u, high_bar = recv_bar + 8u;
   volatile int* s_wide = (volatile int*)(smem_gen + kBarOffset + kMisc + 48);   // 16 bytes, copied to the peers
   static_assert(kMisc + 64 <= Shape::kBarBytes, "barrier block");
 
@@ -105,7 +105,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
     for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8u * s, 1); mbar_init(empty0 + 8u * s, 1); }
     for (int b = 0; b < GROUPS; ++b) { mbar_init(tfull0 + 8u * b, 1); mbar_init(tempty0 + 8u * b, EPIW); }
     mbar_init(epi_bar, EPIW);
-    if constexpr (CLUSTER) mbar_init(recv_bar, 1);
+    if constexpr (CLUSTER) { mbar_init(recv_bar, 1); mbar_init(high_bar, (uint32_t)(p.split_k - 1)); }
     *abort_flag = 0;
     for (int i = 0; i < 4; ++i) s_wide[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");

@@ -250,7 +250,7 @@
       const int to = warp - 2;                           // warp w sends rank w's rows
       if (to < S && to != rank && lane == 0 && rows_of(to) > 0) {
         const int slot = rank < to ? rank : rank - 1;
-        if (*s_wide) fence_acq_rel_cluster();            // peers read the high words with plain loads
+        if (*s_wide) mbar_arrive_release_cluster(mapa_u32(high_bar, (uint32_t)to));   // peers read the high words with plain loads
         const uint32_t bar = mapa_u32(recv_bar, (uint32_t)to);
         bulk_copy_cluster(mapa_u32(smem_base + Shape::kRecvOffset + (uint32_t)(slot * rows_of(to) * 512), (uint32_t)to),
                           smem_base + (uint32_t)(to * rows_per * 512), (uint32_t)(rows_of(to) * 512), bar);
@@ -266,8 +266,18 @@
       wide = (unsigned long long)*s_wide << (8 * rank);
       for (int rr = 0; rr < S - 1; ++rr) wide |= (unsigned long long)flags[rr * 4] << (8 * (rr < rank ? rr : rr + 1));
     }
-    if (wide) fence_acq_rel_cluster();
-    else cluster_arrive();                               // this rank has what was sent to it
+    if (wide) {
+      // the high words of every peer that has some; its own arrivals stand for the other peers
+      if (warp == 2 && lane == 0) {
+        int none = S - 1;
+        for (int r = 0; r < S; ++r) none -= r != rank && ((wide >> (8 * r)) & 0xff);
+        if (none) mbar_arrive_n(high_bar, (uint32_t)none);
+      }
+      __syncwarp();
+      ok = __all_sync(0xffffffffu, mbar_wait_acquire_cluster(high_bar, 0, abort_flag));
+    } else {
+      cluster_arrive();                                  // this rank has what was sent to it
+    }
     if (ok) {
       const int* mine = stage32 + rank * rows_per * 128;
       const int* recv = reinterpret_cast<const int*>(smem_gen + Shape::kRecvOffset);
