@@ -515,6 +515,19 @@ def test_cluster_merges_of_sums_beyond_32_bits(M, split, wide):
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M,split", [(9, 8), (64, 3), (80, 2), (128, 4)])
+def test_cluster_merges_wrap_32_bit_sums(M, split):
+    """1040 partials of 60 * 2^16, all in the fast range: 32-bit sums wrap around in the merge, 64-bit ones do not."""
+    K = 64 * 1040
+    a, b = torch.ones(M, K, dtype=torch.bfloat16, device="cuda"), torch.full((K, 136), 0.9375, dtype=torch.bfloat16, device="cuda")
+    with L.overrides(gemm_k_tile=64, gemm_split_k=split, gemm_flags=4096):         # GEMM_MID above 64 rows
+        narrow, full = (torch.ops.fxpr.gemm_fxp_int(a, b, bits, 16) for bits in (32, 64))
+    total = 1040 * 60 << 16
+    assert (full == total).all()
+    assert (narrow == (total + (1 << 31)) % (1 << 32) - (1 << 31)).all()
+    L.check_device_status()
+
+
 @pytest.mark.parametrize("M,N,K", [
     (65, 128, 64), (96, 256, 200), (97, 264, 1096), (128, 392, 640), (129, 520, 1096), (192, 256, 2056), (193, 1000, 328),
     (257, 384, 712), (333, 776, 456), (700, 520, 136),

@@ -87,6 +87,9 @@ static __device__ __noinline__ void fixup_tile(uint32_t taddr, int ncols, uint32
   }
 }
 
+// 32-bit sums wrap around, which signed addition must not.
+static __device__ __forceinline__ int wrap_add(int a, int b) { return (int)((uint32_t)a + (uint32_t)b); }
+
 // The whole warp probes: 1-7 % faster than one lane probing and a shuffle behind it.
 static __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));

@@ -392,7 +392,7 @@ gemm_tc_mid_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
             int4 q = *reinterpret_cast<const int4*>(mine + mr * 128 + lane * 4);
             for (int rr = 0; rr < S - 1; ++rr) {
               const int4 v = *reinterpret_cast<const int4*>(recv + (rr * my_rows + mr) * 128 + lane * 4);
-              q.x += v.x; q.y += v.y; q.z += v.z; q.w += v.w;
+              q.x = wrap_add(q.x, v.x); q.y = wrap_add(q.y, v.y); q.z = wrap_add(q.z, v.z); q.w = wrap_add(q.w, v.w);
             }
             emit(ks * rows_per + mr, q.x, q.y, q.z, q.w);
           }

@@ -287,7 +287,7 @@
           int4 q = *reinterpret_cast<const int4*>(mine + mr * 128 + lane * 4);
           for (int rr = 0; rr < S - 1; ++rr) {
             const int4 v = *reinterpret_cast<const int4*>(recv + (rr * my_rows + mr) * 128 + lane * 4);
-            q.x += v.x; q.y += v.y; q.z += v.z; q.w += v.w;
+            q.x = wrap_add(q.x, v.x); q.y = wrap_add(q.y, v.y); q.z = wrap_add(q.z, v.z); q.w = wrap_add(q.w, v.w);
           }
           emit(rank * rows_per + mr, n4, q.x, q.y, q.z, q.w);
         }
