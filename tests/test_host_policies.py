@@ -2,11 +2,26 @@
 the same bits) and the arg-max key arithmetic of the fused lm_head GEMM."""
 from __future__ import annotations
 
+import shutil
+import subprocess
+from pathlib import Path
+
 import pytest
 import torch
 
 import fxpr_vllm  # noqa: F401
 from fxpr_vllm import _lib as L
+
+
+def _policy_program(tmp_path, body):
+    """What a C++ program over csrc/host_policy.h prints (the functions that no C entry exports)."""
+    if shutil.which("g++") is None:
+        pytest.skip("no g++")
+    header = Path(fxpr_vllm.__file__).resolve().parent.parent / "csrc" / "host_policy.h"
+    src, exe = tmp_path / "policy.cpp", tmp_path / "policy"
+    src.write_text(f'#include "{header}"\n#include <chrono>\n#include <cstdio>\nusing namespace fxpr;\nint main() {{\n{body}\n}}\n')
+    subprocess.run(["g++", "-O2", "-std=c++17", str(src), "-o", str(exe)], check=True, capture_output=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
 
 
 def test_decode_gemm_split_policy_fills_the_sms_once():
@@ -37,6 +52,32 @@ def test_medium_batches_split_into_clusters():
             for n, k in ((768, 4096), (4096, 14336), (28672, 4096), (1064, 2376)):
                 got = L.pick_split_k(m, n, k, kt, 64, sms)
                 assert 1 <= got <= 16 and got <= -(-k // kt)
+
+
+def test_medium_batch_plan_takes_a_handful_of_steps_and_finds_the_cheapest_row_tiles(tmp_path):
+    """Every call above 64 rows makes this plan on the host: its time must not grow with the rows."""
+    assert float(_policy_program(tmp_path, """
+  const auto t0 = std::chrono::steady_clock::now();
+  volatile int sink = 0;
+  for (int i = 0; i < 1000; ++i) sink = sink + plan_mid_rows(1000000 + i, 4096, 4096, 128, 1, 148).row_tiles;
+  std::printf("%f", std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count() / 1000);
+""")) < 10.0                                                       # us; 98 when it walked all tile counts
+    assert _policy_program(tmp_path, """
+  int calls = 0, worse = 0;
+  for (int64_t M = 65; M < 1500; M += 13)
+    for (int64_t N : {128, 136, 768, 1000, 4096, 6144, 28672})
+      for (int64_t K : {64, 512, 4096, 14336})
+        for (int kt : {64, 128})
+          for (int split = 1; split <= 4; ++split) {
+            double least = 1e30;
+            for (int64_t t = ceil_div(M, split > 1 ? 128 : 256); t <= ceil_div(M, 64); ++t)
+              least = std::min(least, est_mid_us(mid_tile_rows(M, t), t, N, K, kt, split, 148));
+            const MidPlan plan = plan_mid_rows(M, N, K, kt, split, 148);
+            ++calls;
+            worse += plan.us != least || ceil_div(M, plan.row_tiles) > (split > 1 ? 128 : 256);
+          }
+  std::printf("%d %d", calls, worse);
+""") == "24864 0"
 
 
 def test_decode_attention_rank_policy():

@@ -4,7 +4,6 @@
 
 #include <algorithm>
 #include <cstdint>
-#include <climits>
 
 namespace fxpr {
 
@@ -50,21 +49,29 @@ inline double est_pair_us(int64_t M, int64_t N, int64_t K, int64_t k_tile, int n
   return waves * ((double)K / 128 * (k_tile == 64 ? 2690 : 1936) / 1850) + 3.5;
 }
 
+// gemm_tc_mid.cu with `tiles` row tiles of `rows` rows each.
+inline double est_mid_us(int64_t rows, int64_t tiles, int64_t N, int64_t K, int64_t k_tile, int split, int num_sms) {
+  const int64_t cols = ceil_div(N, 256), pairs = std::max(1, num_sms / 2);
+  // clusters of 4, 6 and 8 whole SMs that are resident at once: they do not pack a GPC
+  const int64_t room = split == 1 ? pairs : split == 2 ? num_sms * 34 / 148 : split == 3 ? num_sms * 20 / 148 : num_sms * 14 / 148;
+  const double waves = (double)ceil_div(cols * tiles, std::max<int64_t>(1, room));
+  const double copies = (double)(256 + rows) * (cols * tiles * split * 2 * 3 >= num_sms * 2 ? 3.05 : 2.4);
+  const double convert = (double)rows * (k_tile == 64 ? 14 : 7);
+  return waves * ((double)K / 128 / split * std::max(copies, convert) / 1850 + (waves > 1 ? 8 : 3)) +
+         (split == 1 ? 0.0 : split == 2 ? 2.0 : split == 3 ? 3.0 : 4.5);
+}
 // Row tiles of gemm_tc_mid.cu for a given split (0: it does not take the call) and their estimate.
 struct MidPlan { int row_tiles; double us; };
+inline int64_t mid_tile_rows(int64_t M, int64_t tiles) { return std::max<int64_t>(96, ceil_div(ceil_div(M, tiles), 32) * 32); }
 inline MidPlan plan_mid_rows(int64_t M, int64_t N, int64_t K, int64_t k_tile, int split, int num_sms) {
   MidPlan best = {0, 1e30};
   if (M <= 64 || N < 128 || split < 1 || split > 4 || (k_tile != 64 && k_tile != 128)) return best;
-  const int64_t cols = ceil_div(N, 256), pairs = std::max(1, num_sms / 2), most = split > 1 ? 128 : 256;
-  // clusters of 4, 6 and 8 whole SMs that are resident at once: they do not pack a GPC
-  const int64_t room = split == 1 ? pairs : split == 2 ? num_sms * 34 / 148 : split == 3 ? num_sms * 20 / 148 : num_sms * 14 / 148;
-  for (int64_t t = ceil_div(M, most); t <= ceil_div(M, 64) && t <= 65535; ++t) {
-    const int64_t rows = std::max<int64_t>(96, ceil_div(ceil_div(M, t), 32) * 32);
-    const double waves = (double)ceil_div(cols * t, std::max<int64_t>(1, room));
-    const double copies = (double)(256 + rows) * (cols * t * split * 2 * 3 >= num_sms * 2 ? 3.05 : 2.4);
-    const double convert = (double)rows * (k_tile == 64 ? 14 : 7);
-    const double us = waves * ((double)K / 128 / split * std::max(copies, convert) / 1850 + (waves > 1 ? 8 : 3)) +
-                      (split == 1 ? 0.0 : split == 2 ? 2.0 : split == 3 ? 3.0 : 4.5);
+  // Of the tile counts that round to the same rows the fewest cost least, so six counts at most are looked at,
+  // whatever M (all counts from M / 256 to M / 64 took the host 98 us at a million rows).
+  for (int64_t most = split > 1 ? 128 : 256; most >= 96; most -= 32) {
+    const int64_t t = ceil_div(M, most);
+    if (t > 65535) break;
+    const double us = est_mid_us(mid_tile_rows(M, t), t, N, K, k_tile, split, num_sms);
     if (us < best.us) best = {(int)t, us};
   }
   return best;
