@@ -159,8 +159,11 @@ int fxpr_log_softmax(const void* x, int x_dtype, float* y, int64_t rows,
                      int64_t cols, int frac_bits, void* stream);
 
 /*
- * Bytes of scratch fxpr_gemm needs for this problem (0 when split_k <= 1):
- * tile counters followed by one plane of integer partial tiles per split.
+ * Bytes of scratch that any fxpr_gemm call of this problem can need (0 when split_k <= 1):
+ * tile counters followed by one plane of integer partial tiles per split.  Calls whose
+ * splits a thread-block cluster merges (2 to 8 splits of up to 64 rows, 2 to 4 on the
+ * medium-batch kernel) and the CUDA-core kernel need none; a call that needs it and was given less
+ * returns FXPR_ERR_SCRATCH before it does anything.
  * The buffer must be zero-filled once before its first use; after that it may
  * be reused, without clearing, for calls of any shape that it is large enough
  * for (calls that share a buffer must be ordered on one stream).
@@ -176,8 +179,8 @@ int64_t fxpr_gemm_scratch_bytes(int64_t M, int64_t N, int int_bits, int split_k)
  * accumulators (for the tensor-parallel reduce and for tests).
  * k_tile: conversion granularity (0 = reference default: 128 for f16/bf16, 64
  * for f32).  split_k: 0/1 = none, else the K-tiles are dealt round-robin to
- * split_k CTAs per output tile; each leaves an integer partial tile in the
- * scratch and the last to arrive adds them up (order-free, needs scratch).
+ * split_k CTAs per output tile; a cluster merges their integer partial tiles, or each
+ * leaves its own in the scratch and the last to arrive adds them up (order-free either way).
  * partials_out: optional fp32 [ceil(K/k_tile), M, N] dump of the per-tile
  * float partials (tests only; must be NULL when split_k > 1).
  * status_word: optional device int the tensor-core kernel sets to

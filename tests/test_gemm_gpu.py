@@ -686,6 +686,42 @@ def test_streams_that_split_k_at_the_same_time_do_not_share_scratch():
                 assert torch.equal(g, calls[i // 3][2]), i
 
 
+_CAPTURE_AFTER_WARM_UP = """
+import torch, fxpr_vllm
+from fxpr_vllm import warmup, _lib as L
+M, N, K = %d, %d, %d
+a = torch.randn(M, K, device="cuda").bfloat16()
+b = torch.randn(K, N, device="cuda").bfloat16() * 0.02
+warmup.warmup_gemm(b, 64, 16)
+with L.overrides(gemm_k_tile=64):
+    assert L.pick_split_k(M, N, K, 64, 64, 148) > 1
+    small = torch.ops.fxpr.gemm_fxp_int(a[:, :256], b[:256, :256], 64, 16)     # loads the kernels
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16)
+    graph.replay()
+    torch.cuda.synchronize()
+    with L.overrides(gemm_split_k=1):
+        assert torch.equal(out, torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16))
+L.check_device_status()
+print("captured")
+"""
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 9600, 14336), (65, 10752, 18944)])
+def test_a_split_that_a_cluster_merges_needs_no_scratch_in_a_capture(M, N, K):
+    """Warmed up as a model is, a shape that was never run is captured: its planes would exceed the warmed scratch.
+    In a process of its own, since scratch that other tests grew would hide it."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    pkg = Path(fxpr_vllm.__file__).resolve().parent.parent
+    r = subprocess.run([sys.executable, "-c", _CAPTURE_AFTER_WARM_UP % (M, N, K)], cwd=pkg, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0 and "captured" in r.stdout, r.stderr[-2000:]
+
+
 def test_a_graph_that_splits_k_does_not_share_scratch_with_eager_calls():
     (a, b, want), (a2, b2, want2) = _split_calls(2)
     with L.overrides(gemm_split_k=8):

@@ -80,6 +80,28 @@ def test_medium_batch_plan_takes_a_handful_of_steps_and_finds_the_cheapest_row_t
 """) == "24864 0"
 
 
+def test_splits_that_no_cluster_merges_stay_within_the_scratch_of_the_warm_up(tmp_path):
+    """CUDA-graph capture cannot grow the scratch: whatever the policy picks needs what ``warmup_gemm`` made, or none."""
+    from fxpr_vllm import _native as nat
+
+    planes = _policy_program(tmp_path, """
+  for (int64_t M : {65, 80, 96, 97, 128, 129, 200, 256, 257, 300, 384})
+    for (int64_t N = 128; N <= 20000; N += N < 1500 ? 8 : 328)
+      for (int64_t K : {1024, 4096, 14336, 18944, 70000})
+        for (int kt : {64, 128}) {
+          const int split = pick_gemm_split_k(M, N, K, kt, 64, 148);
+          if (split > 1 && !mid_route(M, N, K, kt, split, 148))
+            std::printf("%d %d %d\\n", (int)M, (int)N, split);
+        }
+""")
+    shapes = {tuple(map(int, line.split())) for line in planes.splitlines()}
+    assert shapes
+    lib = nat.load()
+    for m, n, split in shapes:
+        for bits in (32, 64):
+            assert lib.fxpr_gemm_scratch_bytes(m, n, bits, split) <= L.gemm_scratch_policy_bytes(148, bits), (m, n, split)
+
+
 def test_decode_attention_rank_policy():
     f = L.pick_num_splits_b200
     assert f(5, 64, 1, 32, 8, 8192, 148) == 5                     # an explicit request is kept

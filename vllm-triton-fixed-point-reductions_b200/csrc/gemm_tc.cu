@@ -431,6 +431,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, TcParams& p, 
 
 bool gemm_tc_fast_supported(const GemmArgs& g, int split_k);
 bool gemm_tc_skinny_supported(const GemmArgs& g, int split_k);
+bool gemm_tc_skinny_cluster(const GemmArgs& g, int split_k);
 int gemm_tc_skinny(const GemmArgs& g, TcParams& p, const CUtensorMap& mw, cudaStream_t s);
 int gemm_tc_fast(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb,
                  cudaStream_t s);
@@ -446,18 +447,6 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   const bool b_kmajor = !((g.b_sn == 1) && (g.b_sk % 8 == 0));
   const bool acc64 = g.int_bits == 64;
   const int BN = acc64 ? 128 : 256;
-
-  CUtensorMap ma, mb;
-  if (!tc_make_map(&ma, g.dtype, g.a, g.M, g.K, g.a_sm, kBM)) {
-    set_last_error("cuTensorMapEncodeTiled(A)", cudaErrorInvalidValue);
-    return FXPR_ERR_CUDA;
-  }
-  const bool okb = b_kmajor ? tc_make_map(&mb, g.dtype, g.b, g.N, g.K, g.b_sn, 64)
-                            : tc_make_map(&mb, g.dtype, g.b, g.K, g.N, g.b_sk, 64);
-  if (!okb) {
-    set_last_error("cuTensorMapEncodeTiled(B)", cudaErrorInvalidValue);
-    return FXPR_ERR_CUDA;
-  }
 
   TcParams p;
   p.bias = g.bias; p.c = g.c; p.c_int = g.c_int; p.partials = g.partials;
@@ -476,7 +465,15 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   p.split_k = g.split_k < 1 ? 1 : (g.split_k > k_tiles ? k_tiles : g.split_k);
   p.acc_scratch = nullptr; p.locks = nullptr;
   if (((g.M + kBM - 1) / kBM) * ((g.N + 127) / 128) > kMaxSplitTiles) p.split_k = 1;
-  if (p.split_k > 1) {
+  // decode shapes: weights on the 128-row side of the MMA (same bits, see gemm_tc_skinny.cu)
+  const bool skinny = !(g.flags & (FXPR_GEMM_FORCE_EXACT_TC | FXPR_GEMM_NO_SKINNY)) && gemm_tc_skinny_supported(g, p.split_k);
+  // medium batches: weights on the M side of SM pairs (same bits, see gemm_tc_mid.cu)
+  int mid_rows = 0;
+  if (!(g.flags & (FXPR_GEMM_FORCE_EXACT_TC | FXPR_GEMM_TILE_N128 | FXPR_GEMM_PAIR)) && gemm_tc_mid_supported(g, p.split_k))
+    mid_rows = (g.flags & FXPR_GEMM_MID) ? plan_mid_rows(g.M, g.N, g.K, g.k_tile, p.split_k, sms).row_tiles
+                                         : mid_route(g.M, g.N, g.K, g.k_tile, p.split_k, sms);
+  // splits that a cluster merges need no scratch
+  if (p.split_k > 1 && !(skinny ? gemm_tc_skinny_cluster(g, p.split_k) : mid_rows > 0)) {
     const int64_t need = gemm_tc_scratch_bytes(g.M, g.N, g.int_bits, p.split_k);
     if (!g.scratch || g.scratch_bytes < need) return FXPR_ERR_SCRATCH;
     if ((uintptr_t)g.scratch & 15) return FXPR_ERR_BAD_ARG;
@@ -484,8 +481,19 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
     p.acc_scratch = (char*)g.scratch + tc_lock_bytes(g.M, g.N);
   }
 
-  // decode shapes: weights on the 128-row side of the MMA (same bits, see gemm_tc_skinny.cu)
-  if (!(g.flags & (FXPR_GEMM_FORCE_EXACT_TC | FXPR_GEMM_NO_SKINNY)) && gemm_tc_skinny_supported(g, p.split_k)) {
+  CUtensorMap ma, mb;
+  if (!tc_make_map(&ma, g.dtype, g.a, g.M, g.K, g.a_sm, kBM)) {
+    set_last_error("cuTensorMapEncodeTiled(A)", cudaErrorInvalidValue);
+    return FXPR_ERR_CUDA;
+  }
+  const bool okb = b_kmajor ? tc_make_map(&mb, g.dtype, g.b, g.N, g.K, g.b_sn, 64)
+                            : tc_make_map(&mb, g.dtype, g.b, g.K, g.N, g.b_sk, 64);
+  if (!okb) {
+    set_last_error("cuTensorMapEncodeTiled(B)", cudaErrorInvalidValue);
+    return FXPR_ERR_CUDA;
+  }
+
+  if (skinny) {
     p.silu_mul = (g.flags & FXPR_GEMM_SILU_MUL) ? 1 : 0;
     if (g.best) {
       if (p.split_k != 1 || p.silu_mul) return FXPR_ERR_UNSUPPORTED;
@@ -495,12 +503,7 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   }
   if (g.best) return FXPR_ERR_UNSUPPORTED;                          // only the decode-shape kernel
   if (g.flags & FXPR_GEMM_SILU_MUL) return FXPR_ERR_UNSUPPORTED;   // only the decode-shape kernel fuses it
-  // medium batches: weights on the M side of SM pairs (same bits, see gemm_tc_mid.cu)
-  if (!(g.flags & (FXPR_GEMM_FORCE_EXACT_TC | FXPR_GEMM_TILE_N128 | FXPR_GEMM_PAIR)) && gemm_tc_mid_supported(g, p.split_k)) {
-    const int rows = (g.flags & FXPR_GEMM_MID) ? plan_mid_rows(g.M, g.N, g.K, g.k_tile, p.split_k, sms).row_tiles
-                                               : mid_route(g.M, g.N, g.K, g.k_tile, p.split_k, sms);
-    if (rows) return gemm_tc_mid(g, p, mb, rows, s);
-  }
+  if (mid_rows) return gemm_tc_mid(g, p, mb, mid_rows, s);
   if (!(g.flags & FXPR_GEMM_FORCE_EXACT_TC) && gemm_tc_pair_supported(g, p.split_k)) {
     // 256 x 256 tiles on SM pairs or 128 x 128 tiles on single SMs (same bits).  A full wave of pair
     // tiles has twice the output of a wave of single tiles and takes 1.7 times as long at K-tile 64

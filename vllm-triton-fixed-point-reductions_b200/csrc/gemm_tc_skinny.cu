@@ -231,6 +231,12 @@ bool gemm_tc_skinny_supported(const GemmArgs& g, int split_k) {
   return g.M <= kSkMaxRows && g.partials == nullptr && gemm_tc_fast_supported(g, split_k);
 }
 
+// 2 to 8 splits run as a thread-block cluster (merge through distributed shared memory, no scratch);
+// larger split counts use the partial planes in the caller's scratch.  Same bits either way.
+bool gemm_tc_skinny_cluster(const GemmArgs& g, int split_k) {
+  return split_k >= 2 && split_k <= 8 && (g.N + 127) / 128 <= 65535 && !(g.flags & FXPR_GEMM_NO_CLUSTER);
+}
+
 template <typename T, int MP, bool CLUSTER, int PER_SM>
 static int launch_skinny(const GemmArgs& g, const CUtensorMap& mw, TcParams& p, cudaStream_t s) {
   constexpr int kSmem = SkShape<MP, PER_SM>::kSmem;
@@ -261,9 +267,7 @@ template <typename T, int MP>
 static int route_skinny(const GemmArgs& g, const CUtensorMap& mw, TcParams& p, int sms, cudaStream_t s) {
   p.tiles_m = 1;
   p.tiles_n = (p.N + 127) / 128;
-  // 2 to 8 splits run as a thread-block cluster (merge through distributed shared memory);
-  // larger split counts use the partial planes in the caller's scratch.  Same bits either way.
-  const bool cluster = p.split_k >= 2 && p.split_k <= 8 && p.tiles_n <= 65535 && !(g.flags & FXPR_GEMM_NO_CLUSTER);
+  const bool cluster = gemm_tc_skinny_cluster(g, p.split_k);
   // A grid that does not fill the SMs once gives a CTA the whole SM's memory as its ring; more CTAs share an
   // SM, so that the column tiles of large weights all stream at once (64 x 28672 x 4096, 224 tiles: 46.5 us
   // with one CTA and tile after tile per SM, 38.8 with two).  64 x 4096 x 4096 on 128 CTAs: 11.3 us with the

@@ -364,17 +364,21 @@ GemmOut gemm_common(const Tensor& a, const Tensor& b, const optional<Tensor>& bi
     partials = at::zeros({k_tiles, M, N}, a.options().dtype(at::kFloat));
     t_ovr.last_partials = partials;
   }
-  int64_t scratch_bytes = 0;
-  if (split > 1) {
-    scratch_bytes = fxpr_gemm_scratch_bytes(M, N, (int)int_bits, split);
-    scratch = gemm_scratch(on.dev, scratch_bytes);
+  const auto call = [&](int64_t scratch_bytes) {
+    return fxpr_gemm(a.data_ptr(), b.data_ptr(), ptr(bias), r.c.defined() ? r.c.data_ptr() : nullptr,
+                     r.c_int.defined() ? r.c_int.data_ptr() : nullptr, dtype_code(t), M, N, K, a.stride(0), a.stride(1),
+                     b.stride(0), b.stride(1), r.c.defined() ? r.c.stride(0) : N, (int)int_bits, (int)frac_bits, k_tile,
+                     split, flags, scratch.defined() ? scratch.data_ptr() : nullptr, scratch_bytes,
+                     partials.defined() && partials.numel() ? partials.data_ptr<float>() : nullptr, status_ptr(on.dev),
+                     on.stream());
+  };
+  // Most splits are merged without scratch, and the library says, before it does anything, where they are not.
+  int st = call(0);
+  if (st == FXPR_ERR_SCRATCH) {
+    const int64_t bytes = fxpr_gemm_scratch_bytes(M, N, (int)int_bits, split);
+    scratch = gemm_scratch(on.dev, bytes);
+    st = call(bytes);
   }
-  const int st = fxpr_gemm(a.data_ptr(), b.data_ptr(), ptr(bias), r.c.defined() ? r.c.data_ptr() : nullptr,
-                           r.c_int.defined() ? r.c_int.data_ptr() : nullptr, dtype_code(t), M, N, K, a.stride(0), a.stride(1),
-                           b.stride(0), b.stride(1), r.c.defined() ? r.c.stride(0) : N, (int)int_bits, (int)frac_bits, k_tile,
-                           split, flags, scratch.defined() ? scratch.data_ptr() : nullptr, scratch_bytes,
-                           partials.defined() && partials.numel() ? partials.data_ptr<float>() : nullptr, status_ptr(on.dev),
-                           on.stream());
   if (want.silu_pairs && st == FXPR_ERR_UNSUPPORTED) { r.unsupported = true; return r; }
   check_status(st, "gemm_fxp");
   return r;

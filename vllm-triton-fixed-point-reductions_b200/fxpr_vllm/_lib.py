@@ -202,11 +202,12 @@ def _get_gemm_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
 
 
 def gemm_scratch_policy_bytes(num_sms: int, int_bits: int = 64) -> int:
-    """Largest scratch the automatic split-K policy (``pick_split_k``) can ask for,
-    whatever M, N and K: it doubles the split only while ``tiles * split * 2 <= num_sms``,
-    so at most ``num_sms`` integer partial tiles of 128 x 128 exist, each padded to 256
-    columns in the worst case, after the fixed 256 KiB counter region."""
-    planes = num_sms * 128 * 256 * (8 if int_bits == 64 else 4)
+    """Largest scratch a split of the automatic policy (``pick_split_k``) can need,
+    whatever M, N and K.  Splits that a cluster merges need none.  The others double only while
+    ``tiles * split * 2 <= num_sms``, so at most ``num_sms`` integer partial tiles of 128 x 128 exist, and
+    one more a split (16 at most) where the columns are padded to 256; rows padded to 256 can double
+    that.  In front of them the fixed 256 KiB counter region."""
+    planes = (num_sms + 16) * 128 * 256 * (8 if int_bits == 64 else 4)
     return 256 * 1024 + -(-planes // 256) * 256
 
 
