@@ -322,7 +322,8 @@ int fxpr_gemm_default_k_tile(int dtype);
 
 /*
  * Automatic split counts, from host shapes only (the torch operators ask the same functions; no
- * choice changes a result).  GEMM K-splits; KV splits of the CUDA-core attention route
+ * choice changes a result).  GEMM K-splits (for at most 21 fraction bits and no flag that names
+ * a kernel); KV splits of the CUDA-core attention route
  * (fxpr_vllm/_triton/attention.py:664-689); cluster ranks of the tensor-core attention route.
  */
 int fxpr_pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int k_tile, int int_bits, int num_sms);

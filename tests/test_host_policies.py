@@ -80,6 +80,26 @@ def test_medium_batch_plan_takes_a_handful_of_steps_and_finds_the_cheapest_row_t
 """) == "24864 0"
 
 
+def test_splits_follow_the_kernel_that_runs(tmp_path):
+    """The medium-batch kernel's cluster merges set the split only where that kernel may run: not above 21 fraction
+    bits or in the exact-conversion kernel (planes, at most four), and not where a flag names another kernel."""
+    got = _policy_program(tmp_path, """
+  for (int64_t M : {80, 200, 256})
+    for (int64_t N : {256, 768, 4096})
+      for (auto k : {wide_kernels(16, 0), wide_kernels(32, 0), wide_kernels(16, FXPR_GEMM_FORCE_EXACT_TC),
+                     wide_kernels(16, FXPR_GEMM_TILE_N128), wide_kernels(16, FXPR_GEMM_MID)})
+        std::printf("%d ", pick_gemm_split_k(M, N, 4096, 128, 64, 148, k));
+""").split()
+    # (any kernel, 32 fraction bits, exact, 128 x 128 tiles, the medium-batch flag) by shape
+    rows = [list(map(int, got[i:i + 5])) for i in range(0, len(got), 5)]
+    for (m, n), (free, fine, exact, single, mid) in zip([(m, n) for m in (80, 200, 256) for n in (256, 768, 4096)], rows):
+        tiles = -(-m // 128) * (n // 128)
+        doubled = 1
+        while doubled < 16 and tiles * doubled * 2 <= 148 and 32 // (doubled * 2) >= 4:
+            doubled *= 2
+        assert fine == exact == min(4, 148 // tiles) and single == doubled and mid == free <= 4, (m, n)
+
+
 def test_splits_that_no_cluster_merges_stay_within_the_scratch_of_the_warm_up(tmp_path):
     """CUDA-graph capture cannot grow the scratch: whatever the policy picks needs what ``warmup_gemm`` made, or none."""
     from fxpr_vllm import _native as nat

@@ -469,7 +469,7 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   const bool skinny = !(g.flags & (FXPR_GEMM_FORCE_EXACT_TC | FXPR_GEMM_NO_SKINNY)) && gemm_tc_skinny_supported(g, p.split_k);
   // medium batches: weights on the M side of SM pairs (same bits, see gemm_tc_mid.cu)
   int mid_rows = 0;
-  if (!(g.flags & (FXPR_GEMM_FORCE_EXACT_TC | FXPR_GEMM_TILE_N128 | FXPR_GEMM_PAIR)) && gemm_tc_mid_supported(g, p.split_k))
+  if (wide_kernels(g.frac_bits, g.flags) == WideKernels::any && gemm_tc_mid_supported(g, p.split_k))
     mid_rows = (g.flags & FXPR_GEMM_MID) ? plan_mid_rows(g.M, g.N, g.K, g.k_tile, p.split_k, sms).row_tiles
                                          : mid_route(g.M, g.N, g.K, g.k_tile, p.split_k, sms);
   // splits that a cluster merges need no scratch

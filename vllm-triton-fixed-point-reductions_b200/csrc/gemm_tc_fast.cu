@@ -33,6 +33,7 @@
 
 #include "fxp_common.cuh"
 #include "gemm_common.cuh"
+#include "host_policy.h"
 #include "tc_common.cuh"
 #include "gemm_tc_fast_common.cuh"
 
@@ -239,11 +240,11 @@ static int launch_fast(const CUtensorMap& ma, const CUtensorMap& mb, TcParams& p
 // conversion (gemm_tc.cu) serves those.
 bool gemm_tc_fast_supported(const GemmArgs& g, int split_k) {
   if (g.int_bits == 16) return false;
-  if (g.frac_bits > 21) return false;
+  if (g.frac_bits > kFastFracBits) return false;
   if (g.k_tile != 64 && g.k_tile != 128) return false;
   const int64_t k_tiles = (g.K + g.k_tile - 1) / g.k_tile;
   const int64_t per_item = (k_tiles + split_k - 1) / split_k;
-  return per_item <= 510;
+  return per_item <= kFastKTiles;
 }
 
 int gemm_tc_fast(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb,

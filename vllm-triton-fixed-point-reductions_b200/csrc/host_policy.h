@@ -5,6 +5,8 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "../../include/fxpr_b200.h"
+
 namespace fxpr {
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
@@ -60,12 +62,23 @@ inline double est_mid_us(int64_t rows, int64_t tiles, int64_t N, int64_t K, int6
   return waves * ((double)K / 128 / split * std::max(copies, convert) / 1850 + (waves > 1 ? 8 : 3)) +
          (split == 1 ? 0.0 : split == 2 ? 2.0 : split == 3 ? 3.0 : 4.5);
 }
+// What conversion a call above 64 rows gets and which kernels may run it: any of the three, not the medium-batch one (a
+// flag names another), or, beyond the fast conversion's range (gemm_tc_fast_supported), only the plain-conversion kernel.
+enum class WideKernels { any, no_mid, plain };
+inline constexpr int kFastFracBits = 21;
+inline constexpr int64_t kFastKTiles = 510;              // K-tiles of an item whose 32-bit sums cannot overflow
+inline WideKernels wide_kernels(int frac_bits, int flags) {
+  if (frac_bits > kFastFracBits || (flags & FXPR_GEMM_FORCE_EXACT_TC)) return WideKernels::plain;
+  return (flags & (FXPR_GEMM_TILE_N128 | FXPR_GEMM_PAIR)) ? WideKernels::no_mid : WideKernels::any;
+}
+
 // Row tiles of gemm_tc_mid.cu for a given split (0: it does not take the call) and their estimate.
 struct MidPlan { int row_tiles; double us; };
 inline int64_t mid_tile_rows(int64_t M, int64_t tiles) { return std::max<int64_t>(96, ceil_div(ceil_div(M, tiles), 32) * 32); }
 inline MidPlan plan_mid_rows(int64_t M, int64_t N, int64_t K, int64_t k_tile, int split, int num_sms) {
   MidPlan best = {0, 1e30};
   if (M <= 64 || N < 128 || split < 1 || split > 4 || (k_tile != 64 && k_tile != 128)) return best;
+  if (ceil_div(ceil_div(K, k_tile), split) > kFastKTiles) return best;
   // Of the tile counts that round to the same rows the fewest cost least, so six counts at most are looked at,
   // whatever M (all counts from M / 256 to M / 64 took the host 98 us at a million rows).
   for (int64_t most = split > 1 ? 128 : 256; most >= 96; most -= 32) {
@@ -85,7 +98,8 @@ inline int mid_route(int64_t M, int64_t N, int64_t K, int64_t k_tile, int split,
 }
 
 // K-split of a GEMM: split when the output tiles alone cannot fill the GPU.
-inline int pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int64_t k_tile, int int_bits, int num_sms) {
+inline int pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int64_t k_tile, int int_bits, int num_sms,
+                             WideKernels kernels = WideKernels::any) {
   if (int_bits == 16) return 1;
   const int64_t tiles = ceil_div(M, 128) * ceil_div(N, 128);
   const int64_t k_tiles = ceil_div(K, k_tile);
@@ -98,8 +112,15 @@ inline int pick_gemm_split_k(int64_t M, int64_t N, int64_t K, int64_t k_tile, in
     while (split < 8 && tiles * split * 2 <= num_sms * 9 / 10 && K / (split * 2) >= 384) split *= 2;
     return split;
   }
-  // one wave of CTAs at most: a second, partly filled wave costs more than it hides
+  // One wave of CTAs at most: a second, partly filled wave costs more than it hides.
+  if (kernels == WideKernels::plain) {
+    // this kernel's last arriver adds its planes alone (32 fraction bits, 64-bit sums, us: 80 x 768 x 4096 three splits
+    // 33.9, four 32.7, eight 42.1, sixteen 64.4; 200 x 2560 x 8192 two 63.1, three 52.5, four, a second wave, 89.3;
+    // 80 x 2048 x 2048, sixteen K-tiles, two 24.8, three 27.3, four 27.4)
+    return (int)std::max<int64_t>(1, std::min<int64_t>(k_tiles >= 24 ? 4 : 2, num_sms / tiles));
+  }
   while (split < 16 && tiles * split * 2 <= num_sms && k_tiles / (split * 2) >= 4) split *= 2;
+  if (kernels != WideKernels::any) return split;
   // the splits of a cluster are cheaper to merge
   int best = split;
   double us = est_single_us(M, N, K, k_tile, split, num_sms);

@@ -357,7 +357,8 @@ GemmOut gemm_common(const Tensor& a, const Tensor& b, const optional<Tensor>& bi
   }
 
   int split = o.gemm_split_k >= 0 ? o.gemm_split_k : cfg.gemm_split_k.load();
-  if (split <= 0) split = fxpr::pick_gemm_split_k(M, N, K, k_tile, (int)int_bits, num_sms(on.dev));
+  if (split <= 0)
+    split = fxpr::pick_gemm_split_k(M, N, K, k_tile, (int)int_bits, num_sms(on.dev), fxpr::wide_kernels((int)frac_bits, flags));
   split = (int)std::max<int64_t>(1, std::min<int64_t>(split, std::max<int64_t>(1, k_tiles)));
   Tensor partials, scratch;
   if (o.gemm_partials && split == 1) {
