@@ -528,6 +528,59 @@ def test_cluster_merges_wrap_32_bit_sums(M, split):
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M,N", [(129, 130), (300, 136), (256, 161), (290, 552), (417, 260), (200, 129)])
+@pytest.mark.parametrize("far", [False, True])
+def test_two_sm_kernel_integer_outputs(M, N, far):
+    """Integer sums by TMA where their rows start on 16 bytes (32 or 64 bits a column) and by rows where not, at every
+    edge, with a fix-up in some warps, alone and next to the io outputs: the plain-conversion kernel's integers."""
+    from fxpr_vllm import _native as nat
+
+    K = 320
+    a = _rand((M, K), torch.float16, M, 2.0).cuda()
+    b = _rand((N, K), torch.float16, N, 1.0).cuda().t()
+    if far:
+        a[M // 2, 64:128] = 3.0e4
+    lib = nat.load()
+    for bits, dtype in ((32, torch.int32), (64, torch.int64)):
+        with L.overrides(gemm_k_tile=64, gemm_split_k=1, gemm_flags=nat.GEMM_FORCE_EXACT_TC):
+            want = torch.ops.fxpr.gemm_fxp_int(a, b, bits, 16)
+            want_c = _gemm(a, b, None, bits, 16)
+        with L.overrides(gemm_k_tile=64, gemm_split_k=1, gemm_flags=nat.GEMM_PAIR):
+            assert torch.equal(torch.ops.fxpr.gemm_fxp_int(a, b, bits, 16), want)
+        c = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float16)
+        c_int = torch.full((M, N), -1, device="cuda", dtype=dtype)
+        assert lib.fxpr_gemm(a.data_ptr(), b.data_ptr(), None, c.data_ptr(), c_int.data_ptr(), 0, M, N, K, K, 1, 1, K, N, bits, 16,
+                             64, 1, nat.GEMM_PAIR, None, 0, None, None, torch.cuda.current_stream().cuda_stream) == 0
+        assert torch.equal(c_int, want) and torch.equal(c.view(torch.int16), want_c.view(torch.int16))
+    L.check_device_status()
+
+
+def _fastest_us(fn, n=5):
+    times = []
+    for _ in range(n):
+        start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        fn()
+        stop.record()
+        torch.cuda.synchronize()
+        times.append(start.elapsed_time(stop) * 1e3)
+    return min(times)
+
+
+def test_two_sm_kernel_time_does_not_depend_on_the_size_of_the_sums():
+    """Sums of 64.0 and more (16 fraction bits) are ordinary outputs of operands with a mean: they may not cost a
+    multiple of small sums (2.1 to 2.3 times when they went element by element through local memory)."""
+    a = _rand((4096, 4096), torch.bfloat16, 1).cuda()
+    b = _rand((4096, 4096), torch.bfloat16, 2, 0.02).cuda()
+    far_a, far_b = a + 0.5, b + 0.1
+    for kt in (64, 128):
+        with L.overrides(gemm_k_tile=kt):
+            small = _fastest_us(lambda: _gemm(a, b, None, 64, 16))
+            large = _fastest_us(lambda: _gemm(far_a, far_b, None, 64, 16))
+        assert _gemm(far_a, far_b, None, 64, 16).float().abs().median() > 100
+        assert large < 1.4 * small, (kt, small, large)
+
+
 @pytest.mark.parametrize("M,N,K", [
     (65, 128, 64), (96, 256, 200), (97, 264, 1096), (128, 392, 640), (129, 520, 1096), (192, 256, 2056), (193, 1000, 328),
     (257, 384, 712), (333, 776, 456), (700, 520, 136),

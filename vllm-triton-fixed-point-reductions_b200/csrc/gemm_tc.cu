@@ -354,6 +354,18 @@ bool tc_make_map(CUtensorMap* m, int dtype, const void* base, int64_t rows, int6
   return r == CUDA_SUCCESS;
 }
 
+bool tc_make_map_int(CUtensorMap* m, int int_bits, const void* base, int64_t rows, int64_t cols, int box_rows) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return false;
+  const int bytes = int_bits / 8;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)cols * bytes};
+  cuuint32_t box[2] = {(cuuint32_t)(64 / bytes), (cuuint32_t)box_rows}, estr[2] = {1, 1};
+  return fn(m, int_bits == 64 ? CU_TENSOR_MAP_DATA_TYPE_INT64 : CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<void*>(base),
+            dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool tc_make_map_groups(CUtensorMap* m, int dtype, const void* base, int64_t rows, int64_t cols,
                         int64_t row_stride_elems, int box_rows) {
   EncodeTiledFn fn = get_encode_fn();
@@ -457,7 +469,7 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
   p.idesc = make_idesc(g.dtype == FXPR_BF16 ? 1 : 0, b_kmajor ? 0 : 1, BN, kBM);
   p.c_vec_ok = g.c && !((uintptr_t)g.c & 15) && g.c_sm % 8 == 0;
   p.status = g.status;
-  p.c_tma = 0;
+  p.c_tma = p.ci_tma = 0;
   p.silu_mul = 0;
   p.best = nullptr; p.n_offset = 0;
   p.w_static = (g.flags & FXPR_GEMM_WEIGHTS_STATIC) ? 1 : 0;

@@ -31,6 +31,9 @@
 // Numerics, the conversion with its range screen and exact fix-up are those of gemm_tc_fast.cu
 // (gemm_tc_fast_common.cuh); results are bit-identical to it (the fixed-point contract:
 // fxpr_vllm/_triton/gemm.py:183-204).  Every wait is bounded.
+#include <cstring>
+#include <type_traits>
+
 #include <cuda.h>
 
 #include "fxp_common.cuh"
@@ -54,10 +57,11 @@ static constexpr int kPrSmem = kPrStages * kPrStageBytes + kPrEpiW * kPrOutBytes
 static_assert(kPrSmem <= 227 * 1024, "shared memory of an SM");
 static constexpr int kPrCols = 64;                         // accumulator columns per epilogue thread
 
-template <typename T>
+template <typename T, bool INTS>
 __global__ void __launch_bounds__(kPrThreads, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                    const __grid_constant__ CUtensorMap tma_c, const TcParams p, const int zero /* always 0: keeps the side arrays in local memory */) {
+                    const __grid_constant__ CUtensorMap tma_c, const __grid_constant__ CUtensorMap tma_ci,
+                    const TcParams p, const int zero /* always 0: keeps the side arrays in local memory */) {
   constexpr int kOutOffset = kPrStages * kPrStageBytes, kBarOffset = kOutOffset + kPrEpiW * kPrOutBytes;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -222,81 +226,118 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_cons
       const int col0 = pn * 256 + cgroup * kPrCols;
       const uint32_t bias_bits = (uint32_t)n_kt * mbits;   // what the multiply-adds summed on top
       const T* bias = (const T*)p.bias;
-      // Fast output: with every sum below 2^22 in magnitude, MAGIC + sum is a float whose value minus
-      // MAGIC is the sum, so one fma gives sum * 2^-f exactly (what int -> float -> scale gives).  The rows go
-      // through shared memory and leave by TMA, which clips them to the matrix, while the next tile is
-      // converted.  (Stored by the threads, a row each, an output took the epilogue warps 7700-8400 clocks a tile:
-      // all SMs write at the same time, and the stores wait.)
-      bool fast = !corr_used && p.c_tma;
-      if (fast) {
-        uint32_t off = 0;
+      // Sums fit 32 bits unless a partial took the fix-up, and are converted to float where the outputs are made, one
+      // instruction each, whatever their size.  (Sums below 2^22 allow a shortcut, MAGIC + sum as a float, but its
+      // test, and any second form next to it, spills in the main loop: 4096^3, K-tile 128, us: shortcut and a loop out
+      // of local memory for larger sums 134 and 314, both in registers 138 and 137, this one 130 and 127; K-tile 64:
+      // 187 and 370, 199 and 202, 186 and 187.)  After a fix-up the exact 64-bit sums, as floats, are put together out of
+      // local memory, in a loop.
+      if (corr_used) {
+        uint32_t sums[kPrCols];
+#pragma unroll
+        for (int i = 0; i < kPrCols; ++i) sums[i + zero] = alu_add(i) ? acc[i] : acc[i] - bias_bits;
+#pragma unroll 4
+        for (int c = 0; c < kPrCols; ++c) {
+          // the in-range part is < 2^31 in magnitude, so it is the sign extension of the wrapped sum once
+          // the out-of-range raw values are taken out again
+          long long t = (long long)(int32_t)(sums[c + zero] - corr_raw[c + zero]) + corr_q[c + zero];
+          if (p.int_bits != 64) t = (long long)(int32_t)t;
+          if constexpr (INTS) corr_q[c + zero] = t;
+          sums[c + zero] = __float_as_uint(__ll2float_rn(t));
+        }
+#pragma unroll
+        for (int i = 0; i < kPrCols; ++i) acc[i] = sums[i + zero];
+      } else {
 #pragma unroll
         for (int i = 0; i < kPrCols; ++i) {
-          acc[i] += alu_add(i) ? kMagicBits : kMagicBits - bias_bits;
-          off |= acc[i] ^ kExpBits;
-        }
-        fast = !__any_sync(0xffffffffu, (off >> 23) != 0);
-        if (!fast) {
-#pragma unroll
-          for (int i = 0; i < kPrCols; ++i) acc[i] -= alu_add(i) ? kMagicBits : kMagicBits - bias_bits;
+          if (!alu_add(i)) acc[i] -= bias_bits;
+          if constexpr (INTS) corr_q[i + zero] = (long long)(int)acc[i];
         }
       }
-      if (fast) {
-        if (col0 < p.N && row - lane < p.M) {
-          const float inv = p.inv_scale, minus = -__fmul_rn(__uint_as_float(kMagicBits), inv);
-          const uint32_t out_s = smem_base + kOutOffset + (uint32_t)((warp - kPrFirstEpi) * kPrOutBytes);
+      if (col0 < p.N && row - lane < p.M) {
+        // 32 rows x 64 bytes at a time go through shared memory and leave by TMA, which clips them to the matrix, while
+        // the next tile is converted.  (Stored by the threads, a row each, an output took the epilogue warps 7700-8400
+        // clocks a tile: all SMs write at the same time, and the stores wait.)  A matrix that no tensor map can
+        // describe is written from there by rows.
+        const uint32_t out_s = smem_base + kOutOffset + (uint32_t)((warp - kPrFirstEpi) * kPrOutBytes);
+        auto staging_free = [&]() {
+          tma_store_wait_read();                           // the last store has read it
+          __syncwarp();
+        };
+        // 16-byte chunks swizzled with the row, as the tensor maps say
+        auto at = [&](int r, int chunk) { return out_s + (uint32_t)(r * 64 + ((chunk ^ ((r >> 1) & 3)) << 4)); };
+        auto put = [&](int chunk, const uint32_t* w) {
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                       ::"r"(at(lane, chunk)), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+        };
+        auto leave = [&](const CUtensorMap* map, bool tma, int x, auto* base, int64_t stride) {
+          using E = std::remove_pointer_t<decltype(base)>;
+          if (tma) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0 && x < p.N) {
+              tma_store_2d(map, out_s, x, row);
+              tma_store_commit();
+            }
+          } else {
+            constexpr int kPerRow = 64 / (int)sizeof(E), kRows = 32 / kPerRow;
+            const int e = lane % kPerRow;
+            __syncwarp();
+#pragma unroll 4
+            for (int r = lane / kPerRow; r < 32; r += kRows) {
+              const uint32_t from = at(r, e * (int)sizeof(E) >> 4) + (uint32_t)(e * (int)sizeof(E) & 15);
+              E v;
+              memcpy(&v, smem_gen + (from - smem_base), sizeof(E));
+              if (row - lane + r < p.M && x + e < p.N) base[(int64_t)(row - lane + r) * stride + x + e] = v;
+            }
+          }
+        };
+        if constexpr (INTS) {
+          const long long* q = &corr_q[zero];
+          if (p.int_bits == 64) {
+#pragma unroll 1
+            for (int h = 0; h < kPrCols; h += 8) {
+              staging_free();
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const long long a = q[h + 2 * g], b = q[h + 2 * g + 1];
+                const uint32_t w[4] = {(uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32)};
+                put(g, w);
+              }
+              leave(&tma_ci, p.ci_tma, col0 + h, (long long*)p.c_int, p.N);
+            }
+          } else {
+#pragma unroll 1
+            for (int h = 0; h < kPrCols; h += 16) {
+              staging_free();
+#pragma unroll
+              for (int g = 0; g < 4; ++g) {
+                const int c = h + 4 * g;
+                const uint32_t w[4] = {(uint32_t)q[c], (uint32_t)q[c + 1], (uint32_t)q[c + 2], (uint32_t)q[c + 3]};
+                put(g, w);
+              }
+              leave(&tma_ci, p.ci_tma, col0 + h, (int32_t*)p.c_int, p.N);
+            }
+          }
+        }
+        if (!INTS || p.c) {
+          const float inv = p.inv_scale;
 #pragma unroll
           for (int h = 0; h < kPrCols; h += 32) {
-            tma_store_wait_read();                         // the last store has read the staging
-            __syncwarp();
+            staging_free();
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
               alignas(16) T out[8];
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 const int c = h + g * 8 + i;
-                float v = __fmaf_rn(__uint_as_float(acc[c]), inv, minus);
+                float v = __fmul_rn(corr_used ? __uint_as_float(acc[c]) : __int2float_rn((int)acc[c]), inv);
                 if (bias) v = __fadd_rn(v, col0 + c < p.N ? to_f32<T>(bias[col0 + c]) : 0.0f);
                 out[i] = from_f32<T>(v);
               }
-              const uint32_t* w = reinterpret_cast<const uint32_t*>(out);
-              // 16-byte chunks swizzled with the row, as the tensor map says
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
-                           ::"r"(out_s + (uint32_t)(lane * 64 + ((g ^ ((lane >> 1) & 3)) << 4))), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+              put(g, reinterpret_cast<const uint32_t*>(out));
             }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0 && col0 + h < p.N) {
-              tma_store_2d(&tma_c, out_s, col0 + h, row);
-              tma_store_commit();
-            }
-          }
-        }
-      } else {
-        // integer output, corrections, large sums or an unaligned matrix: element by element out of local
-        // memory, in a loop (unrolled it was most of the kernel's code)
-        uint32_t sums[kPrCols];
-#pragma unroll
-        for (int i = 0; i < kPrCols; ++i) sums[i + zero] = alu_add(i) ? acc[i] : acc[i] - bias_bits;
-        if (row < p.M) {
-#pragma unroll 4
-          for (int c = 0; c < kPrCols; ++c) {
-            const int col = col0 + c;
-            if (col >= p.N) break;
-            // with corrections the in-range part is < 2^31 in magnitude, so it is the sign extension of the
-            // wrapped sum once the out-of-range raw values are taken out again
-            long long t = (long long)(int32_t)(corr_used ? sums[c + zero] - corr_raw[c + zero] : sums[c + zero]);
-            if (corr_used) t += corr_q[c + zero];
-            if (p.int_bits != 64) t = (long long)(int32_t)t;
-            if (p.c_int) {
-              if (p.int_bits == 64) ((long long*)p.c_int)[(int64_t)row * p.N + col] = t;
-              else ((int32_t*)p.c_int)[(int64_t)row * p.N + col] = (int32_t)t;
-            }
-            if (p.c) {
-              float v = fixed_to_float<long long>(t, p.inv_scale);
-              if (bias) v = __fadd_rn(v, to_f32<T>(bias[col]));
-              ((T*)p.c)[(int64_t)row * p.c_sm + col] = from_f32<T>(v);
-            }
+            leave(&tma_c, p.c_tma, col0 + h, (T*)p.c, p.c_sm);
           }
         }
       }
@@ -331,10 +372,10 @@ bool gemm_tc_pair_supported(const GemmArgs& g, int split_k) {
   return split_k == 1 && g.partials == nullptr && g.M > 128 && g.N >= 128 && gemm_tc_fast_supported(g, split_k);
 }
 
-template <typename T>
-static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, TcParams& p, int sms,
-                       cudaStream_t s) {
-  auto k = gemm_tc_pair_kernel<T>;
+template <typename T, bool INTS>
+static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const CUtensorMap& mci,
+                       TcParams& p, int sms, cudaStream_t s) {
+  auto k = gemm_tc_pair_kernel<T, INTS>;
   static bool attr_done_dev[64] = {};            // function attributes are per device
   int dev_id = 0;
   cudaGetDevice(&dev_id);
@@ -357,7 +398,7 @@ static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUten
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, k, ma, mb, mc, (const TcParams)p, 0);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, k, ma, mb, mc, mci, (const TcParams)p, 0);
   if (e != cudaSuccess) { set_last_error("gemm_tc_pair launch", e); return FXPR_ERR_CUDA; }
   return check_launch("gemm_tc_pair");
 }
@@ -367,11 +408,14 @@ int gemm_tc_pair(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CU
   const int sms = tc_device_sms();
   if (sms < 0) return FXPR_ERR_ARCH;
   p.idesc = make_idesc(g.dtype == FXPR_BF16 ? 1 : 0, p.b_kmajor ? 0 : 1, 256, 256);
-  // C by TMA where a tensor map can say where it is: rows that start on 16 bytes
-  CUtensorMap mc = ma;
-  p.c_tma = !p.c_int && p.c_vec_ok && tc_make_map(&mc, g.dtype, g.c, g.M, g.N, g.c_sm, 32, 32);
-  if (g.dtype == FXPR_BF16) return launch_pair<__nv_bfloat16>(ma, mb, mc, p, sms, s);
-  return launch_pair<__half>(ma, mb, mc, p, sms, s);
+  // outputs by TMA where a tensor map can say where they are: rows that start on 16 bytes
+  CUtensorMap mc = ma, mci = ma;
+  p.c_tma = p.c_vec_ok && tc_make_map(&mc, g.dtype, g.c, g.M, g.N, g.c_sm, 32, 32);
+  p.ci_tma = p.c_int && !((uintptr_t)p.c_int & 15) && (int64_t)p.N * (p.int_bits / 8) % 16 == 0 &&
+             tc_make_map_int(&mci, p.int_bits, p.c_int, g.M, g.N, 32);
+  if (g.dtype == FXPR_BF16)
+    return p.c_int ? launch_pair<__nv_bfloat16, true>(ma, mb, mc, mci, p, sms, s) : launch_pair<__nv_bfloat16, false>(ma, mb, mc, mci, p, sms, s);
+  return p.c_int ? launch_pair<__half, true>(ma, mb, mc, mci, p, sms, s) : launch_pair<__half, false>(ma, mb, mc, mci, p, sms, s);
 }
 
 }  // namespace fxpr

@@ -381,7 +381,7 @@ struct TcParams {
   int M, N, K; int64_t c_sm;
   int k_tile, split_k, int_bits; float scale, inv_scale;
   int tiles_m, tiles_n; uint32_t idesc; int b_kmajor; int c_vec_ok;   // rows of c start on 16 bytes
-  int c_tma;             // two-SM kernel: c leaves by TMA
+  int c_tma, ci_tma;     // two-SM kernel: c, c_int leave by TMA
   int silu_mul;          // decode-shape kernel only: c[m, n / 2] = silu(out[m, n]) * out[m, n + 1], n even
   // decode-shape kernel only: best[m] = max over columns of argmax_key(out[m, n], n_offset + n)
   unsigned long long* best; unsigned int n_offset;
@@ -417,6 +417,8 @@ bool tc_make_map(CUtensorMap* m, int dtype, const void* base, int64_t rows, int6
 // tc_make_map in one copy.  cols must be a multiple of 64 (a ragged last group would reach past the last row).
 bool tc_make_map_groups(CUtensorMap* m, int dtype, const void* base, int64_t rows, int64_t cols,
                         int64_t row_stride_elems, int box_rows);
+// A contiguous [rows, cols] matrix of 32- or 64-bit integers, boxes of box_rows x 64 bytes, swizzled over them.
+bool tc_make_map_int(CUtensorMap* m, int int_bits, const void* base, int64_t rows, int64_t cols, int box_rows);
 int tc_device_sms();
 
 }  // namespace fxpr
