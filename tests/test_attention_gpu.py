@@ -305,6 +305,54 @@ def test_tcgen05_prefill_kernel_equals_mma_sync_kernel(case):
     assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
 
 
+def _prefill_inputs(sls, head_dim, mean, seed=0):
+    from fxpr_vllm import synthetic as syn
+
+    q, kv, qsl, sl, bt = syn.paged_attention_inputs(sls, sls, q_heads=32, kv_heads=8, head_dim=head_dim, page=16,
+                                                    dtype=torch.bfloat16, seed=seed)
+    kv[:, 1] += mean
+    return q * 0.2, kv, qsl, sl, bt                                # flat weights: sums of weights of hundreds
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("int_bits", [32, 64])
+def test_prefill_numerators_beyond_the_magic_range(head_dim, int_bits):
+    """Values with a mean: unnormalised numerators of 64.0 and more (2^22 at 16 fraction bits), negative ones too, no
+    partial out of range: the bits of the mma.sync kernel."""
+    from fxpr_vllm import _native as nat
+
+    for mean in (0.5, -0.7):
+        sls = [1500, 70, 1000]
+        q, kv, qsl, sl, bt = _prefill_inputs(sls, head_dim, mean)
+        outs = []
+        for flags in (0, nat.ATTN_NO_TCGEN05):
+            o = torch.full_like(q, float("nan"))
+            with L.overrides(attn_flags=flags):
+                torch.ops.fxpr.unified_attention_fxp(q, kv, o, qsl, sl, bt, max(sls), None, True, None, int_bits, 16, 0.0, 0, 1)
+            outs.append(o)
+        assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
+    L.check_device_status()
+
+
+def test_prefill_time_does_not_depend_on_the_size_of_the_numerators():
+    """1.8 times as long when numerators of 64.0 and more were divided element by element out of local memory."""
+    times = []
+    for mean in (0.0, 0.5):
+        sls = [1024] * 16
+        q, kv, qsl, sl, bt = _prefill_inputs(sls, 128, mean)
+        o = torch.empty_like(q)
+        best = float("inf")
+        for _ in range(6):
+            start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            torch.ops.fxpr.unified_attention_fxp(q, kv, o, qsl, sl, bt, 1024, None, True, None, 64, 16, 0.0, 0, 1)
+            stop.record()
+            torch.cuda.synchronize()
+            best = min(best, start.elapsed_time(stop))
+        times.append(best)
+    assert times[1] < 1.25 * times[0], times
+
+
 @pytest.mark.parametrize("head_dim,case", [
     # (seq_lens, q_lens, q heads, kv heads, page, dtype, int_bits, extra arguments)
     (64, ([1, 16, 63, 64, 65, 127, 128, 129, 385], [1, 16, 63, 64, 65, 127, 128, 129, 385], 32, 8, 16, torch.bfloat16, 64, {})),

@@ -783,52 +783,46 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const float dn = fmaxf(fixed_to_float<long long>(wrap_to_bits(dsum, p.int_bits), p.inv_scale), 1.0e-6f);
       T* op = (T*)p.o + (int64_t)(I.q_start + tok) * p.o_st + (int64_t)head * p.o_sh + half * kHalfCols;
       const uint32_t bias_bits = (uint32_t)n_tiles * mbits;  // what the multiply-adds summed on top
-      // With every sum below 2^22 in magnitude MAGIC + sum is a float whose value minus MAGIC is the sum.
-      uint32_t off = 0;
-#pragma unroll
-      for (int i = 0; i < kHalfCols; ++i) {
-        acc[i] += alu_add(i) ? kMagicBits : kMagicBits - bias_bits;
-        off |= acc[i] ^ kExpBits;
-      }
-      if (__all_sync(0xffffffffu, !corr_used && (off >> 23) == 0)) {
-        // num / dn correctly rounded from the row's one reciprocal (Markstein, IBM J. Res. Dev. 34, 1990: with y the
-        // correctly rounded 1 / b and q within an ulp of a / b, q + (a - b q) y, the remainder by fma, rounds
-        // correctly; the first step brings q there).  num = sum * 2^-f over dn is sum over dn * 2^f.
-        const float b = __fmul_rn(dn, p.scale), y = __frcp_rn(b);
-        const uint64_t y2 = pack2(__float_as_uint(y), __float_as_uint(y)), nb2 = pack2(__float_as_uint(-b), __float_as_uint(-b));
-        const uint64_t minus2 = pack2(kMagicBits | 0x80000000u, kMagicBits | 0x80000000u);
-#pragma unroll
-        for (int g8 = 0; g8 < kHalfCols / 8; ++g8) {
-          uint32_t out[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int c = g8 * 8 + i * 2;
-            uint64_t a, q, r;
-            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(a) : "l"(pack2(acc[c], acc[c + 1])), "l"(minus2));
-            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(a), "l"(y2));
-            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(q), "l"(nb2), "l"(a));
-            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(q) : "l"(r), "l"(y2), "l"(q));
-            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(q), "l"(nb2), "l"(a));
-            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(q) : "l"(r), "l"(y2), "l"(q));
-            out[i] = pack2_tc<T>(__uint_as_float((uint32_t)q), __uint_as_float((uint32_t)(q >> 32)));
-          }
-          if (store) *reinterpret_cast<uint4*>(op + g8 * 8) = make_uint4(out[0], out[1], out[2], out[3]);
-        }
-      } else {
-        // large sums or corrections: element by element out of local memory, in a loop, as unrolled it was most
-        // of the kernel's code
+      // acc becomes the sums as floats.  They fit 32 bits unless a partial took the fix-up: one conversion each, whatever
+      // their size (16 prompts of 1024 tokens, values of zero mean / mean 0.5, us: a shortcut below 2^22 and an element loop out
+      // of local memory above it 296 / 525, this 296 / 297, both in registers, which spilled, 340 / 342).  After a
+      // fix-up the exact sums, as floats, are put together out of local memory, in a loop.
+      if (corr_used) {
         uint32_t sums[kHalfCols];
 #pragma unroll
-        for (int i = 0; i < kHalfCols; ++i) sums[i + zero] = acc[i] - kMagicBits;
-        if (store) {
-#pragma unroll 1
-          for (int c = 0; c < kHalfCols; ++c) {
-            long long tot = (long long)(int32_t)sums[c + zero];
-            if (corr_used)
-              tot = wrap_to_bits((long long)(int32_t)(sums[c + zero] - corr_raw[c + zero]) + corr_q[c + zero], p.int_bits);
-            op[c] = from_f32<T>(__fdiv_rn(fixed_to_float<long long>(tot, p.inv_scale), dn));
-          }
+        for (int i = 0; i < kHalfCols; ++i) sums[i + zero] = alu_add(i) ? acc[i] : acc[i] - bias_bits;
+#pragma unroll 4
+        for (int c = 0; c < kHalfCols; ++c) {
+          const long long t = wrap_to_bits((long long)(int32_t)(sums[c + zero] - corr_raw[c + zero]) + corr_q[c + zero], p.int_bits);
+          sums[c + zero] = __float_as_uint(__ll2float_rn(t));
         }
+#pragma unroll
+        for (int i = 0; i < kHalfCols; ++i) acc[i] = sums[i + zero];
+      } else {
+#pragma unroll
+        for (int i = 0; i < kHalfCols; ++i) acc[i] = __float_as_uint(__int2float_rn((int)(alu_add(i) ? acc[i] : acc[i] - bias_bits)));
+      }
+      // num / dn correctly rounded from the row's one reciprocal (Markstein, IBM J. Res. Dev. 34, 1990: with y the
+      // correctly rounded 1 / b and q within an ulp of a / b, q + (a - b q) y, the remainder by fma, rounds
+      // correctly; the first step brings q there).  num = sum * 2^-f over dn is sum over dn * 2^f.
+      const float b = __fmul_rn(dn, p.scale), y = __frcp_rn(b);
+      const uint64_t y2 = pack2(__float_as_uint(y), __float_as_uint(y)), nb2 = pack2(__float_as_uint(-b), __float_as_uint(-b));
+#pragma unroll
+      for (int g8 = 0; g8 < kHalfCols / 8; ++g8) {
+        uint32_t out[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int c = g8 * 8 + i * 2;
+          const uint64_t a = pack2(acc[c], acc[c + 1]);
+          uint64_t q, r;
+          asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(a), "l"(y2));
+          asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(q), "l"(nb2), "l"(a));
+          asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(q) : "l"(r), "l"(y2), "l"(q));
+          asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(q), "l"(nb2), "l"(a));
+          asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(q) : "l"(r), "l"(y2), "l"(q));
+          out[i] = pack2_tc<T>(__uint_as_float((uint32_t)q), __uint_as_float((uint32_t)(q >> 32)));
+        }
+        if (store) *reinterpret_cast<uint4*>(op + g8 * 8) = make_uint4(out[0], out[1], out[2], out[3]);
       }
     }
   }
