@@ -459,6 +459,29 @@ def test_two_sm_kernel_at_tile_edges(M, N, K, kt, kmajor):
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M", [1, 16])
+@pytest.mark.parametrize("N,K,split,pad", [(1096, 4168, 0, 0), (392, 4168, 8, 0), (1800, 6000, 4, 0), (264, 520, 1, 8), (2008, 3080, 8, 0)])
+@pytest.mark.parametrize("kmajor", [False, True])
+def test_decode_shape_weights_off_the_sectors(M, N, K, split, pad, kmajor):
+    """Up to 16 rows and weights whose rows start inside a 32-byte sector (by their stride, or by their first address):
+    the whole-SM ring, with and without clusters, gives the wide kernel's integers and outputs."""
+    from fxpr_vllm import _native as nat
+
+    a = _rand((M, K), torch.bfloat16, 31).cuda()
+    rows, cols = (N, K) if kmajor else (K, N)
+    store = _rand((rows, cols + 2 * pad), torch.bfloat16, 32, 0.05).cuda()
+    b = store[:, pad:pad + cols]
+    b = b.t() if kmajor else b
+    a[M - 1, 200:264] = 3.0e4                      # partials beyond the fast conversion's range in one row
+    for kt in (64, 128):
+        with L.overrides(gemm_k_tile=kt, gemm_split_k=split or None):
+            got, got_c = torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16), _gemm(a, b, None, 64, 16)
+        with L.overrides(gemm_k_tile=kt, gemm_split_k=1, gemm_flags=nat.GEMM_NO_SKINNY):
+            want, want_c = torch.ops.fxpr.gemm_fxp_int(a, b, 64, 16), _gemm(a, b, None, 64, 16)
+        assert torch.equal(got, want) and torch.equal(got_c.view(torch.int16), want_c.view(torch.int16))
+    L.check_device_status()
+
+
 @pytest.mark.parametrize("M,N", [(129, 130), (300, 136), (256, 161), (290, 552), (417, 288)])
 @pytest.mark.parametrize("big", [False, True])
 def test_two_sm_kernel_output_paths(M, N, big):

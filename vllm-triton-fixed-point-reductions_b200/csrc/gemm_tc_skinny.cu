@@ -272,12 +272,20 @@ static int route_skinny(const GemmArgs& g, const CUtensorMap& mw, TcParams& p, i
   // SM, so that the column tiles of large weights all stream at once (64 x 28672 x 4096, 224 tiles: 46.5 us
   // with one CTA and tile after tile per SM, 38.8 with two).  64 x 4096 x 4096 on 128 CTAs: 11.3 us with the
   // whole ring, 12.1 with half of it; 64 x 6144 x 4096 13.7 / 15.9.  With 16 rows half of it holds as many
-  // weights as are needed in flight: 16 x 4096 x 4096 10.5 / 9.9, 16 x 4096 x 14336 23.9 / 21.8.
+  // weights as are needed in flight: 16 x 4096 x 4096 10.5 / 9.9, 16 x 4096 x 14336 23.9 / 21.8.  Not so where the rows of
+  // the weights start inside a 32-byte sector: every row of a box then touches a sector more at either end, and
+  // latency with it (11 x 11928 x 11888 54.6 / 63.8, 5 x 7080 x 18976 49.9 / 58.7, 12 x 8632 x 6384 28.3 / 35.5; rows of 32 bytes
+  // and more: 5 x 12576 x 3696 19.1 / 18.3; short ranks, which the half ring all but holds: 11 x 5312 x 920 6.5 / 6.3).  Whole-SM clusters of eight do not all fit from fifteen on (2 x 2016 x 8920,
+  // sixteen of them: 17.7 / 11.1).
   // A thousand tiles of 64 rows pay for a CTA's set-up each: 64 x 128256 x 4096 166.6 us with persistent CTAs, 170.5.
-  if constexpr (MP > 16) {
-    if ((int64_t)p.tiles_n * p.split_k <= sms)
-      return cluster ? launch_skinny<T, MP, true, 1>(g, mw, p, s) : launch_skinny<T, MP, false, 1>(g, mw, p, s);
+  const int64_t ctas = (int64_t)p.tiles_n * p.split_k;
+  bool whole = ctas <= sms;
+  if constexpr (MP == 16) {
+    const int64_t row_bytes = 2 * (p.b_kmajor ? g.b_sn : g.b_sk);
+    whole = whole && p.K >= 1024 * (int64_t)p.split_k && ((row_bytes | (int64_t)(uintptr_t)g.b) & 31) != 0 && (p.split_k <= 4 || p.tiles_n <= sms * 14 / 148);
   }
+  if (whole)
+    return cluster ? launch_skinny<T, MP, true, 1>(g, mw, p, s) : launch_skinny<T, MP, false, 1>(g, mw, p, s);
   return cluster ? launch_skinny<T, MP, true, 2>(g, mw, p, s) : launch_skinny<T, MP, false, 2>(g, mw, p, s);
 }
 
