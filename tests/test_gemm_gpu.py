@@ -459,6 +459,35 @@ def test_two_sm_kernel_at_tile_edges(M, N, K, kt, kmajor):
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M,N,K,kt", [(33, 38008, 64, 64), (64, 38008, 136, 64), (64, 38016, 136, 128), (48, 76040, 712, 64),
+                                      (64, 113672, 392, 128), (63, 38008, 1096, 128), (64, 38008, 3080, 64), (40, 57096, 3072, 128)])
+def test_decode_shape_walk_over_large_vocabularies(M, N, K, kt):
+    """More than 32 rows on more column tiles than CTAs fit the GPU: a CTA walks from tile to tile with its ring, its
+    accumulators and its sums, K shorter and longer than the ring, ragged last tiles, and partials beyond the fast range
+    (64-bit sums) in some tiles only, one after the other or not: the wide kernel's integers, outputs and arg-max keys."""
+    from fxpr_vllm import _native as nat
+
+    a = _rand((M, K), torch.bfloat16, 41).cuda()
+    b = _rand((K, N), torch.bfloat16, 42, 0.05).cuda()
+    for first in (300, 128 * 296 + 5, N - 1):                     # a CTA's first, second and last tile
+        b[:, first] = 3.0e4
+    bias = _rand((N,), torch.bfloat16, 43).cuda()
+    with L.overrides(gemm_k_tile=kt):
+        got = [torch.ops.fxpr.gemm_fxp_int(a, b, bits, 16) for bits in (32, 64)]
+        got_c = [_gemm(a, b, x, 64, 16) for x in (None, bias)]
+        c, keys = L.gemm_fxp_argmax(a, b, None, 64, 16)
+        act = L.gemm_silu_mul(a, b, 64, 16)
+    with L.overrides(gemm_k_tile=kt, gemm_split_k=1, gemm_flags=nat.GEMM_NO_SKINNY):
+        for bits, x in zip((32, 64), got):
+            assert torch.equal(x, torch.ops.fxpr.gemm_fxp_int(a, b, bits, 16))
+        for x, y in zip((None, bias), got_c):
+            assert torch.equal(y.view(torch.int16), _gemm(a, b, x, 64, 16).view(torch.int16))
+    assert torch.equal(c.view(torch.int16), got_c[0].view(torch.int16))
+    assert torch.equal(L.argmax_from_keys(keys), got_c[0].argmax(dim=-1))
+    assert torch.equal(act.view(torch.int16), L.silu_mul_pairs(got_c[0]).view(torch.int16))
+    L.check_device_status()
+
+
 @pytest.mark.parametrize("M", [1, 16])
 @pytest.mark.parametrize("N,K,split,pad", [(1096, 4168, 0, 0), (392, 4168, 8, 0), (1800, 6000, 4, 0), (264, 520, 1, 8), (2008, 3080, 8, 0)])
 @pytest.mark.parametrize("kmajor", [False, True])

@@ -43,33 +43,36 @@ constexpr int sk_most_received(int rows) {
   return most;
 }
 
-// MP = activation rows of the tile (MMA N).  PER_SM = CTAs that share an SM's memory.
-template <int MP, int PER_SM> struct SkShape {
-  static constexpr int kStages = (MP == 16 ? 12 : MP == 32 ? 10 : 8) / PER_SM;
+// MP = activation rows of the tile (MMA N).  PER_SM = CTAs that share an SM's memory.  WALK: a CTA takes tile after
+// tile, with the sums beside the ring and not over it.
+template <int MP, int PER_SM, bool WALK> struct SkShape {
+  static constexpr int kStages = (MP == 16 ? 12 : MP == 32 ? 10 : 8) / PER_SM - (WALK ? 1 : 0);
   static constexpr int kXBytes = MP * kBK * 2;
   static constexpr int kStageBytes = kSkWBytes + kXBytes;  // 18, 20 or 24 KB
   static constexpr int kGroups = MP == 64 ? 4 : 8;         // accumulators in tensor memory
-  static constexpr int kBarOffset = kStages * kStageBytes;
+  static constexpr int kSumsOffset = WALK ? kStages * kStageBytes : 0;
+  static constexpr int kBarOffset = kStages * kStageBytes + (WALK ? MP * 512 : 0);
   static constexpr int kBarBytes = 448;
   static constexpr int kSmem = kBarOffset + kBarBytes + 1024;   // barriers, alignment slack
-  // over the stages once they are done: the finished sums, [row][128 columns] of 32 bits; what the
+  // over the stages once they are done: the finished sums, [row][128 columns] of 32 bits; for the cluster merge what the
   // peers send for this rank's rows, their flags, this rank's high words
   static constexpr int kRecvOffset = 32 * 1024, kFlagOffset = 62 * 1024, kHighOffset = 64 * 1024;
   static_assert(MP * 512 <= kRecvOffset && kRecvOffset + sk_most_received(MP) * 512 <= kFlagOffset, "sums and received slices");
   static_assert(kFlagOffset + 7 * 16 <= kHighOffset, "a flag of 16 bytes from each peer");
-  static_assert(kHighOffset + MP * 512 <= kBarOffset, "the merge fits the stages");
+  static_assert(WALK || kHighOffset + MP * 512 <= kBarOffset, "the merge fits the stages");
   static_assert(PER_SM * (kSmem + 1024) <= 228 * 1024, "shared memory of an SM");
   static_assert(kGroups * MP <= kSkTmemCols, "tensor memory");
 };
 
-// One item -- a tile of 128 columns and one K-split -- per CTA.
+// One item -- a tile of 128 columns and one K-split -- per CTA, or, with WALK and without splits, tile after tile.
 // CLUSTER: split-K as a thread-block cluster (grid = splits x tiles): every rank sums a slice of the rows,
 // which the others send it by bulk copies between shared memories -- no global scratch, no fences.
-template <typename T, int MP, bool CLUSTER, int PER_SM>
+template <typename T, int MP, bool CLUSTER, int PER_SM, bool WALK>
 __global__ void __launch_bounds__(kSkWarps * 32, 2)
 gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_constant__ CUtensorMap tma_x,
                       const TcParams p, const int zero /* always 0: keeps the side arrays in local memory */) {
-  using Shape = SkShape<MP, PER_SM>;
+  using Shape = SkShape<MP, PER_SM, WALK>;
+  static_assert(!(CLUSTER && WALK), "a walk has no splits");
   constexpr int STAGES = Shape::kStages, GROUPS = Shape::kGroups;
   constexpr int EPIW = 8;
   constexpr int kCols = MP / (EPIW / 4);                 // activation rows per epilogue thread
@@ -130,8 +133,8 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
   if (warp != 0) pdl_wait();
 
   const int tiles_n = p.tiles_n;                         // 128-column tiles; one row tile (M <= 64)
-  const int tile = CLUSTER ? (int)blockIdx.y : (int)blockIdx.x / p.split_k;
-  const int ks = CLUSTER ? (int)blockIdx.x : (int)blockIdx.x % p.split_k;
+  const int tile0 = CLUSTER ? (int)blockIdx.y : WALK ? (int)blockIdx.x : (int)blockIdx.x / p.split_k;
+  const int ks = CLUSTER ? (int)blockIdx.x : WALK ? 0 : (int)blockIdx.x % p.split_k;
   const int k_tiles_total = (p.K + p.k_tile - 1) / p.k_tile;
   const int n_kt = (k_tiles_total - ks + p.split_k - 1) / p.split_k;
   const int deep = p.k_tile >> 6;                        // stages per K-tile: 1 or 2
@@ -141,7 +144,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
     // ------------------------------ TMA producer --------------------------------
     const uint32_t e = elect_one();
     const bool wk = p.b_kmajor != 0;                     // weights given as an (N, K) row-major view
-    const int n0 = tile * 128;
+    int n0 = tile0 * 128;
     auto k_of = [&](int j) { return deep == 1 ? (ks + j * p.split_k) * 64 : (ks + (j >> 1) * p.split_k) * 128 + (j & 1) * 64; };
     auto load_w = [&](int j, int st) {
       const uint32_t fb = full0 + 8u * st, sw = smem_base + st * kStageBytes;
@@ -164,10 +167,17 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
       for (int j = 0; j < first; ++j) { load_w(j, j); load_x(j, j); }
     }
     int stage = 0; uint32_t phase = 0;
-    for (int j = first; j < n_st; ++j) {
-      if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8u * stage, phase, abort_flag))) break;
-      load_w(j, stage); load_x(j, stage);
-      if (++stage == STAGES) { stage = 0; phase ^= 1; }
+    if (WALK && first < STAGES) { stage = first; phase = 1; }
+    int j = first;
+    for (;;) {
+      bool fetched = true;
+      for (; j < n_st; ++j) {
+        if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8u * stage, phase, abort_flag))) { fetched = false; break; }
+        load_w(j, stage); load_x(j, stage);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (!WALK || !fetched || (n0 += (int)gridDim.x * 128) >= tiles_n * 128) break;
+      j = 0;
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ----------------------------------
@@ -179,6 +189,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
     constexpr uint64_t kStep = kStageBytes >> 4;
     const uint32_t idesc = p.idesc, e = elect_one();
     int stage = 0; uint32_t phase = 0; int grp = 0; uint32_t gphase = 1;
+    for (int t = tile0; t < tiles_n; t += WALK ? (int)gridDim.x : tiles_n)
     for (int kt = 0; kt < n_kt; ++kt) {
       const uint32_t d = tmem_base + (uint32_t)(grp * MP);
       for (int h = 0; h < deep; ++h) {
@@ -237,9 +248,9 @@ bool gemm_tc_skinny_cluster(const GemmArgs& g, int split_k) {
   return split_k >= 2 && split_k <= 8 && (g.N + 127) / 128 <= 65535 && !(g.flags & FXPR_GEMM_NO_CLUSTER);
 }
 
-template <typename T, int MP, bool CLUSTER, int PER_SM>
-static int launch_skinny(const GemmArgs& g, const CUtensorMap& mw, TcParams& p, cudaStream_t s) {
-  constexpr int kSmem = SkShape<MP, PER_SM>::kSmem;
+template <typename T, int MP, bool CLUSTER, int PER_SM, bool WALK = false>
+static int launch_skinny(const GemmArgs& g, const CUtensorMap& mw, TcParams& p, cudaStream_t s, int walkers = 0) {
+  constexpr int kSmem = SkShape<MP, PER_SM, WALK>::kSmem;
   CUtensorMap mx;
   if (!tc_make_map(&mx, g.dtype, g.a, g.M, g.K, g.a_sm, MP)) {
     set_last_error("cuTensorMapEncodeTiled(X)", cudaErrorInvalidValue);
@@ -247,7 +258,7 @@ static int launch_skinny(const GemmArgs& g, const CUtensorMap& mw, TcParams& p, 
   }
   // M = 128 weight columns, N = activation rows; bit 15: the 128-row operand is MN-major
   p.idesc = make_idesc(g.dtype == FXPR_BF16 ? 1 : 0, 0, MP, 128) | (p.b_kmajor ? 0u : (1u << 15));
-  auto k = gemm_tc_skinny_kernel<T, MP, CLUSTER, PER_SM>;
+  auto k = gemm_tc_skinny_kernel<T, MP, CLUSTER, PER_SM, WALK>;
   static bool attr_done_dev[64] = {};            // function attributes are per device
   int dev_id = 0;
   cudaGetDevice(&dev_id);
@@ -257,7 +268,7 @@ static int launch_skinny(const GemmArgs& g, const CUtensorMap& mw, TcParams& p, 
     if (e != cudaSuccess) { set_last_error("gemm_tc_skinny smem attribute", e); return FXPR_ERR_CUDA; }
     attr_done = true;
   }
-  const dim3 grid = CLUSTER ? dim3((unsigned)p.split_k, (unsigned)p.tiles_n, 1) : dim3((unsigned)(p.tiles_n * p.split_k));
+  const dim3 grid = CLUSTER ? dim3((unsigned)p.split_k, (unsigned)p.tiles_n, 1) : dim3((unsigned)(WALK ? walkers : p.tiles_n * p.split_k));
   cudaError_t e = launch_pdl(k, grid, dim3(kSkWarps * 32), kSmem, s, CLUSTER ? (unsigned)p.split_k : 1u, mw, mx, p, 0);
   if (e != cudaSuccess) { set_last_error("gemm_tc_skinny launch", e); return FXPR_ERR_CUDA; }
   return check_launch("gemm_tc_skinny");
@@ -277,12 +288,22 @@ static int route_skinny(const GemmArgs& g, const CUtensorMap& mw, TcParams& p, i
   // latency with it (11 x 11928 x 11888 54.6 / 63.8, 5 x 7080 x 18976 49.9 / 58.7, 12 x 8632 x 6384 28.3 / 35.5; rows of 32 bytes
   // and more: 5 x 12576 x 3696 19.1 / 18.3; short ranks, which the half ring all but holds: 11 x 5312 x 920 6.5 / 6.3).  Whole-SM clusters of eight do not all fit from fifteen on (2 x 2016 x 8920,
   // sixteen of them: 17.7 / 11.1).
-  // A thousand tiles of 64 rows pay for a CTA's set-up each: 64 x 128256 x 4096 166.6 us with persistent CTAs, 170.5.
+  // More tiles of 64 rows than two CTAs an SM: a CTA walks from tile to tile, so that its set-up is paid once and the next
+  // tile's weights come in under the outputs.  One walker an SM, with seven stages, unless K is short (a CTA per
+  // tile / two walkers / one, us): 64 x 128256 x 4096 168 / 168 / 165, 64 x 40008 x 4096 73.1 / 72.1 / 67.2, 64 x 50304 x 4096 73.5 /
+  // 75.5 / 68.4, 64 x 152064 x 3584 180.9 / 180.3 / 177.7; 64 x 60000 x 2048 46.6 / 44.6 / 49.2, 64 x 102400 x 2048 74.1 / 69.2 / 72.8.
+  // With fewer rows a CTA per tile stays (32 x 128256 x 4096 157.0, one persistent CTA an SM 162.5).
   const int64_t ctas = (int64_t)p.tiles_n * p.split_k;
   bool whole = ctas <= sms;
   if constexpr (MP == 16) {
     const int64_t row_bytes = 2 * (p.b_kmajor ? g.b_sn : g.b_sk);
     whole = whole && p.K >= 1024 * (int64_t)p.split_k && ((row_bytes | (int64_t)(uintptr_t)g.b) & 31) != 0 && (p.split_k <= 4 || p.tiles_n <= sms * 14 / 148);
+  }
+  if constexpr (MP == 64) {
+    if (ctas > 2 * sms && p.split_k == 1) {
+      if (p.K >= 3072) return launch_skinny<T, MP, false, 1, true>(g, mw, p, s, sms);
+      return launch_skinny<T, MP, false, 2, true>(g, mw, p, s, 2 * sms);
+    }
   }
   if (whole)
     return cluster ? launch_skinny<T, MP, true, 1>(g, mw, p, s) : launch_skinny<T, MP, false, 1>(g, mw, p, s);

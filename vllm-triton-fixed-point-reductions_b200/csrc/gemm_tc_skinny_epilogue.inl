@@ -31,8 +31,8 @@
   bool corr_used = false;
   bool announced = false;      // cluster merge: this thread has said that the stages are done
 
-  int* stage32 = reinterpret_cast<int*>(smem_gen);              // [MP][128]
-  long long* stage64 = reinterpret_cast<long long*>(smem_gen);  // [MP / 2][128]
+  int* stage32 = reinterpret_cast<int*>(smem_gen + Shape::kSumsOffset);              // [MP][128]
+  long long* stage64 = reinterpret_cast<long long*>(smem_gen + Shape::kSumsOffset);  // [MP / 2][128]
   const bool c_vec4 = ((uintptr_t)p.c & 7) == 0 && p.c_sm % 4 == 0;
   float bias4[4];
 
@@ -90,9 +90,13 @@
     }
   };
 
-  const int n4 = tile * 128 + lane * 4;                  // output columns of this lane
+  int n4 = 0;                                            // output columns of this lane
+  for (int tile = tile0, it = 0;; ++it) {
+  const int flag = WALK ? it & 1 : 0;                    // of s_wide
+  n4 = tile * 128 + lane * 4;
 #pragma unroll
   for (int i = 0; i < 4; ++i) bias4[i] = p.bias && n4 + i < p.N ? to_f32<T>(((const T*)p.bias)[n4 + i]) : 0.0f;
+  corr_used = false;
   uint32_t acc[kCols];
 #pragma unroll
   for (int i = 0; i < kCols; ++i) acc[i] = 0;
@@ -130,6 +134,7 @@
     if (lane == 0) mbar_arrive(tempty0 + 8u * grp);
     if (++grp == GROUPS) { grp = 0; gphase ^= 1; }
   }
+  if (WALK && ok && it) ok = epi_sync();                 // the last tile's sums have been read
   if (ok) {
     const uint32_t bias_bits = (uint32_t)n_kt * mbits;   // the multiply-adds summed one magic per K-tile
     // the sum without corrections is below 2^31 in magnitude (at most 510 K-tiles of less than 2^22)
@@ -191,11 +196,12 @@
         do_store = ok && *s_last != 0;
         if (do_store) __threadfence();
       } else {
-        if (corr_used && p.int_bits == 64) *s_wide = 1;
+        if (corr_used && p.int_bits == 64) s_wide[flag] = 1;
         else park32();                                   // not read when another warp makes the tile a wide one
         do_store = ok = epi_sync();
+        if (WALK && threadIdx.x == 64) s_wide[flag ^ 1] = 0;   // read by all before this tile's first barrier
       }
-      if (do_store && !split && !*s_wide) {
+      if (do_store && !split && !s_wide[flag]) {
         for (int m = warp - 2; m < live_rows; m += EPIW) {
           const int4 v = *reinterpret_cast<const int4*>(stage32 + m * 128 + lane * 4);
           emit(m, n4, v.x, v.y, v.z, v.w);
@@ -231,6 +237,8 @@
       }
       if (split && do_store && threadIdx.x == 64) p.locks[tile] = 0;
     }
+  }
+  if (!WALK || !ok || (tile += (int)gridDim.x) >= tiles_n) break;
   }
 
   if constexpr (CLUSTER) {
