@@ -153,6 +153,18 @@ def test_decode_ranks_of_small_batches_and_last_waves():
                 assert 1 <= f(0, n, 1, hq, hkv, keys, 148) <= 16
 
 
+def test_sixteen_ranks_fall_back_where_the_device_cannot_place_them(tmp_path):
+    """A device that cannot place a cluster of sixteen (asked of a stand-in here) gets eight ranks, not an error."""
+    assert _policy_program(tmp_path, """
+  for (bool can : {false, true})
+    for (int ranks : {1, 8, 9, 16}) {
+      int asked = 0;
+      const int got = ranks_that_fit(ranks, [&](int) { ++asked; return can; });
+      std::printf("%d:%d ", got, asked);
+    }
+""").split() == ["1:0", "8:0", "8:1", "8:1", "1:0", "8:0", "9:1", "16:1"]
+
+
 def test_argmax_keys_pick_the_first_maximum_and_combine_across_shards():
     g = torch.Generator().manual_seed(0)
     for dtype in (torch.bfloat16, torch.float16):

@@ -21,6 +21,10 @@
 //     mma.sync.m16n8k16 with a fixed k order and each output row depends only on its own
 //     query row, so a token's bits are the same in any batch, block or split.
 //   * K/V pages are staged with 16-byte cp.async into XOR-swizzled shared memory.
+#include <map>
+#include <mutex>
+#include <tuple>
+
 #include <cooperative_groups.h>
 
 #include "attention_common.cuh"
@@ -108,6 +112,37 @@ static constexpr int kFastMaxTiles = 500;                 // 500 * 2^22 < 2^31: 
 
 static int stash_bytes_per_key(int stash_rows) { return stash_rows <= 8 ? stash_rows * 4 : 64; }
 
+// A launch asks attention_mma() to come again with eight ranks: this device cannot place a cluster of more (a GPU slice,
+// or a GPC with too few SMs).
+static constexpr int kFewerRanks = 1;
+
+// Whether the device can place one cluster of `ranks` CTAs, asked once per kernel, device and shared memory.
+template <typename K>
+static bool cluster_fits(K k, int ranks, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, int, int, size_t>, bool> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple((const void*)k, dev, ranks, smem);
+  const auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ranks);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, k, &cfg);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return known[key] = e == cudaSuccess && clusters > 0;
+}
+
 template <typename T, int HD, int NW, bool STASH, bool ACC64, bool FAST = false>
 static int launch_mma(const AttnParams& p, const MmaAttnShape& sh, cudaStream_t s) {
   constexpr int BM = 16 * NW;
@@ -122,6 +157,7 @@ static int launch_mma(const AttnParams& p, const MmaAttnShape& sh, cudaStream_t 
   if (p.num_splits > 8) {
     e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) { set_last_error("attention_mma cluster attribute", e); return FXPR_ERR_CUDA; }
+    if (ranks_that_fit(p.num_splits, [&](int ranks) { return cluster_fits(k, ranks, NW * 32, smem); }) != p.num_splits) return kFewerRanks;
   }
   e = launch_pdl(k, dim3((unsigned)p.num_splits, (unsigned)(sh.num_q_blocks * p.num_kv_heads), (unsigned)p.num_reqs),
                  dim3(NW * 32), smem, s, (unsigned)p.num_splits, p, sh);
@@ -145,6 +181,7 @@ static int launch_decode(const AttnParams& p, const MmaAttnShape& sh, int dtype,
   if (p.num_splits > 8) {
     e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) { set_last_error("attention_decode cluster attribute", e); return FXPR_ERR_CUDA; }
+    if (ranks_that_fit(p.num_splits, [&](int ranks) { return cluster_fits(k, ranks, NW * 32, smem); }) != p.num_splits) return kFewerRanks;
   }
   e = launch_pdl(k, dim3((unsigned)p.num_splits, (unsigned)(sh.num_q_blocks * p.num_kv_heads), (unsigned)p.num_reqs),
                  dim3(NW * 32), smem, s, (unsigned)p.num_splits, mk, mv, p, sh);
@@ -158,10 +195,7 @@ bool attention_mma_supported(const AttnParams& p, int dtype) {
                                       p.q, p.k, p.v});
 }
 
-int attention_mma(const AttnParams& p_in, int dtype, int max_query_len, bool force_exact, cudaStream_t s) {
-  AttnParams p = p_in;
-  if (p.num_splits > 16) p.num_splits = 16;        // cluster size limit; results do not depend on it
-  if (p.num_splits < 1) p.num_splits = 1;
+static int attention_mma_ranks(const AttnParams& p, int dtype, int max_query_len, bool force_exact, cudaStream_t s) {
   const int G = p.num_heads / p.num_kv_heads;
   const int mq = max_query_len < 1 ? 1 : max_query_len;
   MmaAttnShape sh;
@@ -209,6 +243,18 @@ int attention_mma(const AttnParams& p_in, int dtype, int max_query_len, bool for
   if (p.head_dim == 128) FXPR_ATTN(__half, 128);
   FXPR_ATTN(__half, 64);
 #undef FXPR_ATTN
+}
+
+int attention_mma(const AttnParams& p_in, int dtype, int max_query_len, bool force_exact, cudaStream_t s) {
+  AttnParams p = p_in;
+  if (p.num_splits > 16) p.num_splits = 16;        // cluster size limit; results do not depend on it
+  if (p.num_splits < 1) p.num_splits = 1;
+  int st = attention_mma_ranks(p, dtype, max_query_len, force_exact, s);
+  if (st == kFewerRanks) {
+    p.num_splits = kPortableRanks;
+    st = attention_mma_ranks(p, dtype, max_query_len, force_exact, s);
+  }
+  return st;
 }
 
 }  // namespace fxpr

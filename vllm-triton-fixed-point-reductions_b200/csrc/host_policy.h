@@ -146,6 +146,13 @@ inline int64_t pick_attention_splits(int64_t requested, int64_t num_requests, in
   return p;
 }
 
+// More ranks than every device can place as one cluster are used where this one can (`fits` asks it), else eight.
+inline constexpr int kPortableRanks = 8;
+template <typename Fits>
+inline int ranks_that_fit(int ranks, Fits fits) {
+  return ranks <= kPortableRanks || fits(ranks) ? ranks : kPortableRanks;
+}
+
 // KV splits of the tensor-core attention route, where splits are cluster ranks.  Decode keeps each
 // CTA's key slice near 1024 keys (small score stash -> more resident CTAs) unless fewer clusters
 // than CTA slots call for more ranks; prefill splits only when the row blocks alone cannot fill
@@ -169,7 +176,10 @@ inline int64_t pick_attention_ranks(int64_t requested, int64_t num_requests, int
     const int64_t clusters = std::max<int64_t>(1, num_requests * num_kv_heads);
     const int64_t by_fill = std::max<int64_t>(1, std::min<int64_t>({8, (4 * num_sms) / clusters, tiles / 2}));
     // A few clusters with long contexts: sixteen, one CTA per SM (1 request x 3588 keys, 8 KV heads: 14.1 us with
-    // eight, 11.3).
+    // eight, 11.3).  The width of the table stands for the contexts; short ones in a wide table lose by it (1 request in 512
+    // pages, eight / sixteen ranks, us, 8 KV heads: 200 keys 5.9 / 6.7, 1000 6.8 / 7.0, 3588 12.0 / 11.0, 8000 17.4 / 13.9;
+    // 2 KV heads: 5.7 / 5.9, 6.8 / 5.9, 11.5 / 9.0, 16.2 / 11.1).  Merging only the ranks that have keys gives
+    // short contexts their time back and costs every other call 1 to 2 %.
     if (clusters * 16 <= num_sms && tiles >= 48) return 16;
     int64_t ranks = std::max(by_keys, by_fill);
     // No last wave of a handful of CTAs: two ranks and not three where two fit one wave at three CTAs per SM (600
