@@ -80,6 +80,14 @@ def test_medium_batch_plan_takes_a_handful_of_steps_and_finds_the_cheapest_row_t
 """) == "24864 0"
 
 
+def test_two_planes_are_taken_where_they_measured_faster(tmp_path):
+    """Calls that went to the medium-batch kernel and lost 4 to 15 % by it: two K-splits through planes."""
+    for m, n, k, kt in ((200, 4096, 14336, 64), (299, 3064, 11912, 128), (402, 2016, 15704, 64), (501, 2120, 4424, 64)):
+        assert L.pick_split_k(m, n, k, kt, 64, 148) == 2
+        assert _policy_program(tmp_path, f'  std::printf("%d", mid_route({m}, {n}, {k}, {kt}, 2, 148));') == "0"
+    assert L.pick_split_k(154, 4808, 8800, 64, 64, 148) == 3          # 48 us in a cluster of three, 54 unsplit
+
+
 def test_splits_follow_the_kernel_that_runs(tmp_path):
     """The medium-batch kernel's cluster merges set the split only where that kernel may run: not above 21 fraction
     bits or in the exact-conversion kernel (planes, at most four), and not where a flag names another kernel."""

@@ -37,14 +37,16 @@ inline bool attention_tensor_core_route(const AttnRoute& r) {
 // scratch), 256 x 256 on pairs (gemm_tc_pair.cu, unsplit) and 256 weight columns x 96 to 256 rows on pairs
 // (gemm_tc_mid.cu, up to four splits in a cluster).  The estimates are clocks per 128 of K at 1850 MHz, fitted to
 // sweeps of 80 to 700 rows over ten weight shapes (within 15 % of the measured times, most within 8 %):
-//   128 x 128     1300 (K-tile 128) or 1665 (64), 3.5 us a call, 8 + splits for the planes of a split
+//   128 x 128     1300 (K-tile 128) or 1665 (64), 3.5 us a call, 8 + splits for the planes of a split, 8 for two
+//                 (with 10 for two: 200 x 4096 x 14336, K-tile 64, 57.7 us in a cluster of two where planes take 55.1,
+//                 299 x 3064 x 11912 59.5 unsplit and 51.9)
 //   256 x 256     1936 or 2690
 //   256 x rows    copies: (256 + rows) requests of 128 bytes a CTA at 2.4 clocks, 3.05 when most SMs fetch; or the
 //                 conversion, 7 (14) clocks a row; 3 us a call, 8 a wave when there are several (its waves do not
 //                 overlap), 2 to 4.5 for the merge
 inline double est_single_us(int64_t M, int64_t N, int64_t K, int64_t k_tile, int split, int num_sms) {
   const double waves = (double)ceil_div(ceil_div(M, 128) * ceil_div(N, 128) * split, num_sms);
-  return waves * ((double)K / 128 / split * (k_tile == 64 ? 1665 : 1300) / 1850) + 3.5 + (split > 1 ? 8.0 + split : 0.0);
+  return waves * ((double)K / 128 / split * (k_tile == 64 ? 1665 : 1300) / 1850) + 3.5 + (split > 2 ? 8.0 + split : split == 2 ? 8.0 : 0.0);
 }
 inline double est_pair_us(int64_t M, int64_t N, int64_t K, int64_t k_tile, int num_sms) {
   const double waves = (double)ceil_div(ceil_div(M, 256) * ceil_div(N, 256), std::max(1, num_sms / 2));
