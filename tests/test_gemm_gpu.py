@@ -663,6 +663,49 @@ def test_medium_batch_kernel(M, N, K, kt, split):
     L.check_device_status()
 
 
+@pytest.mark.parametrize("M,split", [(3, 1), (20, 1), (64, 4), (64, 7), (64, 16), (80, 1), (129, 3), (250, 1)])
+@pytest.mark.parametrize("N", [129, 258, 391])
+def test_columns_that_are_no_multiple_of_four(M, N, split):
+    """Weights as an (N, K) view allow any N: the decode-shape and medium-batch kernels' scalar stores and bias guards at
+    the last columns, an output whose rows start anywhere, and activations that are columns of a wider matrix."""
+    from fxpr_vllm import _native as nat
+
+    K = 1160
+    wide = _rand((M, K + 24), torch.bfloat16, M).cuda()
+    a = wide[:, 8:8 + K]
+    b = _rand((N, K), torch.bfloat16, N, 0.05).cuda().t()
+    bias = _rand((N,), torch.bfloat16, 3).cuda()
+    flag = nat.GEMM_MID if M > 64 else 0
+    for kt in (64, 128):
+        with L.overrides(gemm_k_tile=kt, gemm_split_k=split, gemm_flags=flag):
+            got = [torch.ops.fxpr.gemm_fxp_int(a, b, bits, 16) for bits in (32, 64)] + [_gemm(a, b, x, 64, 16) for x in (None, bias)]
+        with L.overrides(gemm_k_tile=kt, gemm_split_k=1, gemm_flags=nat.GEMM_FORCE_EXACT_TC):
+            want = [torch.ops.fxpr.gemm_fxp_int(a, b, bits, 16) for bits in (32, 64)] + [_gemm(a, b, x, 64, 16) for x in (None, bias)]
+        for x, y in zip(got, want):
+            assert torch.equal(x if x.dtype != torch.bfloat16 else x.view(torch.int16), y if y.dtype != torch.bfloat16 else y.view(torch.int16))
+    L.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K,split", [(16, 256, 520, 1), (64, 384, 1160, 4), (80, 384, 1160, 1), (129, 640, 1160, 3), (300, 256, 520, 1)])
+def test_infinities_and_nan_in_the_newer_kernels(M, N, K, split):
+    """Partials that are infinite or NaN take the fix-up: what the plain-conversion kernel makes of them."""
+    from fxpr_vllm import _native as nat
+
+    a = _rand((M, K), torch.float16, 51).cuda()
+    b = _rand((K, N), torch.float16, 52, 0.05).cuda()
+    a[M // 2, 70] = float("inf")
+    a[0, 130] = float("-inf")
+    b[300, N - 3] = float("nan")
+    flags = {16: 0, 64: 0, 80: nat.GEMM_MID, 129: nat.GEMM_MID, 300: nat.GEMM_PAIR}[M]
+    for bits in (32, 64):
+        with L.overrides(gemm_k_tile=64, gemm_split_k=split, gemm_flags=flags):
+            got, got_c = torch.ops.fxpr.gemm_fxp_int(a, b, bits, 16), _gemm(a, b, None, bits, 16)
+        with L.overrides(gemm_k_tile=64, gemm_split_k=1, gemm_flags=nat.GEMM_FORCE_EXACT_TC):
+            want, want_c = torch.ops.fxpr.gemm_fxp_int(a, b, bits, 16), _gemm(a, b, None, bits, 16)
+        assert torch.equal(got, want) and torch.equal(got_c.view(torch.int16), want_c.view(torch.int16))
+    L.check_device_status()
+
+
 @pytest.mark.parametrize("M,N,K,flag,want", [
     (80, 4096, 4096, 0, "gemm_tc_mid_kernel"), (333, 6144, 4096, 0, "gemm_tc_mid_kernel"),
     (64, 4096, 4096, 0, "gemm_tc_skinny_kernel"), (4096, 4096, 4096, 0, "gemm_tc_pair_kernel"),
