@@ -189,7 +189,8 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
     constexpr uint64_t kStep = kStageBytes >> 4;
     const uint32_t idesc = p.idesc, e = elect_one();
     int stage = 0; uint32_t phase = 0; int grp = 0; uint32_t gphase = 1;
-    for (int t = tile0; t < tiles_n; t += WALK ? (int)gridDim.x : tiles_n)
+    int t = tile0;
+    do
     for (int kt = 0; kt < n_kt; ++kt) {
       const uint32_t d = tmem_base + (uint32_t)(grp * MP);
       for (int h = 0; h < deep; ++h) {
@@ -207,6 +208,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_co
       umma_commit(tfull0 + 8u * grp, e);
       if (++grp == GROUPS) { grp = 0; gphase ^= 1; }
     }
+    while (WALK && (t += (int)gridDim.x) < tiles_n);
   issuer_done:;
   } else {
 #include "gemm_tc_skinny_epilogue.inl"
