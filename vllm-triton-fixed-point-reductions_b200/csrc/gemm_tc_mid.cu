@@ -370,18 +370,7 @@ gemm_tc_mid_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         wide = (unsigned long long)(uint32_t)*s_wide << (16 * ks);
         for (int rr = 0; rr < S - 1; ++rr) wide |= (unsigned long long)(uint32_t)flags[rr * 4] << (16 * (rr < ks ? rr : rr + 1));
       }
-      if (wide) {
-        // the high words of every peer that has some; its own arrivals stand for the other peers
-        if (warp == 2 && lane == 0) {
-          int none = S - 1;
-          for (int s = 0; s < S; ++s) none -= s != ks && ((wide >> (16 * s)) & 0xffff);
-          if (none) mbar_arrive_n(high_bar, (uint32_t)none);
-        }
-        __syncwarp();
-        ok = __all_sync(0xffffffffu, mbar_wait_acquire_cluster(high_bar, 0, abort_flag));
-      } else {
-        cluster_arrive();                                  // this CTA has what was sent to it
-      }
+      if (!wide) cluster_arrive();                         // this CTA has what was sent to it
       if (ok) {
         const int* mine = stage32 + ks * rows_per * 128;
         const int* recv = reinterpret_cast<const int*>(smem_gen + Shape::kRecvOffset);
@@ -397,8 +386,18 @@ gemm_tc_mid_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
             emit(ks * rows_per + mr, q.x, q.y, q.z, q.w);
           }
         } else {
+          if (wide) {
+            // the high words of every peer that has some; its own arrivals stand for the other peers
+            if (warp == 2 && lane == 0) {
+              int none = S - 1;
+              for (int s = 0; s < S; ++s) none -= s != ks && ((wide >> (16 * s)) & 0xffff);
+              if (none) mbar_arrive_n(high_bar, (uint32_t)none);
+            }
+            __syncwarp();
+            ok = __all_sync(0xffffffffu, mbar_wait_acquire_cluster(high_bar, 0, abort_flag));
+          }
 #pragma unroll 1
-          for (int mr = warp - 2; mr < my_rows; mr += EPIW) {
+          for (int mr = warp - 2; ok && mr < my_rows; mr += EPIW) {
             const int m = ks * rows_per + mr;
             long long q[4] = {0, 0, 0, 0};
 #pragma unroll 1
