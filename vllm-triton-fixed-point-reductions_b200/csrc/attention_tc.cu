@@ -79,7 +79,7 @@ struct TcAttnShape {
   int num_q_blocks;
   int page_size;
   int group_shift;         // log2 of the keys per TMA box: 6 when pages are multiples of 64 tokens, else 4
-  int page_mask;           // page_size - 1 when the page size is a power of two, else 0
+  int page_shift;          // log2 of the page size, -1 where it is no power of two
   int head_chunks;         // 64-element chunks from one KV head to the next
   uint32_t idesc_s, idesc_s2, idesc_pv;    // S of 64 keys, S of 128 keys, P.V
 };
@@ -431,9 +431,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int stage_bytes = is_v ? Sm::kVBytes : Sm::kKBytes;
       int stage = 0; uint32_t phase = 1;
       int qb = 0; uint32_t q_phase = 1;                    // qfree: the first waits pass
-      int page_shift = -1;
-#pragma unroll 1
-      for (int b = 4; b < 31; ++b) if ((1 << b) == sh.page_size) page_shift = b;
+      const int page_shift = sh.page_shift;
       // ---- item list (first V producer): kTcListGroup requests at a time, one a lane
       int l_start = 0, l_q = 0, l_seq = 0, l_blocks = 0;     // this lane's request
       int group = -kTcListGroup, level = -1;                 // first of these requests; row block, from the last down
@@ -914,7 +912,8 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
   sh.num_q_blocks = (max_query_len + sh.tokens_per_block - 1) / sh.tokens_per_block;
   sh.page_size = p.page_size;
   sh.group_shift = (p.page_size % 64 == 0) ? 6 : 4;
-  sh.page_mask = (p.page_size & (p.page_size - 1)) == 0 ? p.page_size - 1 : 0;
+  sh.page_shift = -1;
+  for (int b = 4; b < 31; ++b) if ((1 << b) == p.page_size) sh.page_shift = b;
   const int fmt = dtype == FXPR_BF16 ? 1 : 0;
   sh.idesc_s = make_idesc(fmt, 0, kTcTileN, kTcRows);
   sh.idesc_s2 = make_idesc(fmt, 0, kTcOpN, kTcRows);
@@ -941,7 +940,7 @@ int attention_tc(const AttnParams& p, int dtype, int max_query_len, int32_t* sta
     return FXPR_ERR_CUDA;
   }
 
-  // persistent CTAs, one per SM, walking the padded item list
+  // persistent CTAs, one per SM; the list of live items is made on the device
   const int64_t total_items = (int64_t)sh.num_q_blocks * p.num_kv_heads * p.num_reqs;
   if (total_items > 0x7fffffffLL) return FXPR_ERR_UNSUPPORTED;
   dim3 grid((unsigned)std::min<int64_t>(total_items, device_sms()), 1, 1);

@@ -9,7 +9,6 @@
 namespace fxpr {
 
 static constexpr uint32_t kMagicBits = 0x4B400000u;      // 1.5 * 2^23
-static constexpr uint32_t kExpBits = 0x4B000000u;        // exponent pattern of [2^23, 2^24)
 
 static __device__ __forceinline__ float tmem_ld1(uint32_t taddr) {
   uint32_t r;

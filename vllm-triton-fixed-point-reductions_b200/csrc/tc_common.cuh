@@ -265,12 +265,6 @@ __device__ __forceinline__ void tmem_wait_ld_regs(uint32_t (&r)[32]) {
 }
 
 // Two loads in flight, one wait.
-__device__ __forceinline__ void tmem_wait_ld_regs2(uint32_t (&a)[8], uint32_t (&b)[8]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
-                 "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7])
-               :: "memory");
-}
 __device__ __forceinline__ void tmem_wait_ld_regs2(uint32_t (&a)[16], uint32_t (&b)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
