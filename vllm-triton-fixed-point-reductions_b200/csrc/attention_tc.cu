@@ -31,8 +31,8 @@
 // exponentials 512 on the special-function unit, its copies about 1200 at the rate L2 gives all SMs at once.  The
 // schedulers issue 53 % of the time with six warps each, an instruction of a warp at work takes 6 clocks, and the
 // softmax warps wait a third of the time for scores, the conversion warps for P.V.
-// 16 prompts of 128 to 4096 tokens, 32/8 heads (one box, both sides): 1333 -> 1034 us against a kernel with P through
-// shared memory, one issuer for both products, every role decoding every item, and exact divisions per output.
+// 16 prompts of 128 to 4096 tokens, 32/8 heads, a call among others, in turn with a kernel with P through shared memory,
+// one issuer for both products, every role decoding every item, and exact divisions per output: 1414 -> 1181 us.
 // With head size 64 882 us, where the mma.sync kernel takes 3114.
 // KV splits are not handled here (the dispatcher sends them to attention_mma.cu: same bits).
 // Every wait is bounded; on a time-out the CTA sets the status word and leaves.

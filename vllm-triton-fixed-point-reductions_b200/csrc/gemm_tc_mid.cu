@@ -11,9 +11,9 @@
 // tile asks for 256 of weights and MP of activations per 128 of K, where two 128 x 128 tiles on single SMs ask for
 // 1024 together; the rows of a tile follow the batch (333 rows are three tiles of 111); small weights split K without
 // the scratch planes.  Copies and barriers come 128 of K at a time and weights in one box (64 of K, two boxes of 64
-// columns: 10 % slower).  At K-tile 64 the conversion is as long.  Against 128 x 128 tiles with planes, K-tile 128, us:
+// columns: 10 % slower).  At K-tile 64 the conversion is as long.  Against 128 x 128 tiles with planes, K-tile 128, in a graph, us:
 //   80 x 4096 x 4096 21.9 -> 12.4, 80 x 768 x 4096 26.7 -> 10.1, 200 x 4096 x 14336 46.6 -> 37.2,
-//   333 x 6144 x 4096 26.0 -> 23.3, 700 x 4096 x 4096 (256 x 256 tiles) 37.7 -> 28.4.
+//   333 x 6144 x 4096 26.0 -> 23.3 (a call among others, with bias: 30.8 -> 27.8), 700 x 4096 x 4096 (256 x 256 tiles) 37.7 -> 28.4.
 // Which calls come here: mid_route in host_policy.h.
 //
 // Numerics are those of the other tensor-core kernels: one fresh fp32 accumulator per K-tile, rint-half-even to Q-format

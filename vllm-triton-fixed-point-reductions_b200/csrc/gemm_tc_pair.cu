@@ -12,8 +12,9 @@
 // (512 clocks of tensor work, 1350 a K-tile all in) they are at work 84 % of the time, ALU pipe 64 %, and
 // the tensor core waits for accumulators; at K-tile 128 (1024 clocks of tensor work) they wait a quarter
 // of the time and the tensor pipe is busy 63 %: the hand-over, next to operands at 8.4 TB/s out of L2.  Outputs
-// leave by TMA: stored by the threads they held the epilogue warps for 7700-8400 clocks a tile.  4096^3, outputs
-// by the threads -> by TMA: K-tile 64 196 -> 186 us, K-tile 128 139 -> 134.
+// leave by TMA: stored by the threads they held the epilogue warps for 7700-8400 clocks a tile.  4096^3 in a graph,
+// outputs by the threads -> by TMA -> with every sum converted in registers: K-tile 64 196 -> 187 -> 186 us, K-tile 128
+// 139 -> 134 -> 130 (a call among others at K-tile 64: 218 -> 208 -> 203).
 //
 // What it depends on, measured at 4096^3 with the conversion left out:
 //   - MMAs, commits and copies are predicated instructions of a uniform warp (tc_common.cuh);

@@ -12,6 +12,7 @@
 // distributed shared memory and outputs written out of registers (cold weights, CUDA graph, us):
 //   16 x 4096 x 4096 13.0 -> 9.9 (weights alone 5.2), 64 x 4096 x 4096 13.3 -> 11.3, 64 x 6144 x 4096 17.6 -> 13.7,
 //   64 x 28672 x 4096 46.5 -> 38.7 (weights alone 36.4), 64 x 768 x 4096 9.0 -> 6.9, 64 x 4096 x 512 8.2 -> 6.0.
+// More than 32 rows on more tiles than two CTAs an SM are walked by persistent CTAs (route_skinny).
 //
 // Numerics are those of the other tensor-core kernels: one fp32 partial per K-tile and
 // output element from tcgen05.mma (kind::f16, fp32 accumulate, fresh accumulator per
