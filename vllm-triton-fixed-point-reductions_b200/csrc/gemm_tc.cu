@@ -449,7 +449,7 @@ int gemm_tc_fast(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CU
                  cudaStream_t s);
 bool gemm_tc_pair_supported(const GemmArgs& g, int split_k);
 bool gemm_tc_mid_supported(const GemmArgs& g, int split_k);
-int gemm_tc_mid(const GemmArgs& g, TcParams& p, const CUtensorMap& mw, int row_tiles, cudaStream_t s);
+int gemm_tc_mid(const GemmArgs& g, TcParams& p, int row_tiles, cudaStream_t s);
 int gemm_tc_pair(const GemmArgs& g, TcParams& p, const CUtensorMap& ma, const CUtensorMap& mb,
                  cudaStream_t s);
 
@@ -493,29 +493,29 @@ int gemm_tc(const GemmArgs& g, cudaStream_t s) {
     p.acc_scratch = (char*)g.scratch + tc_lock_bytes(g.M, g.N);
   }
 
+  // Tensor maps are made where they are used: a lone call waits for each.
   CUtensorMap ma, mb;
-  if (!tc_make_map(&ma, g.dtype, g.a, g.M, g.K, g.a_sm, kBM)) {
-    set_last_error("cuTensorMapEncodeTiled(A)", cudaErrorInvalidValue);
-    return FXPR_ERR_CUDA;
-  }
-  const bool okb = b_kmajor ? tc_make_map(&mb, g.dtype, g.b, g.N, g.K, g.b_sn, 64)
-                            : tc_make_map(&mb, g.dtype, g.b, g.K, g.N, g.b_sk, 64);
-  if (!okb) {
+  const auto make_b = [&] {
+    if (b_kmajor ? tc_make_map(&mb, g.dtype, g.b, g.N, g.K, g.b_sn, 64) : tc_make_map(&mb, g.dtype, g.b, g.K, g.N, g.b_sk, 64)) return true;
     set_last_error("cuTensorMapEncodeTiled(B)", cudaErrorInvalidValue);
-    return FXPR_ERR_CUDA;
-  }
-
+    return false;
+  };
   if (skinny) {
     p.silu_mul = (g.flags & FXPR_GEMM_SILU_MUL) ? 1 : 0;
     if (g.best) {
       if (p.split_k != 1 || p.silu_mul) return FXPR_ERR_UNSUPPORTED;
       p.best = g.best; p.n_offset = (unsigned int)g.n_offset;
     }
-    return gemm_tc_skinny(g, p, mb, s);
+    return make_b() ? gemm_tc_skinny(g, p, mb, s) : FXPR_ERR_CUDA;
   }
   if (g.best) return FXPR_ERR_UNSUPPORTED;                          // only the decode-shape kernel
   if (g.flags & FXPR_GEMM_SILU_MUL) return FXPR_ERR_UNSUPPORTED;   // only the decode-shape kernel fuses it
-  if (mid_rows) return gemm_tc_mid(g, p, mb, mid_rows, s);
+  if (mid_rows) return gemm_tc_mid(g, p, mid_rows, s);
+  if (!tc_make_map(&ma, g.dtype, g.a, g.M, g.K, g.a_sm, kBM)) {
+    set_last_error("cuTensorMapEncodeTiled(A)", cudaErrorInvalidValue);
+    return FXPR_ERR_CUDA;
+  }
+  if (!make_b()) return FXPR_ERR_CUDA;
   if (!(g.flags & FXPR_GEMM_FORCE_EXACT_TC) && gemm_tc_pair_supported(g, p.split_k)) {
     // 256 x 256 tiles on SM pairs or 128 x 128 tiles on single SMs (same bits).  A full wave of pair
     // tiles has twice the output of a wave of single tiles and takes 1.7 times as long at K-tile 64

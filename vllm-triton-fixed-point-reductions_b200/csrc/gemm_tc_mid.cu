@@ -485,7 +485,7 @@ static int launch_mid(const GemmArgs& g, const CUtensorMap& mw, int w_box, TcPar
 }
 
 template <typename T>
-static int route_mid(const GemmArgs& g, const CUtensorMap& mb, TcParams& p, int row_tiles, cudaStream_t s) {
+static int route_mid(const GemmArgs& g, TcParams& p, int row_tiles, cudaStream_t s) {
   CUtensorMap mw;
   int w_box = 0;
   if (p.b_kmajor) {
@@ -493,9 +493,9 @@ static int route_mid(const GemmArgs& g, const CUtensorMap& mb, TcParams& p, int 
   } else if (tc_make_map_groups(&mw, g.dtype, g.b, g.K, g.N, g.b_sk, 64)) {
     w_box = 3;
   }
-  if (!w_box) {
-    if (p.b_kmajor) { set_last_error("cuTensorMapEncodeTiled(W)", cudaErrorInvalidValue); return FXPR_ERR_CUDA; }
-    mw = mb;
+  if (!w_box && (p.b_kmajor || !tc_make_map(&mw, g.dtype, g.b, g.K, g.N, g.b_sk, 64))) {
+    set_last_error("cuTensorMapEncodeTiled(W)", cudaErrorInvalidValue);
+    return FXPR_ERR_CUDA;
   }
   const int rows = (p.M + row_tiles - 1) / row_tiles;
   if (p.split_k > 1) {
@@ -510,11 +510,10 @@ static int route_mid(const GemmArgs& g, const CUtensorMap& mb, TcParams& p, int 
   return launch_mid<T, 256, false>(g, mw, w_box, p, row_tiles, s);
 }
 
-// mw: the weight tensor map of gemm_tc() (64-row boxes in either layout).  row_tiles: at most 256 rows each, 128
-// where K is split.
-int gemm_tc_mid(const GemmArgs& g, TcParams& p, const CUtensorMap& mw, int row_tiles, cudaStream_t s) {
-  if (g.dtype == FXPR_BF16) return route_mid<__nv_bfloat16>(g, mw, p, row_tiles, s);
-  return route_mid<__half>(g, mw, p, row_tiles, s);
+// row_tiles: at most 256 rows each, 128 where K is split.
+int gemm_tc_mid(const GemmArgs& g, TcParams& p, int row_tiles, cudaStream_t s) {
+  if (g.dtype == FXPR_BF16) return route_mid<__nv_bfloat16>(g, p, row_tiles, s);
+  return route_mid<__half>(g, p, row_tiles, s);
 }
 
 }  // namespace fxpr
